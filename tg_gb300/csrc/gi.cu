@@ -236,128 +236,43 @@ __device__ __forceinline__ uint32_t warp_append(uint32_t* counter, bool want)
     return base + (uint32_t)__popc(mask & ((1u << lane) - 1u));
 }
 
-__device__ __forceinline__ void write_hit(RayHit* h, int res, const RayState& r)
+// The two ray lists of one traversal launch: a (n_a rays), then b.
+struct RayLists
 {
-    RayHit o;
-    o.t = r.t;
-    o.c[0] = r.c[0]; o.c[1] = r.c[1]; o.c[2] = r.c[2];
-    o.axis = r.last_axis;
-    o.res = res;
-    *h = o;
-}
+    const Ray *ra, *rb;
+    RayHit *ha, *hb;
+    uint32_t n_a;
+    __device__ __forceinline__ void load(uint32_t i, float o[3], float d[3]) const
+    {
+        const Ray r = i < n_a ? ra[i] : rb[i - n_a];
+#pragma unroll
+        for (int a = 0; a < 3; a++) { o[a] = r.o[a]; d[a] = r.d[a]; }
+    }
+    __device__ __forceinline__ void store(uint32_t i, int res, float t, const int32_t c[3], int32_t axis) const
+    {
+        RayHit h;
+        h.t = t;
+        h.c[0] = c[0]; h.c[1] = c[1]; h.c[2] = c[2];
+        h.axis = axis;
+        h.res = res;
+        (i < n_a ? ha[i] : hb[i - n_a]) = h;
+    }
+};
 
 // Persistent traversal of two ray lists: a (n * mul_a rays) then b (n * mul_b
-// rays), n read from the device.  No CTA waits on another: a CTA that starts
-// after the queue is drained exits at once.
-//
-// A warp sets rays up 32 at a time, one per lane, and parks the ones whose
-// DDA has to run in a per-warp ring of 64 states in shared memory; a lane
-// whose ray ended takes the next parked state.  The set-up (entry slab, the
-// bottom-up start) then runs on full warps instead of on the few lanes that
-// happen to need a ray at a refill.
-constexpr uint32_t kTraceWarps = 4;     // 128 threads
-constexpr uint32_t kRing = 64;          // parked states per warp
-
-__global__ void __launch_bounds__(32 * kTraceWarps) k_trace_queue(SvoDev s, const Ray* __restrict__ ra,
-                                                                  RayHit* __restrict__ ha, uint32_t mul_a,
-                                                                  const Ray* __restrict__ rb, RayHit* __restrict__ hb,
-                                                                  uint32_t mul_b, const uint32_t* __restrict__ n_dev,
-                                                                  uint32_t max_steps, uint32_t steps_per_round,
-                                                                  uint32_t* __restrict__ queue,
+// rays), n read from the device (svo_trace_queue).
+__global__ void __launch_bounds__(32 * kTraceWarps, kTraceCtas) k_trace_queue(const __grid_constant__ SvoDev s,
+                                                                  const Ray* __restrict__ ra, RayHit* __restrict__ ha,
+                                                                  uint32_t mul_a, const Ray* __restrict__ rb,
+                                                                  RayHit* __restrict__ hb, uint32_t mul_b,
+                                                                  const uint32_t* __restrict__ n_dev, uint32_t max_steps,
+                                                                  uint32_t steps_per_round, uint32_t* __restrict__ queue,
                                                                   uint32_t* __restrict__ exhausted,
                                                                   unsigned long long* __restrict__ work)
 {
-    __shared__ uint32_t occ_off[16];
-    __shared__ LevelDesc lv[16];
-    __shared__ uint8_t first_level[kFirstLevelSize];
-    __shared__ RayState ring[kTraceWarps][kRing];
-    __shared__ uint32_t ring_item[kTraceWarps][kRing];
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int i = 0; i < 16; i++) occ_off[i] = s.occ_off[i];
-    }
-    __syncthreads();
-    svo_level_tables(s.L, s.NL, s.B, s.occ, s.pool, s.sub, occ_off, lv, first_level);
-    __syncthreads();
     const uint32_t n = *n_dev;
-    const uint32_t n_a = n * mul_a, n_tot = n_a + n * mul_b;
-    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-    const uint32_t lt_mask = (1u << lane) - 1u;
-    RayState r;
-    uint32_t item = 0;
-    bool have = false;
-    uint32_t head = 0, count = 0;   // the warp's ring (warp-uniform)
-    bool drained = false;           // the ray queue is exhausted (warp-uniform)
-    uint32_t done_steps = 0, done_rays = 0;   // this lane's finished rays and their DDA steps
-    for (;;) {
-        const uint32_t need_mask = __ballot_sync(0xffffffffu, !have);
-        const uint32_t n_need = (uint32_t)__popc(need_mask);
-        // set up rays, 32 at a time, until the ring can serve every idle lane
-        while (n_need && count < n_need && !drained) {
-            uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(queue, 32u);
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (base + 32u >= n_tot) drained = true;
-            const uint32_t it = base + lane;
-            bool running = false;
-            RayState rs;
-            if (it < n_tot) {
-                const Ray ray = it < n_a ? ra[it] : rb[it - n_a];
-                const int res = svo_trace_begin(s, occ_off, lv, ray.o, ray.d, max_steps, rs);
-                if (res == kTraceRunning) {
-                    running = true;
-                } else {
-                    write_hit(it < n_a ? &ha[it] : &hb[it - n_a], res, rs);
-                    done_steps += rs.steps;
-                    done_rays++;
-                }
-            }
-            const uint32_t run_mask = __ballot_sync(0xffffffffu, running);
-            if (running) {
-                const uint32_t slot = (head + count + (uint32_t)__popc(run_mask & lt_mask)) & (kRing - 1u);
-                ring[w][slot] = rs;
-                ring_item[w][slot] = it;
-            }
-            count += (uint32_t)__popc(run_mask);
-            __syncwarp();
-        }
-        // idle lanes take parked states in lane order
-        const uint32_t take = min(n_need, count);
-        if (!have) {
-            const uint32_t rank = (uint32_t)__popc(need_mask & lt_mask);
-            if (rank < take) {
-                const uint32_t slot = (head + rank) & (kRing - 1u);
-                r = ring[w][slot];
-                item = ring_item[w][slot];
-                have = true;
-            }
-        }
-        head = (head + take) & (kRing - 1u);
-        count -= take;
-        __syncwarp();
-        if (!__any_sync(0xffffffffu, have) && drained && count == 0) break;
-        if (have) {
-            const int res = svo_trace_run(s, lv, first_level, r, max_steps, steps_per_round);
-            if (res != kTraceRunning) {
-                if (res < 0) atomicAdd(exhausted, 1u);
-                write_hit(item < n_a ? &ha[item] : &hb[item - n_a], res, r);
-                done_steps += r.steps;
-                done_rays++;
-                have = false;
-            }
-        }
-    }
-    // the frame's traversal work: one pair of 64-bit atomics per warp
-    unsigned long long ws = done_steps, wr = done_rays;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        ws += __shfl_down_sync(0xffffffffu, ws, o);
-        wr += __shfl_down_sync(0xffffffffu, wr, o);
-    }
-    if (lane == 0 && wr) {
-        atomicAdd(&work[0], ws);
-        atomicAdd(&work[1], wr);
-    }
+    const RayLists io = {ra, rb, ha, hb, n * mul_a};
+    svo_trace_queue(s, io, n * mul_a + n * mul_b, max_steps, steps_per_round, queue, exhausted, work);
 }
 
 // Roots of the geometry pixels; sky pixels get the sky radiance.

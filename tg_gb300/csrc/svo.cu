@@ -1054,39 +1054,34 @@ extern "C" tgx_status tgx_svo_download(tgx_ctx* c, const tgx_svo* s, int32_t* ou
 
 namespace {
 
-__global__ void __launch_bounds__(128) k_svo_trace(SvoDev s, uint32_t n, const float* __restrict__ o,
-                                                  const float* __restrict__ d, uint32_t max_steps,
-                                                  float* __restrict__ out_t, int32_t* __restrict__ out_voxel,
-                                                  uint32_t* __restrict__ n_exhausted)
+// A caller's ray batch: origins and directions in, distance and world voxel out.
+struct RayArrays
 {
-    __shared__ uint32_t occ_off[16];
-    __shared__ LevelDesc lv[16];
-    __shared__ uint8_t first_level[kFirstLevelSize];
-    if (threadIdx.x == 0) {
+    const float *o, *d;
+    float* t;
+    int32_t* voxel;
+    int32_t mn[3];
+    __device__ __forceinline__ void load(uint32_t i, float oi[3], float di[3]) const
+    {
+        const size_t k = 3 * (size_t)i;
 #pragma unroll
-        for (int k = 0; k < 16; k++) occ_off[k] = s.occ_off[k];
+        for (int a = 0; a < 3; a++) { oi[a] = o[k + a]; di[a] = d[k + a]; }
     }
-    __syncthreads();
-    svo_level_tables(s.L, s.NL, s.B, s.occ, s.pool, s.sub, occ_off, lv, first_level);
-    __syncthreads();
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float oi[3] = {o[3 * i], o[3 * i + 1], o[3 * i + 2]};
-    const float di[3] = {d[3 * i], d[3 * i + 1], d[3 * i + 2]};
-    float t;
-    int32_t c[3], ax;
-    uint32_t steps;
-    const int r = svo_trace(s, lv, first_level, oi, di, max_steps, t, c, ax, steps);
-    if (r == 1) {
-        out_t[i] = t;
-        out_voxel[3 * i] = c[0] + (int32_t)s.mn[0];
-        out_voxel[3 * i + 1] = c[1] + (int32_t)s.mn[1];
-        out_voxel[3 * i + 2] = c[2] + (int32_t)s.mn[2];
-    } else {
-        out_t[i] = F32_MAX_TG;
-        out_voxel[3 * i] = out_voxel[3 * i + 1] = out_voxel[3 * i + 2] = 0;
-        if (r < 0) atomicAdd(n_exhausted, 1u);
+    __device__ __forceinline__ void store(uint32_t i, int res, float ti, const int32_t c[3], int32_t) const
+    {
+        const size_t k = 3 * (size_t)i;
+        t[i] = res == 1 ? ti : F32_MAX_TG;
+#pragma unroll
+        for (int a = 0; a < 3; a++) voxel[k + a] = res == 1 ? c[a] + mn[a] : 0;
     }
+};
+
+__global__ void __launch_bounds__(32 * kTraceWarps, kTraceCtas) k_svo_trace(const __grid_constant__ SvoDev s, uint32_t n, RayArrays io,
+                                                               uint32_t max_steps, uint32_t steps_per_round,
+                                                               uint32_t* __restrict__ queue,
+                                                               uint32_t* __restrict__ n_exhausted)
+{
+    svo_trace_queue(s, io, n, max_steps, steps_per_round, queue, n_exhausted, nullptr);
 }
 
 }  // namespace
@@ -1101,7 +1096,21 @@ extern "C" tgx_status tgx_svo_trace(tgx_ctx* c, const tgx_svo* s, uint32_t n, co
     if (n == 0) return TGX_OK;
     TGX_TRY(devbuf_reserve(c->svo_counters, S_COUNT * 4 + 64));
     uint32_t* exhausted = (uint32_t*)c->svo_counters.ptr + S_COUNT;
-    TGX_LAUNCH(c, TR_SVO_TRACE, (n + 127) / 128, 128, 0, k_svo_trace, svo_dev(s), n, d_o, d_d, max_steps, d_t, d_voxel,
-               exhausted);
+    uint32_t* queue = exhausted + 1;
+    if (!c->svo_trace_ctas) {
+        int per_sm = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_svo_trace, 32 * kTraceWarps, 0) != cudaSuccess || per_sm < 1) {
+            cudaGetLastError();
+            per_sm = 1;
+        }
+        c->svo_trace_ctas = (uint32_t)(c->num_sms * per_sm);
+    }
+    const uint32_t per_cta = 32 * kTraceWarps;
+    const uint32_t grid = std::min(c->svo_trace_ctas, (n - 1) / per_cta + 1);
+    // the queue counter is read only when the rays outnumber the launch's lanes
+    if ((uint64_t)grid * per_cta < n) TGX_CUDA(cudaMemsetAsync(queue, 0, 4, c->stream));
+    const RayArrays io = {d_o, d_d, d_t, d_voxel, {(int32_t)s->mn[0], (int32_t)s->mn[1], (int32_t)s->mn[2]}};
+    TGX_LAUNCH(c, TR_SVO_TRACE, grid, per_cta, 0, k_svo_trace, svo_dev(s), n, io, max_steps, c->trace_steps_per_round,
+               queue, exhausted);
     return TGX_OK;
 }

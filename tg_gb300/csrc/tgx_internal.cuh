@@ -133,6 +133,7 @@ struct tgx_ctx
     DevBuf vis_work;       // work counters of the tile kernel's counting variant
     uint64_t mem_budget = 0;           // bytes the context's scene stores may hold (0: no limit)
     uint64_t mem_scenes = 0;           // bytes its live scene stores hold
+    uint32_t svo_trace_ctas = 0;       // resident CTAs of the ray-batch traversal (0: not asked yet)
     uint32_t vis_tile_ctas = 0;        // resident CTAs of the persistent (batched-frame) tile kernel
     bool   vis_count_work = false;
     uint32_t vis_bshift = 1;           // depth buckets per tile: 32 >> vis_bshift
