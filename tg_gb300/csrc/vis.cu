@@ -24,13 +24,14 @@
 //                           (tile, bucket) bins, so every tile's entries are
 //                           contiguous and run near to far.
 //   6. k_vis_tiles          one CTA per tile (heaviest first), one thread per
-//      pixel: batches of the tile's entries arrive by one cp.async.bulk each
-//      on an mbarrier; every pixel skips entries whose depth bound cannot beat
-//      its word and rejects clear misses with a conservative reciprocal slab
-//      test; the surviving (pixel, cluster) pairs are compacted by warp ballot
-//      and run the shader's exact ray/box test and DDA on full warps, keeping
-//      each pixel's minimum packed depth|pointer|voxel word (shared
-//      atomicMin); every pixel is written once (fused clear).
+//      pixel (k_vis_tiles_groups: several, for frames of few tiles): batches of
+//      the tile's entries arrive by one cp.async.bulk each on an mbarrier;
+//      every pixel skips entries whose depth bound cannot beat its word and
+//      rejects clear misses with a conservative reciprocal slab test; the
+//      surviving (pixel, cluster) pairs are compacted by warp ballot and run
+//      the shader's exact ray/box test and DDA on full warps, keeping each
+//      pixel's minimum packed depth|pointer|voxel word (shared atomicMin);
+//      every pixel is written once (fused clear).
 //      k_vis_tiles_queue is the persistent form over many jobs' tiles.
 //
 // Every pair evaluates the same binary32 operations in the same order as the
@@ -852,32 +853,41 @@ struct TileJob
 constexpr uint32_t kBatch = 48;                      // entries per staged batch (k < 64 fits the packed word)
 constexpr uint32_t kQueue = 64;                      // ring entries per warp (an entry adds at most 32)
 constexpr uint32_t kQueueWords = 7 * kQueue;         // 6 float arrays + the packed word
-constexpr uint32_t kSmBar = 0, kSmView = 8, kSmN = 12;
+constexpr uint32_t kSmBar = 0, kSmView = 8, kSmN = 12, kSmLost = 16, kSmBars = 24;   // kSmBars: kStages - 1 more mbarriers
 constexpr uint32_t kSmStage = 128;                   // 16-byte aligned bulk-copy target
-constexpr uint32_t kSmBest = kSmStage + kBatch * sizeof(TileEntry);
-__host__ __device__ constexpr uint32_t tile_smem_bytes(uint32_t threads)
+constexpr uint32_t kStages = 2;                      // stages of a tile with several groups of threads (vis_tile_groups)
+__host__ __device__ constexpr uint32_t tile_best_off(uint32_t groups)
 {
-    return kSmBest + 8u * threads + (threads / 32u) * kQueueWords * 4u;
+    return kSmStage + (groups > 1u ? kStages : 1u) * kBatch * (uint32_t)sizeof(TileEntry);
+}
+__host__ __device__ constexpr uint32_t tile_smem_bytes(uint32_t pixels, uint32_t groups = 1u)
+{
+    return tile_best_off(groups) + 8u * pixels + (pixels * groups / 32u) * kQueueWords * 4u;
 }
 
 struct TileSm
 {
     unsigned char* p;
+    uint32_t best_off, pixels;
     __device__ __forceinline__ uint32_t bar() const { return smem_addr(p + kSmBar); }
+    // mbarrier of stage i (stage 0's is that of the single-stage tiles)
+    __device__ __forceinline__ uint32_t bar(uint32_t i) const { return smem_addr(p + (i ? kSmBars + 8u * (i - 1u) : kSmBar)); }
+    __device__ __forceinline__ volatile uint32_t& lost() const { return *(volatile uint32_t*)(p + kSmLost); }
     __device__ __forceinline__ uint32_t& view() const { return *(uint32_t*)(p + kSmView); }
     __device__ __forceinline__ uint32_t& n() const { return *(uint32_t*)(p + kSmN); }
     __device__ __forceinline__ TileEntry* stage() const { return (TileEntry*)(p + kSmStage); }
-    __device__ __forceinline__ unsigned long long* best() const { return (unsigned long long*)(p + kSmBest); }
+    __device__ __forceinline__ unsigned long long* best() const { return (unsigned long long*)(p + best_off); }
     __device__ __forceinline__ uint32_t* queue(uint32_t warp) const
     {
-        return (uint32_t*)(p + kSmBest + 8u * blockDim.x) + warp * kQueueWords;
+        return (uint32_t*)(p + best_off + 8u * pixels) + warp * kQueueWords;
     }
 };
 
+template <uint32_t kGroups = 1>
 __device__ __forceinline__ TileSm tile_sm()
 {
     extern __shared__ __align__(128) unsigned char tile_dyn_smem[];
-    return TileSm{tile_dyn_smem};
+    return TileSm{tile_dyn_smem, tile_best_off(kGroups), blockDim.x / kGroups};
 }
 
 __device__ __forceinline__ void tile_smem_init(const TileSm& sm)
@@ -888,17 +898,160 @@ __device__ __forceinline__ void tile_smem_init(const TileSm& sm)
     }
 }
 
-// One bulk copy of n contiguous entries into the stage, completing on the
-// CTA's mbarrier (expecting `extra` bytes more than it copies under the
+// One bulk copy of n contiguous entries to dst (in the stage), completing on
+// the mbarrier at bar (expecting `extra` bytes more than it copies under the
 // lost-copy test).  Thread 0 only.
-__device__ __forceinline__ void stage_entries(const TileSm& sm, const TileEntry* src, uint32_t n, uint32_t extra)
+__device__ __forceinline__ void stage_entries(uint32_t bar, const TileEntry* dst, const TileEntry* src, uint32_t n,
+                                              uint32_t extra)
 {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
-                 :: "r"(sm.bar()), "r"(n * (uint32_t)sizeof(TileEntry) + extra) : "memory");
+                 :: "r"(bar), "r"(n * (uint32_t)sizeof(TileEntry) + extra) : "memory");
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 :: "r"(smem_addr(sm.stage())), "l"(src), "r"(n * (uint32_t)sizeof(TileEntry)), "r"(sm.bar())
+                 :: "r"(smem_addr(dst)), "l"(src), "r"(n * (uint32_t)sizeof(TileEntry)), "r"(bar)
                  : "memory");
+}
+
+// A thread's pixel of a tile: its place, its world ray, its nearest depth so
+// far and the cluster-space direction of the last object it met.
+struct TilePixel
+{
+    uint32_t px, py;
+    bool valid;
+    float dws[3];
+    float far_plane, far_rcp;
+    uint32_t best_d24, cur_obj;
+    float dx, dy, dz, ix, iy, iz;
+    uint32_t qh;                 // the warp's ring: first pending entry (warp-uniform)
+};
+
+__device__ __forceinline__ void tile_pixel(const ViewConst& vc, uint32_t tile, uint32_t pix, TilePixel& P)
+{
+    const uint32_t lt = tile - vc.tile_base;
+    P.px = (lt % vc.tiles_x) * vc.tile_w + pix % vc.tile_w;
+    P.py = (lt / vc.tiles_x) * vc.tile_h + pix / vc.tile_w;
+    P.valid = P.px < vc.width && P.py < vc.height;
+    P.far_plane = vc.far_plane;
+    P.far_rcp = pow2_reciprocal(vc.far_plane);
+    // pixel ray in world space (visibility.frag:29-33,68; mix per GLSL 8.3)
+    const float fx = xdiv(xadd((float)P.px, 0.5f), (float)vc.width);
+    const float fy = xsub(1.0f, xdiv(xadd((float)P.py, 0.5f), (float)vc.height));
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const float a = xadd(xmul(vc.bl[i], xsub(1.0f, fy)), xmul(vc.tl[i], fy));
+        const float b = xadd(xmul(vc.br[i], xsub(1.0f, fy)), xmul(vc.tr[i], fy));
+        P.dws[i] = xadd(xmul(a, xsub(1.0f, fx)), xmul(b, fx));
+    }
+    P.best_d24 = 0xffffffu;
+    P.cur_obj = 0xffffffffu;
+    P.dx = P.dy = P.dz = P.ix = P.iy = P.iz = 0.0f;
+    P.qh = 0u;
+}
+
+// Entries k0, k0 + kStep, ... of a staged batch of n: every lane walks them for its own pixel (the
+// depth skip, the cluster-space direction once per object, the conservative
+// slab test); the pairs that survive are compacted by warp ballot into the
+// warp's ring q; whenever it holds J.drain, all 32 lanes take one pair each
+// and run the exact entry test and the voxel DDA (vis_pair), folding the
+// result into the pixel's word (best: the warp's first pixel's) with a
+// shared-memory atomicMin.  The ring is drained at the end.
+template <bool kCount, uint32_t kStep>
+__device__ __forceinline__ void tile_batch(const TileJob& J, const TileEntry* const E, uint32_t k0, const uint32_t n, TilePixel& P,
+                                           uint32_t* const q, unsigned long long* const best, uint32_t* work)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t drain = J.drain;
+    float* const qf = (float*)q;
+    uint32_t qn = 0;     // pending entries (warp-uniform)
+    for (uint32_t k = k0;;) {
+        if (k < n) {
+            bool live = false, sure = false;
+            if (P.valid) {
+                if (P.best_d24 < E[k].d24_lb) {   // cannot produce a smaller word
+                    if (kCount) work[W_DEPTH_SKIPS]++;
+                } else {
+                    if (kCount) work[W_PAIRS]++;
+                    const uint32_t obj = E[k].object_idx;
+                    if (obj != P.cur_obj) {
+                        // normalize((ws2ms * v4(dir, 0)).xyz) (visibility.frag:69) with the
+                        // object's shared linear part (see k_object_setup)
+                        if (kCount) work[W_DIR_SETUPS]++;
+                        P.cur_obj = obj;
+                        const float* L = J.inv_rot + 9u * obj;
+                        const float ux = xadd(xadd(xmul(P.dws[0], L[0]), xmul(P.dws[1], L[1])), xmul(P.dws[2], L[2]));
+                        const float uy = xadd(xadd(xmul(P.dws[0], L[3]), xmul(P.dws[1], L[4])), xmul(P.dws[2], L[5]));
+                        const float uz = xadd(xadd(xmul(P.dws[0], L[6]), xmul(P.dws[1], L[7])), xmul(P.dws[2], L[8]));
+                        const float mag = xsqrt(xadd(xadd(xmul(ux, ux), xmul(uy, uy)), xmul(uz, uz)));
+                        P.dx = xdiv(ux, mag); P.dy = xdiv(uy, mag); P.dz = xdiv(uz, mag);
+                        P.ix = P.dx != 0.0f ? __frcp_rn(P.dx) : 0.0f;
+                        P.iy = P.dy != 0.0f ? __frcp_rn(P.dy) : 0.0f;
+                        P.iz = P.dz != 0.0f ? __frcp_rn(P.dz) : 0.0f;
+                    }
+                    const int sc = slab_class(E[k].ox, E[k].oy, E[k].oz, P.dx, P.dy, P.dz, P.ix, P.iy, P.iz);
+                    live = sc != kMiss;
+                    sure = sc == kHit;
+                    if (kCount) work[sc == kMiss ? W_SLAB_MISSES : sc == kHit ? W_SURE_HITS : W_EXACT_TESTS]++;
+                }
+            }
+            const uint32_t m = __ballot_sync(0xffffffffu, live);
+            if (live) {
+                const uint32_t e = (P.qh + qn + __popc(m & ((1u << lane) - 1u))) & (kQueue - 1u);
+                qf[0 * kQueue + e] = P.dx; qf[1 * kQueue + e] = P.dy; qf[2 * kQueue + e] = P.dz;
+                qf[3 * kQueue + e] = P.ix; qf[4 * kQueue + e] = P.iy; qf[5 * kQueue + e] = P.iz;
+                q[6 * kQueue + e] = lane | (k << 5) | ((uint32_t)sure << 11);
+            }
+            qn += __popc(m);
+            k += kStep;
+            if (qn < drain && k < n) continue;
+        }
+        if (qn == 0u) break;   // k >= n and nothing pending
+        // one pair per lane: the exact test and the DDA; the word goes to its pixel
+        const uint32_t take = min(qn, 32u);
+        __syncwarp();
+        if (lane < take) {
+            const uint32_t e = (P.qh + lane) & (kQueue - 1u);
+            const uint32_t pk = q[6 * kQueue + e];
+            const TileEntry& te = E[(pk >> 5) & 63u];
+            const unsigned long long w = vis_pair<kCount>(
+                te.ox, te.oy, te.oz, qf[0 * kQueue + e], qf[1 * kQueue + e], qf[2 * kQueue + e],
+                qf[3 * kQueue + e], qf[4 * kQueue + e], qf[5 * kQueue + e], (pk >> 11) != 0u, te.bits,
+                te.cluster_pointer, P.far_plane, P.far_rcp, &J.counters[C_DDA_OVERRUN], work);
+            if (w != ULLONG_MAX) atomicMin(best + (pk & 31u), w);
+        }
+        P.qh = (P.qh + take) & (kQueue - 1u);
+        qn -= take;
+        __syncwarp();
+        P.best_d24 = min(P.best_d24, (uint32_t)(best[lane] >> 40));
+    }
+}
+
+__device__ __forceinline__ uint32_t tile_view(const TileJob& J, uint32_t tile)
+{
+    uint32_t v = 0;
+    while (v + 1 < J.n_views && J.views[v + 1].tile_base <= tile) v++;
+    return v;
+}
+
+// Of records base .. base + m - 1, those of the view whose tile rectangle holds
+// tile (tx, ty), copied into the stage (count in sm.n()).  All threads of the CTA.
+__device__ __forceinline__ void gather_records(const TileJob& J, uint32_t base, uint32_t m, uint32_t view, uint32_t tx,
+                                               uint32_t ty, const TileSm& sm)
+{
+    for (uint32_t k = threadIdx.x; k < m; k += blockDim.x) {
+        const uint32_t r = base + k;
+        const uint2 qr = J.rects[r];
+        if (J.records[r].view == view && tx >= (qr.x & 0xffffu) && tx <= (qr.y & 0xffffu) && ty >= (qr.x >> 16) &&
+            ty <= (qr.y >> 16)) {
+            const VisRecord& rec = J.records[r];
+            TileEntry& te = sm.stage()[atomicAdd(&sm.n(), 1u)];
+            te.ox = rec.ox; te.oy = rec.oy; te.oz = rec.oz;
+            te.cluster_pointer = rec.cluster_pointer;
+            te.object_idx = rec.object_idx;
+            te.d24_lb = rec.d24_lb;
+#pragma unroll
+            for (int w = 0; w < 16; w++) te.bits[w] = J.bits[(uint64_t)rec.cluster_idx * 16u + w];
+        }
+    }
 }
 
 // Tile `slot` (in the job's heavy-first order) of one job: every pixel's
@@ -942,8 +1095,7 @@ __device__ __forceinline__ bool vis_tile(const TileJob& J, uint32_t slot, const 
     const uint32_t end = scan_all ? J.counters[C_RECORDS] : si.y + si.z;
     if (!scan_all && si.z == 0u) {
         // no entry: the tile is only cleared (no ray set-up, no barrier; the same in every thread)
-        uint32_t v = 0;
-        while (v + 1 < J.n_views && J.views[v + 1].tile_base <= tile) v++;
+        const uint32_t v = tile_view(J, tile);
         const ViewConst& vc = J.views[v];
         const uint32_t lt = tile - vc.tile_base;
         const uint32_t px = (lt % vc.tiles_x) * vc.tile_w + threadIdx.x % vc.tile_w;
@@ -951,44 +1103,23 @@ __device__ __forceinline__ bool vis_tile(const TileJob& J, uint32_t slot, const 
         if (px < vc.width && py < vc.height) J.outs[v][(size_t)py * vc.width + px] = ULLONG_MAX;
         return true;
     }
+    const TileEntry* const E = sm.stage();
     if (threadIdx.x == 0) {
-        if (!scan_all && end > begin) stage_entries(sm, J.entries + begin, min(J.batch, end - begin), J.extra_tx);
-        uint32_t v = 0;
-        while (v + 1 < J.n_views && J.views[v + 1].tile_base <= tile) v++;
-        sm.view() = v;
+        if (!scan_all && end > begin) stage_entries(sm.bar(), E, J.entries + begin, min(J.batch, end - begin), J.extra_tx);
+        sm.view() = tile_view(J, tile);
     }
     sm.best()[threadIdx.x] = ULLONG_MAX;
     __syncthreads();
     const uint32_t view = sm.view();
     const ViewConst& vc = J.views[view];
-    const uint32_t lt = tile - vc.tile_base;
-    const uint32_t tx = lt % vc.tiles_x, ty = lt / vc.tiles_x;
-    const uint32_t px = tx * vc.tile_w + threadIdx.x % vc.tile_w;
-    const uint32_t py = ty * vc.tile_h + threadIdx.x / vc.tile_w;
-    const bool valid = px < vc.width && py < vc.height;
+    TilePixel P;
+    tile_pixel(vc, tile, threadIdx.x, P);
+    const uint32_t tx = (tile - vc.tile_base) % vc.tiles_x, ty = (tile - vc.tile_base) / vc.tiles_x;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     uint32_t* const q = sm.queue(warp);
-    float* const qf = (float*)q;
-    const float far_plane = vc.far_plane, far_rcp = pow2_reciprocal(far_plane);
-    const TileEntry* const E = sm.stage();
-    const uint32_t drain = J.drain;
+    unsigned long long* const best0 = sm.best() + (warp << 5);
 
-    // pixel ray in world space (visibility.frag:29-33,68; mix per GLSL 8.3)
-    const float fx = xdiv(xadd((float)px, 0.5f), (float)vc.width);
-    const float fy = xsub(1.0f, xdiv(xadd((float)py, 0.5f), (float)vc.height));
-    float dws[3];
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-        const float a = xadd(xmul(vc.bl[i], xsub(1.0f, fy)), xmul(vc.tl[i], fy));
-        const float b = xadd(xmul(vc.br[i], xsub(1.0f, fy)), xmul(vc.tr[i], fy));
-        dws[i] = xadd(xmul(a, xsub(1.0f, fx)), xmul(b, fx));
-    }
-
-    uint32_t best_d24 = 0xffffffu;
-    uint32_t cur_obj = 0xffffffffu;
-    float dx = 0.0f, dy = 0.0f, dz = 0.0f, ix = 0.0f, iy = 0.0f, iz = 0.0f;
     bool lost = false;      // a wait for a batch's copy ran out (the same in every lane of a warp)
-    uint32_t qh = 0;        // the warp's ring: first pending entry (warp-uniform)
     for (uint32_t base = begin; base < end;) {
         uint32_t n;
         if (!scan_all) {
@@ -997,7 +1128,7 @@ __device__ __forceinline__ bool vis_tile(const TileJob& J, uint32_t slot, const 
                 // the previous batch is fully consumed; after a lost copy nobody stages another
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 if (__syncthreads_or(lost)) break;
-                if (threadIdx.x == 0) stage_entries(sm, J.entries + base, n, 0u);
+                if (threadIdx.x == 0) stage_entries(sm.bar(), E, J.entries + base, n, 0u);
             }
             base += n;
             lost = __any_sync(0xffffffffu, !mbar_wait_bounded(sm.bar(), phase));
@@ -1009,93 +1140,18 @@ __device__ __forceinline__ bool vis_tile(const TileJob& J, uint32_t slot, const 
             if (threadIdx.x == 0) sm.n() = 0;
             __syncthreads();
             const uint32_t m = min(J.batch, end - base);
-            for (uint32_t k = threadIdx.x; k < m; k += blockDim.x) {
-                const uint32_t r = base + k;
-                const uint2 qr = J.rects[r];
-                if (J.records[r].view == view && tx >= (qr.x & 0xffffu) && tx <= (qr.y & 0xffffu) &&
-                    ty >= (qr.x >> 16) && ty <= (qr.y >> 16)) {
-                    const VisRecord& rec = J.records[r];
-                    TileEntry& te = sm.stage()[atomicAdd(&sm.n(), 1u)];
-                    te.ox = rec.ox; te.oy = rec.oy; te.oz = rec.oz;
-                    te.cluster_pointer = rec.cluster_pointer;
-                    te.object_idx = rec.object_idx;
-                    te.d24_lb = rec.d24_lb;
-#pragma unroll
-                    for (int w = 0; w < 16; w++) te.bits[w] = J.bits[(uint64_t)rec.cluster_idx * 16u + w];
-                }
-            }
+            gather_records(J, base, m, view, tx, ty, sm);
             base += m;
             __syncthreads();
             n = sm.n();
             if (n == 0) continue;
         }
-        if (kCount && valid) work[W_BATCHES]++;
-        // produce live pairs entry by entry; drain the ring 32 at a time, and what is left at the end
-        uint32_t qn = 0;     // pending entries (warp-uniform)
-        for (uint32_t k = 0;;) {
-            if (k < n) {
-                bool live = false, sure = false;
-                if (valid) {
-                    if (best_d24 < E[k].d24_lb) {   // cannot produce a smaller word
-                        if (kCount) work[W_DEPTH_SKIPS]++;
-                    } else {
-                        if (kCount) work[W_PAIRS]++;
-                        const uint32_t obj = E[k].object_idx;
-                        if (obj != cur_obj) {
-                            // normalize((ws2ms * v4(dir, 0)).xyz) (visibility.frag:69) with the
-                            // object's shared linear part (see k_object_setup)
-                            if (kCount) work[W_DIR_SETUPS]++;
-                            cur_obj = obj;
-                            const float* L = J.inv_rot + 9u * obj;
-                            const float ux = xadd(xadd(xmul(dws[0], L[0]), xmul(dws[1], L[1])), xmul(dws[2], L[2]));
-                            const float uy = xadd(xadd(xmul(dws[0], L[3]), xmul(dws[1], L[4])), xmul(dws[2], L[5]));
-                            const float uz = xadd(xadd(xmul(dws[0], L[6]), xmul(dws[1], L[7])), xmul(dws[2], L[8]));
-                            const float mag = xsqrt(xadd(xadd(xmul(ux, ux), xmul(uy, uy)), xmul(uz, uz)));
-                            dx = xdiv(ux, mag); dy = xdiv(uy, mag); dz = xdiv(uz, mag);
-                            ix = dx != 0.0f ? __frcp_rn(dx) : 0.0f;
-                            iy = dy != 0.0f ? __frcp_rn(dy) : 0.0f;
-                            iz = dz != 0.0f ? __frcp_rn(dz) : 0.0f;
-                        }
-                        const int sc = slab_class(E[k].ox, E[k].oy, E[k].oz, dx, dy, dz, ix, iy, iz);
-                        live = sc != kMiss;
-                        sure = sc == kHit;
-                        if (kCount) work[sc == kMiss ? W_SLAB_MISSES : sc == kHit ? W_SURE_HITS : W_EXACT_TESTS]++;
-                    }
-                }
-                const uint32_t m = __ballot_sync(0xffffffffu, live);
-                if (live) {
-                    const uint32_t e = (qh + qn + __popc(m & ((1u << lane) - 1u))) & (kQueue - 1u);
-                    qf[0 * kQueue + e] = dx; qf[1 * kQueue + e] = dy; qf[2 * kQueue + e] = dz;
-                    qf[3 * kQueue + e] = ix; qf[4 * kQueue + e] = iy; qf[5 * kQueue + e] = iz;
-                    q[6 * kQueue + e] = lane | (k << 5) | ((uint32_t)sure << 11);
-                }
-                qn += __popc(m);
-                k++;
-                if (qn < drain && k < n) continue;
-            }
-            if (qn == 0u) break;   // k == n and nothing pending
-            // one pair per lane: the exact test and the DDA; the word goes to its pixel
-            const uint32_t take = min(qn, 32u);
-            __syncwarp();
-            if (lane < take) {
-                const uint32_t e = (qh + lane) & (kQueue - 1u);
-                const uint32_t pk = q[6 * kQueue + e];
-                const TileEntry& te = E[(pk >> 5) & 63u];
-                const unsigned long long w = vis_pair<kCount>(
-                    te.ox, te.oy, te.oz, qf[0 * kQueue + e], qf[1 * kQueue + e], qf[2 * kQueue + e],
-                    qf[3 * kQueue + e], qf[4 * kQueue + e], qf[5 * kQueue + e], (pk >> 11) != 0u, te.bits,
-                    te.cluster_pointer, far_plane, far_rcp, &J.counters[C_DDA_OVERRUN], work);
-                if (w != ULLONG_MAX) atomicMin(sm.best() + ((warp << 5) | (pk & 31u)), w);
-            }
-            qh = (qh + take) & (kQueue - 1u);
-            qn -= take;
-            __syncwarp();
-            best_d24 = (uint32_t)(sm.best()[threadIdx.x] >> 40);
-        }
+        if (kCount && P.valid) work[W_BATCHES]++;
+        tile_batch<kCount, 1>(J, E, 0u, n, P, q, best0, work);
         // every pixel already nearer than the rest of the (bucket-sorted) entries: the tile is done
         if (!scan_all && base < end) {
             const uint32_t lo = bucket_lo(depth_bucket(E[n - 1].d24_lb, J.bshift), J.bshift);
-            if (__syncthreads_and(!valid || best_d24 < lo)) break;
+            if (__syncthreads_and(!P.valid || P.best_d24 < lo)) break;
         }
     }
     const unsigned long long best = sm.best()[threadIdx.x];
@@ -1108,10 +1164,10 @@ __device__ __forceinline__ bool vis_tile(const TileJob& J, uint32_t slot, const 
             mbar_wait_bounded(sm.bar(), phase ^ 1u);
         }
         __syncthreads();
-        if (valid) J.outs[view][(size_t)py * vc.width + px] = best;
+        if (P.valid) J.outs[view][(size_t)P.py * vc.width + P.px] = best;
         return false;
     }
-    if (valid) J.outs[view][(size_t)py * vc.width + px] = best;
+    if (P.valid) J.outs[view][(size_t)P.py * vc.width + P.px] = best;
     if (kCount) {
         // per warp: sum the lanes' counters, one 64-bit atomic each
 #pragma unroll
@@ -1123,6 +1179,97 @@ __device__ __forceinline__ bool vis_tile(const TileJob& J, uint32_t slot, const 
         }
     }
     return true;
+}
+
+// A tile with kGroups threads per pixel: group g of the CTA's threads covers all
+// of the tile's pixels and takes entries g, g + kGroups, ... of every batch, all
+// folding into the pixels' one set of words.  A frame whose tiles do not fill
+// the GPU takes as long as its heaviest tile, a chain of dependent batches;
+// more warps per tile shorten that chain.  Batches alternate between two stages,
+// each refilled as soon as its batch is consumed.  The words are the same bits:
+// the minimum does not depend on which group finds it.  One tile per CTA: the
+// mbarriers' phases start at zero.
+template <uint32_t kGroups>
+__device__ __forceinline__ void vis_tile_groups(const TileJob& J, uint32_t slot, const TileSm& sm,
+                                                tgx_dev_status* __restrict__ status)
+{
+    const uint32_t n_pix = blockDim.x / kGroups;
+    const uint32_t grp = threadIdx.x / n_pix, pix = threadIdx.x - grp * n_pix;
+    const uint4 si = J.slot_info[slot];
+    const uint32_t tile = si.x;
+    // bins overflowed this frame: gather every record whose tile rectangle holds the tile (slow, exact)
+    const bool scan_all = J.counters[C_OVERFLOW] != 0u;
+    if (!scan_all && si.z == 0u) {   // no entry: the tile is only cleared
+        const uint32_t v = tile_view(J, tile);
+        const ViewConst& vc = J.views[v];
+        const uint32_t lt = tile - vc.tile_base;
+        const uint32_t px = (lt % vc.tiles_x) * vc.tile_w + pix % vc.tile_w;
+        const uint32_t py = (lt / vc.tiles_x) * vc.tile_h + pix / vc.tile_w;
+        if (grp == 0u && px < vc.width && py < vc.height) J.outs[v][(size_t)py * vc.width + px] = ULLONG_MAX;
+        return;
+    }
+    const uint32_t n_batches = scan_all ? 0u : (si.z + J.batch - 1u) / J.batch;
+    uint32_t issued = 0;             // batches staged so far (thread 0)
+    auto stage = [&](uint32_t j) {   // batch j, in order
+        issued = j + 1u;
+        const uint32_t first = j * J.batch;
+        stage_entries(sm.bar(j % kStages), sm.stage() + (j % kStages) * kBatch, J.entries + si.y + first,
+                      min(J.batch, si.z - first), j == 0u ? J.extra_tx : 0u);
+    };
+    if (threadIdx.x == 0) {
+        for (uint32_t j = 0; j < min(n_batches, kStages); j++) stage(j);
+        sm.view() = tile_view(J, tile);
+        sm.lost() = 0u;
+    }
+    if (grp == 0u) sm.best()[pix] = ULLONG_MAX;
+    __syncthreads();
+    const uint32_t view = sm.view();
+    const ViewConst& vc = J.views[view];
+    TilePixel P;
+    tile_pixel(vc, tile, pix, P);
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t* const q = sm.queue(threadIdx.x >> 5);
+    unsigned long long* const best0 = sm.best() + (pix & ~31u);
+    uint32_t j = 0;
+    while (j < n_batches) {
+        const uint32_t n = min(J.batch, si.z - j * J.batch);
+        const TileEntry* const E = sm.stage() + (j % kStages) * kBatch;
+        const bool late = __any_sync(0xffffffffu, !mbar_wait_bounded(sm.bar(j % kStages), (j / kStages) & 1u));
+        uint32_t lo = 0u;
+        if (late) {
+            if (lane == 0) sm.lost() = 1u;
+        } else {
+            P.best_d24 = min(P.best_d24, (uint32_t)(best0[lane] >> 40));   // the other groups' words too
+            tile_batch<false, kGroups>(J, E, grp, n, P, q, best0, nullptr);
+            lo = bucket_lo(depth_bucket(E[n - 1].d24_lb, J.bshift), J.bshift);
+        }
+        // the batch is consumed; every pixel already nearer than the rest of the (bucket-sorted) entries: done
+        const bool done = __syncthreads_and(!P.valid || P.best_d24 < lo);
+        j++;
+        if (done || sm.lost()) break;
+        if (threadIdx.x == 0 && j + kStages - 1u < n_batches) stage(j + kStages - 1u);
+    }
+    if (threadIdx.x == 0) {
+        // no copy may land after the CTA is gone: wait (bounded) for the batches staged and not consumed
+        bool late = sm.lost() != 0u;
+        for (uint32_t k = late ? j - 1u : j; k < issued; k++)
+            late |= !mbar_wait_bounded(sm.bar(k % kStages), (k / kStages) & 1u);
+        if (late) dev_error(status, TGX_ERR_TIMEOUT, 5, tile);
+    }
+    if (scan_all) {
+        const uint32_t tx = (tile - vc.tile_base) % vc.tiles_x, ty = (tile - vc.tile_base) / vc.tiles_x;
+        const uint32_t n_rec = J.counters[C_RECORDS];
+        for (uint32_t base = 0; base < n_rec; base += J.batch) {
+            __syncthreads();
+            if (threadIdx.x == 0) sm.n() = 0;
+            __syncthreads();
+            gather_records(J, base, min(J.batch, n_rec - base), view, tx, ty, sm);
+            __syncthreads();
+            tile_batch<false, kGroups>(J, sm.stage(), grp, sm.n(), P, q, best0, nullptr);
+        }
+    }
+    __syncthreads();
+    if (P.valid && grp == 0u) J.outs[view][(size_t)P.py * vc.width + P.px] = sm.best()[pix];
 }
 
 // Instantiated per block size (= tile pixels) so the register budget can be
@@ -1149,6 +1296,22 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_vis_tiles(TileJob J, t
     uint32_t phase = 0;
     const uint32_t slot = J.interleave ? tile_slot(blockIdx.x, J.n_tiles, J.counters[C_NONEMPTY], true) : blockIdx.x;
     vis_tile<kCount>(J, slot, sm, phase, status);
+}
+
+// kGroups threads per pixel: kThreads = kGroups * the tile's pixels.
+template <int kThreads, uint32_t kGroups>
+__global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_vis_tiles_groups(TileJob J, tgx_dev_status* __restrict__ status)
+{
+    const TileSm sm = tile_sm<kGroups>();
+    tile_smem_init(sm);
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (uint32_t i = 1; i < kStages; i++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(sm.bar(i)));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    pdl_wait();
+    const uint32_t slot = J.interleave ? tile_slot(blockIdx.x, J.n_tiles, J.counters[C_NONEMPTY], true) : blockIdx.x;
+    vis_tile_groups<kGroups>(J, slot, sm, status);
 }
 
 // Persistent form over several jobs (scenes, each with its views): CTAs take
@@ -1328,6 +1491,23 @@ static TileJob tile_job(const tgx_ctx* c, const tgx_scene* s, const ViewConst* d
     return J;
 }
 
+// Threads per pixel of the tile launch: the largest power of two, up to 8 and
+// 1024 threads a CTA, that keeps the launch within 12 times the threads the GPU
+// holds (1024 per SM at the kernels' 64 registers).  Below that the time is the
+// heaviest tile's chain of batches, above it the sum of all tiles' work, which
+// grows with the threads.  Tile kernel over the 512-object scene, 8x8 tiles,
+// 1 / 2 / 4 / 8 threads per pixel: 480x270 239 / 141 / 99 / 76 us, 640x480 133 /
+// 87 / 71 / 100, 960x540 124 / 83 / 99 / 151, 1280x720 107 / 107 / 145 / 231,
+// 1920x1080 146 / 186 / 272 / 447; 16x16 tiles, 1 / 2 / 4: 480x270 554 / 318 / 234,
+// 1280x720 175 / 154 / 216, 1920x1080 181 / 249 / 376.
+static uint32_t vis_groups(const tgx_ctx* c, uint32_t pixels, uint32_t n_tiles)
+{
+    const uint64_t limit = 12ull * 1024ull * (uint64_t)c->num_sms;
+    uint32_t g = 1;
+    while (g < 8u && pixels * g * 2u <= 1024u && (uint64_t)n_tiles * pixels * g * 2u <= limit) g *= 2u;
+    return g;
+}
+
 // The launches of one frame (n_views views of scene s, view table d_vc / d_outs
 // on the device): all of them, or the part up to the tile scan, or the rest.
 static tgx_status vis_launch(tgx_ctx* c, const tgx_scene* s, const ViewConst* d_vc, unsigned long long* const* d_outs,
@@ -1387,6 +1567,19 @@ static tgx_status vis_launch(tgx_ctx* c, const tgx_scene* s, const ViewConst* d_
         else TGX_LAUNCH(c, TR_VIS_TILES, n_tiles, threads, smem, (k_vis_tiles<512, 2, true>), J, c->d_status);
         return TGX_OK;
     }
+    // (the fallthrough: 1 thread per pixel, and the pixel counts that are no power of two from 64 to 512)
+    const uint32_t groups = vis_groups(c, threads, n_tiles);
+#define TILE_GROUPS(px, g)                                                                                      \
+    if (threads == (px) && groups == (g)) {                                                                     \
+        TGX_LAUNCH_PDL(c, TR_VIS_TILES, n_tiles, (px) * (g), tile_smem_bytes((px), (g)),                        \
+                       (k_vis_tiles_groups<(px) * (g), (g)>), J, c->d_status);                                  \
+        return TGX_OK;                                                                                          \
+    }
+    TILE_GROUPS(64, 2) TILE_GROUPS(64, 4) TILE_GROUPS(64, 8)
+    TILE_GROUPS(128, 2) TILE_GROUPS(128, 4) TILE_GROUPS(128, 8)
+    TILE_GROUPS(256, 2) TILE_GROUPS(256, 4)
+    TILE_GROUPS(512, 2)
+#undef TILE_GROUPS
     if (threads == 64) TGX_LAUNCH_PDL(c, TR_VIS_TILES, n_tiles, threads, smem, (k_vis_tiles<64, 16>), J, c->d_status);
     else if (threads == 128) TGX_LAUNCH_PDL(c, TR_VIS_TILES, n_tiles, threads, smem, (k_vis_tiles<128, 10>), J, c->d_status);
     else if (threads == 256) TGX_LAUNCH_PDL(c, TR_VIS_TILES, n_tiles, threads, smem, (k_vis_tiles<256, 5>), J, c->d_status);
@@ -1415,6 +1608,12 @@ tgx_status vis_prepare_device(tgx_ctx* c)
     const uint32_t per_sm = threads == 64 ? vis_queue_per_sm<64, 16>() : threads == 128 ? vis_queue_per_sm<128, 10>()
                           : threads == 256 ? vis_queue_per_sm<256, 5>() : vis_queue_per_sm<512, 2>();
     c->vis_tile_ctas = (uint32_t)c->num_sms * per_sm;
+    // 1024 threads take more dynamic shared memory than a launch gets by default
+#define BIG_SMEM(px, g) \
+    TGX_CUDA(cudaFuncSetAttribute(k_vis_tiles_groups<(px) * (g), (g)>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                  (int)tile_smem_bytes((px), (g))))
+    BIG_SMEM(128, 8); BIG_SMEM(256, 4); BIG_SMEM(512, 2);
+#undef BIG_SMEM
     return TGX_OK;
 }
 
