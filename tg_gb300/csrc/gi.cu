@@ -165,12 +165,12 @@ __device__ __forceinline__ void svo_albedo(const SvoDev& s, const int32_t c[3], 
 // Primary hit of a pixel from its visibility word (shading.frag:116-228):
 // returns false for sky; else the offset origin o2, world normal nw and albedo a.
 __device__ bool primary_hit(const tgx_object* __restrict__ objects, const uint32_t* __restrict__ cluster_pointers,
-                            const uint32_t* __restrict__ c2o, const uint8_t* __restrict__ material,
+                            const uint32_t* __restrict__ cp_obj, const float4* __restrict__ inv, const uint8_t* __restrict__ material,
                             const tgx_material* __restrict__ luts, const tgx_view& cam, const GiParams& p,
                             unsigned long long word, uint32_t px, uint32_t py, float o2[3], float nw[3], float a[3])
 {
     PrimarySurface ps;
-    if (!primary_surface(objects, cluster_pointers, c2o, material, luts, cam, word, px, py, ps)) return false;
+    if (!primary_surface(objects, cluster_pointers, cp_obj, inv, material, luts, cam, word, px, py, ps)) return false;
     // no voxel-box hit in cluster space: face the camera
     const bool none = ps.nw[0] == 0.0f && ps.nw[1] == 0.0f && ps.nw[2] == 0.0f;
 #pragma unroll
@@ -276,9 +276,9 @@ __global__ void __launch_bounds__(32 * kTraceWarps, kTraceCtas) k_trace_queue(co
 }
 
 // Roots of the geometry pixels; sky pixels get the sky radiance.
-__global__ void __launch_bounds__(128) k_gi_roots(const tgx_object* __restrict__ objects,
+__global__ void __launch_bounds__(128, 10) k_gi_roots(const tgx_object* __restrict__ objects,
                                                   const uint32_t* __restrict__ cluster_pointers,
-                                                  const uint32_t* __restrict__ c2o, const uint8_t* __restrict__ material,
+                                                  const uint32_t* __restrict__ cp_obj, const float4* __restrict__ inv, const uint8_t* __restrict__ material,
                                                   const tgx_material* __restrict__ luts, tgx_view cam, GiParams p,
                                                   const unsigned long long* __restrict__ visbuf, float* __restrict__ out,
                                                   PathRoot* __restrict__ roots, uint32_t* __restrict__ n_roots)
@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(128) k_gi_roots(const tgx_object* __restrict__
     if (px >= cam.width || py >= cam.height) return;
     const uint32_t pixel = py * cam.width + px;
     PathRoot rt;
-    const bool geo = primary_hit(objects, cluster_pointers, c2o, material, luts, cam, p, visbuf[pixel], px, py, rt.o,
+    const bool geo = primary_hit(objects, cluster_pointers, cp_obj, inv, material, luts, cam, p, visbuf[pixel], px, py, rt.o,
                                  rt.n, rt.a);
     if (!geo) {
         out[3ull * pixel + 0] = p.sky_radiance[0];
@@ -858,7 +858,7 @@ extern "C" tgx_status tgx_gi_render(tgx_ctx* c, const tgx_scene* sc, const tgx_s
     uint32_t* exhausted = (uint32_t*)c->svo_counters.ptr + 8;
     TGX_CUDA(cudaMemsetAsync(counters, 0, 64 * 4, c->stream));
     const dim3 grid((view->width + 15) / 16, (view->height + 7) / 8);
-    TGX_LAUNCH(c, TR_GI, grid, 128, 0, k_gi_roots, sc->d_objects, sc->d_cluster_pointers, sc->d_c2o, sc->d_material,
+    TGX_LAUNCH(c, TR_GI, grid, 128, 0, k_gi_roots, sc->d_objects, sc->d_cluster_pointers, sc->d_cp_obj, sc->d_inv, sc->d_material,
                sc->d_luts, *view, p, (const unsigned long long*)d_visbuf, d_rgb, b.roots, &counters[CC_ROOTS]);
     return run_paths(c, svo_dev(svo), sc->d_luts, p, b, &counters[CC_ROOTS], (uint32_t)n_pix, p.spp,
                      &counters[CC_QUEUE], exhausted, d_rgb);
@@ -947,7 +947,7 @@ extern "C" tgx_status tgx_gi_render_cached(tgx_ctx* c, const tgx_scene* sc, cons
 
     // primary hits, then the first bounce of every (pixel, sample) in chunks
     const dim3 grid((view->width + 15) / 16, (view->height + 7) / 8);
-    TGX_LAUNCH(c, TR_GI, grid, 128, 0, k_gi_roots, sc->d_objects, sc->d_cluster_pointers, sc->d_c2o, sc->d_material,
+    TGX_LAUNCH(c, TR_GI, grid, 128, 0, k_gi_roots, sc->d_objects, sc->d_cluster_pointers, sc->d_cp_obj, sc->d_inv, sc->d_material,
                sc->d_luts, *view, p, (const unsigned long long*)d_visbuf, d_rgb, b.roots, &counters[CC_ROOTS]);
     const uint32_t eg = stride_grid(c, n_pix * cs + n_pix, 256);
     for (uint32_t s0 = 0; s0 < p.spp; s0 += cs) {

@@ -23,38 +23,82 @@ struct PrimarySurface
     float albedo[3];      // LUT albedo of the voxel (0.5 grey without materials)
 };
 
-// false for a sky pixel
-__device__ __forceinline__ bool primary_surface(const tgx_object* __restrict__ objects,
-                                                const uint32_t* __restrict__ cluster_pointers,
-                                                const uint32_t* __restrict__ c2o, const uint8_t* __restrict__ material,
-                                                const tgx_material* __restrict__ luts, const tgx_view& cam,
-                                                unsigned long long word, uint32_t px, uint32_t py, PrimarySurface& ps)
+// world space -> model space of the object's cluster (offset of the cluster's
+// corner from the object's, `half` the object's half extent in voxels) as the
+// shader multiplies it out: any matrix
+static __device__ __noinline__ void primary_ws2ms(const tgx_object* od, float offx, float offy, float offz, float hx,
+                                                  float hy, float hz, float* ws2ms)
 {
-    const float fx = xdiv(xadd((float)px, 0.5f), (float)cam.width);
-    const float fy = xsub(1.0f, xdiv(xadd((float)py, 0.5f), (float)cam.height));
-    ps.depth = xdiv((float)(word >> 40), 16777215.0f);
-    if (!(ps.depth < 1.0f)) return false;
-    const uint32_t ptr = (uint32_t)(word >> 9) & 2147483647u;
-    const uint32_t voxel = (uint32_t)word & 511u;
-    const uint32_t ci = cluster_pointers[ptr];
-    const uint32_t oi = c2o[ci];
-    ps.ptr = ptr; ps.voxel = voxel; ps.ci = ci; ps.oi = oi;
-    const tgx_object& od = objects[oi];
-    const uint32_t nx = od.n_cluster_pointers_per_dim[0], ny = od.n_cluster_pointers_per_dim[1];
-    const uint32_t rel = ptr - od.first_cluster_pointer;
-    const float offx = (float)((rel % nx) * 8u), offy = (float)(((rel / nx) % ny) * 8u), offz = (float)((rel / (nx * ny)) * 8u);
-    const float half = xmul(8.0f, 0.5f);
-    float rot[16], m0[16], m1[16], m2[16], m3[16], ws2ms[16];
+    float rot[16], m0[16], m1[16], m2[16], m3[16];
 #pragma unroll
-    for (int k = 0; k < 16; k++) rot[k] = od.rotation[k];
-    dm4_translate(-od.translation[0], -od.translation[1], -od.translation[2], m0);
+    for (int k = 0; k < 16; k++) rot[k] = od->rotation[k];
+    dm4_translate(-od->translation[0], -od->translation[1], -od->translation[2], m0);
     dm4_inverse(rot, m1);
-    dm4_translate(xmul(half, (float)od.n_cluster_pointers_per_dim[0]), xmul(half, (float)od.n_cluster_pointers_per_dim[1]),
-                  xmul(half, (float)od.n_cluster_pointers_per_dim[2]), m2);
+    dm4_translate(hx, hy, hz, m2);
     dm4_translate(-offx, -offy, -offz, m3);
     dm4_mul(m3, m2, ws2ms);
     dm4_mul(ws2ms, m1, ws2ms);
     dm4_mul(ws2ms, m0, ws2ms);
+}
+
+// Bound by arithmetic per pixel (the inverse and three 4x4 products were most
+// of it) and the chain of loads word -> pointer -> object.  The inverse is the
+// object's (inv, made at upload); in the products with translations every other
+// term multiplies by 0 or 1, so of 3 x 112 operations 48 are left, with the same
+// value in every element (only the sign of a zero can differ, which no later
+// step sees).  inv's first element is NaN where that does not hold (an element
+// that is infinite, NaN or huge: 0 times it is no zero): those objects take
+// the full products.  cp_obj gives the object beside the pointer's own load.
+// 1080p, 512 objects: the shading pass 44 -> 33 us, k_gi_roots 43 -> 34 us, the
+// larger part of it from the 10 resident CTAs that the fewer registers allow.
+// false for a sky pixel
+__device__ __forceinline__ bool primary_surface(const tgx_object* __restrict__ objects,
+                                                const uint32_t* __restrict__ cluster_pointers,
+                                                const uint32_t* __restrict__ cp_obj, const float4* __restrict__ inv,
+                                                const uint8_t* __restrict__ material,
+                                                const tgx_material* __restrict__ luts, const tgx_view& cam,
+                                                unsigned long long word, uint32_t px, uint32_t py, PrimarySurface& ps)
+{
+    ps.depth = xdiv((float)(word >> 40), 16777215.0f);
+    if (!(ps.depth < 1.0f)) return false;
+    const uint32_t ptr = (uint32_t)(word >> 9) & 2147483647u;
+    const uint32_t voxel = (uint32_t)word & 511u;
+    const uint32_t oi = cp_obj[ptr] & 0x7fffffffu;
+    const uint32_t ci = cluster_pointers[ptr];
+    ps.ptr = ptr; ps.voxel = voxel; ps.ci = ci; ps.oi = oi;
+    const tgx_object& od = objects[oi];
+    const uint32_t nx = od.n_cluster_pointers_per_dim[0], ny = od.n_cluster_pointers_per_dim[1];
+    const uint32_t rel = ptr - od.first_cluster_pointer;
+    const uint32_t row = rel / nx, layer = row / ny;
+    const float offx = (float)((rel - row * nx) * 8u), offy = (float)((row - layer * ny) * 8u), offz = (float)(layer * 8u);
+    const float half = xmul(8.0f, 0.5f);
+    const float hx = xmul(half, (float)nx), hy = xmul(half, (float)ny),
+                hz = xmul(half, (float)od.n_cluster_pointers_per_dim[2]);
+    float rot[12];
+#pragma unroll
+    for (int k = 0; k < 12; k++) rot[k] = od.rotation[k];
+    float ws2ms[16];
+    {
+        const float4 c0 = inv[4u * oi], c1 = inv[4u * oi + 1u], c2 = inv[4u * oi + 2u], c3 = inv[4u * oi + 3u];
+        if (c0.x == c0.x) {
+            // T(half - off) * inverse, then * T(-translation); rows 0..2
+            const float s3[3] = {xadd(hx, -offx), xadd(hy, -offy), xadd(hz, -offz)};
+            const float i0[3] = {c0.x, c0.y, c0.z}, i1[3] = {c1.x, c1.y, c1.z}, i2[3] = {c2.x, c2.y, c2.z},
+                        i3[3] = {c3.x, c3.y, c3.z};
+#pragma unroll
+            for (int r = 0; r < 3; r++) {
+                const float m0 = xadd(i0[r], xmul(s3[r], c0.w)), m1 = xadd(i1[r], xmul(s3[r], c1.w)),
+                            m2 = xadd(i2[r], xmul(s3[r], c2.w)), m3 = xadd(i3[r], xmul(s3[r], c3.w));
+                DM(ws2ms, r, 0) = m0; DM(ws2ms, r, 1) = m1; DM(ws2ms, r, 2) = m2;
+                DM(ws2ms, r, 3) = xadd(xadd(xadd(xmul(m0, -od.translation[0]), xmul(m1, -od.translation[1])),
+                                            xmul(m2, -od.translation[2])), m3);
+            }
+        } else {
+            primary_ws2ms(&od, offx, offy, offz, hx, hy, hz, ws2ms);
+        }
+    }
+    const float fx = xdiv(xadd((float)px, 0.5f), (float)cam.width);
+    const float fy = xsub(1.0f, xdiv(xadd((float)py, 0.5f), (float)cam.height));
     float o4[3];
     dm4_mulv4(ws2ms, cam.camera[0], cam.camera[1], cam.camera[2], 1.0f, o4);
 #pragma unroll
@@ -90,7 +134,10 @@ __device__ __forceinline__ bool primary_surface(const tgx_object* __restrict__ o
             else { nm[2] = sgn(nm[2]); nm[1] = 0.0f; }
         }
         float r4[3];
-        dm4_mulv4(rot, nm[0], nm[1], nm[2], 0.0f, r4);
+        // rotation * (nm, 0): the fourth column's products are zeros
+#pragma unroll
+        for (int r = 0; r < 3; r++)
+            r4[r] = xadd(xadd(xmul(nm[0], DM(rot, r, 0)), xmul(nm[1], DM(rot, r, 1))), xmul(nm[2], DM(rot, r, 2)));
         const float rl = xsqrt(xadd(xadd(xmul(r4[0], r4[0]), xmul(r4[1], r4[1])), xmul(r4[2], r4[2])));
         if (rl > 0.0f) { ps.nw[0] = xdiv(r4[0], rl); ps.nw[1] = xdiv(r4[1], rl); ps.nw[2] = xdiv(r4[2], rl); }
     }

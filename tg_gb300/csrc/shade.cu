@@ -47,7 +47,7 @@ __device__ __forceinline__ float ggx_distribution(float c_ndh, float roughness)
 __device__ __forceinline__ float schlick_ggx(float n_dot_v, float roughness)
 {
     const float r = xadd(roughness, 1.0f);
-    const float k = xdiv(xmul(r, r), 8.0f);
+    const float k = xmul(xmul(r, r), 0.125f);   // = / 8, exactly
     return xdiv(n_dot_v, xadd(xmul(n_dot_v, xsub(1.0f, k)), k));
 }
 
@@ -102,9 +102,9 @@ __device__ __forceinline__ void hash_color(uint32_t v, float* out)
     out[2] = xdiv((float)h2, 4294967295.0f);
 }
 
-__global__ void __launch_bounds__(128) k_shade(const tgx_object* __restrict__ objects,
+__global__ void __launch_bounds__(128, 10) k_shade(const tgx_object* __restrict__ objects,
                                               const uint32_t* __restrict__ cluster_pointers,
-                                              const uint32_t* __restrict__ c2o, const uint8_t* __restrict__ material,
+                                              const uint32_t* __restrict__ cp_obj, const float4* __restrict__ inv, const uint8_t* __restrict__ material,
                                               const tgx_material* __restrict__ luts, tgx_view cam,
                                               const unsigned long long* __restrict__ visbuf, uint32_t mode,
                                               float4* __restrict__ out)
@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(128) k_shade(const tgx_object* __restrict__ ob
     if (px >= cam.width || py >= cam.height) return;
     const uint32_t pixel = py * cam.width + px;
     PrimarySurface ps;
-    if (!primary_surface(objects, cluster_pointers, c2o, material, luts, cam, visbuf[pixel], px, py, ps)) {
+    if (!primary_surface(objects, cluster_pointers, cp_obj, inv, material, luts, cam, visbuf[pixel], px, py, ps)) {
         out[pixel] = make_float4(1.0f, 0.0f, 1.0f, 1.0f);
         return;
     }
@@ -140,8 +140,8 @@ __global__ void __launch_bounds__(128) k_shade(const tgx_object* __restrict__ ob
 #pragma unroll
         for (int i = 0; i < 3; i++) vv[i] = xsub(cam.camera[i], xadd(cam.camera[i], xmul(dm, ps.dws[i])));
         normalize3(vv, v);
-        const float l0[3] = {0.0f, 0.8f, 0.3f};
-        normalize3(l0, l);
+        // normalize((0, 0.8, 0.3)): the same three exactly rounded quotients, as constants
+        l[0] = 0.0f; l[1] = 0x1.df668ap-1f; l[2] = 0x1.678ce8p-2f;
 #pragma unroll
         for (int i = 0; i < 3; i++) spec[i] = xadd(xmul(0.04f, xsub(1.0f, metallic)), xmul(albedo[i], metallic));
         tg_shade(ps.nw, v, l, albedo, spec, metallic, roughness, radiance, lo);
@@ -163,7 +163,7 @@ extern "C" tgx_status tgx_shade(tgx_ctx* c, const tgx_scene* sc, const tgx_view*
         return TGX_ERR_INVALID_ARGUMENT;
     }
     const dim3 grid((view->width + 15) / 16, (view->height + 7) / 8);
-    TGX_LAUNCH(c, TR_GI, grid, 128, 0, k_shade, sc->d_objects, sc->d_cluster_pointers, sc->d_c2o, sc->d_material,
+    TGX_LAUNCH(c, TR_GI, grid, 128, 0, k_shade, sc->d_objects, sc->d_cluster_pointers, sc->d_cp_obj, sc->d_inv, sc->d_material,
                sc->d_luts, *view, (const unsigned long long*)d_visbuf, mode, (float4*)d_rgba);
     return TGX_OK;
 }

@@ -294,7 +294,8 @@ extern "C" tgx_status tgx_last_device_error(tgx_ctx* c, tgx_device_error* out)
 // tgm_m4_inverse's operation order).  For every cluster of an object the
 // first three columns of ws2ms (visibility.frag:62) equal this matrix in
 // value, so the ray direction can be transformed once per (pixel, object).
-__global__ void k_object_setup(const tgx_object* __restrict__ objs, uint32_t n, float* __restrict__ inv_rot)
+__global__ void k_object_setup(const tgx_object* __restrict__ objs, uint32_t n, float* __restrict__ inv_rot,
+                               float4* __restrict__ inv_all)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -306,6 +307,10 @@ __global__ void k_object_setup(const tgx_object* __restrict__ objs, uint32_t n, 
     for (int r = 0; r < 3; r++)
 #pragma unroll
         for (int c = 0; c < 3; c++) inv_rot[9 * i + 3 * r + c] = DM(inv, r, c);
+    if (!inverse_is_plain(inv)) inv[0] = __int_as_float(0x7fffffff);
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+        inv_all[4 * i + c] = make_float4(inv[4 * c], inv[4 * c + 1], inv[4 * c + 2], inv[4 * c + 3]);
 }
 
 // per cluster pointer p: c2o[cluster_pointers[p]], with bit 31 set when that
@@ -328,6 +333,7 @@ void scene_release(tgx_scene* s)
     cudaFree(s->d_cp_obj);
     cudaFree(s->d_objects);
     cudaFree(s->d_inv_rot);
+    cudaFree(s->d_inv);
     cudaFree(s->d_cluster_pointers);
     cudaFree(s->d_c2o);
     cudaFree(s->d_bits);
@@ -353,8 +359,16 @@ tgx_status scene_finish(tgx_ctx* c, tgx_scene* s)
             s->d_cluster_pointers, s->d_c2o, s->d_bits, s->n_cluster_pointers, s->d_cp_obj);
         if (cudaGetLastError() == cudaSuccess) c->launches++;
     }
+    if (!s->d_inv) {
+        const cudaError_t e = cudaMalloc((void**)&s->d_inv, (size_t)s->n_objects * 4 * sizeof(float4));
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            tgx_set_error("scene setup: out of device memory (%u object matrices)", s->n_objects);
+            return e == cudaErrorMemoryAllocation ? TGX_ERR_OUT_OF_MEMORY : TGX_ERR_CUDA;
+        }
+    }
     trace_begin(c, TR_OBJECT_SETUP);
-    k_object_setup<<<(s->n_objects + 127) / 128, 128, 0, c->stream>>>(s->d_objects, s->n_objects, s->d_inv_rot);
+    k_object_setup<<<(s->n_objects + 127) / 128, 128, 0, c->stream>>>(s->d_objects, s->n_objects, s->d_inv_rot, s->d_inv);
     cudaError_t le = cudaGetLastError();
     trace_end(c, TR_OBJECT_SETUP);
     if (le == cudaSuccess) c->launches++;

@@ -163,6 +163,9 @@ struct tgx_scene
     uint64_t    bytes = 0;                 // device bytes of the store, counted against the context's budget
     tgx_object* d_objects = nullptr;
     float*      d_inv_rot = nullptr;       // per object: 3x3 linear part of inverse(rotation), row-major
+    float4*     d_inv = nullptr;           // per object: the 16 floats of inverse(rotation), column-major; the first one
+                                           // is NaN when some element is not a moderate number (inverse_is_plain).
+                                           // Derived from the objects, not counted in `bytes`
     uint32_t*   d_cluster_pointers = nullptr;
     uint32_t*   d_c2o = nullptr;
     uint32_t*   d_bits = nullptr;
@@ -295,6 +298,16 @@ __device__ __forceinline__ void dm4_inverse(const float* m, float* out)
 #undef E
 #pragma unroll
     for (int i = 0; i < 16; i++) out[i] = r[i];
+}
+
+// Whether no element of an inverse rotation is NaN, infinite or so large that
+// its products with whole numbers below 2^24 could overflow.
+__device__ __forceinline__ bool inverse_is_plain(const float* inv)
+{
+    bool ok = true;
+#pragma unroll
+    for (int i = 0; i < 16; i++) ok = ok && fabsf(inv[i]) <= 1e30f;
+    return ok;
 }
 
 // tgm_m4_mulv4 (tg_math.c:2428-2438): row = ((x*m0 + y*m1) + z*m2) + w*m3
