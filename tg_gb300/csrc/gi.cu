@@ -59,12 +59,19 @@ struct __align__(8) Ray
     float o[3], d[3];   // d = 0: no ray
 };
 
-struct __align__(8) RayHit
+// A bounce ray's result, 16 bytes: one store by the lane that finished it.
+struct __align__(16) RayHit
 {
     float t;
-    int32_t c[3];
-    int32_t axis;
-    int32_t res;        // 1 hit, 0 miss, -1 step budget ran out
+    uint32_t xy;        // grid voxel x (14 bits) and y (14 bits), face axis + 1 (2 bits), hit (bit 31)
+    uint32_t z;         // grid voxel z
+    uint32_t pad;
+    __device__ __forceinline__ bool hit() const { return xy >> 31; }
+    __device__ __forceinline__ int32_t axis() const { return (int32_t)((xy >> 28) & 3u) - 1; }
+    __device__ __forceinline__ void voxel(int32_t c[3]) const
+    {
+        c[0] = (int32_t)(xy & 16383u); c[1] = (int32_t)((xy >> 14) & 16383u); c[2] = (int32_t)z;
+    }
 };
 
 struct __align__(8) PathRoot
@@ -75,17 +82,14 @@ struct __align__(8) PathRoot
     uint32_t key;       // Philox key and output index (pixel, or training sample)
 };
 
-struct __align__(16) PathState
+// A path between two passes: the radiance gathered so far and what the last
+// hit's sun light adds if its shadow ray, still to be traced, is clear; and,
+// while bounces are left, the throughput past that hit (w: alive).
+struct __align__(8) PathSum
 {
-    float v[3];         // radiance gathered so far
-    float T[3];         // throughput
-    float a[3];         // albedo of the last hit (its shadow ray is pending)
-    float ndl;
-    uint32_t flags;
-    uint32_t pad;
+    float v[3], c[3];
 };
-enum : uint32_t { P_ALIVE = 1u, P_SHADOW = 2u };
-static_assert(sizeof(Ray) == 24 && sizeof(RayHit) == 24 && sizeof(PathRoot) == 40 && sizeof(PathState) == 48,
+static_assert(sizeof(Ray) == 24 && sizeof(RayHit) == 16 && sizeof(PathRoot) == 40 && sizeof(PathSum) == 24,
               "record sizes: the alignment adds no padding");
 
 __device__ __forceinline__ void philox(uint32_t c[4], uint32_t k0, uint32_t k1)
@@ -209,6 +213,10 @@ __device__ __forceinline__ void null_ray(Ray& r)
     q[0] = q[1] = q[2] = make_float2(0.0f, 0.0f);
 }
 
+// A shadow ray: its origin (its direction is the sun's), w = 0: no ray.
+__device__ __forceinline__ float4 shadow_ray(const float o[3]) { return make_float4(o[0], o[1], o[2], 1.0f); }
+__device__ __forceinline__ float4 no_shadow_ray() { return make_float4(0.0f, 0.0f, 0.0f, 0.0f); }
+
 // face normal of an SVO hit: the face crossed, or the dominant axis when the
 // ray started inside the voxel
 __device__ __forceinline__ void hit_normal(int32_t axis, const float d[3], float n2[3])
@@ -236,43 +244,56 @@ __device__ __forceinline__ uint32_t warp_append(uint32_t* counter, bool want)
     return base + (uint32_t)__popc(mask & ((1u << lane) - 1u));
 }
 
-// The two ray lists of one traversal launch: a (n_a rays), then b.
+// The two ray lists of one traversal launch: a (n_a bounce rays), then b
+// (shadow rays toward the sun, of which only whether they hit is kept).
 struct RayLists
 {
-    const Ray *ra, *rb;
-    RayHit *ha, *hb;
+    const Ray* ra;
+    RayHit* ha;
+    const float4* rb;
+    uint32_t* hb;
     uint32_t n_a;
+    float sun[3];
     __device__ __forceinline__ void load(uint32_t i, float o[3], float d[3]) const
     {
-        const Ray r = i < n_a ? ra[i] : rb[i - n_a];
+        if (i < n_a) {
+            const Ray r = ra[i];
 #pragma unroll
-        for (int a = 0; a < 3; a++) { o[a] = r.o[a]; d[a] = r.d[a]; }
+            for (int a = 0; a < 3; a++) { o[a] = r.o[a]; d[a] = r.d[a]; }
+        } else {
+            const float4 r = rb[i - n_a];
+            o[0] = r.x; o[1] = r.y; o[2] = r.z;
+#pragma unroll
+            for (int a = 0; a < 3; a++) d[a] = r.w != 0.0f ? sun[a] : 0.0f;
+        }
     }
     __device__ __forceinline__ void store(uint32_t i, int res, float t, const int32_t c[3], int32_t axis) const
     {
-        RayHit h;
-        h.t = t;
-        h.c[0] = c[0]; h.c[1] = c[1]; h.c[2] = c[2];
-        h.axis = axis;
-        h.res = res;
-        (i < n_a ? ha[i] : hb[i - n_a]) = h;
+        if (i < n_a) {
+            RayHit h;
+            h.t = t;
+            h.xy = (uint32_t)c[0] | (uint32_t)c[1] << 14 | (uint32_t)(axis + 1) << 28 | 0x80000000u;
+            h.z = (uint32_t)c[2];
+            h.pad = 0u;
+            if (res != 1) h.xy = 0u;
+            ha[i] = h;
+        } else {
+            hb[i - n_a] = res == 1 ? 1u : 0u;
+        }
     }
 };
 
-// Persistent traversal of two ray lists: a (n * mul_a rays) then b (n * mul_b
-// rays), n read from the device (svo_trace_queue).
-__global__ void __launch_bounds__(32 * kTraceWarps, kTraceCtas) k_trace_queue(const __grid_constant__ SvoDev s,
-                                                                  const Ray* __restrict__ ra, RayHit* __restrict__ ha,
-                                                                  uint32_t mul_a, const Ray* __restrict__ rb,
-                                                                  RayHit* __restrict__ hb, uint32_t mul_b,
-                                                                  const uint32_t* __restrict__ n_dev, uint32_t max_steps,
-                                                                  uint32_t steps_per_round, uint32_t* __restrict__ queue,
-                                                                  uint32_t* __restrict__ exhausted,
-                                                                  unsigned long long* __restrict__ work)
+// Persistent traversal of two ray lists: a (n * mul_a bounce rays) then b (n *
+// mul_b shadow rays), n read from the device (svo_trace_queue).
+__global__ void __launch_bounds__(32 * kTraceWarps, kTraceCtas) k_trace_queue(
+    const __grid_constant__ SvoDev s, const Ray* __restrict__ ra, RayHit* __restrict__ ha, uint32_t mul_a,
+    const float4* __restrict__ rb, uint32_t* __restrict__ hb, uint32_t mul_b, GiParams p,
+    const uint32_t* __restrict__ n_dev, uint32_t steps_per_round, uint32_t* __restrict__ queue,
+    uint32_t* __restrict__ exhausted, unsigned long long* __restrict__ work)
 {
     const uint32_t n = *n_dev;
-    const RayLists io = {ra, rb, ha, hb, n * mul_a};
-    svo_trace_queue(s, io, n * mul_a + n * mul_b, max_steps, steps_per_round, queue, exhausted, work);
+    const RayLists io = {ra, ha, rb, hb, n * mul_a, {p.sun_dir[0], p.sun_dir[1], p.sun_dir[2]}};
+    svo_trace_queue(s, io, n * mul_a + n * mul_b, p.max_steps, steps_per_round, queue, exhausted, work);
 }
 
 // Roots of the geometry pixels; sky pixels get the sky radiance.
@@ -302,11 +323,18 @@ __global__ void __launch_bounds__(128, 10) k_gi_roots(const tgx_object* __restri
     }
 }
 
+// The path passes below are bound by memory traffic (a thread per path, long
+// lists).  Per path of one bounce they move 192 bytes: ray 24 out, 24 + 16 in
+// and out of the traversal, 40 in and 40 out here, 16 + 4 through the shadow
+// traversal, 28 into the sum -- against 432 when every pass read and wrote a
+// 48-byte state, null rays and 24-byte shadow results.  1080p, 1 bounce, 4 spp:
+// emit 69 -> 27 us, shade 106 -> 53, finish 44 -> 22.
+
 // First bounce ray of every path (root r, sample s0 + j) of a chunk of cs
 // samples; with root_rays, also the shadow ray of every root.
 __global__ void __launch_bounds__(256) k_gi_emit(const PathRoot* __restrict__ roots, const uint32_t* __restrict__ n_dev,
                                                  uint32_t cs, uint32_t s0, GiParams p, Ray* __restrict__ rays,
-                                                 PathState* __restrict__ st, Ray* __restrict__ root_rays)
+                                                 float4* __restrict__ root_rays)
 {
     const uint32_t n = *n_dev;
     const uint64_t n_paths = (uint64_t)n * cs;
@@ -318,85 +346,90 @@ __global__ void __launch_bounds__(256) k_gi_emit(const PathRoot* __restrict__ ro
             float w[3];
             sample_cosine(rt.n, rt.key, s0 + ((uint32_t)i - r * cs), 0, p, w);
             set_ray(rays[i], rt.o, w);
-            if (!st) continue;   // first-bounce queries keep no path state
-            PathState ps;
-            ps.v[0] = ps.v[1] = ps.v[2] = 0.0f;
-            ps.T[0] = ps.T[1] = ps.T[2] = 1.0f;
-            ps.a[0] = ps.a[1] = ps.a[2] = 0.0f;
-            ps.ndl = 0.0f;
-            ps.flags = P_ALIVE;
-            ps.pad = 0;
-            st[i] = ps;
         } else {
             const uint32_t r = (uint32_t)(i - n_paths);
             const PathRoot& rt = roots[r];
-            if (sun_cos(rt.n, p) > 0.0f) set_ray(root_rays[r], rt.o, p.sun_dir);
-            else null_ray(root_rays[r]);
+            root_rays[r] = sun_cos(rt.n, p) > 0.0f ? shadow_ray(rt.o) : no_shadow_ray();
         }
     }
 }
 
 // Consumes the pending shadow ray of bounce k-1 and the hit of bounce k.
+// kFirst: k = 0, a path starts here with nothing gathered and throughput 1.
+// kLast: no bounce follows, so neither its ray nor the throughput is written.
+// A path that ended in an earlier pass keeps its null rays, so only its sum
+// could still change, and that was settled when it ended.
+template <bool kFirst, bool kLast>
 __global__ void __launch_bounds__(256) k_gi_shade(SvoDev s, const tgx_material* __restrict__ luts,
                                                   const PathRoot* __restrict__ roots, const uint32_t* __restrict__ n_dev,
                                                   uint32_t cs, uint32_t s0, uint32_t k, GiParams p,
                                                   Ray* __restrict__ rb, const RayHit* __restrict__ hb,
-                                                  Ray* __restrict__ rs, const RayHit* __restrict__ hs,
-                                                  PathState* __restrict__ st)
+                                                  float4* __restrict__ rs, const uint32_t* __restrict__ hs,
+                                                  PathSum* __restrict__ sums, float4* __restrict__ through)
 {
     const uint64_t n_paths = (uint64_t)(*n_dev) * cs;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_paths; i += (uint64_t)gridDim.x * blockDim.x) {
-        PathState ps = st[i];
-        if (ps.flags & P_SHADOW) {
-            float D[3] = {0.0f, 0.0f, 0.0f};
-            if (ps.ndl > 0.0f && hs[i].res != 1) sun_term(ps.a, ps.ndl, p, D);
+        float v[3] = {0.0f, 0.0f, 0.0f}, T[3] = {1.0f, 1.0f, 1.0f};
+        if (!kFirst) {
+            const float4 tf = through[i];
+            if (tf.w == 0.0f) continue;
+            T[0] = tf.x; T[1] = tf.y; T[2] = tf.z;
+            const PathSum ps = sums[i];
+            const bool lit = hs[i] == 0u;
+#pragma unroll
+            for (int c = 0; c < 3; c++) v[c] = lit ? xadd(ps.v[c], ps.c[c]) : ps.v[c];
+        }
+        const RayHit h = hb[i];
+        PathSum out;
+        float4 ns = no_shadow_ray(), tn = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (!h.hit()) {
 #pragma unroll
             for (int c = 0; c < 3; c++) {
-                ps.v[c] = xadd(ps.v[c], xmul(ps.T[c], D[c]));
-                ps.T[c] = xmul(ps.T[c], ps.a[c]);
+                out.v[c] = xadd(v[c], xmul(T[c], p.sky_radiance[c]));
+                out.c[c] = 0.0f;
             }
-            ps.flags &= ~P_SHADOW;
-        }
-        Ray nb, ns;
-        null_ray(nb);
-        null_ray(ns);
-        if (ps.flags & P_ALIVE) {
-            const RayHit h = hb[i];
+            if (!kLast) null_ray(rb[i]);
+        } else {
             const Ray ray = rb[i];
-            if (h.res != 1) {
+            float n2[3], o3[3], a[3], D[3] = {0.0f, 0.0f, 0.0f};
+            int32_t cv[3];
+            h.voxel(cv);
+            hit_normal(h.axis(), ray.d, n2);
+            svo_albedo(s, cv, luts, a);
 #pragma unroll
-                for (int c = 0; c < 3; c++) ps.v[c] = xadd(ps.v[c], xmul(ps.T[c], p.sky_radiance[c]));
-                ps.flags &= ~P_ALIVE;
-            } else {
-                float n2[3], o3[3];
-                hit_normal(h.axis, ray.d, n2);
-                svo_albedo(s, h.c, luts, ps.a);
+            for (int c = 0; c < 3; c++) o3[c] = xadd(xadd(ray.o[c], xmul(h.t, ray.d[c])), xmul(n2[c], p.offset));
+            const float ndl = sun_cos(n2, p);
+            if (ndl > 0.0f) {
+                sun_term(a, ndl, p, D);
+                ns = shadow_ray(o3);
+            }
 #pragma unroll
-                for (int c = 0; c < 3; c++) o3[c] = xadd(xadd(ray.o[c], xmul(h.t, ray.d[c])), xmul(n2[c], p.offset));
-                ps.ndl = sun_cos(n2, p);
-                ps.flags |= P_SHADOW;
-                if (ps.ndl > 0.0f) set_ray(ns, o3, p.sun_dir);
-                if (k + 1 < p.bounces) {
-                    float w2[3];
-                    const uint32_t r = (uint32_t)i / cs;
-                    sample_cosine(n2, roots[r].key, s0 + ((uint32_t)i - r * cs), k + 1, p, w2);
-                    set_ray(nb, o3, w2);
-                } else {
-                    ps.flags &= ~P_ALIVE;
-                }
+            for (int c = 0; c < 3; c++) {
+                out.v[c] = v[c];
+                out.c[c] = xmul(T[c], D[c]);
+            }
+            if (!kLast) {
+                float w2[3];
+                const uint32_t r = (uint32_t)i / cs;
+                sample_cosine(n2, roots[r].key, s0 + ((uint32_t)i - r * cs), k + 1, p, w2);
+                set_ray(rb[i], o3, w2);
+                tn = make_float4(xmul(T[0], a[0]), xmul(T[1], a[1]), xmul(T[2], a[2]), 1.0f);
             }
         }
-        rb[i] = nb;
         rs[i] = ns;
-        st[i] = ps;
+        float2* q = reinterpret_cast<float2*>(&sums[i]);
+        q[0] = make_float2(out.v[0], out.v[1]);
+        q[1] = make_float2(out.v[2], out.c[0]);
+        q[2] = make_float2(out.c[1], out.c[2]);
+        if (!kLast) through[i] = tn;
     }
 }
 
 // Per root: the last pending shadows, the chunk's samples added in order to
 // the running sum; on the last chunk out[key] = direct + albedo * sum / spp.
 __global__ void __launch_bounds__(256) k_gi_finish(const PathRoot* __restrict__ roots, const uint32_t* __restrict__ n_dev,
-                                                   uint32_t cs, GiParams p, const RayHit* __restrict__ hs,
-                                                   const PathState* __restrict__ st, const RayHit* __restrict__ root_hits,
+                                                   uint32_t cs, GiParams p, const uint32_t* __restrict__ hs,
+                                                   const PathSum* __restrict__ sums, const uint32_t* __restrict__ root_hits,
                                                    float* __restrict__ acc_buf, bool first, bool last, uint32_t spp,
                                                    float* __restrict__ out)
 {
@@ -406,16 +439,10 @@ __global__ void __launch_bounds__(256) k_gi_finish(const PathRoot* __restrict__ 
         if (!first) { acc[0] = acc_buf[3ull * r]; acc[1] = acc_buf[3ull * r + 1]; acc[2] = acc_buf[3ull * r + 2]; }
         for (uint32_t j = 0; j < cs; j++) {
             const uint64_t i = (uint64_t)r * cs + j;
-            const PathState& ps = st[i];
-            float v[3] = {ps.v[0], ps.v[1], ps.v[2]};
-            if (ps.flags & P_SHADOW) {
-                float D[3] = {0.0f, 0.0f, 0.0f};
-                if (ps.ndl > 0.0f && hs[i].res != 1) sun_term(ps.a, ps.ndl, p, D);
+            const PathSum ps = sums[i];
+            const bool lit = hs[i] == 0u;
 #pragma unroll
-                for (int c = 0; c < 3; c++) v[c] = xadd(v[c], xmul(ps.T[c], D[c]));
-            }
-#pragma unroll
-            for (int c = 0; c < 3; c++) acc[c] = xadd(acc[c], v[c]);
+            for (int c = 0; c < 3; c++) acc[c] = xadd(acc[c], lit ? xadd(ps.v[c], ps.c[c]) : ps.v[c]);
         }
         if (!last) {
             acc_buf[3ull * r] = acc[0]; acc_buf[3ull * r + 1] = acc[1]; acc_buf[3ull * r + 2] = acc[2];
@@ -424,7 +451,7 @@ __global__ void __launch_bounds__(256) k_gi_finish(const PathRoot* __restrict__ 
         const PathRoot& rt = roots[r];
         float L[3] = {0.0f, 0.0f, 0.0f};
         const float ndl = sun_cos(rt.n, p);
-        if (ndl > 0.0f && root_hits[r].res != 1) sun_term(rt.a, ndl, p, L);
+        if (ndl > 0.0f && root_hits[r] == 0u) sun_term(rt.a, ndl, p, L);
         const float inv_spp = xdiv(1.0f, (float)(spp ? spp : 1u));
 #pragma unroll
         for (int c = 0; c < 3; c++) out[3ull * rt.key + c] = xadd(L[c], xmul(rt.a[c], xmul(acc[c], inv_spp)));
@@ -485,21 +512,21 @@ __global__ void __launch_bounds__(256) k_gi_query_shade(SvoDev s, const tgx_mate
         const RayHit h = hb[i];
         const uint32_t r = (uint32_t)i / cs;   // paths in flight < 2^32: 32-bit division
         int32_t* qi = qidx + (uint64_t)r * spp + s0 + ((uint32_t)i - r * cs);
-        const bool hit = h.res == 1;
+        const bool hit = h.hit();
         const uint32_t slot = warp_append(&counters[CC_QUERIES], hit);
         if (!hit) { *qi = -1; continue; }
         if (slot >= capacity) { *qi = -2; continue; }
         *qi = (int32_t)slot;
         const Ray ray = rb[i];
         CacheHit ch;
-        hit_normal(h.axis, ray.d, ch.n);
+        hit_normal(h.axis(), ray.d, ch.n);
+        h.voxel(ch.c);
 #pragma unroll
         for (int c = 0; c < 3; c++) {
             ch.p[c] = xadd(ray.o[c], xmul(h.t, ray.d[c]));
             ch.w[c] = ray.d[c];
-            ch.c[c] = h.c[c];
         }
-        svo_albedo(s, h.c, luts, ch.a);
+        svo_albedo(s, ch.c, luts, ch.a);
         hits[slot] = ch;
         cache_input(q, ch.p, ch.n, ch.w, qx + 9ull * slot);
     }
@@ -559,7 +586,7 @@ __global__ void __launch_bounds__(256) k_gi_primary_batch(GiParams p, CacheGiCon
 // training target.
 __global__ void __launch_bounds__(256) k_gi_cache_resolve(const PathRoot* __restrict__ roots,
                                                          const uint32_t* __restrict__ n_dev, GiParams p,
-                                                         const RayHit* __restrict__ root_hits,
+                                                         const uint32_t* __restrict__ root_hits,
                                                          const int32_t* __restrict__ qidx,
                                                          const float* __restrict__ qrgb,
                                                          const CacheHit* __restrict__ hits,
@@ -583,7 +610,7 @@ __global__ void __launch_bounds__(256) k_gi_cache_resolve(const PathRoot* __rest
         }
         float L[3] = {0.0f, 0.0f, 0.0f};
         const float ndl = sun_cos(rt.n, p);
-        if (ndl > 0.0f && root_hits[r].res != 1) sun_term(rt.a, ndl, p, L);
+        if (ndl > 0.0f && root_hits[r] == 0u) sun_term(rt.a, ndl, p, L);
         const float inv_spp = xdiv(1.0f, (float)(p.spp ? p.spp : 1u));
         float m[3], pr[3];
 #pragma unroll
@@ -630,7 +657,7 @@ constexpr int kBlendRadius = 6;   // a 13x13 window
 
 __global__ void __launch_bounds__(256) k_gi_cache_blend(const PathRoot* __restrict__ roots,
                                                        const uint32_t* __restrict__ n_dev, GiParams p,
-                                                       const RayHit* __restrict__ root_hits,
+                                                       const uint32_t* __restrict__ root_hits,
                                                        const float* __restrict__ pmean, const float* __restrict__ prim_rgb,
                                                        const float2* __restrict__ pstat, uint32_t width, uint32_t height,
                                                        float primary_weight, float variance_scale,
@@ -656,7 +683,7 @@ __global__ void __launch_bounds__(256) k_gi_cache_blend(const PathRoot* __restri
         const float kw = vm > 0.0f ? fminf(primary_weight, vm / (vm + b2)) : 0.0f;
         float L[3] = {0.0f, 0.0f, 0.0f};
         const float ndl = sun_cos(rt.n, p);
-        if (ndl > 0.0f && root_hits[r].res != 1) sun_term(rt.a, ndl, p, L);
+        if (ndl > 0.0f && root_hits[r] == 0u) sun_term(rt.a, ndl, p, L);
 #pragma unroll
         for (int i = 0; i < 3; i++) {
             const float m = pmean[3ull * r + i], pr = fmaxf(prim_rgb[3ull * r + i], 0.0f);
@@ -720,9 +747,12 @@ namespace {
 struct PathBufs
 {
     PathRoot* roots;
-    Ray *rb, *rs, *root_rays;
-    RayHit *hb, *hs, *root_hits;
-    PathState* st;
+    Ray* rb;                 // bounce rays and their results
+    RayHit* hb;
+    float4 *rs, *root_rays;  // shadow rays of the paths and of the roots, and whether they hit
+    uint32_t *hs, *root_hits;
+    PathSum* sums;
+    float4* through;
     float* acc;
     uint64_t max_paths;
 };
@@ -744,14 +774,15 @@ struct Carver
 void carve_paths(Carver& cv, PathBufs& b, uint64_t max_roots, uint64_t max_paths)
 {
     b.roots = cv.take<PathRoot>(max_roots);
-    b.root_rays = cv.take<Ray>(max_roots);
-    b.root_hits = cv.take<RayHit>(max_roots);
+    b.root_rays = cv.take<float4>(max_roots);
+    b.root_hits = cv.take<uint32_t>(max_roots);
     b.acc = cv.take<float>(max_roots * 3);
     b.rb = cv.take<Ray>(max_paths);
-    b.rs = cv.take<Ray>(max_paths);
+    b.rs = cv.take<float4>(max_paths);
     b.hb = cv.take<RayHit>(max_paths);
-    b.hs = cv.take<RayHit>(max_paths);
-    b.st = cv.take<PathState>(max_paths);
+    b.hs = cv.take<uint32_t>(max_paths);
+    b.sums = cv.take<PathSum>(max_paths);
+    b.through = cv.take<float4>(max_paths);
     b.max_paths = max_paths;
 }
 
@@ -784,12 +815,12 @@ __host__ __device__ inline unsigned long long* trace_work(uint32_t* counters)
 }
 
 // queue = &counters[CC_QUEUE] of the frame's counters
-tgx_status trace_lists(tgx_ctx* c, const SvoDev& s, const Ray* ra, RayHit* ha, uint32_t mul_a, const Ray* rb,
-                       RayHit* hb, uint32_t mul_b, const uint32_t* n_dev, uint32_t max_steps, uint32_t* queue,
+tgx_status trace_lists(tgx_ctx* c, const SvoDev& s, const GiParams& p, const Ray* ra, RayHit* ha, uint32_t mul_a,
+                       const float4* rb, uint32_t* hb, uint32_t mul_b, const uint32_t* n_dev, uint32_t* queue,
                        uint32_t* exhausted)
 {
     TGX_CUDA(cudaMemsetAsync(queue, 0, 4, c->stream));
-    TGX_LAUNCH(c, TR_GI_TRACE, trace_grid(c), 128, 0, k_trace_queue, s, ra, ha, mul_a, rb, hb, mul_b, n_dev, max_steps,
+    TGX_LAUNCH(c, TR_GI_TRACE, trace_grid(c), 128, 0, k_trace_queue, s, ra, ha, mul_a, rb, hb, mul_b, p, n_dev,
                c->trace_steps_per_round, queue, exhausted, trace_work(queue - CC_QUEUE));
     return TGX_OK;
 }
@@ -802,9 +833,9 @@ tgx_status run_paths(tgx_ctx* c, const SvoDev& s, const tgx_material* luts, cons
     const uint32_t cs = chunk_samples(spp, max_roots);
     const uint32_t rg = stride_grid(c, max_roots, 256);
     if (spp == 0 || p.bounces == 0) {   // direct term only
-        TGX_LAUNCH(c, TR_GI, rg, 256, 0, k_gi_emit, b.roots, n_dev, 0u, 0u, p, b.rb, b.st, b.root_rays);
-        TGX_TRY(trace_lists(c, s, nullptr, nullptr, 0u, b.root_rays, b.root_hits, 1u, n_dev, p.max_steps, queue, exhausted));
-        TGX_LAUNCH(c, TR_GI, rg, 256, 0, k_gi_finish, b.roots, n_dev, 0u, p, b.hs, b.st, b.root_hits, b.acc, true, true,
+        TGX_LAUNCH(c, TR_GI, rg, 256, 0, k_gi_emit, b.roots, n_dev, 0u, 0u, p, b.rb, b.root_rays);
+        TGX_TRY(trace_lists(c, s, p, nullptr, nullptr, 0u, b.root_rays, b.root_hits, 1u, n_dev, queue, exhausted));
+        TGX_LAUNCH(c, TR_GI, rg, 256, 0, k_gi_finish, b.roots, n_dev, 0u, p, b.hs, b.sums, b.root_hits, b.acc, true, true,
                    spp, out);
         return TGX_OK;
     }
@@ -812,16 +843,20 @@ tgx_status run_paths(tgx_ctx* c, const SvoDev& s, const tgx_material* luts, cons
     for (uint32_t s0 = 0; s0 < spp; s0 += cs) {
         const uint32_t n = std::min(cs, spp - s0);
         const bool first = s0 == 0, last = s0 + n >= spp;
-        TGX_LAUNCH(c, TR_GI, eg, 256, 0, k_gi_emit, b.roots, n_dev, n, s0, p, b.rb, b.st, first ? b.root_rays : nullptr);
-        TGX_TRY(trace_lists(c, s, b.rb, b.hb, n, b.root_rays, b.root_hits, first ? 1u : 0u, n_dev, p.max_steps, queue,
-                            exhausted));
+        TGX_LAUNCH(c, TR_GI, eg, 256, 0, k_gi_emit, b.roots, n_dev, n, s0, p, b.rb, first ? b.root_rays : nullptr);
+        TGX_TRY(trace_lists(c, s, p, b.rb, b.hb, n, b.root_rays, b.root_hits, first ? 1u : 0u, n_dev, queue, exhausted));
         for (uint32_t k = 0; k < p.bounces; k++) {
-            TGX_LAUNCH(c, TR_GI, eg, 256, 0, k_gi_shade, s, luts, b.roots, n_dev, n, s0, k, p, b.rb, b.hb, b.rs, b.hs,
-                       b.st);
-            TGX_TRY(trace_lists(c, s, b.rb, b.hb, k + 1 < p.bounces ? n : 0u, b.rs, b.hs, n, n_dev, p.max_steps, queue,
-                                exhausted));
+            const bool more = k + 1 < p.bounces;
+#define SHADE(f, l) TGX_LAUNCH(c, TR_GI, eg, 256, 0, (k_gi_shade<f, l>), s, luts, b.roots, n_dev, n, s0, k, p, b.rb, b.hb, \
+                               b.rs, b.hs, b.sums, b.through)
+            if (k == 0 && more) SHADE(true, false);
+            else if (k == 0) SHADE(true, true);
+            else if (more) SHADE(false, false);
+            else SHADE(false, true);
+#undef SHADE
+            TGX_TRY(trace_lists(c, s, p, b.rb, b.hb, more ? n : 0u, b.rs, b.hs, n, n_dev, queue, exhausted));
         }
-        TGX_LAUNCH(c, TR_GI, rg, 256, 0, k_gi_finish, b.roots, n_dev, n, p, b.hs, b.st, b.root_hits, b.acc, first, last,
+        TGX_LAUNCH(c, TR_GI, rg, 256, 0, k_gi_finish, b.roots, n_dev, n, p, b.hs, b.sums, b.root_hits, b.acc, first, last,
                    spp, out);
     }
     return TGX_OK;
@@ -953,10 +988,10 @@ extern "C" tgx_status tgx_gi_render_cached(tgx_ctx* c, const tgx_scene* sc, cons
     for (uint32_t s0 = 0; s0 < p.spp; s0 += cs) {
         const uint32_t n = std::min(cs, p.spp - s0);
         const bool first = s0 == 0;
-        TGX_LAUNCH(c, TR_GI, eg, 256, 0, k_gi_emit, b.roots, &counters[CC_ROOTS], n, s0, p, b.rb, (PathState*)nullptr,
+        TGX_LAUNCH(c, TR_GI, eg, 256, 0, k_gi_emit, b.roots, &counters[CC_ROOTS], n, s0, p, b.rb,
                    first ? b.root_rays : nullptr);
-        TGX_TRY(trace_lists(c, s, b.rb, b.hb, n, b.root_rays, b.root_hits, first ? 1u : 0u, &counters[CC_ROOTS],
-                            p.max_steps, &counters[CC_QUEUE], exhausted));
+        TGX_TRY(trace_lists(c, s, p, b.rb, b.hb, n, b.root_rays, b.root_hits, first ? 1u : 0u, &counters[CC_ROOTS],
+                            &counters[CC_QUEUE], exhausted));
         TGX_LAUNCH(c, TR_GI, eg, 256, 0, k_gi_query_shade, s, sc->d_luts, q, &counters[CC_ROOTS], n, s0, p.spp, b.rb,
                    b.hb, qidx, qx, hits, counters, (uint32_t)capacity);
     }
