@@ -43,12 +43,10 @@ static __device__ __noinline__ void primary_ws2ms(const tgx_object* od, float of
 
 // Bound by arithmetic per pixel (the inverse and three 4x4 products were most
 // of it) and the chain of loads word -> pointer -> object.  The inverse is the
-// object's (inv, made at upload); in the products with translations every other
-// term multiplies by 0 or 1, so of 3 x 112 operations 48 are left, with the same
-// value in every element (only the sign of a zero can differ, which no later
-// step sees).  inv's first element is NaN where that does not hold (an element
-// that is infinite, NaN or huge: 0 times it is no zero): those objects take
-// the full products.  cp_obj gives the object beside the pointer's own load.
+// object's (inv, made at upload), and of 3 x 112 operations of the products 48
+// are left (dm4_ws2ms).  inv's first element is NaN where that does not hold (an
+// element that is infinite, NaN or huge: 0 times it is no zero): those objects
+// take the full products.  cp_obj gives the object beside the pointer's own load.
 // 1080p, 512 objects: the shading pass 44 -> 33 us, k_gi_roots 43 -> 34 us, the
 // larger part of it from the 10 resident CTAs that the fewer registers allow.
 // false for a sky pixel
@@ -81,18 +79,8 @@ __device__ __forceinline__ bool primary_surface(const tgx_object* __restrict__ o
     {
         const float4 c0 = inv[4u * oi], c1 = inv[4u * oi + 1u], c2 = inv[4u * oi + 2u], c3 = inv[4u * oi + 3u];
         if (c0.x == c0.x) {
-            // T(half - off) * inverse, then * T(-translation); rows 0..2
             const float s3[3] = {xadd(hx, -offx), xadd(hy, -offy), xadd(hz, -offz)};
-            const float i0[3] = {c0.x, c0.y, c0.z}, i1[3] = {c1.x, c1.y, c1.z}, i2[3] = {c2.x, c2.y, c2.z},
-                        i3[3] = {c3.x, c3.y, c3.z};
-#pragma unroll
-            for (int r = 0; r < 3; r++) {
-                const float m0 = xadd(i0[r], xmul(s3[r], c0.w)), m1 = xadd(i1[r], xmul(s3[r], c1.w)),
-                            m2 = xadd(i2[r], xmul(s3[r], c2.w)), m3 = xadd(i3[r], xmul(s3[r], c3.w));
-                DM(ws2ms, r, 0) = m0; DM(ws2ms, r, 1) = m1; DM(ws2ms, r, 2) = m2;
-                DM(ws2ms, r, 3) = xadd(xadd(xadd(xmul(m0, -od.translation[0]), xmul(m1, -od.translation[1])),
-                                            xmul(m2, -od.translation[2])), m3);
-            }
+            dm4_ws2ms(c0, c1, c2, c3, s3, od.translation, ws2ms);
         } else {
             primary_ws2ms(&od, offx, offy, offz, hx, hy, hz, ws2ms);
         }

@@ -12,15 +12,15 @@
 //      whose whole path passes becomes a (cluster, block) pair; the block is
 //      marked in the dense block table.
 //   2. k_svo_alloc       gives every marked block a slot in the block pool.
-//   3. k_svo_voxelize    the pairs grouped by block (count, scan, place),
-//      then one CTA per block, one warp per pair: the leaf voxelisation of
-//      tg__construct_leaf_node (:102-317) -- corner lerp, [0,8)^3 test, bit
-//      fetch -- into the block's image (and material grid) in shared
-//      memory, written out whole and coalesced, with no global atomics.
-//   4. k_svo_pyramid     bottom-up occupancy: one bit per non-empty block and
-//      per non-empty node of every coarser level, and inside each block one
-//      bit per non-empty 4^3 and 8^3 cell (the sub-block levels the
+//   3. k_svo_voxelize    the pairs grouped by block (count, ranges, place),
+//      then one CTA per marked block, one warp per pair: the leaf voxelisation
+//      of tg__construct_leaf_node (:102-317) -- corner lerp, [0,8)^3 test, bit
+//      fetch -- into the block's image (and material grid) in shared memory,
+//      written out whole and coalesced, with no global atomics; and inside each
+//      block one bit per non-empty 4^3 and 8^3 cell (the sub-block levels the
 //      traversal steps through before single voxels).
+//   4. k_svo_pyramid     one bit per non-empty block and per non-empty node of
+//      every coarser level.
 //
 // The node encoding of the reference (u16 relative child pointers, 64-entry
 // leaf lists) is not kept; the voxel set is.  Side length 2^6 .. 2^14.
@@ -172,26 +172,15 @@ __device__ __forceinline__ bool aabb_obb(const dv3* c)
 // 1. candidates
 // ---------------------------------------------------------------------------
 
-__global__ void __launch_bounds__(128) k_svo_candidates(
-    const tgx_object* __restrict__ objects, const uint32_t* __restrict__ cluster_pointers,
-    const uint32_t* __restrict__ c2o, const uint32_t* __restrict__ bits, uint32_t n_cp, float mnx, float mny,
-    float mnz, uint32_t L, uint32_t B, uint32_t* __restrict__ table, SvoPair* __restrict__ pairs,
-    uint32_t pair_capacity, uint32_t* __restrict__ counters, tgx_dev_status* __restrict__ status,
-    const uint8_t* __restrict__ dirty /* null: every block; else only blocks marked dirty */)
+// The blocks the conservative world box of a cluster reaches (clamped to the
+// cube); false when it misses the cube.  lo, hi: the box.
+__device__ __forceinline__ bool cluster_blocks(const tgx_object& od, uint32_t rel, const float mn[3], uint32_t B,
+                                               float lo[3], float hi[3], int b0[3], int b1[3])
 {
-    const uint32_t cp = blockIdx.x * blockDim.x + threadIdx.x;
-    if (cp >= n_cp) return;
-    const uint32_t ci = cluster_pointers[cp];
-    const uint4* w = reinterpret_cast<const uint4*>(bits + (uint64_t)ci * 16u);
-    const uint4 a = w[0], b = w[1], c = w[2], d = w[3];
-    if (!(a.x | a.y | a.z | a.w | b.x | b.y | b.z | b.w | c.x | c.y | c.z | c.w | d.x | d.y | d.z | d.w)) return;
-    const tgx_object& od = objects[c2o[ci]];
-    const uint32_t rel = cp - od.first_cluster_pointer;
-
-    // conservative world box of the cluster (only selects blocks to test)
     float off[3], ohe[3];
     cluster_offsets(od, rel, off, ohe);
-    float lo[3] = {1e30f, 1e30f, 1e30f}, hi[3] = {-1e30f, -1e30f, -1e30f};
+#pragma unroll
+    for (int r = 0; r < 3; r++) { lo[r] = 1e30f; hi[r] = -1e30f; }
 #pragma unroll
     for (int k = 0; k < 8; k++) {
         const float lx = off[0] + ((k & 1) ? 8.0f : 0.0f) - ohe[0];
@@ -205,24 +194,86 @@ __global__ void __launch_bounds__(128) k_svo_candidates(
             hi[r] = fmaxf(hi[r], p);
         }
     }
-    const float mn[3] = {mnx, mny, mnz};
-    int b0[3], b1[3];
+    bool some = true;
 #pragma unroll
     for (int r = 0; r < 3; r++) {
         const float slack = 0.5f + 1e-5f * fabsf(lo[r]) + 1e-5f * fabsf(hi[r]);
-        b0[r] = (int)floorf((lo[r] - slack - mn[r]) / 32.0f);
-        b1[r] = (int)floorf((hi[r] + slack - mn[r]) / 32.0f);
-        b0[r] = max(b0[r], 0);
-        b1[r] = min(b1[r], (int)B - 1);
-        if (b0[r] > b1[r]) return;
+        b0[r] = max((int)floorf((lo[r] - slack - mn[r]) / 32.0f), 0);
+        b1[r] = min((int)floorf((hi[r] + slack - mn[r]) / 32.0f), (int)B - 1);
+        some = some && b0[r] <= b1[r];
+    }
+    return some;
+}
+
+// Bound by instruction issue (the box tests).  A node that holds the cluster's
+// world box with a margin surely passes: no axis can separate them, and the
+// margin (1 + 2e-5 of the coordinates) is far above the test's rounding.  Most
+// levels of most paths are like that (a 32^3 cluster box lies inside its
+// parent's cell of 2^k voxels in all but 45 / 2^k of the cases), so their tests
+// are left out.  That needs a matrix that is a rotation to 10^-3 and node
+// corners that are exact; other objects run every test.  Emptiness comes with the
+// object in cp_obj instead of from the 64-byte bitmask.
+// 386k clusters at 4096^3: CC us -> DD us; with a dirty map (8 moved objects) 83 -> EE.
+__global__ void __launch_bounds__(128) k_svo_candidates(
+    const tgx_object* __restrict__ objects, const float4* __restrict__ inv, const uint32_t* __restrict__ cp_obj,
+    uint32_t n_cp, float mnx, float mny, float mnz, uint32_t L, uint32_t B, uint32_t* __restrict__ table,
+    SvoPair* __restrict__ pairs, uint32_t* __restrict__ marked, uint32_t pair_capacity, uint32_t* __restrict__ counters,
+    tgx_dev_status* __restrict__ status, const uint32_t* __restrict__ dirty /* null: every block; else a bit per block */)
+{
+    const uint32_t cp = blockIdx.x * blockDim.x + threadIdx.x;
+    if (cp >= n_cp) return;
+    const uint32_t po = cp_obj[cp];
+    if (po >> 31) return;   // no set voxel
+    const tgx_object& od = objects[po];
+    const uint32_t rel = cp - od.first_cluster_pointer;
+
+    // conservative world box of the cluster (only selects blocks to test)
+    const float mn[3] = {mnx, mny, mnz};
+    float lo[3], hi[3];
+    int b0[3], b1[3];
+    if (!cluster_blocks(od, rel, mn, B, lo, hi, b0, b1)) return;
+    if (dirty) {
+        bool any = false;
+        for (int bz = b0[2]; bz <= b1[2]; bz++)
+            for (int by = b0[1]; by <= b1[1]; by++)
+                for (int bx = b0[0]; bx <= b1[0]; bx++) {
+                    const uint32_t blk = ((uint32_t)bz * B + (uint32_t)by) * B + (uint32_t)bx;
+                    any = any || (dirty[blk >> 5] >> (blk & 31u)) & 1u;
+                }
+        if (!any) return;
     }
     float ws2ms[16];
-    svo_ws2ms(od, rel, ws2ms);
+    const float4 c0 = inv[4u * po], c1 = inv[4u * po + 1u], c2 = inv[4u * po + 2u], c3 = inv[4u * po + 3u];
+    if (c0.x == c0.x) {
+        float off[3], ohe[3];
+        cluster_offsets(od, rel, off, ohe);
+        const float s3[3] = {xadd(ohe[0], -off[0]), xadd(ohe[1], -off[1]), xadd(ohe[2], -off[2])};
+        dm4_ws2ms(c0, c1, c2, c3, s3, od.translation, ws2ms);
+    } else {
+        svo_ws2ms(od, rel, ws2ms);
+    }
     const float ext = (float)(1u << L);
+    // whether nodes around the cluster can be passed without the test, and the margin they need
+    bool skip = true;
+    float margin = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const float* r = od.rotation + 4 * i;
+#pragma unroll
+        for (int j = 0; j <= i; j++) {
+            const float* q = od.rotation + 4 * j;
+            skip = skip && fabsf(r[0] * q[0] + r[1] * q[1] + r[2] * q[2] - (i == j ? 1.0f : 0.0f)) <= 1e-3f;
+        }
+        // the rows' last column and the last row are those of a rotation
+        skip = skip && od.rotation[4 * i + 3] == 0.0f && od.rotation[12 + i] == 0.0f && fabsf(mn[i]) + ext <= 16777216.0f;
+        margin = fmaxf(margin, 1.0f + 2e-5f * (fabsf(lo[i]) + fabsf(hi[i]) + fabsf(mn[i]) + ext + fabsf(od.translation[i])));
+    }
+    skip = skip && od.rotation[15] == 1.0f;
     for (int bz = b0[2]; bz <= b1[2]; bz++)
         for (int by = b0[1]; by <= b1[1]; by++)
             for (int bx = b0[0]; bx <= b1[0]; bx++) {
-                if (dirty && !dirty[((uint32_t)bz * B + (uint32_t)by) * B + (uint32_t)bx]) continue;
+                const uint32_t blk = ((uint32_t)bz * B + (uint32_t)by) * B + (uint32_t)bx;
+                if (dirty && !((dirty[blk >> 5] >> (blk & 31u)) & 1u)) continue;
                 // walk the reference's recursion from the root to this block
                 dv3 pmin = dv3{mnx, mny, mnz};
                 dv3 pmax = dv3{xadd(mnx, ext), xadd(mny, ext), xadd(mnz, ext)};
@@ -233,24 +284,29 @@ __global__ void __launch_bounds__(128) k_svo_candidates(
                     const uint32_t sh = (uint32_t)lev - 5;
                     const uint32_t cx = ((uint32_t)bx >> sh) & 1u, cy = ((uint32_t)by >> sh) & 1u,
                                    cz = ((uint32_t)bz >> sh) & 1u;
-                    const dv3 cmin = dv3{xadd(pmin.x, xmul((float)cx, ce.x)), xadd(pmin.y, xmul((float)cy, ce.y)),
-                                         xadd(pmin.z, xmul((float)cz, ce.z))};
-                    const dv3 cmax = dv3{xadd(cmin.x, ce.x), xadd(cmin.y, ce.y), xadd(cmin.z, ce.z)};
-                    dv3 bc[8];
+                    pmin = dv3{xadd(pmin.x, xmul((float)cx, ce.x)), xadd(pmin.y, xmul((float)cy, ce.y)),
+                               xadd(pmin.z, xmul((float)cz, ce.z))};
+                    pmax = dv3{xadd(pmin.x, ce.x), xadd(pmin.y, ce.y), xadd(pmin.z, ce.z)};
+                    const bool holds = skip && lo[0] - margin >= pmin.x && lo[1] - margin >= pmin.y && lo[2] - margin >= pmin.z &&
+                                       hi[0] + margin <= pmax.x && hi[1] + margin <= pmax.y && hi[2] + margin <= pmax.z;
+                    if (!holds) {
+                        dv3 bc[8];
 #pragma unroll
-                    for (int k = 0; k < 8; k++)
-                        bc[k] = mulv4p(ws2ms, (k & 1) ? cmax.x : cmin.x, (k & 2) ? cmax.y : cmin.y,
-                                       (k & 4) ? cmax.z : cmin.z);
-                    if (!aabb_obb(bc)) { pass = false; break; }
-                    pmin = cmin;
-                    pmax = cmax;
+                        for (int k = 0; k < 8; k++)
+                            bc[k] = mulv4p(ws2ms, (k & 1) ? pmax.x : pmin.x, (k & 2) ? pmax.y : pmin.y,
+                                           (k & 4) ? pmax.z : pmin.z);
+                        if (!aabb_obb(bc)) { pass = false; break; }
+                    }
                 }
                 if (!pass) continue;
-                const uint32_t blk = ((uint32_t)bz * B + (uint32_t)by) * B + (uint32_t)bx;
                 const uint32_t slot = atomicAdd(&counters[S_PAIRS], 1u);
                 if (slot < pair_capacity) pairs[slot] = SvoPair{cp, blk};
                 else dev_error(status, TGX_ERR_CAPACITY, 11, slot);
-                if (atomicCAS(&table[blk], 0u, kMark) == 0u) atomicAdd(&counters[S_MARKED], 1u);
+                // every marked block has a pair, so the list is no longer than the pairs' storage
+                if (atomicCAS(&table[blk], 0u, kMark) == 0u) {
+                    const uint32_t m = atomicAdd(&counters[S_MARKED], 1u);
+                    if (m < pair_capacity) marked[m] = blk;
+                }
             }
 }
 
@@ -258,22 +314,23 @@ __global__ void __launch_bounds__(128) k_svo_candidates(
 // 2. slot allocation
 // ---------------------------------------------------------------------------
 
-// Marked blocks take slots from the end of the free list first (free[n_free-1],
-// free[n_free-2], ...), then fresh slots from `next_slot` on.
-__global__ void __launch_bounds__(256) k_svo_alloc(uint32_t* __restrict__ table, uint64_t n_table,
-                                                  uint32_t* __restrict__ counters, const uint32_t* __restrict__ free_list,
-                                                  uint32_t n_free, uint32_t next_slot, uint32_t pool_blocks,
-                                                  tgx_dev_status* __restrict__ status)
+// Marked block m of n takes a slot from the end of the free list first
+// (free[n_free-1], free[n_free-2], ...), then fresh slots from `next_slot` on.
+// The table entry holds m + 1 until k_svo_publish puts the slot there: the
+// passes between group the pairs by m.
+__global__ void __launch_bounds__(256) k_svo_alloc(uint32_t* __restrict__ table, const uint32_t* __restrict__ marked,
+                                                  uint32_t n, const uint32_t* __restrict__ free_list, uint32_t n_free,
+                                                  uint32_t next_slot, uint32_t* __restrict__ slots,
+                                                  uint32_t* __restrict__ slot_block, uint32_t* __restrict__ cnt)
 {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_table;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        if (table[i] == kMark) {
-            const uint32_t s = atomicAdd(&counters[S_SLOTS], 1u);
-            const uint32_t slot = s < n_free ? free_list[n_free - 1u - s] : next_slot + (s - n_free);
-            if (slot < pool_blocks) table[i] = slot + 1u;
-            else { table[i] = 0u; dev_error(status, TGX_ERR_CAPACITY, 12, s); }
-        }
-    }
+    const uint32_t m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= n) return;
+    const uint32_t blk = marked[m];
+    const uint32_t slot = m < n_free ? free_list[n_free - 1u - m] : next_slot + (m - n_free);
+    table[blk] = m + 1u;
+    slots[m] = slot;
+    slot_block[slot] = blk;
+    cnt[m] = 0u;
 }
 
 // ---------------------------------------------------------------------------
@@ -297,58 +354,45 @@ __device__ __forceinline__ void smem_max_u16(uint32_t* words, uint32_t idx, uint
     }
 }
 
-// 3a. pairs grouped by their block's slot: counts, one scan, placement
-__global__ void __launch_bounds__(256) k_svo_pair_count(const SvoPair* __restrict__ pairs,
-                                                       const uint32_t* __restrict__ counters, uint32_t pair_capacity,
+// 3a. pairs grouped by their (marked) block: counts, a range each, placement.
+// The order of the ranges is free, so a block's range comes from a counter
+// (one atomic per warp) instead of a scan.
+__global__ void __launch_bounds__(256) k_svo_pair_count(const SvoPair* __restrict__ pairs, uint32_t n,
                                                        const uint32_t* __restrict__ table, uint32_t* __restrict__ cnt)
 {
-    const uint32_t n = min(counters[S_PAIRS], pair_capacity);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t tv = table[pairs[i].block];
-        if (tv) atomicAdd(&cnt[tv - 1u], 1u);
-    }
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        atomicAdd(&cnt[table[pairs[i].block] - 1u], 1u);
 }
 
-// exclusive scan of cnt[0, n) into off[0, n] (off[n] = total): one CTA, each
-// thread a contiguous run
-__global__ void __launch_bounds__(1024) k_svo_pair_scan(const uint32_t* __restrict__ cnt, uint32_t n,
-                                                       uint32_t* __restrict__ off)
+__global__ void __launch_bounds__(256) k_svo_pair_ranges(const uint32_t* __restrict__ cnt, uint32_t n,
+                                                        uint32_t* __restrict__ total, uint32_t* __restrict__ off,
+                                                        uint32_t* __restrict__ cursor)
 {
-    __shared__ uint32_t part[1024];
-    const uint32_t t = threadIdx.x, per = (n + 1023u) / 1024u;
-    const uint32_t b = min(n, t * per), e = min(n, b + per);
-    uint32_t sum = 0;
-    for (uint32_t i = b; i < e; i++) sum += cnt[i];
-    part[t] = sum;
-    __syncthreads();
-    for (uint32_t o = 1; o < 1024u; o <<= 1) {
-        const uint32_t v = t >= o ? part[t - o] : 0u;
-        __syncthreads();
-        part[t] += v;
-        __syncthreads();
+    const uint32_t m = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+    const uint32_t c = m < n ? cnt[m] : 0u;
+    uint32_t incl = c;
+#pragma unroll
+    for (uint32_t o = 1; o < 32u; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
     }
-    uint32_t run = t ? part[t - 1u] : 0u;
-    for (uint32_t i = b; i < e; i++) {
-        off[i] = run;
-        run += cnt[i];
-    }
-    if (t == 1023u) off[n] = part[1023];
+    uint32_t base = 0;
+    if (lane == 31u && incl) base = atomicAdd(total, incl);
+    base = __shfl_sync(0xffffffffu, base, 31);
+    if (m < n) off[m] = cursor[m] = base + incl - c;
 }
 
-__global__ void __launch_bounds__(256) k_svo_pair_fill(const SvoPair* __restrict__ pairs,
-                                                      const uint32_t* __restrict__ counters, uint32_t pair_capacity,
-                                                      const uint32_t* __restrict__ table, const uint32_t* __restrict__ off,
-                                                      uint32_t* __restrict__ cursor, SvoPair* __restrict__ sorted)
+__global__ void __launch_bounds__(256) k_svo_pair_fill(const SvoPair* __restrict__ pairs, uint32_t n,
+                                                      const uint32_t* __restrict__ table, uint32_t* __restrict__ cursor,
+                                                      SvoPair* __restrict__ sorted)
 {
-    const uint32_t n = min(counters[S_PAIRS], pair_capacity);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const SvoPair pr = pairs[i];
-        const uint32_t tv = table[pr.block];
-        if (tv) sorted[off[tv - 1u] + atomicAdd(&cursor[tv - 1u], 1u)] = pr;
+        sorted[atomicAdd(&cursor[table[pr.block] - 1u], 1u)] = pr;
     }
 }
 
-// 3b. voxelisation: one CTA per block slot.  Its warps take the block's
+// 3b. voxelisation: one CTA per marked block.  Its warps take the block's
 // (cluster, block) pairs; every set voxel goes into the CTA's shared image of
 // the block and its material code into the shared material grid, then the
 // block is written out whole, coalesced, with no global atomics.
@@ -463,6 +507,58 @@ __device__ __noinline__ void voxelize_any(const float* bc, uint32_t x0, uint32_t
     }
 }
 
+// The masks of a block's 4^3 and 8^3 cells from its bit words, by one warp (lane
+// y reads the 32 rows (y, z)), and whether it holds a voxel.
+__device__ __forceinline__ void block_masks(const uint32_t* blk, uint32_t* __restrict__ sb, uint32_t* __restrict__ nonempty)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t any = 0;
+    uint32_t n4[8];   // per 4-voxel z-slab: which 4-voxel x-groups of row y hold a voxel
+#pragma unroll
+    for (int k = 0; k < 8; k++) n4[k] = 0;
+#pragma unroll
+    for (int z = 0; z < 32; z++) {
+        const uint32_t row = blk[z * 32 + lane];
+        any |= row;
+        uint32_t f = 0;
+#pragma unroll
+        for (int gx = 0; gx < 8; gx++) f |= ((row >> (4 * gx)) & 15u) ? (1u << gx) : 0u;
+        n4[z >> 2] |= f;
+    }
+    any = __any_sync(0xffffffffu, any != 0u);
+    if (lane == 0) *nonempty = any ? 1u : 0u;
+    // 4^3 cells: bit ((cz * 8 + cy) * 8 + cx), cy = lane / 4
+#pragma unroll
+    for (int cz = 0; cz < 8; cz++) {
+        uint32_t b = n4[cz];
+        b |= __shfl_xor_sync(0xffffffffu, b, 1);
+        b |= __shfl_xor_sync(0xffffffffu, b, 2);
+        uint32_t w = (lane & 3u) == 0u ? b << (((lane >> 2) & 3u) * 8u) : 0u;
+        w |= __shfl_xor_sync(0xffffffffu, w, 4);
+        w |= __shfl_xor_sync(0xffffffffu, w, 8);
+        if ((lane & 15u) == 0u) sb[cz * 2 + (lane >> 4)] = w;
+    }
+    // 8^3 cells: bit ((cz * 4 + cy) * 4 + cx), cy = lane / 8
+    uint32_t w8[2] = {0u, 0u};
+#pragma unroll
+    for (int cz = 0; cz < 4; cz++) {
+        const uint32_t b = n4[2 * cz] | n4[2 * cz + 1];
+        uint32_t c3 = 0;
+#pragma unroll
+        for (int cx = 0; cx < 4; cx++) c3 |= ((b >> (2 * cx)) & 3u) ? (1u << cx) : 0u;
+        c3 |= __shfl_xor_sync(0xffffffffu, c3, 1);
+        c3 |= __shfl_xor_sync(0xffffffffu, c3, 2);
+        c3 |= __shfl_xor_sync(0xffffffffu, c3, 4);
+        if ((lane & 7u) == 0u) w8[cz >> 1] |= c3 << ((cz & 1) * 16 + (lane >> 3) * 4);
+    }
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        w8[k] |= __shfl_xor_sync(0xffffffffu, w8[k], 8);
+        w8[k] |= __shfl_xor_sync(0xffffffffu, w8[k], 16);
+    }
+    if (lane == 0) { sb[16] = w8[0]; sb[17] = w8[1]; }
+}
+
 // Bound by instruction issue.  The pairs are taken kVoxRound at a time.  First a
 // lane per pair computes its matrices, trimmed range and corners (with a warp
 // per pair that set-up was half of all instructions) and the ranges' voxel
@@ -483,8 +579,9 @@ template <bool kMat>
 __global__ void __launch_bounds__(32 * kWarpsPerVoxCta, 2) k_svo_voxelize(
     const tgx_object* __restrict__ objects, const uint32_t* __restrict__ cluster_pointers,
     const uint32_t* __restrict__ c2o, const uint32_t* __restrict__ bits, const SvoPair* __restrict__ sorted,
-    const uint32_t* __restrict__ off, uint32_t* __restrict__ pool, const uint8_t* __restrict__ material,
-    uint16_t* __restrict__ mat_pool, float mnx, float mny, float mnz, uint32_t B)
+    const uint32_t* __restrict__ off, const uint32_t* __restrict__ cnt, const uint32_t* __restrict__ slots,
+    uint32_t* __restrict__ pool, uint32_t* __restrict__ sub, uint32_t* __restrict__ nonempty,
+    const uint8_t* __restrict__ material, uint16_t* __restrict__ mat_pool, float mnx, float mny, float mnz, uint32_t B)
 {
     extern __shared__ __align__(16) uint32_t s_blk[];   // 1024 bit words, then 16384 words of u16 codes
     __shared__ PairRec s_rec[kVoxRound];
@@ -495,9 +592,8 @@ __global__ void __launch_bounds__(32 * kWarpsPerVoxCta, 2) k_svo_voxelize(
     __shared__ uint32_t s_next;                          // the next entry of s_order to take
     uint32_t* img = s_blk;
     uint16_t* smat = reinterpret_cast<uint16_t*>(s_blk + kBlockWords);
-    const uint32_t slot = blockIdx.x;
-    const uint32_t pb = off[slot], pe = off[slot + 1];
-    if (pb == pe) return;
+    const uint32_t slot = slots[blockIdx.x];
+    const uint32_t pb = off[blockIdx.x], pe = pb + cnt[blockIdx.x];   // at least one pair
     const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
     bool again = false;                  // the pass over the doubly set voxels (the same in every thread)
     for (;;) {
@@ -628,80 +724,43 @@ __global__ void __launch_bounds__(32 * kWarpsPerVoxCta, 2) k_svo_voxelize(
         uint4* md = reinterpret_cast<uint4*>(mat_pool + (uint64_t)slot * 32768u);
         for (uint32_t k = threadIdx.x; k < 16384u / 4u; k += blockDim.x) md[k] = reinterpret_cast<const uint4*>(smat)[k];
     }
+    // the block's occupancy masks, from the image while it is here
+    if (wid == kWarpsPerVoxCta - 1u) block_masks(img, sub + (uint64_t)slot * 32u, &nonempty[slot]);
 }
 
 // ---------------------------------------------------------------------------
 // 4. occupancy pyramid
 // ---------------------------------------------------------------------------
 
-__global__ void __launch_bounds__(256) k_svo_pyramid(const uint32_t* __restrict__ table, uint64_t n_table,
-                                                    const uint32_t* __restrict__ pool, uint32_t* __restrict__ nonempty,
-                                                    uint32_t* __restrict__ sub, uint32_t* __restrict__ occ,
+// The slots of the marked blocks go into the table (which held m + 1).
+__global__ void __launch_bounds__(256) k_svo_publish(uint32_t* __restrict__ table, const uint32_t* __restrict__ marked,
+                                                    const uint32_t* __restrict__ slots, uint32_t n)
+{
+    const uint32_t m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m < n) table[marked[m]] = slots[m] + 1u;
+}
+
+// One thread per slot: a slot whose block holds a voxel sets its bit on every
+// level.  The words are zero before; a bit is read first, because the coarse
+// levels' few words would otherwise take an atomic from every block.
+__global__ void __launch_bounds__(256) k_svo_pyramid(const uint32_t* __restrict__ slot_block, uint32_t n_slots,
+                                                    const uint32_t* __restrict__ nonempty, uint32_t* occ,
                                                     const uint64_t* __restrict__ occ_off, uint32_t n_levels, uint32_t B,
                                                     uint32_t* __restrict__ counters)
 {
-    // one warp per table entry; lane y reads the 32 rows (y, z) of the block
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t n_warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t i = warp; i < n_table; i += n_warps) {
-        const uint32_t tv = table[i];
-        if (tv == 0u) continue;
-        const uint32_t* blk = pool + (uint64_t)(tv - 1u) * kBlockWords;
-        uint32_t any = 0;
-        uint32_t n4[8];   // per 4-voxel z-slab: which 4-voxel x-groups of row y hold a voxel
-#pragma unroll
-        for (int k = 0; k < 8; k++) n4[k] = 0;
-#pragma unroll
-        for (int z = 0; z < 32; z++) {
-            const uint32_t row = blk[z * 32 + lane];
-            any |= row;
-            uint32_t f = 0;
-#pragma unroll
-            for (int gx = 0; gx < 8; gx++) f |= ((row >> (4 * gx)) & 15u) ? (1u << gx) : 0u;
-            n4[z >> 2] |= f;
-        }
-        any = __any_sync(0xffffffffu, any != 0u);
-        if (lane == 0) nonempty[tv - 1u] = any ? 1u : 0u;
-        if (!any) continue;
-        // 4^3 cells: bit ((cz * 8 + cy) * 8 + cx), cy = lane / 4
-        uint32_t* sb = sub + (uint64_t)(tv - 1u) * 32u;
-#pragma unroll
-        for (int cz = 0; cz < 8; cz++) {
-            uint32_t b = n4[cz];
-            b |= __shfl_xor_sync(0xffffffffu, b, 1);
-            b |= __shfl_xor_sync(0xffffffffu, b, 2);
-            uint32_t w = (lane & 3u) == 0u ? b << (((lane >> 2) & 3u) * 8u) : 0u;
-            w |= __shfl_xor_sync(0xffffffffu, w, 4);
-            w |= __shfl_xor_sync(0xffffffffu, w, 8);
-            if ((lane & 15u) == 0u) sb[cz * 2 + (lane >> 4)] = w;
-        }
-        // 8^3 cells: bit ((cz * 4 + cy) * 4 + cx), cy = lane / 8
-        uint32_t w8[2] = {0u, 0u};
-#pragma unroll
-        for (int cz = 0; cz < 4; cz++) {
-            const uint32_t b = n4[2 * cz] | n4[2 * cz + 1];
-            uint32_t c3 = 0;
-#pragma unroll
-            for (int cx = 0; cx < 4; cx++) c3 |= ((b >> (2 * cx)) & 3u) ? (1u << cx) : 0u;
-            c3 |= __shfl_xor_sync(0xffffffffu, c3, 1);
-            c3 |= __shfl_xor_sync(0xffffffffu, c3, 2);
-            c3 |= __shfl_xor_sync(0xffffffffu, c3, 4);
-            if ((lane & 7u) == 0u) w8[cz >> 1] |= c3 << ((cz & 1) * 16 + (lane >> 3) * 4);
-        }
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-            w8[k] |= __shfl_xor_sync(0xffffffffu, w8[k], 8);
-            w8[k] |= __shfl_xor_sync(0xffffffffu, w8[k], 16);
-        }
-        if (lane == 0) { sb[16] = w8[0]; sb[17] = w8[1]; }
-        if (lane == 0) atomicAdd(&counters[S_NONEMPTY], 1u);
-        const uint32_t bx = (uint32_t)(i % B), by = (uint32_t)((i / B) % B), bz = (uint32_t)(i / ((uint64_t)B * B));
-        if (lane < n_levels) {
-            const uint32_t s = lane, n = B >> s;
-            const uint64_t idx = ((uint64_t)(bz >> s) * n + (by >> s)) * n + (bx >> s);
-            atomicOr(&occ[occ_off[s] + (idx >> 5)], 1u << (idx & 31u));
-        }
+    const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t i = slot < n_slots ? slot_block[slot] : 0xffffffffu;
+    const bool any = i != 0xffffffffu && nonempty[slot] != 0u;
+    const uint32_t mask = __ballot_sync(0xffffffffu, any);
+    if ((threadIdx.x & 31u) == 0u && mask) atomicAdd(&counters[S_NONEMPTY], (uint32_t)__popc(mask));
+    if (!any) return;
+    const uint32_t bx = i % B, by = (i / B) % B, bz = i / (B * B);
+    for (uint32_t s = 0; s < n_levels; s++) {
+        const uint32_t n = B >> s;
+        const uint64_t idx = ((uint64_t)(bz >> s) * n + (by >> s)) * n + (bx >> s);
+        uint32_t* w = &occ[occ_off[s] + (idx >> 5)];
+        const uint32_t bit = 1u << (idx & 31u);
+        if (!(*(volatile uint32_t*)w & bit)) atomicOr(w, bit);
     }
 }
 
@@ -710,105 +769,82 @@ __global__ void __launch_bounds__(256) k_svo_pyramid(const uint32_t* __restrict_
 // ---------------------------------------------------------------------------
 
 // Conservative world box of every non-empty cluster of one object -- the box
-// k_svo_candidates selects blocks with -- marked into the dirty-block map.
-__device__ void mark_object_blocks(const tgx_object& od, const uint32_t* __restrict__ cluster_pointers,
-                                   const uint32_t* __restrict__ bits, const float mn[3], uint32_t B,
-                                   uint8_t* __restrict__ dirty)
+// k_svo_candidates selects blocks with -- marked into the dirty-block map (a
+// bit per block).  The CTAs of a grid column share the object's clusters.
+__device__ void mark_object_blocks(const tgx_object& od, const uint32_t* __restrict__ cp_obj, const float mn[3], uint32_t B,
+                                   uint32_t* __restrict__ dirty)
 {
     const uint32_t n = od.n_cluster_pointers_per_dim[0] * od.n_cluster_pointers_per_dim[1] * od.n_cluster_pointers_per_dim[2];
-    for (uint32_t rel = threadIdx.x; rel < n; rel += blockDim.x) {
-        const uint32_t ci = cluster_pointers[od.first_cluster_pointer + rel];
-        const uint4* w = reinterpret_cast<const uint4*>(bits + (uint64_t)ci * 16u);
-        const uint4 a = w[0], b = w[1], c = w[2], d = w[3];
-        if (!(a.x | a.y | a.z | a.w | b.x | b.y | b.z | b.w | c.x | c.y | c.z | c.w | d.x | d.y | d.z | d.w)) continue;
-        float off[3], ohe[3];
-        cluster_offsets(od, rel, off, ohe);
-        float lo[3] = {1e30f, 1e30f, 1e30f}, hi[3] = {-1e30f, -1e30f, -1e30f};
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const float lx = off[0] + ((k & 1) ? 8.0f : 0.0f) - ohe[0];
-            const float ly = off[1] + ((k & 2) ? 8.0f : 0.0f) - ohe[1];
-            const float lz = off[2] + ((k & 4) ? 8.0f : 0.0f) - ohe[2];
-#pragma unroll
-            for (int r = 0; r < 3; r++) {
-                const float p = DM(od.rotation, r, 0) * lx + DM(od.rotation, r, 1) * ly + DM(od.rotation, r, 2) * lz +
-                                od.translation[r];
-                lo[r] = fminf(lo[r], p);
-                hi[r] = fmaxf(hi[r], p);
-            }
-        }
+    for (uint32_t rel = blockIdx.y * blockDim.x + threadIdx.x; rel < n; rel += gridDim.y * blockDim.x) {
+        if (cp_obj[od.first_cluster_pointer + rel] >> 31) continue;   // no set voxel
+        float lo[3], hi[3];
         int b0[3], b1[3];
-        bool empty = false;
-#pragma unroll
-        for (int r = 0; r < 3; r++) {
-            const float slack = 0.5f + 1e-5f * fabsf(lo[r]) + 1e-5f * fabsf(hi[r]);
-            b0[r] = max((int)floorf((lo[r] - slack - mn[r]) / 32.0f), 0);
-            b1[r] = min((int)floorf((hi[r] + slack - mn[r]) / 32.0f), (int)B - 1);
-            empty |= b0[r] > b1[r];
-        }
-        if (empty) continue;
+        if (!cluster_blocks(od, rel, mn, B, lo, hi, b0, b1)) continue;
         for (int bz = b0[2]; bz <= b1[2]; bz++)
             for (int by = b0[1]; by <= b1[1]; by++)
-                for (int bx = b0[0]; bx <= b1[0]; bx++) dirty[((uint32_t)bz * B + (uint32_t)by) * B + (uint32_t)bx] = 1;
+                for (int bx = b0[0]; bx <= b1[0]; bx++) {
+                    const uint32_t blk = ((uint32_t)bz * B + (uint32_t)by) * B + (uint32_t)bx;
+                    atomicOr(&dirty[blk >> 5], 1u << (blk & 31u));
+                }
     }
 }
 
-// One CTA per object: when the scene's record differs from the one the SVO
-// was built from, the blocks its clusters touched before (old record) and
-// touch now (new record) become dirty, and the stored record is replaced.
-__global__ void __launch_bounds__(128) k_svo_mark_dirty(const tgx_object* __restrict__ cur, tgx_object* __restrict__ built,
-                                                       const uint32_t* __restrict__ cluster_pointers,
-                                                       const uint32_t* __restrict__ bits, float mnx, float mny,
-                                                       float mnz, uint32_t B, uint8_t* __restrict__ dirty,
-                                                       uint32_t* __restrict__ counters)
+__device__ __forceinline__ bool same_record(const tgx_object& x, const tgx_object& y)
 {
-    const tgx_object now = cur[blockIdx.x], was = built[blockIdx.x];
-    const uint32_t* a = reinterpret_cast<const uint32_t*>(&now);
-    const uint32_t* b = reinterpret_cast<const uint32_t*>(&was);
+    const uint32_t* a = reinterpret_cast<const uint32_t*>(&x);
+    const uint32_t* b = reinterpret_cast<const uint32_t*>(&y);
     bool same = true;
 #pragma unroll
     for (int k = 0; k < (int)(sizeof(tgx_object) / 4); k++) same &= a[k] == b[k];
-    if (same) return;
-    const float mn[3] = {mnx, mny, mnz};
-    mark_object_blocks(was, cluster_pointers, bits, mn, B, dirty);
-    mark_object_blocks(now, cluster_pointers, bits, mn, B, dirty);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        built[blockIdx.x] = now;
-        atomicAdd(&counters[S_MOVED], 1u);
-    }
+    return same;
 }
 
-// One warp per dirty block that holds a slot: its voxel bits, sub-block masks,
-// non-empty flag and materials are zeroed, the table entry is emptied and the
-// slot goes on the free list.  k_svo_candidates re-marks the block if any
-// cluster still reaches it.
-__global__ void __launch_bounds__(256) k_svo_release_dirty(uint32_t* __restrict__ table, uint64_t n_table,
-                                                          const uint8_t* __restrict__ dirty, uint32_t* __restrict__ pool,
-                                                          uint32_t* __restrict__ sub, uint32_t* __restrict__ nonempty,
-                                                          uint16_t* __restrict__ mat, uint32_t* __restrict__ free_tail,
-                                                          uint32_t* __restrict__ counters)
+// A grid column per object: when the scene's record differs from the one the
+// SVO was built from, the blocks its clusters touched before (old record) and
+// touch now (new record) become dirty.
+__global__ void __launch_bounds__(128) k_svo_mark_dirty(const tgx_object* __restrict__ cur,
+                                                       const tgx_object* __restrict__ built,
+                                                       const uint32_t* __restrict__ cp_obj, float mnx, float mny,
+                                                       float mnz, uint32_t B, uint32_t* __restrict__ dirty)
 {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t n_warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t i = warp; i < n_table; i += n_warps) {
-        if (!dirty[i]) continue;
-        const uint32_t tv = table[i];
-        if (tv == 0u) continue;
-        const uint32_t slot = tv - 1u;
-        uint4* blk = reinterpret_cast<uint4*>(pool + (uint64_t)slot * kBlockWords);
-        for (uint32_t k = lane; k < kBlockWords / 4u; k += 32) blk[k] = make_uint4(0u, 0u, 0u, 0u);
-        sub[(uint64_t)slot * 32u + lane] = 0u;
-        if (mat) {
-            uint4* m = reinterpret_cast<uint4*>(mat + (uint64_t)slot * 32768u);
-            for (uint32_t k = lane; k < 32768u / 8u; k += 32) m[k] = make_uint4(0u, 0u, 0u, 0u);
-        }
-        if (lane == 0) {
-            nonempty[slot] = 0u;
+    const tgx_object now = cur[blockIdx.x], was = built[blockIdx.x];
+    if (same_record(now, was)) return;
+    const float mn[3] = {mnx, mny, mnz};
+    mark_object_blocks(was, cp_obj, mn, B, dirty);
+    mark_object_blocks(now, cp_obj, mn, B, dirty);
+}
+
+// Every dirty block that holds a slot gives it back: the table entry is emptied
+// and the slot goes on the free list (a thread per 32 blocks of the map).
+// k_svo_candidates re-marks the block if any cluster still reaches it, and what
+// a slot holds is written whole before it is used again.  Moved objects are
+// counted and their records taken over, a thread each.
+__global__ void __launch_bounds__(256) k_svo_release_dirty(uint32_t* __restrict__ table, uint64_t n_words,
+                                                          const uint32_t* __restrict__ dirty, uint64_t n_table,
+                                                          uint32_t* __restrict__ nonempty, uint32_t* __restrict__ slot_block,
+                                                          uint32_t* __restrict__ free_tail,
+                                                          const tgx_object* __restrict__ cur, tgx_object* __restrict__ built,
+                                                          uint32_t n_objects, uint32_t* __restrict__ counters)
+{
+    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t w = t; w < n_words; w += stride) {
+        uint32_t m = dirty[w];
+        while (m) {
+            const uint64_t i = w * 32u + (uint32_t)(__ffs((int)m) - 1);
+            m &= m - 1u;
+            const uint32_t tv = i < n_table ? table[i] : 0u;
+            if (tv == 0u) continue;
+            nonempty[tv - 1u] = 0u;
+            slot_block[tv - 1u] = 0xffffffffu;
             table[i] = 0u;
-            free_tail[atomicAdd(&counters[S_FREED], 1u)] = slot;
+            free_tail[atomicAdd(&counters[S_FREED], 1u)] = tv - 1u;
         }
+    }
+    for (uint64_t o = t; o < n_objects; o += stride) {
+        const tgx_object now = cur[o];
+        if (same_record(now, built[o])) continue;
+        built[o] = now;
+        atomicAdd(&counters[S_MOVED], 1u);
     }
 }
 
@@ -835,9 +871,17 @@ static void svo_free(tgx_svo* s)
     cudaFree(s->d_nonempty);
     cudaFree(s->d_mat);
     cudaFree(s->d_free);
+    cudaFree(s->d_slot_block);
     cudaFree(s->d_counters);
     cudaFree(s->d_objs);
     delete s;
+}
+
+// The pair storage: pairs, then as many words for the list of the marked blocks.
+constexpr uint64_t kPairBytes = sizeof(SvoPair) + 4;
+static uint32_t* svo_marked(tgx_ctx* c)
+{
+    return (uint32_t*)((SvoPair*)c->svo_pairs.ptr + c->svo_pairs.bytes / kPairBytes);
 }
 
 static uint64_t svo_device_bytes(const tgx_svo* s)
@@ -847,18 +891,18 @@ static uint64_t svo_device_bytes(const tgx_svo* s)
            s->occ_words * 4 + (uint64_t)s->n_objects * sizeof(tgx_object);
 }
 
-// Per-slot arrays (pool, sub masks, non-empty flags, free list, materials)
-// sized for `cap` slots; the first `keep` slots are carried over.  The rest
-// of the small arrays start zero; pool and material slots are written whole
+// Per-slot arrays (pool, sub masks, non-empty flags, free list, block indices,
+// materials) sized for `cap` slots; the first `keep` slots are carried over.  The
+// rest of the small arrays start zero (no block: ~0); pool and material slots are written whole
 // by the voxeliser before anything reads them.
 static tgx_status svo_resize_slots(tgx_ctx* c, tgx_svo* s, uint32_t cap, uint32_t keep, bool materials)
 {
     struct Arr { void** p; uint64_t per_slot; };
     void* mat = s->d_mat;
-    Arr arrs[5] = {{(void**)&s->d_pool, kBlockWords * 4}, {(void**)&s->d_sub, 128}, {(void**)&s->d_nonempty, 4},
-                   {(void**)&s->d_free, 4}, {&mat, 65536}};
-    const int n_arr = materials ? 5 : 4;
-    void* fresh[5] = {};
+    Arr arrs[6] = {{(void**)&s->d_pool, kBlockWords * 4}, {(void**)&s->d_sub, 128}, {(void**)&s->d_nonempty, 4},
+                   {(void**)&s->d_free, 4}, {(void**)&s->d_slot_block, 4}, {&mat, 65536}};
+    const int n_arr = materials ? 6 : 5;
+    void* fresh[6] = {};
     for (int a = 0; a < n_arr; a++)
         if (cudaMalloc(&fresh[a], (uint64_t)cap * arrs[a].per_slot) != cudaSuccess) {
             for (int k = 0; k < a; k++) cudaFree(fresh[k]);
@@ -869,7 +913,7 @@ static tgx_status svo_resize_slots(tgx_ctx* c, tgx_svo* s, uint32_t cap, uint32_
     for (int a = 0; a < n_arr; a++) {
         const uint64_t kept = (uint64_t)keep * arrs[a].per_slot, total = (uint64_t)cap * arrs[a].per_slot;
         if (kept) TGX_CUDA(cudaMemcpyAsync(fresh[a], *arrs[a].p, kept, cudaMemcpyDeviceToDevice, c->stream));
-        if (a != 0 && a != 4) TGX_CUDA(cudaMemsetAsync((char*)fresh[a] + kept, 0, total - kept, c->stream));
+        if (a != 0 && a != 5) TGX_CUDA(cudaMemsetAsync((char*)fresh[a] + kept, a == 4 ? 0xff : 0, total - kept, c->stream));
     }
     TGX_CUDA(cudaStreamSynchronize(c->stream));
     for (int a = 0; a < n_arr; a++) {
@@ -883,18 +927,21 @@ static tgx_status svo_resize_slots(tgx_ctx* c, tgx_svo* s, uint32_t cap, uint32_
 
 // Candidate pass over every cluster pointer (only blocks marked in `dirty` when
 // it is given), with the pair storage grown to the exact count and the pass
-// rerun once when the first estimate was short.  Leaves the counters on the host.
-static tgx_status svo_candidates(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc, const uint8_t* dirty, uint64_t cap)
+// rerun once when the first estimate was short.  The list of the marked blocks
+// follows the pairs.  Leaves the counters on the host.
+static tgx_status svo_candidates(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc, const uint32_t* dirty, uint64_t cap)
 {
     const uint64_t n_table = (uint64_t)s->B * s->B * s->B;
     uint32_t* counters = s->d_counters;
     for (int attempt = 0; attempt < 2; attempt++) {
-        TGX_TRY(devbuf_reserve(c->svo_pairs, cap * sizeof(SvoPair)));
+        TGX_TRY(devbuf_reserve(c->svo_pairs, cap * kPairBytes));
+        cap = c->svo_pairs.bytes / kPairBytes;   // svo_marked() places the list by the buffer's size
         TGX_CUDA(cudaMemsetAsync(counters + S_PAIRS, 0, 2 * 4, c->stream));   // pairs, marks
         if (sc->n_cluster_pointers)
             TGX_LAUNCH(c, TR_SVO_CANDIDATES, (sc->n_cluster_pointers + 127) / 128, 128, 0, k_svo_candidates, sc->d_objects,
-                       sc->d_cluster_pointers, sc->d_c2o, sc->d_bits, sc->n_cluster_pointers, s->mn[0], s->mn[1], s->mn[2],
-                       s->L, s->B, s->d_table, (SvoPair*)c->svo_pairs.ptr, (uint32_t)cap, counters, c->d_status, dirty);
+                       sc->d_inv, sc->d_cp_obj, sc->n_cluster_pointers, s->mn[0], s->mn[1], s->mn[2], s->L, s->B,
+                       s->d_table, (SvoPair*)c->svo_pairs.ptr, svo_marked(c), (uint32_t)std::min<uint64_t>(cap, 0xffffffffu),
+                       counters, c->d_status, dirty);
         if (cudaMemcpyAsync(c->h_counter, counters, S_COUNT * 4, cudaMemcpyDeviceToHost, c->stream) != cudaSuccess ||
             cudaStreamSynchronize(c->stream) != cudaSuccess) {
             tgx_set_error("tgx_svo: %s", cudaGetErrorString(cudaGetLastError()));
@@ -912,51 +959,50 @@ static tgx_status svo_candidates(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc, co
     return TGX_ERR_CAPACITY;
 }
 
-// Slots for the marked blocks, voxelisation of the pairs, and the occupancy
-// pyramid of the whole table (cleared first).
-static tgx_status svo_fill(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc, uint32_t n_free, uint32_t next_slot)
+// Slots for the n_marked marked blocks, voxelisation of the pairs, and the
+// occupancy pyramid of all n_slots slots (cleared first).
+static tgx_status svo_fill(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc, uint32_t n_marked, uint32_t n_free,
+                           uint32_t next_slot, uint32_t n_slots)
 {
-    const uint64_t n_table = (uint64_t)s->B * s->B * s->B;
     uint32_t* counters = s->d_counters;
-    const uint32_t grid = (uint32_t)std::min<uint64_t>((n_table + 255) / 256, (uint64_t)c->num_sms * 32);
-    TGX_CUDA(cudaMemsetAsync(counters + S_SLOTS, 0, 2 * 4, c->stream));   // slots, non-empty
-    TGX_CUDA(cudaMemsetAsync(s->d_occ, 0, s->occ_words * 4, c->stream));
-    TGX_LAUNCH(c, TR_SVO_ALLOC, grid, 256, 0, k_svo_alloc, s->d_table, n_table, counters, s->d_free, n_free, next_slot,
-               s->pool_cap, c->d_status);
-    // group the pairs by block slot: counts, offsets, placement
-    const uint32_t cap = (uint32_t)(c->svo_pairs.bytes / sizeof(SvoPair));
-    const uint64_t n_slots = s->pool_cap;
-    const size_t sort_bytes = (size_t)(n_slots + 1) * 4 * 2 + (size_t)std::max<uint64_t>(s->n_pairs, 1) * sizeof(SvoPair) + 64;
+    const size_t sort_bytes = (size_t)n_marked * 4 * 4 + (size_t)s->n_pairs * sizeof(SvoPair) + 64;
     TGX_TRY(devbuf_reserve(c->svo_sort, sort_bytes));
-    uint32_t* cnt = (uint32_t*)c->svo_sort.ptr;
-    uint32_t* off = cnt + (n_slots + 1);
-    SvoPair* sorted = (SvoPair*)(((uintptr_t)(off + n_slots + 1) + 15) & ~(uintptr_t)15);
-    const uint32_t pgrid_pairs = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((s->n_pairs + 255) / 256, (uint64_t)c->num_sms * 16));
-    TGX_CUDA(cudaMemsetAsync(cnt, 0, n_slots * 4, c->stream));
-    TGX_LAUNCH(c, TR_SVO_VOXELIZE, pgrid_pairs, 256, 0, k_svo_pair_count, (const SvoPair*)c->svo_pairs.ptr, counters, cap,
-               s->d_table, cnt);
-    TGX_LAUNCH(c, TR_SVO_VOXELIZE, 1, 1024, 0, k_svo_pair_scan, cnt, (uint32_t)n_slots, off);
-    TGX_CUDA(cudaMemsetAsync(cnt, 0, n_slots * 4, c->stream));
-    TGX_LAUNCH(c, TR_SVO_VOXELIZE, pgrid_pairs, 256, 0, k_svo_pair_fill, (const SvoPair*)c->svo_pairs.ptr, counters, cap,
-               s->d_table, off, cnt, sorted);
-    // one CTA per slot: the block's image and material grid in shared memory
-    static bool attr = false;
-    if (!attr) {
-        TGX_CUDA(cudaFuncSetAttribute(k_svo_voxelize<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (kBlockWords + 16384) * 4));
-        attr = true;
+    TGX_CUDA(cudaMemsetAsync(counters + S_SLOTS, 0, 2 * 4, c->stream));   // pair ranges handed out, non-empty
+    TGX_CUDA(cudaMemsetAsync(s->d_occ, 0, s->occ_words * 4, c->stream));
+    if (n_marked) {
+        // group the pairs by marked block: counts, ranges, placement
+        const uint32_t* marked = svo_marked(c);
+        uint32_t* cnt = (uint32_t*)c->svo_sort.ptr;
+        uint32_t *off = cnt + n_marked, *cursor = off + n_marked, *slots = cursor + n_marked;
+        SvoPair* sorted = (SvoPair*)(((uintptr_t)(slots + n_marked) + 15) & ~(uintptr_t)15);
+        const uint32_t mgrid = (n_marked + 255) / 256;
+        const uint32_t pgrid = (uint32_t)std::min<uint64_t>(((uint64_t)s->n_pairs + 255) / 256, (uint64_t)c->num_sms * 16);
+        TGX_LAUNCH(c, TR_SVO_ALLOC, mgrid, 256, 0, k_svo_alloc, s->d_table, marked, n_marked, s->d_free, n_free, next_slot,
+                   slots, s->d_slot_block, cnt);
+        TGX_LAUNCH(c, TR_SVO_VOXELIZE, pgrid, 256, 0, k_svo_pair_count, (const SvoPair*)c->svo_pairs.ptr, s->n_pairs,
+                   s->d_table, cnt);
+        TGX_LAUNCH(c, TR_SVO_VOXELIZE, mgrid, 256, 0, k_svo_pair_ranges, cnt, n_marked, counters + S_SLOTS, off, cursor);
+        TGX_LAUNCH(c, TR_SVO_VOXELIZE, pgrid, 256, 0, k_svo_pair_fill, (const SvoPair*)c->svo_pairs.ptr, s->n_pairs,
+                   s->d_table, cursor, sorted);
+        // one CTA per marked block: its image and material grid in shared memory
+        if (s->d_mat) {
+            TGX_CUDA(cudaFuncSetAttribute(k_svo_voxelize<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (kBlockWords + 16384) * 4));
+            TGX_LAUNCH(c, TR_SVO_VOXELIZE, n_marked, 32 * kWarpsPerVoxCta, (kBlockWords + 16384) * 4, k_svo_voxelize<true>,
+                       sc->d_objects, sc->d_cluster_pointers, sc->d_c2o, sc->d_bits, sorted, off, cnt, slots, s->d_pool,
+                       s->d_sub, s->d_nonempty, sc->d_material, s->d_mat, s->mn[0], s->mn[1], s->mn[2], s->B);
+        } else {
+            TGX_LAUNCH(c, TR_SVO_VOXELIZE, n_marked, 32 * kWarpsPerVoxCta, kBlockWords * 4, k_svo_voxelize<false>,
+                       sc->d_objects, sc->d_cluster_pointers, sc->d_c2o, sc->d_bits, sorted, off, cnt, slots, s->d_pool,
+                       s->d_sub, s->d_nonempty, (const uint8_t*)nullptr, (uint16_t*)nullptr, s->mn[0], s->mn[1], s->mn[2],
+                       s->B);
+        }
+        TGX_LAUNCH(c, TR_SVO_PYRAMID, mgrid, 256, 0, k_svo_publish, s->d_table, marked, slots, n_marked);
     }
-    if (s->d_mat)
-        TGX_LAUNCH(c, TR_SVO_VOXELIZE, (uint32_t)n_slots, 32 * kWarpsPerVoxCta, (kBlockWords + 16384) * 4,
-                   k_svo_voxelize<true>, sc->d_objects, sc->d_cluster_pointers, sc->d_c2o, sc->d_bits, sorted, off,
-                   s->d_pool, sc->d_material, s->d_mat, s->mn[0], s->mn[1], s->mn[2], s->B);
-    else
-        TGX_LAUNCH(c, TR_SVO_VOXELIZE, (uint32_t)n_slots, 32 * kWarpsPerVoxCta, kBlockWords * 4, k_svo_voxelize<false>,
-                   sc->d_objects, sc->d_cluster_pointers, sc->d_c2o, sc->d_bits, sorted, off, s->d_pool,
-                   (const uint8_t*)nullptr, (uint16_t*)nullptr, s->mn[0], s->mn[1], s->mn[2], s->B);
-    const uint32_t pgrid = (uint32_t)std::min<uint64_t>((n_table * 32 + 255) / 256, (uint64_t)c->num_sms * 32);
-    TGX_LAUNCH(c, TR_SVO_PYRAMID, pgrid, 256, 0, k_svo_pyramid, s->d_table, n_table, s->d_pool, s->d_nonempty, s->d_sub,
-               s->d_occ, (const uint64_t*)((char*)s->d_occ + svo_occ_off_bytes(s->occ_words)), s->n_levels, s->B, counters);
+    if (n_slots)
+        TGX_LAUNCH(c, TR_SVO_PYRAMID, (n_slots + 255) / 256, 256, 0, k_svo_pyramid, s->d_slot_block, n_slots, s->d_nonempty,
+                   s->d_occ, (const uint64_t*)((char*)s->d_occ + svo_occ_off_bytes(s->occ_words)), s->n_levels, s->B,
+                   counters);
     return TGX_OK;
 }
 
@@ -1022,7 +1068,7 @@ extern "C" tgx_status tgx_svo_build_flags(tgx_ctx* c, const tgx_scene* sc, const
     s->n_slots = s->n_blocks;
     const bool materials = sc->d_material && sc->d_luts && !(flags & TGX_SVO_NO_MATERIALS);
     if ((st = svo_resize_slots(c, s, std::max(s->n_blocks, 1u), 0, materials)) != TGX_OK) return fail(st);
-    if ((st = svo_fill(c, s, sc, 0, 0)) != TGX_OK) return fail(st);
+    if ((st = svo_fill(c, s, sc, s->n_blocks, 0, 0, s->n_slots)) != TGX_OK) return fail(st);
     s->device_bytes = svo_device_bytes(s);
     *out = s;
     return TGX_OK;
@@ -1040,28 +1086,36 @@ extern "C" tgx_status tgx_svo_update(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc
     if (sc->n_objects == 0) return TGX_OK;
     TGX_CUDA(cudaSetDevice(c->device));
     const uint64_t n_table = (uint64_t)s->B * s->B * s->B;
-    TGX_TRY(devbuf_reserve(c->svo_scratch, n_table));
-    uint8_t* dirty = (uint8_t*)c->svo_scratch.ptr;
+    const uint64_t n_words = (n_table + 31) / 32;
+    TGX_TRY(devbuf_reserve(c->svo_scratch, n_words * 4));
+    uint32_t* dirty = (uint32_t*)c->svo_scratch.ptr;
     uint32_t* counters = s->d_counters;
-    TGX_CUDA(cudaMemsetAsync(dirty, 0, n_table, c->stream));
+    TGX_CUDA(cudaMemsetAsync(dirty, 0, n_words * 4, c->stream));
     TGX_CUDA(cudaMemsetAsync(counters + S_FREED, 0, 2 * 4, c->stream));   // freed, moved
-    TGX_LAUNCH(c, TR_SVO_CANDIDATES, sc->n_objects, 128, 0, k_svo_mark_dirty, sc->d_objects, s->d_objs, sc->d_cluster_pointers,
-               sc->d_bits, s->mn[0], s->mn[1], s->mn[2], s->B, dirty, counters);
-    const uint32_t wgrid = (uint32_t)std::min<uint64_t>((n_table * 32 + 255) / 256, (uint64_t)c->num_sms * 32);
-    TGX_LAUNCH(c, TR_SVO_ALLOC, wgrid, 256, 0, k_svo_release_dirty, s->d_table, n_table, dirty, s->d_pool, s->d_sub,
-               s->d_nonempty, s->d_mat, s->d_free + s->n_free, counters);
+    TGX_LAUNCH(c, TR_SVO_CANDIDATES, dim3(sc->n_objects, 8), 128, 0, k_svo_mark_dirty, sc->d_objects, s->d_objs,
+               sc->d_cp_obj, s->mn[0], s->mn[1], s->mn[2], s->B, dirty);
+    const uint64_t items = std::max<uint64_t>(n_words, sc->n_objects);
+    const uint32_t wgrid = (uint32_t)std::min<uint64_t>((items + 255) / 256, (uint64_t)c->num_sms * 16);
+    TGX_LAUNCH(c, TR_SVO_ALLOC, wgrid, 256, 0, k_svo_release_dirty, s->d_table, n_words, dirty, n_table, s->d_nonempty,
+               s->d_slot_block, s->d_free + s->n_free, sc->d_objects, s->d_objs, sc->n_objects, counters);
     // pairs of the dirty blocks, into the pair storage the last build left (grown when short)
-    TGX_TRY(svo_candidates(c, s, sc, dirty, std::max<uint64_t>(1024, c->svo_pairs.bytes / sizeof(SvoPair))));
+    TGX_TRY(svo_candidates(c, s, sc, dirty, std::max<uint64_t>(1024, c->svo_pairs.bytes / kPairBytes)));
     const uint32_t* hc = (const uint32_t*)c->h_counter;
-    const uint32_t n_moved = hc[S_MOVED], n_freed = hc[S_FREED], n_marked = hc[S_MARKED];
+    const uint32_t n_moved = hc[S_MOVED], n_freed = hc[S_FREED], n_marked = hc[S_MARKED], hc_pairs = hc[S_PAIRS];
     if (out_n_moved) *out_n_moved = n_moved;
     if (n_moved == 0) return TGX_OK;
     const uint32_t n_free = s->n_free + n_freed;
     const uint32_t fresh = n_marked > n_free ? n_marked - n_free : 0u;
     const uint32_t need = s->n_slots + fresh;
-    if (need > s->pool_cap) TGX_TRY(svo_resize_slots(c, s, need + need / 4 + 64, s->n_slots, s->d_mat != nullptr));
-    s->n_pairs = hc[S_PAIRS];
-    TGX_TRY(svo_fill(c, s, sc, n_free, s->n_slots));
+    tgx_status st = TGX_OK;
+    if (need > s->pool_cap) st = svo_resize_slots(c, s, need + need / 4 + 64, s->n_slots, s->d_mat != nullptr);
+    s->n_pairs = hc_pairs;
+    if (st == TGX_OK) st = svo_fill(c, s, sc, n_marked, n_free, s->n_slots, need);
+    if (st != TGX_OK) {   // no mark stays in the table: a traversal would take it for a slot
+        const uint32_t grid = (uint32_t)std::min<uint64_t>((n_table + 255) / 256, (uint64_t)c->num_sms * 32);
+        TGX_LAUNCH(c, TR_SVO_ALLOC, grid, 256, 0, k_svo_unmark, s->d_table, n_table);
+        return st;
+    }
     s->n_free = n_free - (n_marked - fresh);
     s->n_slots = need;
     s->n_blocks = s->n_blocks - n_freed + n_marked;

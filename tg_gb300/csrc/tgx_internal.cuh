@@ -186,6 +186,7 @@ struct tgx_svo
     uint32_t  pool_cap = 0;       // slots the pool, sub, nonempty, material and free arrays hold
     uint32_t  n_free = 0;         // slots released by updates, d_free[0 .. n_free)
     uint32_t* d_free = nullptr;
+    uint32_t* d_slot_block = nullptr;   // per slot: its block's table index, ~0 for a slot without one
     uint32_t* d_counters = nullptr;  // this SVO's build counters (pairs, marks, slots, non-empty, freed)
     tgx_object* d_objs = nullptr; // object records the SVO reflects (updates diff the scene against them)
     uint32_t  n_objects = 0, n_cluster_pointers = 0;
@@ -308,6 +309,24 @@ __device__ __forceinline__ bool inverse_is_plain(const float* inv)
 #pragma unroll
     for (int i = 0; i < 16; i++) ok = ok && fabsf(inv[i]) <= 1e30f;
     return ok;
+}
+
+// Rows 0..2 of T(s) * inverse * T(-t) for a plain inverse (c0 .. c3 its columns):
+// the two products with translations, of which every term is left out that is
+// 0 or 1 times something.  The same value in every element as the full products
+// (only the sign of a zero can differ, which no use of these matrices sees).
+__device__ __forceinline__ void dm4_ws2ms(const float4 c0, const float4 c1, const float4 c2, const float4 c3,
+                                          const float s[3], const float t[3], float* m)
+{
+    const float i0[3] = {c0.x, c0.y, c0.z}, i1[3] = {c1.x, c1.y, c1.z}, i2[3] = {c2.x, c2.y, c2.z},
+                i3[3] = {c3.x, c3.y, c3.z};
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+        const float m0 = xadd(i0[r], xmul(s[r], c0.w)), m1 = xadd(i1[r], xmul(s[r], c1.w)),
+                    m2 = xadd(i2[r], xmul(s[r], c2.w)), m3 = xadd(i3[r], xmul(s[r], c3.w));
+        DM(m, r, 0) = m0; DM(m, r, 1) = m1; DM(m, r, 2) = m2;
+        DM(m, r, 3) = xadd(xadd(xadd(xmul(m0, -t[0]), xmul(m1, -t[1])), xmul(m2, -t[2])), m3);
+    }
 }
 
 // tgm_m4_mulv4 (tg_math.c:2428-2438): row = ((x*m0 + y*m1) + z*m2) + w*m3
