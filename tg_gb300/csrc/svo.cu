@@ -36,7 +36,8 @@ namespace {
 
 constexpr uint32_t kBlockSide = 32;
 constexpr uint32_t kBlockWords = 1024;
-constexpr uint32_t kMark = 0xffffffffu;
+constexpr uint32_t kMark = 0xffffffffu;      // table entry of a marked block
+constexpr uint32_t kNoBlock = 0xffffffffu;   // block of a candidate pair that failed its test
 constexpr uint32_t kWarpsPerVoxCta = 16;
 
 struct SvoPair
@@ -45,7 +46,7 @@ struct SvoPair
     uint32_t block;
 };
 
-enum SvoCounter { S_PAIRS = 0, S_MARKED = 1, S_SLOTS = 2, S_NONEMPTY = 3, S_FREED = 4, S_MOVED = 5, S_COUNT = 8 };
+enum SvoCounter { S_PAIRS = 0, S_MARKED = 1, S_SLOTS = 2, S_NONEMPTY = 3, S_FREED = 4, S_MOVED = 5, S_CAND = 6, S_COUNT = 8 };
 
 struct dv3 { float x, y, z; };
 
@@ -205,109 +206,150 @@ __device__ __forceinline__ bool cluster_blocks(const tgx_object& od, uint32_t re
     return some;
 }
 
-// Bound by instruction issue (the box tests).  A node that holds the cluster's
-// world box with a margin surely passes: no axis can separate them, and the
-// margin (1 + 2e-5 of the coordinates) is far above the test's rounding.  Most
-// levels of most paths are like that (a 32^3 cluster box lies inside its
-// parent's cell of 2^k voxels in all but 45 / 2^k of the cases), so their tests
-// are left out.  That needs a matrix that is a rotation to 10^-3 and node
-// corners that are exact; other objects run every test.  Emptiness comes with the
-// object in cp_obj instead of from the 64-byte bitmask.
-// 386k clusters at 4096^3: CC us -> DD us; with a dirty map (8 moved objects) 83 -> EE.
-__global__ void __launch_bounds__(128) k_svo_candidates(
-    const tgx_object* __restrict__ objects, const float4* __restrict__ inv, const uint32_t* __restrict__ cp_obj,
-    uint32_t n_cp, float mnx, float mny, float mnz, uint32_t L, uint32_t B, uint32_t* __restrict__ table,
-    SvoPair* __restrict__ pairs, uint32_t* __restrict__ marked, uint32_t pair_capacity, uint32_t* __restrict__ counters,
-    tgx_dev_status* __restrict__ status, const uint32_t* __restrict__ dirty /* null: every block; else a bit per block */)
+// Every (cluster, block) pair whose block the cluster's conservative box
+// reaches, one thread per cluster pointer, appended by one atomic per warp.  The
+// tests of a pair are long (seven levels at 4096^3), so they run in a kernel of
+// their own with a thread per pair: with a thread per cluster a warp took as
+// long as its cluster with the most blocks.  Emptiness comes with the object in
+// cp_obj instead of from the 64-byte bitmask.
+__global__ void __launch_bounds__(128) k_svo_candidates(const tgx_object* __restrict__ objects,
+                                                       const uint32_t* __restrict__ cp_obj, uint32_t n_cp, float mnx,
+                                                       float mny, float mnz, uint32_t B, SvoPair* __restrict__ pairs,
+                                                       uint32_t pair_capacity, uint32_t* __restrict__ counters,
+                                                       tgx_dev_status* __restrict__ status,
+                                                       const uint32_t* __restrict__ dirty /* null: every block; else a bit per block */)
 {
-    const uint32_t cp = blockIdx.x * blockDim.x + threadIdx.x;
-    if (cp >= n_cp) return;
-    const uint32_t po = cp_obj[cp];
-    if (po >> 31) return;   // no set voxel
-    const tgx_object& od = objects[po];
-    const uint32_t rel = cp - od.first_cluster_pointer;
-
-    // conservative world box of the cluster (only selects blocks to test)
+    const uint32_t cp = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
     const float mn[3] = {mnx, mny, mnz};
     float lo[3], hi[3];
-    int b0[3], b1[3];
-    if (!cluster_blocks(od, rel, mn, B, lo, hi, b0, b1)) return;
+    int b0[3] = {0, 0, 0}, b1[3] = {-1, -1, -1};
+    const uint32_t po = cp < n_cp ? cp_obj[cp] : 0x80000000u;
+    bool some = false;
+    if (!(po >> 31)) {   // some set voxel
+        const tgx_object& od = objects[po];
+        some = cluster_blocks(od, cp - od.first_cluster_pointer, mn, B, lo, hi, b0, b1);
+    }
+    const uint32_t nx = some ? (uint32_t)(b1[0] - b0[0] + 1) : 0u, ny = some ? (uint32_t)(b1[1] - b0[1] + 1) : 0u;
+    const uint32_t total = some ? nx * ny * (uint32_t)(b1[2] - b0[2] + 1) : 0u;
+    auto block = [&](uint32_t k) {
+        const uint32_t q = k / nx, x = k - q * nx, z = q / ny, y = q - z * ny;
+        return (((uint32_t)b0[2] + z) * B + (uint32_t)b0[1] + y) * B + (uint32_t)b0[0] + x;
+    };
+    uint32_t n = total;
     if (dirty) {
-        bool any = false;
-        for (int bz = b0[2]; bz <= b1[2]; bz++)
-            for (int by = b0[1]; by <= b1[1]; by++)
-                for (int bx = b0[0]; bx <= b1[0]; bx++) {
-                    const uint32_t blk = ((uint32_t)bz * B + (uint32_t)by) * B + (uint32_t)bx;
-                    any = any || (dirty[blk >> 5] >> (blk & 31u)) & 1u;
-                }
-        if (!any) return;
-    }
-    float ws2ms[16];
-    const float4 c0 = inv[4u * po], c1 = inv[4u * po + 1u], c2 = inv[4u * po + 2u], c3 = inv[4u * po + 3u];
-    if (c0.x == c0.x) {
-        float off[3], ohe[3];
-        cluster_offsets(od, rel, off, ohe);
-        const float s3[3] = {xadd(ohe[0], -off[0]), xadd(ohe[1], -off[1]), xadd(ohe[2], -off[2])};
-        dm4_ws2ms(c0, c1, c2, c3, s3, od.translation, ws2ms);
-    } else {
-        svo_ws2ms(od, rel, ws2ms);
-    }
-    const float ext = (float)(1u << L);
-    // whether nodes around the cluster can be passed without the test, and the margin they need
-    bool skip = true;
-    float margin = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-        const float* r = od.rotation + 4 * i;
-#pragma unroll
-        for (int j = 0; j <= i; j++) {
-            const float* q = od.rotation + 4 * j;
-            skip = skip && fabsf(r[0] * q[0] + r[1] * q[1] + r[2] * q[2] - (i == j ? 1.0f : 0.0f)) <= 1e-3f;
+        n = 0;
+        for (uint32_t k = 0; k < total; k++) {
+            const uint32_t blk = block(k);
+            n += (dirty[blk >> 5] >> (blk & 31u)) & 1u;
         }
-        // the rows' last column and the last row are those of a rotation
-        skip = skip && od.rotation[4 * i + 3] == 0.0f && od.rotation[12 + i] == 0.0f && fabsf(mn[i]) + ext <= 16777216.0f;
-        margin = fmaxf(margin, 1.0f + 2e-5f * (fabsf(lo[i]) + fabsf(hi[i]) + fabsf(mn[i]) + ext + fabsf(od.translation[i])));
     }
-    skip = skip && od.rotation[15] == 1.0f;
-    for (int bz = b0[2]; bz <= b1[2]; bz++)
-        for (int by = b0[1]; by <= b1[1]; by++)
-            for (int bx = b0[0]; bx <= b1[0]; bx++) {
-                const uint32_t blk = ((uint32_t)bz * B + (uint32_t)by) * B + (uint32_t)bx;
-                if (dirty && !((dirty[blk >> 5] >> (blk & 31u)) & 1u)) continue;
-                // walk the reference's recursion from the root to this block
-                dv3 pmin = dv3{mnx, mny, mnz};
-                dv3 pmax = dv3{xadd(mnx, ext), xadd(mny, ext), xadd(mnz, ext)};
-                bool pass = true;
-                for (int lev = (int)L - 1; lev >= 5; lev--) {
-                    const dv3 ce = dv3{xmul(xsub(pmax.x, pmin.x), 0.5f), xmul(xsub(pmax.y, pmin.y), 0.5f),
-                                       xmul(xsub(pmax.z, pmin.z), 0.5f)};
-                    const uint32_t sh = (uint32_t)lev - 5;
-                    const uint32_t cx = ((uint32_t)bx >> sh) & 1u, cy = ((uint32_t)by >> sh) & 1u,
-                                   cz = ((uint32_t)bz >> sh) & 1u;
-                    pmin = dv3{xadd(pmin.x, xmul((float)cx, ce.x)), xadd(pmin.y, xmul((float)cy, ce.y)),
-                               xadd(pmin.z, xmul((float)cz, ce.z))};
-                    pmax = dv3{xadd(pmin.x, ce.x), xadd(pmin.y, ce.y), xadd(pmin.z, ce.z)};
-                    const bool holds = skip && lo[0] - margin >= pmin.x && lo[1] - margin >= pmin.y && lo[2] - margin >= pmin.z &&
-                                       hi[0] + margin <= pmax.x && hi[1] + margin <= pmax.y && hi[2] + margin <= pmax.z;
-                    if (!holds) {
-                        dv3 bc[8];
+    uint32_t incl = n;
 #pragma unroll
-                        for (int k = 0; k < 8; k++)
-                            bc[k] = mulv4p(ws2ms, (k & 1) ? pmax.x : pmin.x, (k & 2) ? pmax.y : pmin.y,
-                                           (k & 4) ? pmax.z : pmin.z);
-                        if (!aabb_obb(bc)) { pass = false; break; }
-                    }
+    for (uint32_t o = 1; o < 32u; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    uint32_t base = 0;
+    if (lane == 31u && incl) base = atomicAdd(&counters[S_CAND], incl);
+    base = __shfl_sync(0xffffffffu, base, 31) + incl - n;
+    if (n == 0u) return;
+    if ((uint64_t)base + n > pair_capacity) dev_error(status, TGX_ERR_CAPACITY, 11, base);
+    for (uint32_t k = 0; k < total; k++) {
+        const uint32_t blk = block(k);
+        if (dirty && !((dirty[blk >> 5] >> (blk & 31u)) & 1u)) continue;
+        if (base < pair_capacity) pairs[base] = SvoPair{cp, blk};
+        base++;
+    }
+}
+
+// The reference's test of every candidate pair, a thread each: a pair that fails
+// gets the block ~0, one that passes marks its block (and lists it the first
+// time).  Bound by instruction issue.  A node that holds the cluster's world box
+// with a margin surely passes: no axis can separate them, and the margin
+// (1 + 2e-5 of the coordinates) is far above the test's rounding.  Most levels of
+// most paths are like that (a cluster's box lies inside its cell of 2^k voxels in
+// all but about 45 / 2^k of the cases), so their tests are left out.  That needs a
+// matrix that is a rotation to 10^-3 and node corners that are exact; other
+// objects run every test.
+// 386k clusters at 4096^3, both kernels: 385 -> CC us with every test and a thread
+// per cluster; with a dirty map (8 moved objects) 83 -> EE us.
+__global__ void __launch_bounds__(128) k_svo_test_pairs(
+    const tgx_object* __restrict__ objects, const float4* __restrict__ inv, const uint32_t* __restrict__ cp_obj, float mnx,
+    float mny, float mnz, uint32_t L, uint32_t B, uint32_t* __restrict__ table, SvoPair* __restrict__ pairs,
+    uint32_t* __restrict__ marked, uint32_t pair_capacity, uint32_t* __restrict__ counters)
+{
+    const uint32_t n = min(counters[S_CAND], pair_capacity), lane = threadIdx.x & 31u;
+    const float mn[3] = {mnx, mny, mnz};
+    const float ext = (float)(1u << L);
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); i0 < n; i0 += stride) {
+        const uint32_t i = i0 + lane;
+        bool pass = i < n;
+        uint32_t blk = 0;
+        if (pass) {
+            const SvoPair pr = pairs[i];
+            blk = pr.block;
+            const uint32_t bx = blk % B, by = (blk / B) % B, bz = blk / (B * B);
+            const uint32_t po = cp_obj[pr.cluster_pointer];
+            const tgx_object& od = objects[po];
+            const uint32_t rel = pr.cluster_pointer - od.first_cluster_pointer;
+            float lo[3], hi[3], ws2ms[16];
+            int b0[3], b1[3];
+            cluster_blocks(od, rel, mn, B, lo, hi, b0, b1);
+            const float4 c0 = inv[4u * po], c1 = inv[4u * po + 1u], c2 = inv[4u * po + 2u], c3 = inv[4u * po + 3u];
+            if (c0.x == c0.x) {
+                float off[3], ohe[3];
+                cluster_offsets(od, rel, off, ohe);
+                const float s3[3] = {xadd(ohe[0], -off[0]), xadd(ohe[1], -off[1]), xadd(ohe[2], -off[2])};
+                dm4_ws2ms(c0, c1, c2, c3, s3, od.translation, ws2ms);
+            } else {
+                svo_ws2ms(od, rel, ws2ms);
+            }
+            // whether nodes around the cluster can be passed without the test, and the margin they need
+            bool skip = od.rotation[15] == 1.0f;
+            float margin = 0.0f;
+#pragma unroll
+            for (int r = 0; r < 3; r++) {
+                const float* p = od.rotation + 4 * r;
+#pragma unroll
+                for (int j = 0; j <= r; j++) {
+                    const float* q = od.rotation + 4 * j;
+                    skip = skip && fabsf(p[0] * q[0] + p[1] * q[1] + p[2] * q[2] - (r == j ? 1.0f : 0.0f)) <= 1e-3f;
                 }
-                if (!pass) continue;
-                const uint32_t slot = atomicAdd(&counters[S_PAIRS], 1u);
-                if (slot < pair_capacity) pairs[slot] = SvoPair{cp, blk};
-                else dev_error(status, TGX_ERR_CAPACITY, 11, slot);
-                // every marked block has a pair, so the list is no longer than the pairs' storage
-                if (atomicCAS(&table[blk], 0u, kMark) == 0u) {
-                    const uint32_t m = atomicAdd(&counters[S_MARKED], 1u);
-                    if (m < pair_capacity) marked[m] = blk;
+                // the last column and row are those of a rotation; node corners below 2^24 are exact
+                skip = skip && p[3] == 0.0f && od.rotation[12 + r] == 0.0f && fabsf(mn[r]) + ext <= 16777216.0f;
+                margin = fmaxf(margin, 1.0f + 2e-5f * (fabsf(lo[r]) + fabsf(hi[r]) + fabsf(mn[r]) + ext + fabsf(od.translation[r])));
+            }
+            // walk the reference's recursion from the root to this block
+            dv3 pmin = dv3{mnx, mny, mnz};
+            dv3 pmax = dv3{xadd(mnx, ext), xadd(mny, ext), xadd(mnz, ext)};
+            for (int lev = (int)L - 1; lev >= 5; lev--) {
+                const dv3 ce = dv3{xmul(xsub(pmax.x, pmin.x), 0.5f), xmul(xsub(pmax.y, pmin.y), 0.5f),
+                                   xmul(xsub(pmax.z, pmin.z), 0.5f)};
+                const uint32_t sh = (uint32_t)lev - 5;
+                const uint32_t cx = (bx >> sh) & 1u, cy = (by >> sh) & 1u, cz = (bz >> sh) & 1u;
+                pmin = dv3{xadd(pmin.x, xmul((float)cx, ce.x)), xadd(pmin.y, xmul((float)cy, ce.y)),
+                           xadd(pmin.z, xmul((float)cz, ce.z))};
+                pmax = dv3{xadd(pmin.x, ce.x), xadd(pmin.y, ce.y), xadd(pmin.z, ce.z)};
+                const bool holds = skip && lo[0] - margin >= pmin.x && lo[1] - margin >= pmin.y && lo[2] - margin >= pmin.z &&
+                                   hi[0] + margin <= pmax.x && hi[1] + margin <= pmax.y && hi[2] + margin <= pmax.z;
+                if (pass && !holds) {
+                    dv3 bc[8];
+#pragma unroll
+                    for (int k = 0; k < 8; k++)
+                        bc[k] = mulv4p(ws2ms, (k & 1) ? pmax.x : pmin.x, (k & 2) ? pmax.y : pmin.y,
+                                       (k & 4) ? pmax.z : pmin.z);
+                    pass = aabb_obb(bc);
                 }
             }
+            if (!pass) pairs[i].block = kNoBlock;
+        }
+        const uint32_t mask = __ballot_sync(0xffffffffu, pass);
+        if (lane == 0u && mask) atomicAdd(&counters[S_PAIRS], (uint32_t)__popc(mask));
+        // a read before the swap: most blocks are marked by an earlier pair
+        if (pass && *(volatile uint32_t*)&table[blk] == 0u && atomicCAS(&table[blk], 0u, kMark) == 0u)
+            marked[atomicAdd(&counters[S_MARKED], 1u)] = blk;   // no more blocks than pairs: the list holds them
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -321,7 +363,8 @@ __global__ void __launch_bounds__(128) k_svo_candidates(
 __global__ void __launch_bounds__(256) k_svo_alloc(uint32_t* __restrict__ table, const uint32_t* __restrict__ marked,
                                                   uint32_t n, const uint32_t* __restrict__ free_list, uint32_t n_free,
                                                   uint32_t next_slot, uint32_t* __restrict__ slots,
-                                                  uint32_t* __restrict__ slot_block, uint32_t* __restrict__ cnt)
+                                                  uint32_t* __restrict__ slot_block, uint32_t* __restrict__ nonempty,
+                                                  uint32_t* __restrict__ cnt)
 {
     const uint32_t m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= n) return;
@@ -330,6 +373,7 @@ __global__ void __launch_bounds__(256) k_svo_alloc(uint32_t* __restrict__ table,
     table[blk] = m + 1u;
     slots[m] = slot;
     slot_block[slot] = blk;
+    nonempty[slot] = 0u;
     cnt[m] = 0u;
 }
 
@@ -354,14 +398,17 @@ __device__ __forceinline__ void smem_max_u16(uint32_t* words, uint32_t idx, uint
     }
 }
 
-// 3a. pairs grouped by their (marked) block: counts, a range each, placement.
+// 3a. the n candidates that passed grouped by their (marked) block: counts, a
+// range each, placement.
 // The order of the ranges is free, so a block's range comes from a counter
 // (one atomic per warp) instead of a scan.
 __global__ void __launch_bounds__(256) k_svo_pair_count(const SvoPair* __restrict__ pairs, uint32_t n,
                                                        const uint32_t* __restrict__ table, uint32_t* __restrict__ cnt)
 {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        atomicAdd(&cnt[table[pairs[i].block] - 1u], 1u);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t blk = pairs[i].block;
+        if (blk != kNoBlock) atomicAdd(&cnt[table[blk] - 1u], 1u);
+    }
 }
 
 __global__ void __launch_bounds__(256) k_svo_pair_ranges(const uint32_t* __restrict__ cnt, uint32_t n,
@@ -388,7 +435,7 @@ __global__ void __launch_bounds__(256) k_svo_pair_fill(const SvoPair* __restrict
 {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const SvoPair pr = pairs[i];
-        sorted[atomicAdd(&cursor[table[pr.block] - 1u], 1u)] = pr;
+        if (pr.block != kNoBlock) sorted[atomicAdd(&cursor[table[pr.block] - 1u], 1u)] = pr;
     }
 }
 
@@ -408,13 +455,14 @@ struct alignas(16) PairRec
 };
 static_assert(sizeof(PairRec) == 112, "seven 16-byte shared loads");
 
-// Returns the pair's trimmed voxel count.  `plain`: the block side is exactly 32
+// Returns the pair's trimmed voxel count in the `layers` layers from slab0 on (the
+// record is written only when there are any).  `plain`: the block side is exactly 32
 // (min not so large that min + extent rounds) and no corner coordinate is NaN or
 // beyond 10^6, which the row loop's arithmetic needs.
 __device__ __forceinline__ uint32_t pair_setup(const tgx_object* __restrict__ objects,
                                                const uint32_t* __restrict__ cluster_pointers,
                                                const uint32_t* __restrict__ c2o, const SvoPair& pr, float mnx, float mny,
-                                               float mnz, uint32_t B, PairRec* out)
+                                               float mnz, uint32_t B, uint32_t slab0, uint32_t layers, PairRec* out)
 {
     const uint32_t cp = pr.cluster_pointer;
     const uint32_t ci = cluster_pointers[cp];
@@ -439,8 +487,11 @@ __device__ __forceinline__ uint32_t pair_setup(const tgx_object* __restrict__ ob
     const dv3 max_c = vmax(vmax(vmax(cw[0], cw[1]), vmax(cw[2], cw[2])), vmax(vmax(cw[4], cw[6]), vmax(cw[5], cw[7])));
     const dv3 tmin = vmax(pmin, dv3{floorf(min_c.x), floorf(min_c.y), floorf(min_c.z)});
     const dv3 tmax = vmin(pmax, dv3{ceilf(max_c.x), ceilf(max_c.y), ceilf(max_c.z)});
-    const uint32_t x0 = trim_u32(xsub(tmin.x, pmin.x)), y0 = trim_u32(xsub(tmin.y, pmin.y)), z0 = trim_u32(xsub(tmin.z, pmin.z));
-    const uint32_t x1 = trim_u32(xsub(tmax.x, pmin.x)), y1 = trim_u32(xsub(tmax.y, pmin.y)), z1 = trim_u32(xsub(tmax.z, pmin.z));
+    const uint32_t x0 = trim_u32(xsub(tmin.x, pmin.x)), y0 = trim_u32(xsub(tmin.y, pmin.y));
+    const uint32_t x1 = trim_u32(xsub(tmax.x, pmin.x)), y1 = trim_u32(xsub(tmax.y, pmin.y));
+    const uint32_t z0 = max(trim_u32(xsub(tmin.z, pmin.z)), slab0);
+    const uint32_t z1 = layers == 32u ? trim_u32(xsub(tmax.z, pmin.z)) : min(trim_u32(xsub(tmax.z, pmin.z)), slab0 + layers);
+    if (x0 >= x1 || y0 >= y1 || z0 >= z1) return 0u;
     dm4_inverse(cs2ws, ws2cs);
     bool plain = pext.x == 32.0f && pext.y == 32.0f && pext.z == 32.0f;
 #pragma unroll
@@ -453,7 +504,7 @@ __device__ __forceinline__ uint32_t pair_setup(const tgx_object* __restrict__ ob
     out->hi = x1 | y1 << 8 | z1 << 16;
     out->ci = ci;
     out->lut = ((od.lut_idx << 8) & 0x7fffffffu) | (plain ? 0u : 0x80000000u);
-    return x0 >= x1 || y0 >= y1 || z0 >= z1 ? 0u : (x1 - x0) * (y1 - y0) * (z1 - z0);
+    return (x1 - x0) * (y1 - y0) * (z1 - z0);
 }
 
 // The z- and y-lerps of tg__construct_leaf_node for row (iy, iz) of a block:
@@ -478,8 +529,8 @@ __device__ __forceinline__ void row_ends(const float* bc, float ty, float tz, fl
 template <bool kMat>
 __device__ __noinline__ void voxelize_any(const float* bc, uint32_t x0, uint32_t x1, uint32_t y0, uint32_t z0, uint32_t ny,
                                           uint32_t rows, float rny, uint32_t lut, const uint32_t* cw, const uint8_t* cm,
-                                          float mnx, float mny, float mnz, uint32_t B, uint32_t block, uint32_t* img,
-                                          uint32_t* smat)
+                                          float mnx, float mny, float mnz, uint32_t B, uint32_t block, uint32_t word0,
+                                          uint32_t n_words, uint32_t* img, uint32_t* smat)
 {
     const uint32_t bx = block % B, by = (block / B) % B, bz = block / (B * B);
     const float px = xadd(mnx, (float)(bx * kBlockSide)), py = xadd(mny, (float)(by * kBlockSide)),
@@ -501,62 +552,54 @@ __device__ __noinline__ void voxelize_any(const float* bc, uint32_t x0, uint32_t
             const uint32_t rvi = 64u * (uint32_t)cz + 8u * (uint32_t)cy + (uint32_t)cx;
             if (!(cw[rvi >> 5] & (1u << (rvi & 31u)))) continue;
             const uint32_t bvi = (uint32_t)xadd(row_base, (float)ix);
-            atomicOr(&img[bvi >> 5], 1u << (bvi & 31u));
-            if (kMat) smem_max_u16(smat, bvi, ((lut | cm[rvi]) + 1u) & 0xffffu);
+            if ((bvi >> 5) - word0 >= n_words) continue;   // a side that rounds above 32
+            atomicOr(&img[(bvi >> 5) - word0], 1u << (bvi & 31u));
+            if (kMat) smem_max_u16(smat, bvi - word0 * 32u, ((lut | cm[rvi]) + 1u) & 0xffffu);
         }
     }
 }
 
-// The masks of a block's 4^3 and 8^3 cells from its bit words, by one warp (lane
-// y reads the 32 rows (y, z)), and whether it holds a voxel.
-__device__ __forceinline__ void block_masks(const uint32_t* blk, uint32_t* __restrict__ sb, uint32_t* __restrict__ nonempty)
+// The masks of the 4^3 and 8^3 cells of 8 layers of a block (layers 8 u .. 8 u + 7,
+// rows: their bit words), by one warp (lane y reads the rows (y, z)).  Sets
+// *nonempty (zero before) when they hold a voxel.
+__device__ __forceinline__ void layer_masks(const uint32_t* rows, uint32_t u, uint32_t* __restrict__ sb,
+                                            uint32_t* __restrict__ nonempty)
 {
     const uint32_t lane = threadIdx.x & 31u;
-    uint32_t any = 0;
-    uint32_t n4[8];   // per 4-voxel z-slab: which 4-voxel x-groups of row y hold a voxel
+    uint32_t n4[2] = {0u, 0u};   // per 4 layers: which 4-voxel x-groups of row y hold a voxel
 #pragma unroll
-    for (int k = 0; k < 8; k++) n4[k] = 0;
-#pragma unroll
-    for (int z = 0; z < 32; z++) {
-        const uint32_t row = blk[z * 32 + lane];
-        any |= row;
-        uint32_t f = 0;
-#pragma unroll
-        for (int gx = 0; gx < 8; gx++) f |= ((row >> (4 * gx)) & 15u) ? (1u << gx) : 0u;
-        n4[z >> 2] |= f;
+    for (int z = 0; z < 8; z++) {
+        const uint32_t row = rows[z * 32 + lane];
+        uint32_t f = row | row >> 1;
+        f = (f | f >> 2) & 0x11111111u;   // bit 4 gx: some of the group's four voxels
+        f = (f | f >> 3) & 0x03030303u;   // gather the eight bits
+        f = (f | f >> 6) & 0x000f000fu;
+        n4[z >> 2] |= (f | f >> 12) & 0xffu;
     }
-    any = __any_sync(0xffffffffu, any != 0u);
-    if (lane == 0) *nonempty = any ? 1u : 0u;
+    if (__any_sync(0xffffffffu, (n4[0] | n4[1]) != 0u) && lane == 0u) *nonempty = 1u;
     // 4^3 cells: bit ((cz * 8 + cy) * 8 + cx), cy = lane / 4
 #pragma unroll
-    for (int cz = 0; cz < 8; cz++) {
-        uint32_t b = n4[cz];
+    for (int h = 0; h < 2; h++) {
+        uint32_t b = n4[h];
         b |= __shfl_xor_sync(0xffffffffu, b, 1);
         b |= __shfl_xor_sync(0xffffffffu, b, 2);
         uint32_t w = (lane & 3u) == 0u ? b << (((lane >> 2) & 3u) * 8u) : 0u;
         w |= __shfl_xor_sync(0xffffffffu, w, 4);
         w |= __shfl_xor_sync(0xffffffffu, w, 8);
-        if ((lane & 15u) == 0u) sb[cz * 2 + (lane >> 4)] = w;
+        if ((lane & 15u) == 0u) sb[(2u * u + h) * 2u + (lane >> 4)] = w;
     }
-    // 8^3 cells: bit ((cz * 4 + cy) * 4 + cx), cy = lane / 8
-    uint32_t w8[2] = {0u, 0u};
+    // 8^3 cells: bit ((cz * 4 + cy) * 4 + cx), cy = lane / 8: 16 bits for cz = u
+    const uint32_t b = n4[0] | n4[1];
+    uint32_t c3 = 0;
 #pragma unroll
-    for (int cz = 0; cz < 4; cz++) {
-        const uint32_t b = n4[2 * cz] | n4[2 * cz + 1];
-        uint32_t c3 = 0;
-#pragma unroll
-        for (int cx = 0; cx < 4; cx++) c3 |= ((b >> (2 * cx)) & 3u) ? (1u << cx) : 0u;
-        c3 |= __shfl_xor_sync(0xffffffffu, c3, 1);
-        c3 |= __shfl_xor_sync(0xffffffffu, c3, 2);
-        c3 |= __shfl_xor_sync(0xffffffffu, c3, 4);
-        if ((lane & 7u) == 0u) w8[cz >> 1] |= c3 << ((cz & 1) * 16 + (lane >> 3) * 4);
-    }
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-        w8[k] |= __shfl_xor_sync(0xffffffffu, w8[k], 8);
-        w8[k] |= __shfl_xor_sync(0xffffffffu, w8[k], 16);
-    }
-    if (lane == 0) { sb[16] = w8[0]; sb[17] = w8[1]; }
+    for (int cx = 0; cx < 4; cx++) c3 |= ((b >> (2 * cx)) & 3u) ? (1u << cx) : 0u;
+    c3 |= __shfl_xor_sync(0xffffffffu, c3, 1);
+    c3 |= __shfl_xor_sync(0xffffffffu, c3, 2);
+    c3 |= __shfl_xor_sync(0xffffffffu, c3, 4);
+    uint32_t w8 = (lane & 7u) == 0u ? c3 << ((lane >> 3) * 4u) : 0u;
+    w8 |= __shfl_xor_sync(0xffffffffu, w8, 8);
+    w8 |= __shfl_xor_sync(0xffffffffu, w8, 16);
+    if (lane == 0) reinterpret_cast<uint16_t*>(sb + 16)[u] = (uint16_t)w8;
 }
 
 // Bound by instruction issue.  The pairs are taken kVoxRound at a time.  First a
@@ -575,7 +618,7 @@ __device__ __forceinline__ void block_masks(const uint32_t* blk, uint32_t* __res
 // 512 objects, 4096^3, 565k pairs in 18.4k blocks: 2350 -> 1520 us.
 constexpr uint32_t kVoxRound = 128;     // pairs set up at a time
 
-template <bool kMat>
+template <bool kMat, uint32_t kSlabs>
 __global__ void __launch_bounds__(32 * kWarpsPerVoxCta, 2) k_svo_voxelize(
     const tgx_object* __restrict__ objects, const uint32_t* __restrict__ cluster_pointers,
     const uint32_t* __restrict__ c2o, const uint32_t* __restrict__ bits, const SvoPair* __restrict__ sorted,
@@ -583,17 +626,19 @@ __global__ void __launch_bounds__(32 * kWarpsPerVoxCta, 2) k_svo_voxelize(
     uint32_t* __restrict__ pool, uint32_t* __restrict__ sub, uint32_t* __restrict__ nonempty,
     const uint8_t* __restrict__ material, uint16_t* __restrict__ mat_pool, float mnx, float mny, float mnz, uint32_t B)
 {
-    extern __shared__ __align__(16) uint32_t s_blk[];   // 1024 bit words, then 16384 words of u16 codes
+    constexpr uint32_t kLayers = 32u / kSlabs, kWords = kBlockWords / kSlabs;
+    extern __shared__ __align__(16) uint32_t s_blk[];   // the slab's bit words, then 16 words of u16 codes for each
     __shared__ PairRec s_rec[kVoxRound];
     __shared__ uint32_t s_cw[kWarpsPerVoxCta][16];       // each warp's current cluster bits
     __shared__ uint4 s_cm[kMat ? kWarpsPerVoxCta : 1][32];  // and its 512 material bytes
-    __shared__ uint32_t s_conf[kMat ? kBlockWords : 1];  // voxels more than one pair set
+    __shared__ uint32_t s_conf[kMat ? kWords : 1];       // voxels more than one pair set
     __shared__ uint8_t s_order[kVoxRound];               // per chunk of 32: the round's pairs, heaviest first (255: none)
     __shared__ uint32_t s_next;                          // the next entry of s_order to take
     uint32_t* img = s_blk;
-    uint16_t* smat = reinterpret_cast<uint16_t*>(s_blk + kBlockWords);
-    const uint32_t slot = slots[blockIdx.x];
-    const uint32_t pb = off[blockIdx.x], pe = pb + cnt[blockIdx.x];   // at least one pair
+    uint16_t* smat = reinterpret_cast<uint16_t*>(s_blk + kWords);
+    const uint32_t m = blockIdx.x / kSlabs, slab0 = (blockIdx.x % kSlabs) * kLayers;   // the slab's first layer
+    const uint32_t slot = slots[m];
+    const uint32_t pb = off[m], pe = pb + cnt[m];   // at least one pair
     const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
     bool again = false;                  // the pass over the doubly set voxels (the same in every thread)
     for (;;) {
@@ -608,7 +653,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerVoxCta, 2) k_svo_voxelize(
                 int32_t key = -1;
                 uint32_t idx = i;
                 if (i < np)
-                    key = (int32_t)pair_setup(objects, cluster_pointers, c2o, sorted[r0 + i], mnx, mny, mnz, B, &s_rec[i]);
+                    key = (int32_t)pair_setup(objects, cluster_pointers, c2o, sorted[r0 + i], mnx, mny, mnz, B, slab0, kLayers, &s_rec[i]);
                 // ascending bitonic sort over the warp's 32 lanes
 #pragma unroll
                 for (uint32_t k = 2; k <= 32; k <<= 1) {
@@ -624,11 +669,11 @@ __global__ void __launch_bounds__(32 * kWarpsPerVoxCta, 2) k_svo_voxelize(
                 // descending rank 31 - lane; pairs without voxels are left out
                 s_order[wid * 32u + (31u - lane)] = (uint8_t)(key > 0 ? idx : 255u);
             } else if (r0 == pb && !again) {   // the other warps clear the block
-                const uint32_t words = kBlockWords + (kMat ? 16384u : 0u), first = n_chunks * 32u;
+                const uint32_t words = kWords * (kMat ? 17u : 1u), first = n_chunks * 32u;
                 for (uint32_t k = threadIdx.x - first; k < words / 4u; k += blockDim.x - first)
                     reinterpret_cast<uint4*>(s_blk)[k] = make_uint4(0u, 0u, 0u, 0u);
                 if (kMat)
-                    for (uint32_t k = threadIdx.x - first; k < kBlockWords; k += blockDim.x - first) s_conf[k] = 0u;
+                    for (uint32_t k = threadIdx.x - first; k < kWords; k += blockDim.x - first) s_conf[k] = 0u;
             }
             if (threadIdx.x == 0) s_next = 0u;
             __syncthreads();
@@ -665,15 +710,16 @@ __global__ void __launch_bounds__(32 * kWarpsPerVoxCta, 2) k_svo_voxelize(
                 if (rm.w >> 31) {
                     // (again as well: it only takes maxima)
                     voxelize_any<kMat>(bc, x0, x1, y0, z0, ny, rows, rny, lut, cw, cm, mnx, mny, mnz, B,
-                                       sorted[r0 + k].block, img, s_blk + kBlockWords);
+                                       sorted[r0 + k].block, slab0 * 32u, kWords, img, s_blk + kWords);
                     continue;
                 }
                 for (uint32_t row = lane; row < rows; row += 32) {
                     const uint32_t q = (uint32_t)(((float)row + 0.5f) * rny);
                     const uint32_t iy = y0 + (row - q * ny), iz = z0 + q;
+                    const uint32_t word = (iz - slab0) * 32u + iy;   // the row's word of the image
                     uint32_t want = 0xffffffffu;
                     if (again) {
-                        want = s_conf[iz * 32u + iy];
+                        want = s_conf[word];
                         if (!want) continue;
                     }
                     // (i + 0.5) / 32 is an exact scaling: the reciprocal multiply gives the same bits
@@ -681,7 +727,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerVoxCta, 2) k_svo_voxelize(
                     row_ends(bc, xmul(xadd((float)iy, 0.5f), 0.03125f), xmul(xadd((float)iz, 0.5f), 0.03125f), p0, p1);
                     // tx = (ix + 0.5) / 32 is a multiple of 2^-6 below 1, so adding 1/32 per voxel is exact
                     float tx = xmul(xadd((float)x0, 0.5f), 0.03125f);
-                    uint16_t* const codes = smat + (iz * 32u + iy) * 32u;
+                    uint16_t* const codes = smat + word * 32u;
                     uint32_t mask = 0;
                     for (uint32_t ix = x0; ix < x1; ix++, tx = xadd(tx, 0.03125f)) {
                         const float omtx = xsub(1.0f, tx);
@@ -696,16 +742,15 @@ __global__ void __launch_bounds__(32 * kWarpsPerVoxCta, 2) k_svo_voxelize(
                             mask |= 1u << ix;
                             if (kMat) codes[ix] = (uint16_t)((lut | cm[rvi]) + 1u);
                         } else if ((want >> ix) & 1u) {
-                            smem_max_u16(s_blk + kBlockWords, (iz * 32u + iy) * 32u + ix,
-                                         ((lut | cm[rvi]) + 1u) & 0xffffu);
+                            smem_max_u16(s_blk + kWords, word * 32u + ix, ((lut | cm[rvi]) + 1u) & 0xffffu);
                         }
                     }
                     if (mask) {
                         if (kMat) {
-                            const uint32_t twice = atomicOr(&img[iz * 32u + iy], mask) & mask;
-                            if (twice) { atomicOr(&s_conf[iz * 32u + iy], twice); conflict = true; }
+                            const uint32_t twice = atomicOr(&img[word], mask) & mask;
+                            if (twice) { atomicOr(&s_conf[word], twice); conflict = true; }
                         } else {
-                            atomicOr(&img[iz * 32u + iy], mask);
+                            atomicOr(&img[word], mask);
                         }
                     }
                 }
@@ -713,19 +758,19 @@ __global__ void __launch_bounds__(32 * kWarpsPerVoxCta, 2) k_svo_voxelize(
         }
         if (!kMat || again || !__syncthreads_or(conflict)) break;
         // doubly set voxels: forget their codes, then take the maximum over the pairs
-        for (uint32_t w = wid; w < kBlockWords; w += kWarpsPerVoxCta)
+        for (uint32_t w = wid; w < kWords; w += kWarpsPerVoxCta)
             if ((s_conf[w] >> lane) & 1u) smat[w * 32u + lane] = 0u;
         again = true;
     }
     __syncthreads();
-    uint4* dst = reinterpret_cast<uint4*>(pool + (uint64_t)slot * kBlockWords);
-    for (uint32_t k = threadIdx.x; k < kBlockWords / 4u; k += blockDim.x) dst[k] = reinterpret_cast<const uint4*>(img)[k];
+    uint4* dst = reinterpret_cast<uint4*>(pool + (uint64_t)slot * kBlockWords + slab0 * 32u);
+    for (uint32_t k = threadIdx.x; k < kWords / 4u; k += blockDim.x) dst[k] = reinterpret_cast<const uint4*>(img)[k];
     if (kMat) {
-        uint4* md = reinterpret_cast<uint4*>(mat_pool + (uint64_t)slot * 32768u);
-        for (uint32_t k = threadIdx.x; k < 16384u / 4u; k += blockDim.x) md[k] = reinterpret_cast<const uint4*>(smat)[k];
+        uint4* md = reinterpret_cast<uint4*>(mat_pool + (uint64_t)slot * 32768u + slab0 * 1024u);
+        for (uint32_t k = threadIdx.x; k < kWords * 4u; k += blockDim.x) md[k] = reinterpret_cast<const uint4*>(smat)[k];
     }
-    // the block's occupancy masks, from the image while it is here
-    if (wid == kWarpsPerVoxCta - 1u) block_masks(img, sub + (uint64_t)slot * 32u, &nonempty[slot]);
+    // the occupancy masks of every 8 layers, from the image while it is here
+    if (wid < 4u / kSlabs) layer_masks(img + wid * 256u, slab0 / 8u + wid, sub + (uint64_t)slot * 32u, &nonempty[slot]);
 }
 
 // ---------------------------------------------------------------------------
@@ -740,9 +785,10 @@ __global__ void __launch_bounds__(256) k_svo_publish(uint32_t* __restrict__ tabl
     if (m < n) table[marked[m]] = slots[m] + 1u;
 }
 
-// One thread per slot: a slot whose block holds a voxel sets its bit on every
-// level.  The words are zero before; a bit is read first, because the coarse
-// levels' few words would otherwise take an atomic from every block.
+// One thread per slot: a slot whose block holds a voxel sets its bit level by
+// level up to the first one that is set already (whoever set that one goes on
+// to the coarser ones), so the few words of the coarse levels do not take an
+// atomic from every block.  The words are zero before.
 __global__ void __launch_bounds__(256) k_svo_pyramid(const uint32_t* __restrict__ slot_block, uint32_t n_slots,
                                                     const uint32_t* __restrict__ nonempty, uint32_t* occ,
                                                     const uint64_t* __restrict__ occ_off, uint32_t n_levels, uint32_t B,
@@ -760,7 +806,7 @@ __global__ void __launch_bounds__(256) k_svo_pyramid(const uint32_t* __restrict_
         const uint64_t idx = ((uint64_t)(bz >> s) * n + (by >> s)) * n + (bx >> s);
         uint32_t* w = &occ[occ_off[s] + (idx >> 5)];
         const uint32_t bit = 1u << (idx & 31u);
-        if (!(*(volatile uint32_t*)w & bit)) atomicOr(w, bit);
+        if ((*(volatile uint32_t*)w & bit) || (atomicOr(w, bit) & bit)) break;
     }
 }
 
@@ -937,23 +983,28 @@ static tgx_status svo_candidates(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc, co
         TGX_TRY(devbuf_reserve(c->svo_pairs, cap * kPairBytes));
         cap = c->svo_pairs.bytes / kPairBytes;   // svo_marked() places the list by the buffer's size
         TGX_CUDA(cudaMemsetAsync(counters + S_PAIRS, 0, 2 * 4, c->stream));   // pairs, marks
-        if (sc->n_cluster_pointers)
+        TGX_CUDA(cudaMemsetAsync(counters + S_CAND, 0, 4, c->stream));
+        if (sc->n_cluster_pointers) {
+            const uint32_t cap32 = (uint32_t)std::min<uint64_t>(cap, 0xffffffffu);
             TGX_LAUNCH(c, TR_SVO_CANDIDATES, (sc->n_cluster_pointers + 127) / 128, 128, 0, k_svo_candidates, sc->d_objects,
-                       sc->d_inv, sc->d_cp_obj, sc->n_cluster_pointers, s->mn[0], s->mn[1], s->mn[2], s->L, s->B,
-                       s->d_table, (SvoPair*)c->svo_pairs.ptr, svo_marked(c), (uint32_t)std::min<uint64_t>(cap, 0xffffffffu),
-                       counters, c->d_status, dirty);
+                       sc->d_cp_obj, sc->n_cluster_pointers, s->mn[0], s->mn[1], s->mn[2], s->B, (SvoPair*)c->svo_pairs.ptr,
+                       cap32, counters, c->d_status, dirty);
+            TGX_LAUNCH(c, TR_SVO_CANDIDATES, (uint32_t)c->num_sms * 16, 128, 0, k_svo_test_pairs, sc->d_objects, sc->d_inv,
+                       sc->d_cp_obj, s->mn[0], s->mn[1], s->mn[2], s->L, s->B, s->d_table, (SvoPair*)c->svo_pairs.ptr,
+                       svo_marked(c), cap32, counters);
+        }
         if (cudaMemcpyAsync(c->h_counter, counters, S_COUNT * 4, cudaMemcpyDeviceToHost, c->stream) != cudaSuccess ||
             cudaStreamSynchronize(c->stream) != cudaSuccess) {
             tgx_set_error("tgx_svo: %s", cudaGetErrorString(cudaGetLastError()));
             return TGX_ERR_CUDA;
         }
-        const uint32_t n_pairs = ((uint32_t*)c->h_counter)[S_PAIRS];
-        if (n_pairs <= cap) return TGX_OK;
+        const uint32_t n_cand = ((uint32_t*)c->h_counter)[S_CAND];
+        if (n_cand <= cap) return TGX_OK;
         // the capacity error recorded by the first attempt is expected; clear it and the marks it left
         TGX_CUDA(cudaMemsetAsync(c->d_status, 0, sizeof(tgx_dev_status), c->stream));
         const uint32_t grid = (uint32_t)std::min<uint64_t>((n_table + 255) / 256, (uint64_t)c->num_sms * 32);
         TGX_LAUNCH(c, TR_SVO_ALLOC, grid, 256, 0, k_svo_unmark, s->d_table, n_table);
-        cap = (uint64_t)n_pairs + 1024;
+        cap = (uint64_t)n_cand + 1024;
     }
     tgx_set_error("tgx_svo: pair count grew between two identical passes");
     return TGX_ERR_CAPACITY;
@@ -961,8 +1012,8 @@ static tgx_status svo_candidates(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc, co
 
 // Slots for the n_marked marked blocks, voxelisation of the pairs, and the
 // occupancy pyramid of all n_slots slots (cleared first).
-static tgx_status svo_fill(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc, uint32_t n_marked, uint32_t n_free,
-                           uint32_t next_slot, uint32_t n_slots)
+static tgx_status svo_fill(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc, uint32_t n_cand, uint32_t n_marked,
+                           uint32_t n_free, uint32_t next_slot, uint32_t n_slots)
 {
     uint32_t* counters = s->d_counters;
     const size_t sort_bytes = (size_t)n_marked * 4 * 4 + (size_t)s->n_pairs * sizeof(SvoPair) + 64;
@@ -976,27 +1027,34 @@ static tgx_status svo_fill(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc, uint32_t
         uint32_t *off = cnt + n_marked, *cursor = off + n_marked, *slots = cursor + n_marked;
         SvoPair* sorted = (SvoPair*)(((uintptr_t)(slots + n_marked) + 15) & ~(uintptr_t)15);
         const uint32_t mgrid = (n_marked + 255) / 256;
-        const uint32_t pgrid = (uint32_t)std::min<uint64_t>(((uint64_t)s->n_pairs + 255) / 256, (uint64_t)c->num_sms * 16);
+        const uint32_t pgrid = (uint32_t)std::min<uint64_t>(((uint64_t)n_cand + 255) / 256, (uint64_t)c->num_sms * 16);
         TGX_LAUNCH(c, TR_SVO_ALLOC, mgrid, 256, 0, k_svo_alloc, s->d_table, marked, n_marked, s->d_free, n_free, next_slot,
-                   slots, s->d_slot_block, cnt);
-        TGX_LAUNCH(c, TR_SVO_VOXELIZE, pgrid, 256, 0, k_svo_pair_count, (const SvoPair*)c->svo_pairs.ptr, s->n_pairs,
+                   slots, s->d_slot_block, s->d_nonempty, cnt);
+        TGX_LAUNCH(c, TR_SVO_VOXELIZE, pgrid, 256, 0, k_svo_pair_count, (const SvoPair*)c->svo_pairs.ptr, n_cand,
                    s->d_table, cnt);
         TGX_LAUNCH(c, TR_SVO_VOXELIZE, mgrid, 256, 0, k_svo_pair_ranges, cnt, n_marked, counters + S_SLOTS, off, cursor);
-        TGX_LAUNCH(c, TR_SVO_VOXELIZE, pgrid, 256, 0, k_svo_pair_fill, (const SvoPair*)c->svo_pairs.ptr, s->n_pairs,
+        TGX_LAUNCH(c, TR_SVO_VOXELIZE, pgrid, 256, 0, k_svo_pair_fill, (const SvoPair*)c->svo_pairs.ptr, n_cand,
                    s->d_table, cursor, sorted);
-        // one CTA per marked block: its image and material grid in shared memory
-        if (s->d_mat) {
-            TGX_CUDA(cudaFuncSetAttribute(k_svo_voxelize<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (kBlockWords + 16384) * 4));
-            TGX_LAUNCH(c, TR_SVO_VOXELIZE, n_marked, 32 * kWarpsPerVoxCta, (kBlockWords + 16384) * 4, k_svo_voxelize<true>,
-                       sc->d_objects, sc->d_cluster_pointers, sc->d_c2o, sc->d_bits, sorted, off, cnt, slots, s->d_pool,
-                       s->d_sub, s->d_nonempty, sc->d_material, s->d_mat, s->mn[0], s->mn[1], s->mn[2], s->B);
-        } else {
-            TGX_LAUNCH(c, TR_SVO_VOXELIZE, n_marked, 32 * kWarpsPerVoxCta, kBlockWords * 4, k_svo_voxelize<false>,
-                       sc->d_objects, sc->d_cluster_pointers, sc->d_c2o, sc->d_bits, sorted, off, cnt, slots, s->d_pool,
-                       s->d_sub, s->d_nonempty, (const uint8_t*)nullptr, (uint16_t*)nullptr, s->mn[0], s->mn[1], s->mn[2],
-                       s->B);
-        }
+        // one CTA per marked block, or four (8 layers each) when there are so few blocks
+        // that the heaviest ones (up to 190 pairs against 30 on average) would decide the
+        // time: 280 blocks of an update 222 -> SS us; 18.4k blocks take UU us whole and WW split
+        // (and only where every block's side is exactly 32, so that a voxel's index stays in its layers)
+        bool split = (uint64_t)n_marked < (uint64_t)c->num_sms * 16u;
+        for (int i = 0; i < 3; i++) split = split && fabsf(s->mn[i]) + (float)(1u << s->L) <= 16777216.0f;
+#define VOXELIZE(mat, slabs)                                                                                          \
+        do {                                                                                                          \
+            const uint32_t smem = kBlockWords / (slabs) * ((mat) ? 17u : 1u) * 4u;                                     \
+            TGX_CUDA(cudaFuncSetAttribute(k_svo_voxelize<mat, slabs>, cudaFuncAttributeMaxDynamicSharedMemorySize,     \
+                                          (int)smem));                                                                \
+            TGX_LAUNCH(c, TR_SVO_VOXELIZE, n_marked * (slabs), 32 * kWarpsPerVoxCta, smem, (k_svo_voxelize<mat, slabs>), \
+                       sc->d_objects, sc->d_cluster_pointers, sc->d_c2o, sc->d_bits, sorted, off, cnt, slots, s->d_pool, \
+                       s->d_sub, s->d_nonempty, sc->d_material, s->d_mat, s->mn[0], s->mn[1], s->mn[2], s->B);         \
+        } while (0)
+        if (s->d_mat && split) VOXELIZE(true, 4);
+        else if (s->d_mat) VOXELIZE(true, 1);
+        else if (split) VOXELIZE(false, 4);
+        else VOXELIZE(false, 1);
+#undef VOXELIZE
         TGX_LAUNCH(c, TR_SVO_PYRAMID, mgrid, 256, 0, k_svo_publish, s->d_table, marked, slots, n_marked);
     }
     if (n_slots)
@@ -1065,10 +1123,11 @@ extern "C" tgx_status tgx_svo_build_flags(tgx_ctx* c, const tgx_scene* sc, const
     const uint32_t* hc = (const uint32_t*)c->h_counter;
     s->n_pairs = hc[S_PAIRS];
     s->n_blocks = hc[S_MARKED];
+    const uint32_t n_cand = hc[S_CAND];
     s->n_slots = s->n_blocks;
     const bool materials = sc->d_material && sc->d_luts && !(flags & TGX_SVO_NO_MATERIALS);
     if ((st = svo_resize_slots(c, s, std::max(s->n_blocks, 1u), 0, materials)) != TGX_OK) return fail(st);
-    if ((st = svo_fill(c, s, sc, s->n_blocks, 0, 0, s->n_slots)) != TGX_OK) return fail(st);
+    if ((st = svo_fill(c, s, sc, n_cand, s->n_blocks, 0, 0, s->n_slots)) != TGX_OK) return fail(st);
     s->device_bytes = svo_device_bytes(s);
     *out = s;
     return TGX_OK;
@@ -1101,7 +1160,7 @@ extern "C" tgx_status tgx_svo_update(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc
     // pairs of the dirty blocks, into the pair storage the last build left (grown when short)
     TGX_TRY(svo_candidates(c, s, sc, dirty, std::max<uint64_t>(1024, c->svo_pairs.bytes / kPairBytes)));
     const uint32_t* hc = (const uint32_t*)c->h_counter;
-    const uint32_t n_moved = hc[S_MOVED], n_freed = hc[S_FREED], n_marked = hc[S_MARKED], hc_pairs = hc[S_PAIRS];
+    const uint32_t n_moved = hc[S_MOVED], n_freed = hc[S_FREED], n_marked = hc[S_MARKED], hc_pairs = hc[S_PAIRS], n_cand = hc[S_CAND];
     if (out_n_moved) *out_n_moved = n_moved;
     if (n_moved == 0) return TGX_OK;
     const uint32_t n_free = s->n_free + n_freed;
@@ -1110,7 +1169,7 @@ extern "C" tgx_status tgx_svo_update(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc
     tgx_status st = TGX_OK;
     if (need > s->pool_cap) st = svo_resize_slots(c, s, need + need / 4 + 64, s->n_slots, s->d_mat != nullptr);
     s->n_pairs = hc_pairs;
-    if (st == TGX_OK) st = svo_fill(c, s, sc, n_marked, n_free, s->n_slots, need);
+    if (st == TGX_OK) st = svo_fill(c, s, sc, n_cand, n_marked, n_free, s->n_slots, need);
     if (st != TGX_OK) {   // no mark stays in the table: a traversal would take it for a slot
         const uint32_t grid = (uint32_t)std::min<uint64_t>((n_table + 255) / 256, (uint64_t)c->num_sms * 32);
         TGX_LAUNCH(c, TR_SVO_ALLOC, grid, 256, 0, k_svo_unmark, s->d_table, n_table);
