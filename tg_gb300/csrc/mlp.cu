@@ -40,16 +40,15 @@ constexpr int NI = 9, NE = 216, NEP = 224, NH = 64, NO = 3;
 constexpr int OFF_W0 = 0, OFF_W1 = OFF_W0 + NH * NE, OFF_W2 = OFF_W1 + NH * NH, OFF_W3 = OFF_W2 + NH * NH,
               OFF_W4 = OFF_W3 + NH * NH, N_PARAMS = OFF_W4 + NO * NH;
 
-// BF16 weight image, row-major [out][in] per layer (row strides padded)
-constexpr int S0 = 232;   // W0  [64][S0]   k < 216 real
-constexpr int SH = 72;    // W1..W3 [64][SH]
-// offsets in bf16 elements inside the packed image
-constexpr int B_W0 = 0;
-constexpr int B_W1 = B_W0 + NH * S0;
-constexpr int B_W2 = B_W1 + NH * SH;
-constexpr int B_W3 = B_W2 + NH * SH;
-constexpr int B_W4 = B_W3 + NH * SH;         // [8][SH], rows >= 3 zero
-constexpr int B_TOTAL = B_W4 + 8 * SH;
+// BF16 weight image: every layer's [out][in] matrix as the tensor core reads it
+// from shared memory, 8 x 8 core matrices (8 outputs of 8 inputs, 128 bytes)
+// ordered [in / 8][out / 8], so that a CTA stages all layers with one bulk copy.
+// Offsets in BF16 elements; inputs 216..223 of layer 0 and outputs 3..15 of the
+// last layer are zero.
+constexpr int B_W0 = 0;                       // 28 x 8 core matrices
+constexpr int B_W1 = B_W0 + (NEP / 8) * 8 * 64;   // 8 x 8, three layers
+constexpr int B_W4 = B_W1 + 3 * 8 * 8 * 64;       // 8 x 2
+constexpr int B_TOTAL = B_W4 + 8 * 2 * 64;
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
 {
@@ -93,9 +92,10 @@ constexpr int A1 = A0;                                  //   [8 kg][16 mg][128 B
                                                         //   A0's first 16 KB: written only after layer 0's
                                                         //   MMAs completed, and A0 again only after layer 4's
 constexpr int GROUP_BYTES = KG0 * 16 * 128;
-constexpr int BAR = GROUP + NG * GROUP_BYTES;           // NG mbarriers, TMEM address
+constexpr int BAR = GROUP + NG * GROUP_BYTES;           // NG mbarriers, the weights' one, TMEM address
 constexpr int SMEM = BAR + 64;
 static_assert(SMEM <= 232448, "shared memory per CTA");
+static_assert(GROUP == B_TOTAL * 2, "the image is the weights' shared-memory layout");
 constexpr uint32_t TMEM_COLS = 256;                     // 64 per group, allocated as a power of two
 
 // instruction descriptor, kind::f16: D = F32, A = B = BF16, both K-major
@@ -165,27 +165,21 @@ __device__ __forceinline__ void put8(unsigned char* a, int kg, int row, const fl
     *reinterpret_cast<uint4*>(a + kg * (16 * 128) + (row >> 3) * 128 + (row & 7) * 16) = q;
 }
 
-// copies rows [0, n_rows) of a BF16 image matrix ([row][stride], K real columns
-// padded to kgs * 8) into the core-matrix layout [kg][row / 8][128 B]; rows up
-// to pad_rows are zero
-__device__ __forceinline__ void stage_weights(unsigned char* dst, const __nv_bfloat16* src, int stride, int n_rows,
-                                              int pad_rows, int kgs)
+// Starts the copy of the weight image into shared memory at dst, completing on
+// the mbarrier at bar (phase 0).  One thread.
+__device__ __forceinline__ void stage_weights(uint32_t dst, const __nv_bfloat16* wimg, uint32_t bar)
 {
-    const int ngs = pad_rows / 8;
-    for (int e = threadIdx.x; e < pad_rows * kgs; e += blockDim.x) {
-        const int row = e % pad_rows, kg = e / pad_rows;
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (row < n_rows) v = *reinterpret_cast<const uint4*>(src + (size_t)row * stride + kg * 8);
-        *reinterpret_cast<uint4*>(dst + kg * (ngs * 128) + (row >> 3) * 128 + (row & 7) * 16) = v;
-    }
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(B_TOTAL * 2) : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 :: "r"(dst), "l"(wimg), "r"(B_TOTAL * 2), "r"(bar) : "memory");
 }
 
-// The 24 features of one input (sin, cos of 2^k pi x for k = 0..11) into core
-// columns 3i .. 3i+2 of the A tile.  sincospif anchors octaves 0 and 6; the
-// others follow by angle doubling (sin 2a = 2 sin a cos a, cos 2a =
+// The 24 features of one input (sin, cos of 2^k pi x for k = 0..11): core columns
+// 3i .. 3i+2 of the A tile, 8 BF16 values each.  sincospif anchors octaves 0 and
+// 6; the others follow by angle doubling (sin 2a = 2 sin a cos a, cos 2a =
 // (cos a - sin a)(cos a + sin a)), whose error (a few ulp times 2^5) stays far
 // below the BF16 rounding of the features.
-__device__ __forceinline__ void encode_input(unsigned char* a, int i, int row, float x)
+__device__ __forceinline__ void features(float x, uint4 out[3])
 {
     float f[24];
 #pragma unroll
@@ -201,9 +195,23 @@ __device__ __forceinline__ void encode_input(unsigned char* a, int i, int row, f
             cv = c2;
         }
     }
-    put8(a, 3 * i + 0, row, f);
-    put8(a, 3 * i + 1, row, f + 8);
-    put8(a, 3 * i + 2, row, f + 16);
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+        const float* v = f + 8 * q;
+        out[q] = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+    }
+}
+__device__ __forceinline__ void put_features(unsigned char* a, int i, int row, const uint4 f[3])
+{
+#pragma unroll
+    for (int q = 0; q < 3; q++)
+        *reinterpret_cast<uint4*>(a + (3 * i + q) * (16 * 128) + (row >> 3) * 128 + (row & 7) * 16) = f[q];
+}
+__device__ __forceinline__ void encode_input(unsigned char* a, int i, int row, float x)
+{
+    uint4 f[3];
+    features(x, f);
+    put_features(a, i, row, f);
 }
 
 }  // namespace tc
@@ -218,22 +226,37 @@ __global__ void __launch_bounds__(tc::THREADS, 1) k_mlp_forward_tc(const __nv_bf
     const uint32_t tid = threadIdx.x, warp = tid >> 5;
     const uint32_t g = warp >> 2, gt = tid & 127u;         // group, thread (= tile row) in the group
     uint64_t* bars = reinterpret_cast<uint64_t*>(sm + BAR);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + BAR + 16);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + BAR + 32);
     unsigned char* ga = sm + GROUP + g * GROUP_BYTES;
+    const uint32_t wbar = saddr(&bars[NG]);
     if (n_dev) n = min(n, *n_dev);
-    stage_weights(sm + W0, wimg + B_W0, S0, NH, NH, KG0);
-    stage_weights(sm + W1 + 0 * KGH * 8 * 128, wimg + B_W1, SH, NH, NH, KGH);
-    stage_weights(sm + W1 + 1 * KGH * 8 * 128, wimg + B_W2, SH, NH, NH, KGH);
-    stage_weights(sm + W1 + 2 * KGH * 8 * 128, wimg + B_W3, SH, NH, NH, KGH);
-    stage_weights(sm + W4, wimg + B_W4, SH, 8, 16, KGH);
     if (tid == 0) {
-        for (int q = 0; q < NG; q++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(saddr(&bars[q])));
+        for (int q = 0; q <= NG; q++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(saddr(&bars[q])));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        stage_weights(saddr(sm), wimg, wbar);
     }
+    __syncwarp();
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      :: "r"(saddr(tmem_slot)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    // this thread's query of the group's first tile, then of its next one (loaded
+    // a tile ahead of its encoding, so its HBM latency hides behind a tile's layers)
+    const uint32_t tiles = (n + M - 1) / M, step = gridDim.x * NG;
+    uint32_t tile = blockIdx.x * NG + g;
+    float xn[NI];
+    auto load = [&](uint32_t t) {
+        const uint32_t row = t * M + gt;
+#pragma unroll
+        for (int i = 0; i < NI; i++) xn[i] = row < n ? __ldg(&x[(uint64_t)row * NI + i]) : 0.0f;
+    };
+    load(tile);
+    if (tile < tiles) {
+#pragma unroll
+        for (int i = 0; i < NI; i++) encode_input(ga + A0, i, (int)gt, xn[i]);
+        *reinterpret_cast<uint4*>(ga + A0 + (KG0 - 1) * (16 * 128) + (gt >> 3) * 128 + (gt & 7) * 16) = make_uint4(0, 0, 0, 0);   // features 216..223
+        load(tile + step);
     }
     fence_async_smem();
     fence_before();
@@ -243,85 +266,94 @@ __global__ void __launch_bounds__(tc::THREADS, 1) k_mlp_forward_tc(const __nv_bf
     const uint32_t lanes = tmem + (((warp & 3u) * 32u) << 16);           // this warp's 32 lanes
     const uint32_t b = saddr(&bars[g]);
     uint32_t phase = 0;
-    bool ok = true;
-    const uint32_t tiles = (n + M - 1) / M;
-    // this thread's query of the group's next tile, loaded one tile ahead so
-    // its HBM latency hides behind the current tile's layers
-    float xn[NI];
-    {
-        const uint32_t row = (blockIdx.x * NG + g) * M + gt;
-#pragma unroll
-        for (int i = 0; i < NI; i++) xn[i] = row < n ? __ldg(&x[(uint64_t)row * NI + i]) : 0.0f;
-    }
-    for (uint32_t tile = blockIdx.x * NG + g; tile < tiles && ok; tile += gridDim.x * NG) {
+    bool weights = false, ok = true;
+    // One tile per turn.  Its layer-0 tile is encoded when the turn begins.  While
+    // the tensor core works on a layer, the group's threads encode part of the next
+    // tile: inputs 3..8 straight into the columns of the layer-0 tile that the
+    // hidden layers' operand (its first 16 KB, columns 0..7) leaves free, inputs
+    // 0..2 into registers until the last layer has read that operand.
+    for (; tile < tiles; tile += step) {
         const uint32_t row = tile * M + gt;
-        float xc[NI];
-#pragma unroll
-        for (int i = 0; i < NI; i++) xc[i] = xn[i];
-        {
-            const uint32_t next = (tile + gridDim.x * NG) * M + gt;
-#pragma unroll
-            for (int i = 0; i < NI; i++) xn[i] = next < n ? __ldg(&x[(uint64_t)next * NI + i]) : 0.0f;
-        }
-#pragma unroll
-        for (int i = 0; i < NI; i++) encode_input(ga + A0, i, (int)gt, xc[i]);
-        {
-            const float z[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            put8(ga + A0, KG0 - 1, (int)gt, z);   // features 216..223
-        }
-        fence_async_smem();
-        fence_before();
-        group_sync(g);
-        // five layers; the hidden ones write the next A operand into A1
-        for (int l = 0; l < 5 && ok; l++) {
-            if (gt == 0) {
-                fence_after();
-                const int kgs = l == 0 ? KG0 : KGH;
-                const uint32_t a_base = saddr(ga + (l == 0 ? A0 : A1));
-                const uint32_t w_base = saddr(sm + (l == 0 ? W0 : l < 4 ? W1 + (l - 1) * KGH * 8 * 128 : W4));
-                const uint32_t n_out = l < 4 ? 64u : 16u;
-                const uint32_t w_sbo = 128, w_lbo = (n_out / 8) * 128;
-                for (int k = 0; k < kgs / 2; k++)
-                    mma(tmem, sdesc(a_base + 2 * k * (16 * 128), 16 * 128, 128),
-                        sdesc(w_base + 2 * k * w_lbo, w_lbo, w_sbo), idesc(n_out), k > 0);
-                commit(b);
+        const bool more = tile + step < tiles;   // the same in every thread of the group
+        uint4 hold[3][3];
+        auto issue = [&](int l) {
+            if (gt != 0) return;
+            if (!weights) {
+                if (!wait(wbar, 0u)) { dev_error(status, TGX_ERR_TIMEOUT, 45, tile); ok = false; }
+                weights = true;
             }
-            // every thread of the group waits; one that gives up stops the group
-            if (group_sync_or(g, !wait(b, phase))) {
-                if (gt == 0) dev_error(status, TGX_ERR_TIMEOUT, 40 + l, tile);
+            fence_after();
+            const int kgs = l == 0 ? KG0 : KGH;
+            const uint32_t a_base = saddr(ga + (l == 0 ? A0 : A1));
+            const uint32_t w_base = saddr(sm + (l == 0 ? W0 : l < 4 ? W1 + (l - 1) * KGH * 8 * 128 : W4));
+            const uint32_t n_out = l < 4 ? 64u : 16u;
+            const uint32_t w_sbo = 128, w_lbo = (n_out / 8) * 128;
+            for (int k = 0; k < kgs / 2; k++)
+                mma(tmem, sdesc(a_base + 2 * k * (16 * 128), 16 * 128, 128),
+                    sdesc(w_base + 2 * k * w_lbo, w_lbo, w_sbo), idesc(n_out), k > 0);
+            commit(b);
+        };
+#pragma unroll
+        for (int l = 0; l < 5; l++) {
+            issue(l);
+            if (more) {
+                if (l == 0) {
+#pragma unroll
+                    for (int i = 0; i < 3; i++) features(xn[i], hold[i]);
+                } else if (l == 1) {
+                    encode_input(ga + A0, 3, (int)gt, xn[3]);
+                    encode_input(ga + A0, 4, (int)gt, xn[4]);
+                } else if (l == 2) {
+                    encode_input(ga + A0, 5, (int)gt, xn[5]);
+                    encode_input(ga + A0, 6, (int)gt, xn[6]);
+                } else if (l == 3) {
+                    encode_input(ga + A0, 7, (int)gt, xn[7]);
+                } else {
+                    encode_input(ga + A0, 8, (int)gt, xn[8]);
+                    load(tile + 2 * step);
+                }
+            }
+            // a wait that gives up is noted; the group stops at the end of the tile
+            if (wait(b, phase)) {
+                phase ^= 1u;
+            } else {
+                dev_error(status, TGX_ERR_TIMEOUT, 40 + l, tile);
                 ok = false;
-                break;
             }
-            phase ^= 1u;
+            __syncwarp();
             fence_after();
             if (l < 4) {
                 // the 64 accumulator columns in one TMEM round trip
-                {
-                    float v[64];
+                float v[64];
 #pragma unroll
-                    for (int q = 0; q < 4; q++) ld16(lanes + q * 16, v + 16 * q);
-                    ld_wait();
+                for (int q = 0; q < 4; q++) ld16(lanes + q * 16, v + 16 * q);
+                ld_wait();
 #pragma unroll
-                    for (int j = 0; j < 64; j++) v[j] = fmaxf(v[j], 0.0f);
+                for (int j = 0; j < 64; j++) v[j] = fmaxf(v[j], 0.0f);
 #pragma unroll
-                    for (int q = 0; q < 8; q++) put8(ga + A1, q, (int)gt, v + 8 * q);
-                }
-                fence_async_smem();
+                for (int q = 0; q < 8; q++) put8(ga + A1, q, (int)gt, v + 8 * q);
             } else {
                 float v[16];
                 ld16(lanes, v);
                 ld_wait();
+                if (more) {
+#pragma unroll
+                    for (int i = 0; i < 3; i++) put_features(ga + A0, i, (int)gt, hold[i]);
+                }
                 if (row < n) {
                     y[(uint64_t)row * NO + 0] = v[0];
                     y[(uint64_t)row * NO + 1] = v[1];
                     y[(uint64_t)row * NO + 2] = v[2];
                 }
             }
+            fence_async_smem();
             fence_before();
-            group_sync(g);
+            if (l < 4) group_sync(g);
         }
+        if (group_sync_or(g, !ok)) break;   // the same in every thread of the group
     }
-    if (!ok) wait(b, phase);   // let MMAs still in flight land (bounded) before the columns are freed
+    if (!ok) wait(b, phase);      // let MMAs still in flight land (bounded) before the columns are freed
+    if (tid == 0) wait(wbar, 0u); // no copy lands after the CTA is gone
     fence_before();
     __syncthreads();
     fence_after();
@@ -364,6 +396,7 @@ constexpr int CS = 2;                                 // threads per sample (col
 constexpr int CW = 64 / CS;                           // accumulator columns per thread
 constexpr int THREADS = 128 * CS;
 static_assert(CW % 16 == 0 && CW <= 32, "column parts");
+static_assert(KG0 * 8 * 128 == B_W1 * 2 && (KG0 + 3 * KGH) * 8 * 128 == B_W4 * 2, "the image is the weights' shared-memory layout");
 constexpr int W0 = 0;                                 // [28 kg][8 ng][128 B]
 constexpr int W1 = W0 + KG0 * 8 * 128;                // [8 kg][8 ng][128 B] x 3 (W1, W2, W3)
 constexpr int W4 = W1 + 3 * KGH * 8 * 128;            // [8 kg][2 ng][128 B] (16 rows, 3 real)
@@ -372,7 +405,7 @@ constexpr int H = X0 + KG0 * 16 * 128;                // h1..h4: [8 kg][16 mg][1
 constexpr int TILE64 = KGH * 16 * 128;
 constexpr int DA = H + 4 * TILE64;                    // delta tiles (dy uses the first 2 kg of DB)
 constexpr int DB = DA + TILE64;
-constexpr int BAR = DB + TILE64;                      // mbarrier, TMEM address
+constexpr int BAR = DB + TILE64;                      // the MMAs' and the weights' mbarriers, TMEM address
 constexpr int SMEM = BAR + 64;
 // gradient reads of M = 128 rows run 16 column groups past a tile's base
 static_assert(X0 + 32 * 16 * 128 <= SMEM && H + 3 * TILE64 + 16 * 16 * 128 <= SMEM, "gradient operand over-read");
@@ -428,15 +461,13 @@ __global__ void __launch_bounds__(tt::THREADS, 1) k_mlp_train_tc(TrainJobs jobs,
     float* warp_loss = reinterpret_cast<float*>(sm + tt::BAR + 32);   // the 4 sample warps' loss sums
     pdl_wait();      // the weight image and the batch come from earlier kernels of the stream
     pdl_trigger();
-    stage_weights(sm + tt::W0, wimg + B_W0, S0, NH, NH, KG0);
-    stage_weights(sm + tt::W1 + 0 * KGH * 8 * 128, wimg + B_W1, SH, NH, NH, KGH);
-    stage_weights(sm + tt::W1 + 1 * KGH * 8 * 128, wimg + B_W2, SH, NH, NH, KGH);
-    stage_weights(sm + tt::W1 + 2 * KGH * 8 * 128, wimg + B_W3, SH, NH, NH, KGH);
-    stage_weights(sm + tt::W4, wimg + B_W4, SH, 8, 16, KGH);
     if (t == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(saddr(bar)));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(saddr(bar + 1)));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        stage_weights(saddr(sm), wimg, saddr(bar + 1));
     }
+    __syncwarp();
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      :: "r"(saddr(tmem_slot)), "r"(tt::TMEM_COLS) : "memory");
@@ -490,6 +521,7 @@ __global__ void __launch_bounds__(tt::THREADS, 1) k_mlp_train_tc(TrainJobs jobs,
         for (int l = 0; l < 5 && ok; l++) {
             publish();
             if (t == 0) {
+                if (l == 0 && tile == cta && !wait(saddr(bar + 1), 0u)) dev_error(status, TGX_ERR_TIMEOUT, 55, tile);
                 fence_after();
                 if (l == 0) {
                     for (int k = 0; k < KG0 / 2; k++)
@@ -633,6 +665,7 @@ __global__ void __launch_bounds__(tt::THREADS, 1) k_mlp_train_tc(TrainJobs jobs,
     for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
     if ((t & 31) == 0 && part == 0) warp_loss[warp] = lsum;
     if (!ok) wait(b, phase);   // let MMAs still in flight land (bounded) before the columns are freed
+    if (t == 0) wait(saddr(bar + 1), 0u);   // no copy lands after the CTA is gone
     fence_before();
     __syncthreads();
     fence_after();
@@ -695,16 +728,15 @@ __global__ void __launch_bounds__(256) k_mlp_reduce(const float* __restrict__ pa
     g[p] += sum_slices(partial, n_parts, p);
 }
 
-// bf16 image position of master parameter p
+// BF16 image position of master parameter p
 __device__ __forceinline__ int image_pos(int p)
 {
-    if (p < OFF_W1) return B_W0 + (p / NE) * S0 + p % NE;
-    if (p < OFF_W4) {
-        const int l = (p - OFF_W1) / (NH * NH), r = (p - OFF_W1) % (NH * NH);
-        return B_W1 + l * NH * SH + (r / NH) * SH + r % NH;
-    }
-    const int r = p - OFF_W4;
-    return B_W4 + (r / NH) * SH + r % NH;
+    const bool first = p < OFF_W1, last = p >= OFF_W4;
+    const int l = (p - OFF_W1) / (NH * NH);
+    const int r = first ? p : last ? p - OFF_W4 : (p - OFF_W1) % (NH * NH);
+    const int out = r / (first ? NE : NH), in = r % (first ? NE : NH);
+    const int base = first ? B_W0 : last ? B_W4 : B_W1 + l * (8 * 8 * 64);
+    return base + (in / 8) * (last ? 2 * 64 : 8 * 64) + (out / 8) * 64 + (out % 8) * 8 + in % 8;
 }
 
 // Adam for up to two networks (blockIdx.y).  The gradient is g plus the
