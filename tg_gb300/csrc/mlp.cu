@@ -59,14 +59,20 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
 // Inference on the 5th-generation tensor cores (tcgen05, accumulators in TMEM)
 // ---------------------------------------------------------------------------
 //
-// A CTA of 384 threads holds three independent groups of 4 warps that share
-// the weights in shared memory.  Each group works through tiles of 128 queries:
-// thread t of the group owns query t of its tile, which is row t of every
-// GEMM and TMEM lane t.  While one group waits for its MMAs the others encode
-// or drain their accumulators, so the tensor core and the CUDA cores overlap.
-// A group's layer-0 feature tile (56 KB) also holds, in its first 16 KB, the
-// A operand of layers 1-4, which is written only once layer 0's MMAs have
-// completed; that is what leaves room for a third group.
+// A CTA of 768 threads holds six independent groups of 4 warps that share the
+// weights in shared memory.  Each group works through tiles of 128 queries:
+// thread t of the group owns query t of its tile, which is row t of every GEMM
+// and TMEM lane t.  While one group waits for its MMAs the others encode or
+// drain their accumulators, so the tensor core and the CUDA cores overlap.
+// The kernel is bound by the CUDA cores' issue (about 1,800 instructions per 32
+// queries, two thirds of them the encoding), so what counts is having enough
+// warps to fill it.  The features of a tile are made in two halves of 14 core
+// columns, the second accumulating onto the first, so that a group needs 28 KB
+// of operands instead of 56 and six fit; the operand of layers 1-4 takes the
+// same place.
+// 2^20 queries: 137 us with three groups and the features whole, 123 with the
+// next tile's encoding moved behind the MMAs, 96 with five groups in this form,
+// 89 with ReLU on packed values, 82 with six.
 // Operands use the canonical no-swizzle K-major layout: 8 x 8 BF16 core
 // matrices (8 rows of 16 contiguous bytes), K-adjacent core matrices LBO
 // bytes apart and row-group-adjacent ones SBO bytes apart.  Per layer one
@@ -80,23 +86,21 @@ namespace tc {
 constexpr int M = 128;                      // queries per tile
 constexpr int KG0 = NEP / 8;                // 28 K core-matrix columns of layer 0
 constexpr int KGH = NH / 8;                 // 8 of the hidden layers
-constexpr int NG = 3;                       // query groups per CTA
-constexpr int THREADS = 128 * NG;           // three groups of 128
+constexpr int KGF = KG0 / 2;                // core columns of a feature half
+constexpr int NG = 6;                       // query groups per CTA
+constexpr int THREADS = 128 * NG;
 // byte offsets in dynamic shared memory (all 1024-aligned)
 constexpr int W0 = 0;                                   // [28 kg][8 ng][128 B]
 constexpr int W1 = W0 + KG0 * 8 * 128;                  // [8 kg][8 ng][128 B] x 3
 constexpr int W4 = W1 + 3 * KGH * 8 * 128;              // [8 kg][2 ng][128 B] (16 rows, 3 real)
-constexpr int GROUP = W4 + KGH * 2 * 128;               // per group:
-constexpr int A0 = 0;                                   //   [28 kg][16 mg][128 B] layer 0's A operand
-constexpr int A1 = A0;                                  //   [8 kg][16 mg][128 B] layers 1-4's A operand, in
-                                                        //   A0's first 16 KB: written only after layer 0's
-                                                        //   MMAs completed, and A0 again only after layer 4's
-constexpr int GROUP_BYTES = KG0 * 16 * 128;
+constexpr int GROUP = W4 + KGH * 2 * 128;               // per group: [14 kg][16 mg][128 B], half of layer 0's A operand,
+                                                        //   then (first 8 kg) that of layers 1-4
+constexpr int GROUP_BYTES = KGF * 16 * 128;
 constexpr int BAR = GROUP + NG * GROUP_BYTES;           // NG mbarriers, the weights' one, TMEM address
 constexpr int SMEM = BAR + 64;
 static_assert(SMEM <= 232448, "shared memory per CTA");
 static_assert(GROUP == B_TOTAL * 2, "the image is the weights' shared-memory layout");
-constexpr uint32_t TMEM_COLS = 256;                     // 64 per group, allocated as a power of two
+constexpr uint32_t TMEM_COLS = 512;                     // 64 per group, allocated as a power of two
 
 // instruction descriptor, kind::f16: D = F32, A = B = BF16, both K-major
 __host__ __device__ constexpr uint32_t idesc(uint32_t n)
@@ -132,7 +136,7 @@ __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::be
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// barrier of the 128 threads of one group (ids 1 and 2)
+// barrier of the 128 threads of one group (ids 1 .. NG)
 __device__ __forceinline__ void group_sync(uint32_t g) { asm volatile("bar.sync %0, 128;" :: "r"(g + 1u) : "memory"); }
 // the same barrier, returning whether any thread of the group passed pred = true
 __device__ __forceinline__ bool group_sync_or(uint32_t g, bool pred)
@@ -156,13 +160,29 @@ __device__ __forceinline__ void ld16(uint32_t taddr, float* v)
 }
 __device__ __forceinline__ void ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// row `row` of an A tile: the 8 BF16 values of core-matrix column kg
+// row `row` of an A tile: core-matrix column kg
+__device__ __forceinline__ void put_column(unsigned char* a, int kg, int row, uint4 q)
+{
+    *reinterpret_cast<uint4*>(a + kg * (16 * 128) + (row >> 3) * 128 + (row & 7) * 16) = q;
+}
+// ... its 8 BF16 values
 __device__ __forceinline__ void put8(unsigned char* a, int kg, int row, const float* v)
 {
     uint4 q;
     q.x = pack_bf16(v[0], v[1]); q.y = pack_bf16(v[2], v[3]);
     q.z = pack_bf16(v[4], v[5]); q.w = pack_bf16(v[6], v[7]);
-    *reinterpret_cast<uint4*>(a + kg * (16 * 128) + (row >> 3) * 128 + (row & 7) * 16) = q;
+    put_column(a, kg, row, q);
+}
+
+// ... with ReLU after the rounding, two values at a time: rounding keeps the order
+// of numbers and zero, and the maximum of NaN and 0 is 0 in both forms
+__device__ __forceinline__ void put8_relu(unsigned char* a, int kg, int row, const float* v)
+{
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        asm("max.bf16x2 %0, %1, %2;" : "=r"(w[i]) : "r"(pack_bf16(v[2 * i], v[2 * i + 1])), "r"(0u));
+    put_column(a, kg, row, make_uint4(w[0], w[1], w[2], w[3]));
 }
 
 // Starts the copy of the weight image into shared memory at dst, completing on
@@ -201,17 +221,13 @@ __device__ __forceinline__ void features(float x, uint4 out[3])
         out[q] = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
     }
 }
-__device__ __forceinline__ void put_features(unsigned char* a, int i, int row, const uint4 f[3])
-{
-#pragma unroll
-    for (int q = 0; q < 3; q++)
-        *reinterpret_cast<uint4*>(a + (3 * i + q) * (16 * 128) + (row >> 3) * 128 + (row & 7) * 16) = f[q];
-}
+// ... of input i into an A tile that holds all 28 columns
 __device__ __forceinline__ void encode_input(unsigned char* a, int i, int row, float x)
 {
     uint4 f[3];
     features(x, f);
-    put_features(a, i, row, f);
+#pragma unroll
+    for (int q = 0; q < 3; q++) put_column(a, 3 * i + q, row, f[q]);
 }
 
 }  // namespace tc
@@ -226,7 +242,7 @@ __global__ void __launch_bounds__(tc::THREADS, 1) k_mlp_forward_tc(const __nv_bf
     const uint32_t tid = threadIdx.x, warp = tid >> 5;
     const uint32_t g = warp >> 2, gt = tid & 127u;         // group, thread (= tile row) in the group
     uint64_t* bars = reinterpret_cast<uint64_t*>(sm + BAR);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + BAR + 32);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + BAR + 8 * (NG + 1));
     unsigned char* ga = sm + GROUP + g * GROUP_BYTES;
     const uint32_t wbar = saddr(&bars[NG]);
     if (n_dev) n = min(n, *n_dev);
@@ -241,24 +257,16 @@ __global__ void __launch_bounds__(tc::THREADS, 1) k_mlp_forward_tc(const __nv_bf
                      :: "r"(saddr(tmem_slot)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    // this thread's query of the group's first tile, then of its next one (loaded
-    // a tile ahead of its encoding, so its HBM latency hides behind a tile's layers)
+    // this thread's query of the group's current tile, and its next one, loaded a tile ahead
     const uint32_t tiles = (n + M - 1) / M, step = gridDim.x * NG;
-    uint32_t tile = blockIdx.x * NG + g;
-    float xn[NI];
+    uint32_t tile = g * gridDim.x + blockIdx.x;   // few tiles spread over the CTAs first
+    float xc[NI], xn[NI];
     auto load = [&](uint32_t t) {
         const uint32_t row = t * M + gt;
 #pragma unroll
         for (int i = 0; i < NI; i++) xn[i] = row < n ? __ldg(&x[(uint64_t)row * NI + i]) : 0.0f;
     };
     load(tile);
-    if (tile < tiles) {
-#pragma unroll
-        for (int i = 0; i < NI; i++) encode_input(ga + A0, i, (int)gt, xn[i]);
-        *reinterpret_cast<uint4*>(ga + A0 + (KG0 - 1) * (16 * 128) + (gt >> 3) * 128 + (gt & 7) * 16) = make_uint4(0, 0, 0, 0);   // features 216..223
-        load(tile + step);
-    }
-    fence_async_smem();
     fence_before();
     __syncthreads();
     fence_after();
@@ -267,89 +275,92 @@ __global__ void __launch_bounds__(tc::THREADS, 1) k_mlp_forward_tc(const __nv_bf
     const uint32_t b = saddr(&bars[g]);
     uint32_t phase = 0;
     bool weights = false, ok = true;
-    // One tile per turn.  Its layer-0 tile is encoded when the turn begins.  While
-    // the tensor core works on a layer, the group's threads encode part of the next
-    // tile: inputs 3..8 straight into the columns of the layer-0 tile that the
-    // hidden layers' operand (its first 16 KB, columns 0..7) leaves free, inputs
-    // 0..2 into registers until the last layer has read that operand.
+    // the MMAs of operand columns 0 .. kgs - 1 against the weight columns from w_off on
+    auto issue = [&](int kgs, int w_off, uint32_t n_out, bool accumulate) {
+        if (gt != 0) return;
+        if (!weights) {
+            if (!wait(wbar, 0u)) { dev_error(status, TGX_ERR_TIMEOUT, 45, tile); ok = false; }
+            weights = true;
+        }
+        fence_after();
+        const uint32_t a_base = saddr(ga), w_base = saddr(sm + w_off);
+        const uint32_t w_lbo = (n_out / 8) * 128;
+        for (int k = 0; k < kgs / 2; k++)
+            mma(tmem, sdesc(a_base + 2 * k * (16 * 128), 16 * 128, 128), sdesc(w_base + 2 * k * w_lbo, w_lbo, 128),
+                idesc(n_out), accumulate || k > 0);
+        commit(b);
+    };
+    // a wait that gives up is noted; the group stops at the end of the tile
+    auto finish = [&](int where) {
+        if (wait(b, phase)) {
+            phase ^= 1u;
+        } else {
+            dev_error(status, TGX_ERR_TIMEOUT, where, tile);
+            ok = false;
+        }
+        __syncwarp();
+        fence_after();
+    };
+    auto publish = [&]() {   // this thread's operand rows, visible to the tensor core
+        fence_async_smem();
+        fence_before();
+        group_sync(g);
+    };
     for (; tile < tiles; tile += step) {
         const uint32_t row = tile * M + gt;
-        const bool more = tile + step < tiles;   // the same in every thread of the group
-        uint4 hold[3][3];
-        auto issue = [&](int l) {
-            if (gt != 0) return;
-            if (!weights) {
-                if (!wait(wbar, 0u)) { dev_error(status, TGX_ERR_TIMEOUT, 45, tile); ok = false; }
-                weights = true;
-            }
-            fence_after();
-            const int kgs = l == 0 ? KG0 : KGH;
-            const uint32_t a_base = saddr(ga + (l == 0 ? A0 : A1));
-            const uint32_t w_base = saddr(sm + (l == 0 ? W0 : l < 4 ? W1 + (l - 1) * KGH * 8 * 128 : W4));
-            const uint32_t n_out = l < 4 ? 64u : 16u;
-            const uint32_t w_sbo = 128, w_lbo = (n_out / 8) * 128;
-            for (int k = 0; k < kgs / 2; k++)
-                mma(tmem, sdesc(a_base + 2 * k * (16 * 128), 16 * 128, 128),
-                    sdesc(w_base + 2 * k * w_lbo, w_lbo, w_sbo), idesc(n_out), k > 0);
-            commit(b);
-        };
 #pragma unroll
-        for (int l = 0; l < 5; l++) {
-            issue(l);
-            if (more) {
-                if (l == 0) {
+        for (int i = 0; i < NI; i++) xc[i] = xn[i];
+        load(tile + step);
+        // layer 0, columns 0..13: inputs 0..3 and two thirds of input 4
+        uint4 f[3];
 #pragma unroll
-                    for (int i = 0; i < 3; i++) features(xn[i], hold[i]);
-                } else if (l == 1) {
-                    encode_input(ga + A0, 3, (int)gt, xn[3]);
-                    encode_input(ga + A0, 4, (int)gt, xn[4]);
-                } else if (l == 2) {
-                    encode_input(ga + A0, 5, (int)gt, xn[5]);
-                    encode_input(ga + A0, 6, (int)gt, xn[6]);
-                } else if (l == 3) {
-                    encode_input(ga + A0, 7, (int)gt, xn[7]);
-                } else {
-                    encode_input(ga + A0, 8, (int)gt, xn[8]);
-                    load(tile + 2 * step);
-                }
-            }
-            // a wait that gives up is noted; the group stops at the end of the tile
-            if (wait(b, phase)) {
-                phase ^= 1u;
-            } else {
-                dev_error(status, TGX_ERR_TIMEOUT, 40 + l, tile);
-                ok = false;
-            }
-            __syncwarp();
-            fence_after();
-            if (l < 4) {
-                // the 64 accumulator columns in one TMEM round trip
-                float v[64];
+        for (int i = 0; i < 5; i++) {
+            features(xc[i], f);
 #pragma unroll
-                for (int q = 0; q < 4; q++) ld16(lanes + q * 16, v + 16 * q);
-                ld_wait();
-#pragma unroll
-                for (int j = 0; j < 64; j++) v[j] = fmaxf(v[j], 0.0f);
-#pragma unroll
-                for (int q = 0; q < 8; q++) put8(ga + A1, q, (int)gt, v + 8 * q);
-            } else {
-                float v[16];
-                ld16(lanes, v);
-                ld_wait();
-                if (more) {
-#pragma unroll
-                    for (int i = 0; i < 3; i++) put_features(ga + A0, i, (int)gt, hold[i]);
-                }
-                if (row < n) {
-                    y[(uint64_t)row * NO + 0] = v[0];
-                    y[(uint64_t)row * NO + 1] = v[1];
-                    y[(uint64_t)row * NO + 2] = v[2];
-                }
-            }
-            fence_async_smem();
-            fence_before();
-            if (l < 4) group_sync(g);
+            for (int q = 0; q < (i < 4 ? 3 : 2); q++) put_column(ga, 3 * i + q, (int)gt, f[q]);
         }
+        publish();
+        issue(KGF, W0, 64u, false);
+        // columns 14..27: the rest of input 4, inputs 5..8 and the zero column
+        const uint4 rest = f[2];
+        features(xc[5], f);
+        finish(40);
+        put_column(ga, 0, (int)gt, rest);
+#pragma unroll
+        for (int i = 5; i < 9; i++) {
+            if (i > 5) features(xc[i], f);
+#pragma unroll
+            for (int q = 0; q < 3; q++) put_column(ga, 3 * i + q - KGF, (int)gt, f[q]);
+        }
+        put_column(ga, KGF - 1, (int)gt, make_uint4(0u, 0u, 0u, 0u));
+        publish();
+        issue(KGF, W0 + KGF * 8 * 128, 64u, true);
+#pragma unroll
+        for (int l = 0; l < 4; l++) {
+            finish(40 + l);
+            // the 64 accumulator columns, 32 at a time, into the next layer's operand
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                float v[32];
+                ld16(lanes + h * 32, v);
+                ld16(lanes + h * 32 + 16, v + 16);
+                ld_wait();
+#pragma unroll
+                for (int q = 0; q < 4; q++) put8_relu(ga, 4 * h + q, (int)gt, v + 8 * q);
+            }
+            publish();
+            issue(KGH, l < 3 ? W1 + l * KGH * 8 * 128 : W4, l < 3 ? 64u : 16u, false);
+        }
+        finish(44);
+        float v[16];
+        ld16(lanes, v);
+        ld_wait();
+        if (row < n) {
+            y[(uint64_t)row * NO + 0] = v[0];
+            y[(uint64_t)row * NO + 1] = v[1];
+            y[(uint64_t)row * NO + 2] = v[2];
+        }
+        fence_before();
         if (group_sync_or(g, !ok)) break;   // the same in every thread of the group
     }
     if (!ok) wait(b, phase);      // let MMAs still in flight land (bounded) before the columns are freed
@@ -907,7 +918,7 @@ static tgx_status cache_forward(tgx_ctx* c, tgx_cache* k, const uint32_t* d_n, u
         attr = true;
     }
     const uint32_t tiles = (n + tc::M - 1) / tc::M;
-    const uint32_t grid = std::max(1u, std::min<uint32_t>((tiles + tc::NG - 1) / tc::NG, (uint32_t)c->num_sms));
+    const uint32_t grid = std::max(1u, std::min<uint32_t>(tiles, (uint32_t)c->num_sms));
     TGX_LAUNCH(c, TR_MLP, grid, tc::THREADS, tc::SMEM, k_mlp_forward_tc, k->img, n, d_n, d_x, d_rgb, c->d_status);
     return TGX_OK;
 }
