@@ -1035,7 +1035,7 @@ extern "C" tgx_status tgx_gi_render_cached(tgx_ctx* c, const tgx_scene* sc, cons
         uint32_t m = 0;
         if (per) { nets[m] = cache; ns[m] = per; xs[m] = tx + 9ull * per * k; ts[m] = tt + 3ull * per * k; m++; }
         if (pper) { nets[m] = pnet; ns[m] = pper; xs[m] = ptx + 9ull * pper * k; ts[m] = ptt + 3ull * pper * k; m++; }
-        TGX_TRY(cache_train_pair(c, nets, ns, xs, ts, m, cp->lr));
+        TGX_TRY(cache_train_pair(c, nets, ns, xs, ts, m, cp->lr, k > 0));
     }
     return TGX_OK;
 }

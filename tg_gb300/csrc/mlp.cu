@@ -449,6 +449,7 @@ struct TrainJob
 struct TrainJobs
 {
     TrainJob j[2];
+    uint32_t batch_ready;        // the batches were written before the kernel this launch depends on even started
 };
 
 __global__ void __launch_bounds__(tt::THREADS, 1) k_mlp_train_tc(TrainJobs jobs, tgx_dev_status* __restrict__ status)
@@ -470,7 +471,22 @@ __global__ void __launch_bounds__(tt::THREADS, 1) k_mlp_train_tc(TrainJobs jobs,
     uint64_t* bar = reinterpret_cast<uint64_t*>(sm + tt::BAR);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + tt::BAR + 16);
     float* warp_loss = reinterpret_cast<float*>(sm + tt::BAR + 32);   // the 4 sample warps' loss sums
-    pdl_wait();      // the weight image and the batch come from earlier kernels of the stream
+    // The first tile's features, before or after the wait for the kernel before:
+    // the batch comes from an earlier kernel of the stream, the weight image from
+    // the one before (Adam) or an earlier one.  Read from L2: an L1 line could be
+    // older than the batch when this runs before the wait.
+    auto encode_tile = [&](uint32_t tile) {
+        const uint32_t row = tile * 128 + r;
+        for (int i = (int)part; i < NI; i += tt::CS)
+            encode_input(sm + tt::X0, i, (int)r, row < n ? __ldcg(&x[(uint64_t)row * NI + i]) : 0.0f);
+        if (part == tt::CS - 1) {
+            const float z[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+            put8(sm + tt::X0, KG0 - 1, (int)r, z);   // features 216..223
+        }
+    };
+    const uint32_t tiles = (n + 127) / 128;
+    if (jobs.batch_ready && cta < tiles) encode_tile(cta);
+    pdl_wait();
     pdl_trigger();
     if (t == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(saddr(bar)));
@@ -498,7 +514,6 @@ __global__ void __launch_bounds__(tt::THREADS, 1) k_mlp_train_tc(TrainJobs jobs,
     bool ok = true;
     const float inv = 1.0f / (3.0f * (float)n);
     float lsum = 0.0f;
-    const uint32_t tiles = (n + 127) / 128;
     uint32_t acc_g = 0;   // gradient accumulators hold a previous tile's sums
     // all threads wait for the MMAs of one commit; any thread that gives up stops the CTA
     auto sync_mma = [&](int where, uint32_t tile) -> bool {
@@ -511,6 +526,36 @@ __global__ void __launch_bounds__(tt::THREADS, 1) k_mlp_train_tc(TrainJobs jobs,
         fence_after();
         return true;
     };
+    // layer l's gradient sums into this CTA's slice of the partial buffer (zeros
+    // without `sums`): dW_l^T, row = layer input = TMEM lane, a thread's columns
+    // in one TMEM round trip
+    float* const P = partial + (uint64_t)cta * N_PARAMS;
+    auto write_block = [&](uint32_t col, int off, int i, int ni, bool sums) {
+        float v[CW];
+#pragma unroll
+        for (int q = 0; q < CW / 16; q++) ld16(lanes + col + cols + q * 16, v + 16 * q);
+        ld_wait();
+        if (i < ni) {
+#pragma unroll
+            for (int j = 0; j < CW; j++) P[off + ((int)cols + j) * ni + i] = sums ? v[j] : 0.0f;
+        }
+    };
+    auto write_gradient = [&](int l, bool sums) {
+        if (l == 0) {
+            write_block(tt::G0A, OFF_W0, (int)r, NE, sums);
+            write_block(tt::G0B, OFF_W0, 128 + (int)r, NE, sums);
+        } else if (l < 4) {
+            write_block(l == 1 ? tt::G1 : l == 2 ? tt::G2 : tt::G3, l == 1 ? OFF_W1 : l == 2 ? OFF_W2 : OFF_W3, (int)r, NH, sums);
+        } else if (part == 0) {   // dW4^T: 3 real columns
+            float v[16];
+            ld16(lanes + tt::G4, v);
+            ld_wait();
+            if (r < NH) {
+#pragma unroll
+                for (int j = 0; j < NO; j++) P[OFF_W4 + j * NH + (int)r] = sums ? v[j] : 0.0f;
+            }
+        }
+    };
     auto publish = [&]() {   // this thread's shared-memory writes, visible to the tensor core
         fence_async_smem();
         fence_before();
@@ -519,12 +564,8 @@ __global__ void __launch_bounds__(tt::THREADS, 1) k_mlp_train_tc(TrainJobs jobs,
     for (uint32_t tile = cta; tile < tiles && ok; tile += n_ctas) {
         const uint32_t row = tile * 128 + r;
         const bool valid = row < n;
-        for (int i = (int)part; i < NI; i += tt::CS)
-            encode_input(sm + tt::X0, i, (int)r, valid ? x[(uint64_t)row * NI + i] : 0.0f);
-        if (part == tt::CS - 1) {
-            const float z[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            put8(sm + tt::X0, KG0 - 1, (int)r, z);   // features 216..223
-        }
+        const bool last = tile + n_ctas >= tiles;    // the gradient sums are final after this tile
+        if (tile != cta || !jobs.batch_ready) encode_tile(tile);
         // ---- forward ----
         uint32_t mask[4];   // relu'(z) of the thread's columns per hidden layer
         float y[3] = {0.0f, 0.0f, 0.0f};
@@ -623,6 +664,9 @@ __global__ void __launch_bounds__(tt::THREADS, 1) k_mlp_train_tc(TrainJobs jobs,
                             sdesc(din + 2 * k * 128, 128, 2048), tt::idesc_t(nout, true, true), (acc_g | k) ? 1u : 0u);
                 commit(b);
             }
+            // the sums of the stage before are final on the last tile: they go out behind this stage's MMAs
+            __syncwarp();
+            if (last && s > 0) write_gradient(5 - s, true);
             if (!(ok = sync_mma(60 + s, tile))) break;
             if (s == 4) break;
             // mask with relu'(z) of the layer's input and store the next delta into the other tile
@@ -639,39 +683,14 @@ __global__ void __launch_bounds__(tt::THREADS, 1) k_mlp_train_tc(TrainJobs jobs,
         }
         acc_g = 1u;
     }
-    // ---- this CTA's gradient sums into its slice of the partial buffer ----
     fence_before();
     __syncthreads();
     fence_after();
-    float* P = partial + (uint64_t)cta * N_PARAMS;
-    {
-#pragma unroll 1
-        for (int blk = 0; blk < 5; blk++) {
-            const uint32_t col = blk == 0 ? tt::G0A : blk == 1 ? tt::G0B : blk == 2 ? tt::G1 : blk == 3 ? tt::G2 : tt::G3;
-            const int i = (blk == 1 ? 128 : 0) + (int)r;                  // layer input (TMEM row)
-            const int ni = blk < 2 ? NE : NH;
-            const int off = blk < 2 ? OFF_W0 : blk == 2 ? OFF_W1 : blk == 3 ? OFF_W2 : OFF_W3;
-            // the thread's columns of the block in one TMEM round trip
-            float v[CW];
-#pragma unroll
-            for (int q = 0; q < CW / 16; q++) ld16(lanes + col + cols + q * 16, v + 16 * q);
-            ld_wait();
-            if (i < ni) {
-#pragma unroll
-                for (int j = 0; j < CW; j++) P[off + ((int)cols + j) * ni + i] = ok && acc_g ? v[j] : 0.0f;
-            }
-        }
-        if (part == 0) {   // dW4^T: 3 real columns
-            float v[16];
-            ld16(lanes + tt::G4, v);
-            ld_wait();
-            const int i = (int)r;
-            if (i < NH) {
-#pragma unroll
-                for (int j = 0; j < NO; j++) P[OFF_W4 + j * NH + i] = ok && acc_g ? v[j] : 0.0f;
-            }
-        }
-    }
+    // layer 0's sums (written after the last tile's last MMAs), and all of them
+    // where no tile was finished
+    if (!ok || !acc_g)
+        for (int l = 4; l > 0; l--) write_gradient(l, false);
+    write_gradient(0, ok && acc_g);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
     if ((t & 31) == 0 && part == 0) warp_loss[warp] = lsum;
@@ -720,13 +739,23 @@ __device__ __forceinline__ float sum_slices(const float* __restrict__ partial, u
     return s + tail;
 }
 
-// The CTAs' losses (after the n_parts gradient slices), added in CTA order.
-__device__ __forceinline__ float sum_losses(const float* __restrict__ partial, uint32_t n_parts)
+// The CTAs' losses (after the n_parts <= 1024 gradient slices), added in CTA
+// order by the last warp of the grid's last CTA, which has no parameters: loaded
+// side by side, then added from shared memory.
+static_assert(N_PARAMS % 256 != 0 && 256 - N_PARAMS % 256 >= 32, "the last CTA's last warp is free");
+constexpr uint32_t kMaxParts = 1024;
+__device__ __forceinline__ void sum_losses(const float* __restrict__ partial, uint32_t n_parts, float* __restrict__ loss)
 {
+    __shared__ float part[kMaxParts];
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t c = lane; c < n_parts; c += 32u) part[c] = partial[(uint64_t)n_parts * N_PARAMS + c];
+    __syncwarp();
+    if (lane != 0u) return;
     float l = 0.0f;
-    for (uint32_t c = 0; c < n_parts; c++) l += partial[(uint64_t)n_parts * N_PARAMS + c];
-    return l;
+    for (uint32_t c = 0; c < n_parts; c++) l += part[c];
+    *loss = l;
 }
+__device__ __forceinline__ bool loss_warp() { return blockIdx.x == gridDim.x - 1u && threadIdx.x >= 224u; }
 
 // The slices' sum added to the gradient; the loss.
 __global__ void __launch_bounds__(256) k_mlp_reduce(const float* __restrict__ partial, uint32_t n_parts,
@@ -734,7 +763,7 @@ __global__ void __launch_bounds__(256) k_mlp_reduce(const float* __restrict__ pa
 {
     pdl_wait();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p == 0) *loss = sum_losses(partial, n_parts);
+    if (loss_warp()) sum_losses(partial, n_parts, loss);
     if (p >= N_PARAMS) return;
     g[p] += sum_slices(partial, n_parts, p);
 }
@@ -772,8 +801,6 @@ struct AdamJobs
 
 __global__ void __launch_bounds__(256) k_mlp_adam(AdamJobs jobs, float lr, float b1, float b2, float eps)
 {
-    pdl_wait();      // the training kernel's slices
-    pdl_trigger();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     const AdamJob& J = jobs.j[0];
     const AdamJob& K = jobs.j[1];
@@ -786,15 +813,24 @@ __global__ void __launch_bounds__(256) k_mlp_adam(AdamJobs jobs, float lr, float
     const uint32_t n_parts = second ? K.n_parts : J.n_parts;
     const float c1 = second ? K.c1 : J.c1, c2 = second ? K.c2 : J.c2;
     __nv_bfloat16* img = second ? K.img : J.img;
-    if (p == 0) *(second ? K.loss : J.loss) = sum_losses(partial, n_parts);
-    if (p >= N_PARAMS) return;
-    const float gp = g[p] + sum_slices(partial, n_parts, p);
+    // The parameter's own numbers are read before the wait for the training
+    // kernel: it writes none of them, and whatever wrote them was complete before
+    // its own wait ended, hence before it let this launch begin (read from L2: an
+    // L1 line could be older).
+    const bool real = p < N_PARAMS;
+    const float g0 = real ? __ldcg(&g[p]) : 0.0f, m0 = real ? __ldcg(&m[p]) : 0.0f, v0 = real ? __ldcg(&v[p]) : 0.0f,
+                w0 = real ? __ldcg(&w[p]) : 0.0f;
+    pdl_wait();      // the training kernel's slices
+    pdl_trigger();
+    if (loss_warp()) sum_losses(partial, n_parts, second ? K.loss : J.loss);
+    if (!real) return;
+    const float gp = g0 + sum_slices(partial, n_parts, p);
     g[p] = 0.0f;
-    const float mp = b1 * m[p] + (1.0f - b1) * gp;
-    const float vp = b2 * v[p] + (1.0f - b2) * gp * gp;
+    const float mp = b1 * m0 + (1.0f - b1) * gp;
+    const float vp = b2 * v0 + (1.0f - b2) * gp * gp;
     m[p] = mp;
     v[p] = vp;
-    const float wp = w[p] - lr * (mp / c1) / (sqrtf(vp / c2) + eps);
+    const float wp = w0 - lr * (mp / c1) / (sqrtf(vp / c2) + eps);
     w[p] = wp;
     img[image_pos(p)] = __float2bfloat16_rn(wp);
 }
@@ -942,7 +978,7 @@ tgx_status cache_infer_counted(tgx_ctx* c, tgx_cache* k, const uint32_t* d_n, ui
 // networks' batches side by side in one launch; leaves each network's per-CTA
 // gradient slices in its scratch (parts[i] of them).
 static tgx_status cache_grad_parts(tgx_ctx* c, tgx_cache* const* k, const uint32_t* n, const float* const* d_x,
-                                   const float* const* d_t, uint32_t n_nets, uint32_t* parts)
+                                   const float* const* d_t, uint32_t n_nets, bool batch_ready, uint32_t* parts)
 {
     static bool attr = false;
     if (!attr) {
@@ -950,6 +986,7 @@ static tgx_status cache_grad_parts(tgx_ctx* c, tgx_cache* const* k, const uint32
         attr = true;
     }
     TrainJobs jobs;
+    jobs.batch_ready = batch_ready ? 1u : 0u;
     uint32_t grid = 0;
     // One wave of CTAs (one per SM: the kernel holds most of an SM's shared
     // memory) shared between the jobs in proportion to their 128-sample tiles,
@@ -986,7 +1023,7 @@ static tgx_status cache_grad_parts(tgx_ctx* c, tgx_cache* const* k, const uint32
 static tgx_status cache_grad(tgx_ctx* c, tgx_cache* k, uint32_t n, const float* d_x, const float* d_t)
 {
     uint32_t parts = 0;
-    TGX_TRY(cache_grad_parts(c, &k, &n, &d_x, &d_t, 1, &parts));
+    TGX_TRY(cache_grad_parts(c, &k, &n, &d_x, &d_t, 1, false, &parts));
     TGX_LAUNCH(c, TR_MLP_WGRAD, (N_PARAMS + 255) / 256, 256, 0, k_mlp_reduce, (const float*)k->scratch.ptr, parts, k->g,
                k->loss);
     return TGX_OK;
@@ -1006,12 +1043,13 @@ extern "C" tgx_status tgx_cache_gradient(tgx_ctx* c, tgx_cache* k, uint32_t n, c
 }
 
 // One Adam step of one network, or of two networks side by side (shared
-// training and Adam launches); n[i] samples each.
+// training and Adam launches); n[i] samples each.  batch_ready: the stream's
+// previous work is the step before, and the batches are older than that step.
 tgx_status cache_train_pair(tgx_ctx* c, tgx_cache* const* k, const uint32_t* n, const float* const* d_x,
-                            const float* const* d_t, uint32_t n_nets, float lr)
+                            const float* const* d_t, uint32_t n_nets, float lr, bool batch_ready)
 {
     uint32_t parts[2] = {0, 0};
-    TGX_TRY(cache_grad_parts(c, k, n, d_x, d_t, n_nets, parts));
+    TGX_TRY(cache_grad_parts(c, k, n, d_x, d_t, n_nets, batch_ready, parts));
     const float b1 = 0.9f, b2 = 0.99f, eps = 1e-15f;
     AdamJobs jobs;
     for (uint32_t i = 0; i < n_nets; i++) {
@@ -1034,7 +1072,7 @@ extern "C" tgx_status tgx_cache_train_step(tgx_ctx* c, tgx_cache* k, uint32_t n,
                                            float lr)
 {
     if (!c || !k || !n || !d_x || !d_t) return TGX_ERR_INVALID_ARGUMENT;
-    return cache_train_pair(c, &k, &n, &d_x, &d_t, 1, lr);
+    return cache_train_pair(c, &k, &n, &d_x, &d_t, 1, lr, false);
 }
 
 extern "C" tgx_status tgx_cache_last_loss(tgx_ctx* c, const tgx_cache* k, float* out_loss)

@@ -449,7 +449,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
 // cache inference over min(max_n, *d_n) inputs (mlp.cu)
 tgx_status cache_primary(tgx_ctx* c, tgx_cache* k, tgx_cache** out);
 tgx_status cache_train_pair(tgx_ctx* c, tgx_cache* const* k, const uint32_t* n, const float* const* d_x,
-                            const float* const* d_t, uint32_t n_nets, float lr);
+                            const float* const* d_t, uint32_t n_nets, float lr, bool batch_ready);
 tgx_status cache_infer_counted(tgx_ctx* c, tgx_cache* k, const uint32_t* d_n, uint32_t max_n, const float* d_x,
                                float* d_rgb);
 
