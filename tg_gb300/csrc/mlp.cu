@@ -124,6 +124,19 @@ __device__ __forceinline__ void mma(uint32_t d_tmem, uint64_t a, uint64_t b, uin
                  :: "r"(d_tmem), "l"(a), "l"(b), "r"(id), "r"(acc) : "memory");
 }
 
+// kSteps MMAs along K: the descriptors' addresses (in 16-byte units, the low bits)
+// advance by a_step and b_step bytes.  One thread issues all of them, so what a
+// step costs it counts: building both descriptors anew took 75 cycles a step,
+// twice the tensor core's time for it.
+template <int kSteps>
+__device__ __forceinline__ void mma_steps(uint32_t d_tmem, uint64_t a, uint32_t a_step, uint64_t b, uint32_t b_step, uint32_t id,
+                                          uint32_t acc)
+{
+#pragma unroll
+    for (int k = 0; k < kSteps; k++)
+        mma(d_tmem, a + (uint64_t)(k * (a_step >> 4)), b + (uint64_t)(k * (b_step >> 4)), id, k > 0 ? 1u : acc);
+}
+
 __device__ __forceinline__ void commit(uint32_t bar)
 {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar) : "memory");
@@ -275,19 +288,27 @@ __global__ void __launch_bounds__(tc::THREADS, 1) k_mlp_forward_tc(const __nv_bf
     const uint32_t b = saddr(&bars[g]);
     uint32_t phase = 0;
     bool weights = false, ok = true;
-    // the MMAs of operand columns 0 .. kgs - 1 against the weight columns from w_off on
-    auto issue = [&](int kgs, int w_off, uint32_t n_out, bool accumulate) {
-        if (gt != 0) return;
+    // the MMAs of a layer (or of a half of layer 0) against the weights at w_off
+    auto begin = [&]() {   // the issuing thread
         if (!weights) {
             if (!wait(wbar, 0u)) { dev_error(status, TGX_ERR_TIMEOUT, 45, tile); ok = false; }
             weights = true;
         }
         fence_after();
-        const uint32_t a_base = saddr(ga), w_base = saddr(sm + w_off);
-        const uint32_t w_lbo = (n_out / 8) * 128;
-        for (int k = 0; k < kgs / 2; k++)
-            mma(tmem, sdesc(a_base + 2 * k * (16 * 128), 16 * 128, 128), sdesc(w_base + 2 * k * w_lbo, w_lbo, 128),
-                idesc(n_out), accumulate || k > 0);
+    };
+    const uint64_t a_desc = sdesc(saddr(ga), 16 * 128, 128);
+    auto issue_half = [&](int w_off, uint32_t acc) {
+        if (gt != 0) return;
+        begin();
+        mma_steps<KGF / 2>(tmem, a_desc, 2 * 16 * 128, sdesc(saddr(sm + w_off), 8 * 128, 128), 2 * 8 * 128, idesc(64), acc);
+        commit(b);
+    };
+    auto issue_hidden = [&](int l) {
+        if (gt != 0) return;
+        fence_after();
+        if (l < 4) mma_steps<KGH / 2>(tmem, a_desc, 2 * 16 * 128, sdesc(saddr(sm + W1 + (l - 1) * KGH * 8 * 128), 8 * 128, 128),
+                                      2 * 8 * 128, idesc(64), 0u);
+        else mma_steps<KGH / 2>(tmem, a_desc, 2 * 16 * 128, sdesc(saddr(sm + W4), 2 * 128, 128), 2 * 2 * 128, idesc(16), 0u);
         commit(b);
     };
     // a wait that gives up is noted; the group stops at the end of the tile
@@ -320,7 +341,7 @@ __global__ void __launch_bounds__(tc::THREADS, 1) k_mlp_forward_tc(const __nv_bf
             for (int q = 0; q < (i < 4 ? 3 : 2); q++) put_column(ga, 3 * i + q, (int)gt, f[q]);
         }
         publish();
-        issue(KGF, W0, 64u, false);
+        issue_half(W0, 0u);
         // columns 14..27: the rest of input 4, inputs 5..8 and the zero column
         const uint4 rest = f[2];
         features(xc[5], f);
@@ -334,7 +355,7 @@ __global__ void __launch_bounds__(tc::THREADS, 1) k_mlp_forward_tc(const __nv_bf
         }
         put_column(ga, KGF - 1, (int)gt, make_uint4(0u, 0u, 0u, 0u));
         publish();
-        issue(KGF, W0 + KGF * 8 * 128, 64u, true);
+        issue_half(W0 + KGF * 8 * 128, 1u);
 #pragma unroll
         for (int l = 0; l < 4; l++) {
             finish(40 + l);
@@ -349,7 +370,7 @@ __global__ void __launch_bounds__(tc::THREADS, 1) k_mlp_forward_tc(const __nv_bf
                 for (int q = 0; q < 4; q++) put8_relu(ga, 4 * h + q, (int)gt, v + 8 * q);
             }
             publish();
-            issue(KGH, l < 3 ? W1 + l * KGH * 8 * 128 : W4, l < 3 ? 64u : 16u, false);
+            issue_hidden(l + 1);
         }
         finish(44);
         float v[16];
@@ -475,14 +496,21 @@ __global__ void __launch_bounds__(tt::THREADS, 1) k_mlp_train_tc(TrainJobs jobs,
     // the batch comes from an earlier kernel of the stream, the weight image from
     // the one before (Adam) or an earlier one.  Read from L2: an L1 line could be
     // older than the batch when this runs before the wait.
-    auto encode_tile = [&](uint32_t tile) {
+    auto encode_tile = [&](uint32_t tile) {   // inputs part, part + CS, ...: their loads first, then side by side
         const uint32_t row = tile * 128 + r;
-        for (int i = (int)part; i < NI; i += tt::CS)
-            encode_input(sm + tt::X0, i, (int)r, row < n ? __ldcg(&x[(uint64_t)row * NI + i]) : 0.0f);
-        if (part == tt::CS - 1) {
-            const float z[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            put8(sm + tt::X0, KG0 - 1, (int)r, z);   // features 216..223
+        constexpr int kMine = (NI + tt::CS - 1) / tt::CS;
+        float xi[kMine];
+#pragma unroll
+        for (int k = 0; k < kMine; k++) {
+            const int i = (int)part + k * tt::CS;
+            xi[k] = i < NI && row < n ? __ldcg(&x[(uint64_t)row * NI + i]) : 0.0f;
         }
+#pragma unroll
+        for (int k = 0; k < kMine; k++) {
+            const int i = (int)part + k * tt::CS;
+            if (i < NI) encode_input(sm + tt::X0, i, (int)r, xi[k]);
+        }
+        if (part == tt::CS - 1) put_column(sm + tt::X0, KG0 - 1, (int)r, make_uint4(0u, 0u, 0u, 0u));   // features 216..223
     };
     const uint32_t tiles = (n + 127) / 128;
     if (jobs.batch_ready && cta < tiles) encode_tile(cta);
@@ -576,19 +604,13 @@ __global__ void __launch_bounds__(tt::THREADS, 1) k_mlp_train_tc(TrainJobs jobs,
                 if (l == 0 && tile == cta && !wait(saddr(bar + 1), 0u)) dev_error(status, TGX_ERR_TIMEOUT, 55, tile);
                 fence_after();
                 if (l == 0) {
-                    for (int k = 0; k < KG0 / 2; k++)
-                        mma(tmem + tt::ACC, sdesc(x0 + 2 * k * 2048, 2048, 128), sdesc(w0 + 2 * k * 1024, 1024, 128),
-                            idesc(64), k > 0);
+                    mma_steps<KG0 / 2>(tmem + tt::ACC, sdesc(x0, 2048, 128), 4096, sdesc(w0, 1024, 128), 2048, idesc(64), 0u);
                 } else if (l < 4) {
-                    const uint32_t a = hb + (l - 1) * tt::TILE64, w = w1 + (l - 1) * KGH * 8 * 128;
-                    for (int k = 0; k < KGH / 2; k++)
-                        mma(tmem + tt::ACC, sdesc(a + 2 * k * 2048, 2048, 128), sdesc(w + 2 * k * 1024, 1024, 128),
-                            idesc(64), k > 0);
+                    mma_steps<KGH / 2>(tmem + tt::ACC, sdesc(hb + (l - 1) * tt::TILE64, 2048, 128), 4096,
+                                       sdesc(w1 + (l - 1) * KGH * 8 * 128, 1024, 128), 2048, idesc(64), 0u);
                 } else {
-                    const uint32_t a = hb + 3 * tt::TILE64;
-                    for (int k = 0; k < KGH / 2; k++)
-                        mma(tmem + tt::ACC, sdesc(a + 2 * k * 2048, 2048, 128), sdesc(w4 + 2 * k * 256, 256, 128),
-                            idesc(16), k > 0);
+                    mma_steps<KGH / 2>(tmem + tt::ACC, sdesc(hb + 3 * tt::TILE64, 2048, 128), 4096, sdesc(w4, 256, 128), 512,
+                                       idesc(16), 0u);
                 }
                 commit(b);
             }
@@ -644,24 +666,20 @@ __global__ void __launch_bounds__(tt::THREADS, 1) k_mlp_train_tc(TrainJobs jobs,
                 const int l = 4 - s;                       // weight layer
                 if (s < 4) {
                     // next delta (pre-mask) = din * W_l: B = W_l read MN-major (N = inputs, K = outputs)
-                    if (l == 4) {
+                    if (l == 4)
                         mma(tmem + tt::ACC, sdesc(din, 2048, 128), sdesc(w4, 128, 256), tt::idesc_t(64, false, true), 0u);
-                    } else {
-                        const uint32_t w = w1 + (l - 1) * KGH * 8 * 128;
-                        for (int k = 0; k < KGH / 2; k++)
-                            mma(tmem + tt::ACC, sdesc(din + 2 * k * 2048, 2048, 128), sdesc(w + 2 * k * 128, 128, 1024),
-                                tt::idesc_t(64, false, true), k > 0);
-                    }
+                    else
+                        mma_steps<KGH / 2>(tmem + tt::ACC, sdesc(din, 2048, 128), 4096,
+                                           sdesc(w1 + (l - 1) * KGH * 8 * 128, 128, 1024), 256, tt::idesc_t(64, false, true), 0u);
                 }
                 // dW_l^T += input_l^T din: A = the layer's input tile, B = din, both MN-major, K = samples
                 const uint32_t nout = l == 4 ? 16u : 64u;
                 const uint32_t gcol = l == 4 ? tt::G4 : l == 3 ? tt::G3 : l == 2 ? tt::G2 : l == 1 ? tt::G1 : tt::G0A;
                 const uint32_t ain = l == 0 ? x0 : hb + (l - 1) * tt::TILE64;
-                const int parts = l == 0 ? 2 : 1;
-                for (int part = 0; part < parts; part++)
-                    for (int k = 0; k < 8; k++)
-                        mma(tmem + gcol + part * 64u, sdesc(ain + part * 16 * 2048 + 2 * k * 128, 128, 2048),
-                            sdesc(din + 2 * k * 128, 128, 2048), tt::idesc_t(nout, true, true), (acc_g | k) ? 1u : 0u);
+                const uint32_t id = tt::idesc_t(nout, true, true);
+                mma_steps<8>(tmem + gcol, sdesc(ain, 128, 2048), 256, sdesc(din, 128, 2048), 256, id, acc_g);
+                if (l == 0)
+                    mma_steps<8>(tmem + gcol + 64u, sdesc(ain + 16 * 2048, 128, 2048), 256, sdesc(din, 128, 2048), 256, id, acc_g);
                 commit(b);
             }
             // the sums of the stage before are final on the last tile: they go out behind this stage's MMAs
