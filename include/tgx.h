@@ -311,7 +311,7 @@ typedef struct tgx_vis_work
     uint64_t pairs;               /* pairs evaluated: past the per-pixel depth skip */
     uint64_t depth_skips;         /* pairs skipped: the pixel already holds a nearer word */
     uint64_t dir_setups;          /* cluster-space ray directions computed (per pixel and object) */
-    uint64_t slab_misses;         /* pairs the conservative slab test rejects */
+    uint64_t slab_misses;         /* pairs the conservative tests reject (the warp's or the pixel's) */
     uint64_t sure_hits;           /* pairs whose box entry is certain (entry distance only) */
     uint64_t exact_tests;         /* pairs that run the shader's full ray/box test */
     uint64_t ddas;                /* pairs that run the voxel DDA */
