@@ -19,13 +19,14 @@
 //                           first); then per group: tile offsets and order.
 //                           Up to 512 groups, k_vis_finalize_direct does both:
 //                           each CTA reads all groups' sums and histograms.
-//   5. k_vis_bin_fill       a half-warp per record: writes it, with its cluster's
-//                           64-byte bitmask, as a 96-byte entry into each of its
-//                           (tile, bucket) bins, so every tile's entries are
-//                           contiguous and run near to far.
+//   5. k_vis_bin_fill       a half-warp per record, a warp per 256 tiles of the
+//                           records of many: an 8-byte reference into each of
+//                           its (tile, bucket) bins, so every tile's references
+//                           are contiguous and run near to far.
 //   6. k_vis_tiles          one CTA per tile (heaviest first), one thread per
 //      pixel (k_vis_tiles_groups: several, for frames of few tiles): batches of
-//      the tile's entries arrive by one cp.async.bulk each on an mbarrier;
+//      the tile's entries (record and 64-byte bitmask) are gathered by cp.async
+//      on an mbarrier;
 //      each warp drops, 32 at a time, the entries that none of its pixels can
 //      take; every pixel skips entries whose depth bound cannot beat its word and
 //      rejects clear misses with a conservative reciprocal slab test; the
@@ -55,30 +56,53 @@ struct alignas(16) VisRecord
 {
     float    ox, oy, oz;        // camera position in cluster space (visibility.frag:66)
     uint32_t cluster_idx;
-    uint32_t cluster_pointer;
     uint32_t object_idx;
     uint32_t d24_lb;            // lower bound of the 24-bit depth field any pixel can get from it
+    uint32_t cluster_pointer;
     uint32_t view;
 };
 static_assert(sizeof(VisRecord) == 32, "record layout");
 
 enum Counter { C_RECORDS = 0, C_ENTRIES = 1, C_DDA_OVERRUN = 2, C_OVERFLOW = 3, C_TILE_QUEUE = 4, C_NONEMPTY = 5,
-               C_COUNT = 8 };
+               C_CHUNKS = 6, C_COUNT = 8 };
 
-// One binned (tile, cluster) entry as the tile kernel stages it: the record's
-// fields the DDA needs and the cluster's 64-byte bitmask, so a batch of a
-// tile's entries is one contiguous bulk copy.
+// One (tile, cluster) pair as the tile kernel stages it: the record and the
+// cluster's 64-byte bitmask.  The tile's bin holds only where the two are (a
+// TileRef); the copies into shared memory gather them.
 struct alignas(16) TileEntry
 {
-    float    ox, oy, oz;        // camera position in cluster space
-    uint32_t cluster_pointer;
-    uint32_t object_idx;
-    uint32_t d24_lb;
-    uint32_t pad[2];
+    VisRecord rec;
     uint32_t bits[16];
 };
 static_assert(sizeof(TileEntry) == 96, "entry layout");
-constexpr uint32_t kEntryWords = sizeof(TileEntry) / 4;
+struct alignas(8) TileRef
+{
+    uint32_t record, cluster_idx;
+};
+
+// A record's tile rectangle: x = tx0 | ty0 << 16, y = tx1 | ty1 << 16 (at most
+// 4095 tiles a side); bit 31 of y: the record's tiles are in the chunk list.
+constexpr uint32_t kListed = 0x80000000u;
+struct TileRect
+{
+    uint32_t tx0, ty0, w, n;    // first tile, tiles per row, tiles
+};
+__device__ __forceinline__ TileRect tile_rect(uint2 r)
+{
+    TileRect t;
+    t.tx0 = r.x & 0xffffu;
+    t.ty0 = r.x >> 16;
+    t.w = (r.y & 0xffffu) - t.tx0 + 1u;
+    t.n = t.w * (((r.y & ~kListed) >> 16) - t.ty0 + 1u);
+    return t;
+}
+
+// Records of more than kHalfWarpTiles tiles are cut into chunks of kChunkTiles,
+// a list of (record, first tile) that the counting and the binning pass spread
+// over the GPU, a warp per chunk; the others take a half-warp each.  A cluster
+// next to the camera covers every tile: a half-warp alone was at 129,600 of them
+// for 6 ms.  A record whose chunks find no room in the list goes the other way.
+constexpr uint32_t kHalfWarpTiles = 64, kChunkTiles = 256;
 // work counters of the tile kernel's counting variant (tgx_vis_work, same order)
 enum Work { W_PAIRS = 0, W_DEPTH_SKIPS, W_DIR_SETUPS, W_SLAB_MISSES, W_SURE_HITS, W_EXACT_TESTS, W_DDAS, W_DDA_STEPS,
             W_HITS, W_BATCHES, W_COUNT };
@@ -130,7 +154,8 @@ __global__ void __launch_bounds__(256, 4) k_vis_cluster_setup(
     const uint32_t* __restrict__ c2o, const uint32_t* __restrict__ bits, const uint32_t* __restrict__ cp_obj,
     uint32_t n_cp, const ViewConst* __restrict__ views, uint32_t n_views, VisRecord* __restrict__ records,
     uint2* __restrict__ rects, uint32_t record_capacity, uint32_t* __restrict__ counters,
-    uint32_t* __restrict__ zero, uint32_t n_zero, tgx_dev_status* __restrict__ status)
+    uint32_t* __restrict__ zero, uint32_t n_zero, uint2* __restrict__ chunks, uint32_t chunk_cap,
+    tgx_dev_status* __restrict__ status)
 {
     pdl_wait();
     pdl_trigger();
@@ -264,14 +289,25 @@ __global__ void __launch_bounds__(256, 4) k_vis_cluster_setup(
         return;
     }
     records[slot] = rec;
-    rects[slot] = make_uint2(tx0 | (ty0 << 16), tx1 | (ty1 << 16));
+    uint32_t listed = 0u;
+    const uint32_t n = (tx1 - tx0 + 1u) * (ty1 - ty0 + 1u);
+    if (n > kHalfWarpTiles) {
+        const uint32_t n_chunks = (n + kChunkTiles - 1u) / kChunkTiles;
+        const uint32_t first = atomicAdd(&counters[C_CHUNKS], n_chunks);
+        const bool room = first <= chunk_cap && n_chunks <= chunk_cap - first;
+        for (uint32_t k = 0; k < n_chunks && first + k < chunk_cap && first + k >= first; k++)
+            chunks[first + k] = make_uint2(room ? slot : 0xffffffffu, k * kChunkTiles);
+        if (room) listed = kListed;
+    }
+    rects[slot] = make_uint2(tx0 | (ty0 << 16), tx1 | (ty1 << 16) | listed);
 }
 
 // ---------------------------------------------------------------------------
 // 2. per record: the exact ws2ms and ray origin (visibility.frag:57-66), one
-//    thread per record; then its per-(tile, bucket) counts, a half-warp per
-//    record with the lanes over its tiles.  The two loops write different
-//    fields and buffers; the cull kept apart runs at high occupancy.
+//    thread per record; then its per-(tile, bucket) counts, a warp per listed
+//    chunk and a half-warp per other record (records span ~17 tiles on average)
+//    with the lanes over the tiles.  The loops write different fields and
+//    buffers; the cull kept apart runs at high occupancy.
 // ---------------------------------------------------------------------------
 
 __global__ void __launch_bounds__(256) k_vis_count(VisRecord* __restrict__ records, const uint2* __restrict__ rects,
@@ -279,7 +315,7 @@ __global__ void __launch_bounds__(256) k_vis_count(VisRecord* __restrict__ recor
                                                   const tgx_object* __restrict__ objects,
                                                   const ViewConst* __restrict__ views,
                                                   uint32_t* __restrict__ bucket_cnt, uint32_t n_tiles,
-                                                  uint32_t bshift)
+                                                  uint32_t bshift, const uint2* __restrict__ chunks, uint32_t chunk_cap)
 {
     pdl_wait();
     pdl_trigger();
@@ -308,18 +344,24 @@ __global__ void __launch_bounds__(256) k_vis_count(VisRecord* __restrict__ recor
         dm4_mulv4(ws2ms, vc.cam[0], vc.cam[1], vc.cam[2], 1.0f, o);
         rec.ox = o[0]; rec.oy = o[1]; rec.oz = o[2];
     }
-    const uint32_t lane = threadIdx.x & 15u;   // a half-warp per record: records span ~17 tiles on average
+    auto count = [&](uint32_t i, const TileRect& t, uint32_t k) {
+        const ViewConst& vc = views[records[i].view];
+        const uint32_t tile = vc.tile_base + (t.ty0 + k / t.w) * vc.tiles_x + t.tx0 + k % t.w;
+        atomicAdd(&bucket_cnt[depth_bucket(records[i].d24_lb, bshift) * n_tiles + tile], 1u);
+    };
+    const uint32_t n_chunks = min(counters[C_CHUNKS], chunk_cap);
+    for (uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < n_chunks; c += (gridDim.x * blockDim.x) >> 5) {
+        const uint2 ch = chunks[c];
+        if (ch.x >= n) continue;
+        const TileRect t = tile_rect(rects[ch.x]);
+        const uint32_t end = min(t.n, ch.y + kChunkTiles);
+        for (uint32_t k = ch.y + (threadIdx.x & 31u); k < end; k += 32u) count(ch.x, t, k);
+    }
     for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 4; i < n; i += (gridDim.x * blockDim.x) >> 4) {
         const uint2 r = rects[i];
-        const uint32_t view = records[i].view;
-        const ViewConst& vc = views[view];
-        const uint32_t b = depth_bucket(records[i].d24_lb, bshift);
-        const uint32_t tx0 = r.x & 0xffffu, ty0 = r.x >> 16, tx1 = r.y & 0xffffu, ty1 = r.y >> 16;
-        const uint32_t w = tx1 - tx0 + 1, cnt = w * (ty1 - ty0 + 1);
-        for (uint32_t k = lane; k < cnt; k += 16) {
-            const uint32_t t = vc.tile_base + (ty0 + k / w) * vc.tiles_x + tx0 + k % w;
-            atomicAdd(&bucket_cnt[b * n_tiles + t], 1u);
-        }
+        if (r.y & kListed) continue;
+        const TileRect t = tile_rect(r);
+        for (uint32_t k = threadIdx.x & 15u; k < t.n; k += 16u) count(i, t, k);
     }
 }
 
@@ -593,9 +635,11 @@ __global__ void __launch_bounds__(kScanTiles) k_vis_finalize_direct(const uint32
 }
 
 // ---------------------------------------------------------------------------
-// 5. bin fill: a half-warp per record; its lanes take the record's tiles'
-//    slots (16 at a time), then 12 lanes write the 96-byte entry into each
-//    slot with 8-byte stores
+// 5. bin fill: as in the count, a warp per listed chunk and a half-warp per
+//    other record, a lane per tile, which takes the next place of the tile's
+//    bucket and writes the 8-byte reference there.  (Writing the 96-byte entry
+//    itself took 26 us at 1080p, 512 objects, and 210 us for 7.3 M entries;
+//    the tile kernel gathers it as quickly from the record as from a copy.)
 // ---------------------------------------------------------------------------
 
 __global__ void __launch_bounds__(256) k_vis_bin_fill(const VisRecord* __restrict__ records,
@@ -604,62 +648,51 @@ __global__ void __launch_bounds__(256) k_vis_bin_fill(const VisRecord* __restric
                                                      const ViewConst* __restrict__ views,
                                                      const uint32_t* __restrict__ tile_off,
                                                      const uint32_t* __restrict__ bucket_off,
-                                                     uint32_t* __restrict__ cursor, TileEntry* __restrict__ entries,
-                                                     const uint32_t* __restrict__ bits,
+                                                     uint32_t* __restrict__ cursor, TileRef* __restrict__ refs,
                                                      uint32_t n_tiles, uint32_t bin_capacity, uint32_t bshift,
+                                                     const uint2* __restrict__ chunks, uint32_t chunk_cap,
                                                      tgx_dev_status* __restrict__ status)
 {
     pdl_wait();
     pdl_trigger();
     if (counters[C_OVERFLOW]) return;   // the tile kernel scans all records instead
-    const uint32_t lane = threadIdx.x & 15u;
-    const uint32_t src0 = threadIdx.x & 16u;   // this half-warp's first lane in the warp
     const uint32_t n = counters[C_RECORDS];
-    uint2* const ew = reinterpret_cast<uint2*>(entries);
-    const uint32_t stride = (gridDim.x * blockDim.x) >> 4;
-    // every half-warp runs the same number of iterations, so the shuffles see full warps
-    const uint32_t rounds = (n + stride - 1) / stride;
-    for (uint32_t it = 0; it < rounds; it++) {
-        const uint32_t i = ((blockIdx.x * blockDim.x + threadIdx.x) >> 4) + it * stride;
-        const bool have = i < n;
-        // entry words 2 lane, 2 lane + 1: ox oy | oz pointer | object lb | 0 0 | bitmask (16 words)
-        uint2 word = make_uint2(0u, 0u);
-        uint32_t cnt = 0, w = 1, tx0 = 0, ty0 = 0, b = 0, tile_base = 0, tiles_x = 0;
-        if (have) {
-            const uint32_t* rw = reinterpret_cast<const uint32_t*>(records + i);
-            if (lane == 0) word = make_uint2(rw[0], rw[1]);
-            else if (lane == 1) word = make_uint2(rw[2], rw[4]);
-            else if (lane == 2) word = make_uint2(rw[5], rw[6]);
-            else if (lane >= 4 && lane < 12) {
-                const uint2* bw = reinterpret_cast<const uint2*>(bits + (uint64_t)rw[3] * 16u);
-                word = bw[lane - 4];
+    // tiles k, k + step, ... below end of record i, four at a time so that their atomics are in flight together
+    auto fill = [&](uint32_t i, const TileRect& t, uint32_t k, uint32_t end, uint32_t step) {
+        const VisRecord& rec = records[i];
+        const ViewConst& vc = views[rec.view];
+        const uint32_t row = depth_bucket(rec.d24_lb, bshift) * n_tiles;
+        const uint32_t base = vc.tile_base + t.ty0 * vc.tiles_x + t.tx0;
+        const TileRef ref = {i, rec.cluster_idx};
+        for (; k < end; k += 4u * step) {
+            uint32_t pos[4];
+#pragma unroll
+            for (uint32_t j = 0; j < 4u; j++) {
+                const uint32_t kj = k + j * step;
+                if (kj >= end) continue;
+                const uint32_t tile = base + (kj / t.w) * vc.tiles_x + kj % t.w;
+                pos[j] = tile_off[tile] + bucket_off[row + tile] + atomicAdd(&cursor[row + tile], 1u);
             }
-            const uint2 r = rects[i];
-            const VisRecord& rec = records[i];
-            const ViewConst& vc = views[rec.view];
-            b = depth_bucket(rec.d24_lb, bshift);
-            tx0 = r.x & 0xffffu; ty0 = r.x >> 16;
-            const uint32_t tx1 = r.y & 0xffffu, ty1 = r.y >> 16;
-            w = tx1 - tx0 + 1;
-            cnt = w * (ty1 - ty0 + 1);
-            tile_base = vc.tile_base;
-            tiles_x = vc.tiles_x;
-        }
-        // the longer record of the warp's two sets the trip count
-        const uint32_t cnt_max = max(cnt, __shfl_xor_sync(0xffffffffu, cnt, 16));
-        for (uint32_t k0 = 0; k0 < cnt_max; k0 += 16u) {
-            uint32_t pos = 0xffffffffu;
-            const uint32_t k = k0 + lane;
-            if (k < cnt) {
-                const uint32_t t = tile_base + (ty0 + k / w) * tiles_x + tx0 + k % w;
-                pos = tile_off[t] + bucket_off[b * n_tiles + t] + atomicAdd(&cursor[b * n_tiles + t], 1u);
-                if (pos >= bin_capacity) { dev_error(status, TGX_ERR_DEVICE_FAULT, 3, pos); pos = 0xffffffffu; }
-            }
-            for (uint32_t q = 0; q < 16u; q++) {
-                const uint32_t pq = __shfl_sync(0xffffffffu, pos, src0 + q);
-                if (pq != 0xffffffffu && lane < 12u) ew[(uint64_t)pq * 12u + lane] = word;
+#pragma unroll
+            for (uint32_t j = 0; j < 4u; j++) {
+                if (k + j * step >= end) continue;
+                if (pos[j] >= bin_capacity) dev_error(status, TGX_ERR_DEVICE_FAULT, 3, pos[j]);
+                else refs[pos[j]] = ref;
             }
         }
+    };
+    const uint32_t n_chunks = min(counters[C_CHUNKS], chunk_cap);
+    for (uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < n_chunks; c += (gridDim.x * blockDim.x) >> 5) {
+        const uint2 ch = chunks[c];
+        if (ch.x >= n) continue;
+        const TileRect t = tile_rect(rects[ch.x]);
+        fill(ch.x, t, ch.y + (threadIdx.x & 31u), min(t.n, ch.y + kChunkTiles), 32u);
+    }
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 4; i < n; i += (gridDim.x * blockDim.x) >> 4) {
+        const uint2 r = rects[i];
+        if (r.y & kListed) continue;
+        const TileRect t = tile_rect(r);
+        fill(i, t, threadIdx.x & 15u, t.n, 16u);
     }
 }
 
@@ -851,7 +884,7 @@ struct TileJob
 {
     const VisRecord* records;
     const uint2* rects;
-    const TileEntry* entries;
+    const TileRef* refs;         // the bins, tile after tile
     const uint32_t* tile_off;
     const uint4* slot_info;      // per launch slot (heavy first): tile, first entry, entry count
     const ViewConst* views;
@@ -865,14 +898,14 @@ struct TileJob
     uint32_t bshift;             // depth buckets: 32 >> bshift
     uint32_t batch;              // entries per staged batch (1..kBatch)
     uint32_t drain;              // live pairs a warp collects before its lanes run their DDAs (1..32)
-    uint32_t extra_tx;           // bytes the first batch's barrier expects beyond its copies: 0, or 64
+    uint32_t extra_tx;           // bytes the first batch's barrier expects that nobody copies: 0, or 64
                                  // under TGX_FLAG_TEST_LOST_COPY (its wait then runs out)
     uint32_t interleave;         // k_vis_tiles: spread the tiles without entries evenly over the launch
                                  // (outputs in host memory), instead of launching them last
 };
 
 // Shared memory of a tile CTA (dynamic, tile_smem_bytes(threads)):
-//   the mbarrier of the bulk copies, the tile's view and a gather count;
+//   the mbarrier of the copies, the tile's view and a gather count;
 //   the staged batch: up to kBatch of the tile's 96-byte entries;
 //   every pixel's best packed word so far (the pair lanes' atomicMin target);
 //   per warp, a ring of kQueue live (pixel, entry) pairs waiting for a lane:
@@ -883,7 +916,7 @@ constexpr uint32_t kQueue = 64;                      // ring entries per warp (a
 constexpr uint32_t kWarpRays = 7 * kQueue;           // then the bounds of the warp's rays (warp_rays): 6 floats
 constexpr uint32_t kQueueWords = kWarpRays + 8;      // the ring: 6 float arrays + the packed word
 constexpr uint32_t kSmBar = 0, kSmView = 8, kSmN = 12, kSmLost = 16, kSmBars = 24;   // kSmBars: kStages - 1 more mbarriers
-constexpr uint32_t kSmStage = 128;                   // 16-byte aligned bulk-copy target
+constexpr uint32_t kSmStage = 128;                   // 16-byte aligned copy target
 constexpr uint32_t kStages = 2;                      // stages of a tile with several groups of threads (vis_tile_groups)
 __host__ __device__ constexpr uint32_t tile_best_off(uint32_t groups)
 {
@@ -922,24 +955,41 @@ __device__ __forceinline__ TileSm tile_sm()
 __device__ __forceinline__ void tile_smem_init(const TileSm& sm)
 {
     if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(sm.bar()));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(sm.bar()), "r"(blockDim.x));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
 }
 
-// One bulk copy of n contiguous entries to dst (in the stage), completing on
-// the mbarrier at bar (expecting `extra` bytes more than it copies under the
-// lost-copy test).  Thread 0 only.
-__device__ __forceinline__ void stage_entries(uint32_t bar, const TileEntry* dst, const TileEntry* src, uint32_t n,
+__device__ __forceinline__ void copy16(uint32_t to, const char* from)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(to), "l"(from) : "memory");
+}
+
+// Entries first .. first + n - 1 of the job's bins gathered to dst, a thread per
+// entry: its reference, then 32 bytes of the record and 64 of the bitmask.
+// (Spreading an entry's six copies over lanes: 106.7 to 108.6 us against 106.5
+// at 1080p, 512 objects.)  Every thread of the CTA arrives once on the mbarrier
+// at bar when its own copies have landed; `extra` more bytes are expected under
+// the lost-copy test.
+__device__ __forceinline__ void stage_entries(const TileJob& J, uint32_t bar, const TileEntry* dst, uint32_t first, uint32_t n,
                                               uint32_t extra)
 {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
-                 :: "r"(bar), "r"(n * (uint32_t)sizeof(TileEntry) + extra) : "memory");
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 :: "r"(smem_addr(dst)), "l"(src), "r"(n * (uint32_t)sizeof(TileEntry)), "r"(bar)
-                 : "memory");
+    for (uint32_t e = threadIdx.x; e < n; e += blockDim.x) {
+        const TileRef ref = J.refs[first + e];
+        const char* rec = reinterpret_cast<const char*>(J.records + ref.record);
+        const char* bits = reinterpret_cast<const char*>(J.bits + (uint64_t)ref.cluster_idx * 16u);
+        const uint32_t to = smem_addr(dst + e);
+#pragma unroll
+        for (uint32_t q = 0; q < 2u; q++) copy16(to + 16u * q, rec + 16u * q);
+#pragma unroll
+        for (uint32_t q = 0; q < 4u; q++) copy16(to + 32u + 16u * q, bits + 16u * q);
+    }
+    if (extra && threadIdx.x == 0)
+        asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" :: "r"(bar), "r"(extra) : "memory");
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" :: "r"(bar) : "memory");
 }
+// this thread's copies have landed
+__device__ __forceinline__ void own_copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // A thread's pixel of a tile: its place, its world ray, its nearest depth so
 // far and the cluster-space direction of the last object it met.
@@ -1017,11 +1067,12 @@ __device__ __forceinline__ void warp_rays(const TilePixel& P, float* __restrict_
 // squares could underflow or overflow in the normalisation.
 __device__ __forceinline__ bool warp_may_hit(const TileEntry& E, const float* __restrict__ bounds, const float* __restrict__ inv_rot)
 {
-    const float* L = inv_rot + 9u * E.object_idx;
+    const float* L = inv_rot + 9u * E.rec.object_idx;
     const float mx = bounds[0], my = bounds[1], mz = bounds[2];
     const float hx = bounds[4], hy = bounds[5], hz = bounds[6];
     float u[3], s[3], c[3], a[3];
-    const float o[3] = {E.ox, E.oy, E.oz};
+    const float4 oc = *reinterpret_cast<const float4*>(&E.rec.ox);
+    const float o[3] = {oc.x, oc.y, oc.z};
 #pragma unroll
     for (int i = 0; i < 3; i++) {
         const float l0 = L[3 * i], l1 = L[3 * i + 1], l2 = L[3 * i + 2];
@@ -1076,14 +1127,14 @@ __device__ __forceinline__ void tile_batch(const TileJob& J, const TileEntry* co
             const uint32_t e = next + kStep * lane;
             bool keep = e < n;
             if (keep) {
-                lb = E[e].d24_lb;
+                lb = E[e].rec.d24_lb;
                 keep = farthest >= lb && warp_may_hit(E[e], qf + kWarpRays, J.inv_rot);
             }
             todo = __ballot_sync(0xffffffffu, keep);
             if (kCount && P.valid) {
                 for (uint32_t i = 0, k = next; i < 32u && k < n; i++, k += kStep)
                     if (!((todo >> i) & 1u)) {
-                        if (P.best_d24 < E[k].d24_lb) work[W_DEPTH_SKIPS]++;
+                        if (P.best_d24 < E[k].rec.d24_lb) work[W_DEPTH_SKIPS]++;
                         else { work[W_PAIRS]++; work[W_SLAB_MISSES]++; }
                     }
             }
@@ -1093,7 +1144,7 @@ __device__ __forceinline__ void tile_batch(const TileJob& J, const TileEntry* co
             const uint32_t k = next - kStep * (33u - __ffs(todo));
             todo &= todo - 1u;
             bool live = false, sure = false;
-            const uint2 ol = *reinterpret_cast<const uint2*>(&E[k].object_idx);   // object, depth bound
+            const uint2 ol = *reinterpret_cast<const uint2*>(&E[k].rec.object_idx);   // object, depth bound
             if (P.valid) {
                 if (P.best_d24 < ol.y) {   // cannot produce a smaller word
                     if (kCount) work[W_DEPTH_SKIPS]++;
@@ -1115,7 +1166,7 @@ __device__ __forceinline__ void tile_batch(const TileJob& J, const TileEntry* co
                         P.iy = P.dy != 0.0f ? __frcp_rn(P.dy) : nan;
                         P.iz = P.dz != 0.0f ? __frcp_rn(P.dz) : nan;
                     }
-                    const float4 o = *reinterpret_cast<const float4*>(&E[k].ox);
+                    const float4 o = *reinterpret_cast<const float4*>(&E[k].rec.ox);
                     const int sc = slab_class(o.x, o.y, o.z, P.ix, P.iy, P.iz);
                     live = sc != kMiss;
                     sure = sc == kHit;
@@ -1140,10 +1191,11 @@ __device__ __forceinline__ void tile_batch(const TileJob& J, const TileEntry* co
             const uint32_t e = (P.qh + lane) & (kQueue - 1u);
             const uint32_t pk = q[6 * kQueue + e];
             const TileEntry& te = E[(pk >> 5) & 63u];
+            const float4 o = *reinterpret_cast<const float4*>(&te.rec.ox);
             const unsigned long long w = vis_pair<kCount>(
-                te.ox, te.oy, te.oz, qf[0 * kQueue + e], qf[1 * kQueue + e], qf[2 * kQueue + e],
+                o.x, o.y, o.z, qf[0 * kQueue + e], qf[1 * kQueue + e], qf[2 * kQueue + e],
                 qf[3 * kQueue + e], qf[4 * kQueue + e], qf[5 * kQueue + e], (pk >> 11) != 0u, te.bits,
-                te.cluster_pointer, P.far_plane, P.far_rcp, &J.counters[C_DDA_OVERRUN], work);
+                te.rec.cluster_pointer, P.far_plane, P.far_rcp, &J.counters[C_DDA_OVERRUN], work);
             // the minimum of 64 bits is a compare-and-swap loop: only where it can lower the word
             unsigned long long* const word = best + (pk & 31u);
             if (w < *(volatile unsigned long long*)word) atomicMin(word, w);
@@ -1172,16 +1224,12 @@ __device__ __forceinline__ void gather_records(const TileJob& J, uint32_t base, 
     for (uint32_t k = threadIdx.x; k < m; k += blockDim.x) {
         const uint32_t r = base + k;
         const uint2 qr = J.rects[r];
-        if (J.records[r].view == view && tx >= (qr.x & 0xffffu) && tx <= (qr.y & 0xffffu) && ty >= (qr.x >> 16) &&
-            ty <= (qr.y >> 16)) {
-            const VisRecord& rec = J.records[r];
+        const uint2 q1 = make_uint2(qr.y & 0xffffu, (qr.y & ~kListed) >> 16);
+        if (J.records[r].view == view && tx >= (qr.x & 0xffffu) && tx <= q1.x && ty >= (qr.x >> 16) && ty <= q1.y) {
             TileEntry& te = sm.stage()[atomicAdd(&sm.n(), 1u)];
-            te.ox = rec.ox; te.oy = rec.oy; te.oz = rec.oz;
-            te.cluster_pointer = rec.cluster_pointer;
-            te.object_idx = rec.object_idx;
-            te.d24_lb = rec.d24_lb;
+            te.rec = J.records[r];
 #pragma unroll
-            for (int w = 0; w < 16; w++) te.bits[w] = J.bits[(uint64_t)rec.cluster_idx * 16u + w];
+            for (int w = 0; w < 16; w++) te.bits[w] = J.bits[(uint64_t)te.rec.cluster_idx * 16u + w];
         }
     }
 }
@@ -1189,15 +1237,14 @@ __device__ __forceinline__ void gather_records(const TileJob& J, uint32_t base, 
 // Tile `slot` (in the job's heavy-first order) of one job: every pixel's
 // nearest packed word over the entries binned to the tile.  `phase` is the
 // parity of the CTA's bulk-copy mbarrier, carried across tiles.  Returns
-// false (the same in every thread) when a batch's copy did not complete in
+// false (the same in every thread) when a batch's copies did not complete in
 // time: the status word then holds TGX_ERR_TIMEOUT, the CTA has issued no
-// further copy, has waited once more (bounded) for the one in flight and has
-// written its pixels' words so far; it must not stage another tile.
+// further copy, every thread's own have landed and it has written its pixels'
+// words so far; it must not stage another tile.
 //
-// The tile's entries (record fields and bitmask, contiguous and sorted near
-// to far by depth bucket) arrive kBatch at a time by one cp.async.bulk; the
-// first copy is issued before the pixels' rays are set up, so the two
-// overlap.  Per batch every lane walks the entries for its own pixel: the
+// The tile's entries (sorted near to far by depth bucket) arrive kBatch at a
+// time (stage_entries); the first copies are issued before the pixels' rays are
+// set up, so the two overlap.  Per batch every lane walks the entries for its own pixel: the
 // depth skip, the cluster-space direction (once per object), and the
 // conservative slab test.  The pairs that survive are compacted by warp
 // ballot into the warp's ring; whenever it holds 32, all 32 lanes take one
@@ -1215,10 +1262,7 @@ __device__ __forceinline__ bool vis_tile(const TileJob& J, uint32_t slot, const 
 #pragma unroll
         for (int i = 0; i < W_COUNT; i++) work[i] = 0u;
     }
-    // the CTA's previous tile is done with the shared state (its generic reads of the stage
-    // ordered before the bulk copy that overwrites it)
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
+    __syncthreads();   // the CTA's previous tile is done with the shared state
     const uint4 si = J.slot_info[slot];   // one load: the tile and its entry range
     const uint32_t tile = si.x;
     // bins overflowed this frame: gather every record whose tile rectangle holds the tile (slow, exact)
@@ -1236,10 +1280,8 @@ __device__ __forceinline__ bool vis_tile(const TileJob& J, uint32_t slot, const 
         return true;
     }
     const TileEntry* const E = sm.stage();
-    if (threadIdx.x == 0) {
-        if (!scan_all && end > begin) stage_entries(sm.bar(), E, J.entries + begin, min(J.batch, end - begin), J.extra_tx);
-        sm.view() = tile_view(J, tile);
-    }
+    if (!scan_all && end > begin) stage_entries(J, sm.bar(), E, begin, min(J.batch, end - begin), J.extra_tx);
+    if (threadIdx.x == 0) sm.view() = tile_view(J, tile);
     sm.best()[threadIdx.x] = ULLONG_MAX;
     __syncthreads();
     const uint32_t view = sm.view();
@@ -1259,9 +1301,8 @@ __device__ __forceinline__ bool vis_tile(const TileJob& J, uint32_t slot, const 
             n = min(J.batch, end - base);
             if (base != begin) {
                 // the previous batch is fully consumed; after a lost copy nobody stages another
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 if (__syncthreads_or(lost)) break;
-                if (threadIdx.x == 0) stage_entries(sm.bar(), E, J.entries + base, n, 0u);
+                stage_entries(J, sm.bar(), E, base, n, 0u);
             }
             base += n;
             lost = __any_sync(0xffffffffu, !mbar_wait_bounded(sm.bar(), phase));
@@ -1283,20 +1324,16 @@ __device__ __forceinline__ bool vis_tile(const TileJob& J, uint32_t slot, const 
         tile_batch<kCount, 1>(J, E, 0u, n, P, q, best0, work);
         // every pixel already nearer than the rest of the (bucket-sorted) entries: the tile is done
         if (!scan_all && base < end) {
-            const uint32_t lo = bucket_lo(depth_bucket(E[n - 1].d24_lb, J.bshift), J.bshift);
+            const uint32_t lo = bucket_lo(depth_bucket(E[n - 1].rec.d24_lb, J.bshift), J.bshift);
             if (__syncthreads_and(!P.valid || P.best_d24 < lo)) break;
         }
     }
     const unsigned long long best = sm.best()[threadIdx.x];
     if (__syncthreads_or(lost)) {
-        // a batch's copy did not complete: report it, give the copy still in
-        // flight one more bounded wait so it does not land after the CTA is
-        // gone, and write the words found so far
-        if (threadIdx.x == 0) {
-            dev_error(status, TGX_ERR_TIMEOUT, 5, tile);
-            mbar_wait_bounded(sm.bar(), phase ^ 1u);
-        }
-        __syncthreads();
+        // a batch's copies did not complete: report it, let this thread's own
+        // land before the CTA is gone, and write the words found so far
+        if (threadIdx.x == 0) dev_error(status, TGX_ERR_TIMEOUT, 5, tile);
+        own_copies_wait();
         if (P.valid) J.outs[view][(size_t)P.py * vc.width + P.px] = best;
         return false;
     }
@@ -1342,15 +1379,13 @@ __device__ __forceinline__ void vis_tile_groups(const TileJob& J, uint32_t slot,
         return;
     }
     const uint32_t n_batches = scan_all ? 0u : (si.z + J.batch - 1u) / J.batch;
-    uint32_t issued = 0;             // batches staged so far (thread 0)
     auto stage = [&](uint32_t j) {   // batch j, in order
-        issued = j + 1u;
         const uint32_t first = j * J.batch;
-        stage_entries(sm.bar(j % kStages), sm.stage() + (j % kStages) * kBatch, J.entries + si.y + first,
-                      min(J.batch, si.z - first), j == 0u ? J.extra_tx : 0u);
+        stage_entries(J, sm.bar(j % kStages), sm.stage() + (j % kStages) * kBatch, si.y + first, min(J.batch, si.z - first),
+                      j == 0u ? J.extra_tx : 0u);
     };
+    for (uint32_t j = 0; j < min(n_batches, kStages); j++) stage(j);
     if (threadIdx.x == 0) {
-        for (uint32_t j = 0; j < min(n_batches, kStages); j++) stage(j);
         sm.view() = tile_view(J, tile);
         sm.lost() = 0u;
     }
@@ -1375,21 +1410,16 @@ __device__ __forceinline__ void vis_tile_groups(const TileJob& J, uint32_t slot,
         } else {
             P.best_d24 = min(P.best_d24, (uint32_t)(best0[lane] >> 40));   // the other groups' words too
             tile_batch<false, kGroups>(J, E, grp, n, P, q, best0, nullptr);
-            lo = bucket_lo(depth_bucket(E[n - 1].d24_lb, J.bshift), J.bshift);
+            lo = bucket_lo(depth_bucket(E[n - 1].rec.d24_lb, J.bshift), J.bshift);
         }
         // the batch is consumed; every pixel already nearer than the rest of the (bucket-sorted) entries: done
         const bool done = __syncthreads_and(!P.valid || P.best_d24 < lo);
         j++;
         if (done || sm.lost()) break;
-        if (threadIdx.x == 0 && j + kStages - 1u < n_batches) stage(j + kStages - 1u);
+        if (j + kStages - 1u < n_batches) stage(j + kStages - 1u);
     }
-    if (threadIdx.x == 0) {
-        // no copy may land after the CTA is gone: wait (bounded) for the batches staged and not consumed
-        bool late = sm.lost() != 0u;
-        for (uint32_t k = late ? j - 1u : j; k < issued; k++)
-            late |= !mbar_wait_bounded(sm.bar(k % kStages), (k / kStages) & 1u);
-        if (late) dev_error(status, TGX_ERR_TIMEOUT, 5, tile);
-    }
+    own_copies_wait();   // none may land after the CTA is gone
+    if (threadIdx.x == 0 && sm.lost()) dev_error(status, TGX_ERR_TIMEOUT, 5, tile);
     if (scan_all) {
         const uint32_t tx = (tile - vc.tile_base) % vc.tiles_x, ty = (tile - vc.tile_base) / vc.tiles_x;
         const uint32_t n_rec = J.counters[C_RECORDS];
@@ -1440,10 +1470,12 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_vis_tiles_groups(
     tile_smem_init(sm);
     if (threadIdx.x == 0) {
 #pragma unroll
-        for (uint32_t i = 1; i < kStages; i++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(sm.bar(i)));
+        for (uint32_t i = 1; i < kStages; i++)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(sm.bar(i)), "r"(blockDim.x));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     pdl_wait();
+    __syncthreads();   // every thread arrives on the mbarriers
     const uint32_t slot = J.interleave ? tile_slot(blockIdx.x, J.n_tiles, J.counters[C_NONEMPTY], true) : blockIdx.x;
     vis_tile_groups<kGroups>(J, slot, sm, status);
 }
@@ -1569,16 +1601,22 @@ struct VisScratch
     uint32_t* cta_aux;
     uint32_t* tile_off;
     uint4* slot_info;
-    TileEntry* entries;
-    uint32_t bin_capacity;     // entries
+    TileRef* refs;
+    uint32_t bin_capacity;     // references
+    uint2* chunks;             // chunk list of the records of many tiles
+    uint32_t chunk_cap;
 };
+
+// places of the chunk list: a frame lists about entries / kChunkTiles + (records of many tiles)
+static uint32_t vis_chunk_cap(uint32_t n_tiles) { return std::max<uint32_t>(1u << 16, n_tiles); }
 
 // bytes of the tile-sized part of the scratch
 // (the bucket arrays are sized for the finest setting, kMaxBuckets per tile)
 static size_t vis_tile_bytes(uint32_t n_tiles)
 {
     const uint32_t n_scan_ctas = (n_tiles + kScanTiles - 1) / kScanTiles;
-    return (size_t)n_tiles * kMaxBuckets * 4 * 2 + (size_t)n_tiles * 4 + (size_t)n_scan_ctas * (1 + kOrderClasses) * 4;
+    return (size_t)n_tiles * kMaxBuckets * 4 * 2 + (size_t)n_tiles * 4 + (size_t)n_scan_ctas * (1 + kOrderClasses) * 4 + 8 +
+           (size_t)vis_chunk_cap(n_tiles) * sizeof(uint2);
 }
 
 // bytes of the tile offsets (n_tiles + 1 words, padded to 16 bytes) and the slot records
@@ -1593,6 +1631,9 @@ static void vis_carve_tiles(VisScratch& w, uint32_t* tile_cnt, uint32_t* tile_of
     w.bucket_off = w.bucket_cnt + (size_t)n_tiles * kMaxBuckets;
     w.tile_total = w.bucket_off + (size_t)n_tiles * kMaxBuckets;
     w.cta_aux = w.tile_total + n_tiles;
+    const size_t words = (size_t)n_tiles * (2 * kMaxBuckets + 1) + (size_t)((n_tiles + kScanTiles - 1) / kScanTiles) * (1 + kOrderClasses);
+    w.chunks = reinterpret_cast<uint2*>(tile_cnt + ((words + 1) & ~(size_t)1));
+    w.chunk_cap = vis_chunk_cap(n_tiles);
     w.tile_off = tile_off;
     w.slot_info = reinterpret_cast<uint4*>(w.tile_off + ((n_tiles + 4u) & ~3u));
 }
@@ -1608,7 +1649,7 @@ static TileJob tile_job(const tgx_ctx* c, const tgx_scene* s, const ViewConst* d
     J.drain = c->vis_drain;
     J.records = w.records;
     J.rects = w.rects;
-    J.entries = w.entries;
+    J.refs = w.refs;
     J.tile_off = w.tile_off;
     J.slot_info = w.slot_info;
     J.views = d_vc;
@@ -1658,10 +1699,10 @@ static tgx_status vis_launch(tgx_ctx* c, const tgx_scene* s, const ViewConst* d_
         TGX_LAUNCH(c, TR_VIS_SETUP, setup_blocks, 256, 0, k_vis_cluster_setup<true>,
                    s->d_objects, s->d_cluster_pointers, s->d_c2o, s->d_bits, s->d_cp_obj, s->n_cluster_pointers,
                    d_vc, n_views, w.records, w.rects, w.rec_cap, w.counters, w.bucket_cnt,
-                   n_tiles * (kMaxBuckets >> bshift), c->d_status);
+                   n_tiles * (kMaxBuckets >> bshift), w.chunks, w.chunk_cap, c->d_status);
         // each later pass is a programmatic dependent of the one before
         TGX_LAUNCH_PDL(c, TR_VIS_COUNT, warp_grid, 256, 0, k_vis_count, w.records, w.rects, w.counters, w.rec_cap,
-                       s->d_objects, d_vc, w.bucket_cnt, n_tiles, bshift);
+                       s->d_objects, d_vc, w.bucket_cnt, n_tiles, bshift, w.chunks, w.chunk_cap);
         if (bshift == 0)
             TGX_LAUNCH_PDL(c, TR_VIS_PREFIX, n_scan_ctas, kScanTiles, 0, k_vis_prefix<32>, w.bucket_cnt, w.bucket_off,
                            w.tile_total, n_tiles, w.cta_aux);
@@ -1683,8 +1724,8 @@ static tgx_status vis_launch(tgx_ctx* c, const tgx_scene* s, const ViewConst* d_
     }
     if (phase == VIS_TO_SCAN) return TGX_OK;
     TGX_LAUNCH_PDL(c, TR_VIS_BIN, warp_grid, 256, 0, k_vis_bin_fill,
-                   w.records, w.rects, w.counters, d_vc, w.tile_off, w.bucket_off, w.bucket_cnt, w.entries,
-                   s->d_bits, n_tiles, w.bin_capacity, bshift, c->d_status);
+                   w.records, w.rects, w.counters, d_vc, w.tile_off, w.bucket_off, w.bucket_cnt, w.refs,
+                   n_tiles, w.bin_capacity, bshift, w.chunks, w.chunk_cap, c->d_status);
     if (phase == VIS_NO_TILES) return TGX_OK;
     TileJob J = tile_job(c, s, d_vc, d_outs, n_views, n_tiles, w);
     J.interleave = interleave ? 1u : 0u;
@@ -1816,7 +1857,7 @@ tgx_status vis_render_device(tgx_ctx* c, const tgx_scene* s, const tgx_view* vie
     if (n_pairs > 0xffffffffull) { tgx_set_error("too many (view, cluster) pairs"); return TGX_ERR_CAPACITY; }
     VisScratch w;
     bool exact = false;
-    constexpr size_t kEntry = sizeof(TileEntry);
+    constexpr size_t kEntry = sizeof(TileRef);
     if (c->flags & TGX_FLAG_MIN_BIN_CAPACITY) {
         TGX_TRY(devbuf_reserve(c->vis_bins, 64 * kEntry));
         w.bin_capacity = 64;
@@ -1840,7 +1881,7 @@ tgx_status vis_render_device(tgx_ctx* c, const tgx_scene* s, const tgx_view* vie
     w.records = (VisRecord*)c->vis_records.ptr;
     w.rects = (uint2*)(w.records + w.rec_cap);
     w.counters = (uint32_t*)c->vis_counters.ptr;
-    w.entries = (TileEntry*)c->vis_bins.ptr;
+    w.refs = (TileRef*)c->vis_bins.ptr;
     vis_carve_tiles(w, (uint32_t*)c->vis_tile_cnt.ptr, (uint32_t*)c->vis_tile_off.ptr, n_tiles);
     if (!exact) {
         TGX_TRY(vis_launch(c, s, d_vc, d_outs, n_views, n_tiles, w, VIS_ALL, host_out));
@@ -1851,7 +1892,7 @@ tgx_status vis_render_device(tgx_ctx* c, const tgx_scene* s, const tgx_view* vie
         const uint32_t entries = ((const uint32_t*)c->h_vis_counters)[C_ENTRIES];
         if (entries > w.bin_capacity) {
             TGX_TRY(devbuf_reserve(c->vis_bins, (size_t)entries * kEntry));
-            w.entries = (TileEntry*)c->vis_bins.ptr;
+            w.refs = (TileRef*)c->vis_bins.ptr;
             w.bin_capacity = (uint32_t)std::min<size_t>(c->vis_bins.bytes / kEntry, 0xffffffffu);
             if (entries <= w.bin_capacity) TGX_CUDA(cudaMemsetAsync(w.counters + C_OVERFLOW, 0, 4, c->stream));
         }
@@ -1914,7 +1955,7 @@ extern "C" tgx_status tgx_frame_graph_create(tgx_ctx* c, const tgx_vis_job* jobs
     std::vector<std::vector<unsigned char>> tables(n_jobs);
     auto job_bytes = [&](const tgx_frame_graph::Job& job) {
         return al((size_t)job.rec_cap * (sizeof(VisRecord) + sizeof(uint2))) + 256 + al(vis_tile_bytes(job.n_tiles)) +
-               al(vis_off_bytes(job.n_tiles)) + al((size_t)job.bin_cap * sizeof(TileEntry));
+               al(vis_off_bytes(job.n_tiles)) + al((size_t)job.bin_cap * sizeof(TileRef));
     };
     for (uint32_t j = 0; j < n_jobs; j++) {
         const tgx_vis_job& jb = jobs[j];
@@ -1974,7 +2015,7 @@ extern "C" tgx_status tgx_frame_graph_create(tgx_ctx* c, const tgx_vis_job* jobs
         p += al(vis_tile_bytes(job.n_tiles));
         uint32_t* tile_off = (uint32_t*)p;
         p += al(vis_off_bytes(job.n_tiles));
-        w.entries = (TileEntry*)p;
+        w.refs = (TileRef*)p;
         w.bin_capacity = (uint32_t)job.bin_cap;
         vis_carve_tiles(w, tile_cnt, tile_off, job.n_tiles);
         const ViewConst* d_vc = (const ViewConst*)(base + job.table_off);
@@ -2299,7 +2340,9 @@ constexpr size_t kNaScanAux = kNaTileTotal + na_align((size_t)kNaMaxTiles * 4);
 constexpr size_t kNaTileOff = kNaScanAux + na_align(((size_t)kNaMaxTiles / kScanTiles + 1) * (1 + kOrderClasses) * 4);
 constexpr size_t kNaSlotInfo = kNaTileOff + na_align(((size_t)kNaMaxTiles + 4) * 4);
 constexpr size_t kNaBinsOff = kNaSlotInfo + na_align((size_t)kNaMaxTiles * 16);
-constexpr size_t kNaBytes = kNaBinsOff + na_align((size_t)kNaBins * sizeof(TileEntry));   // about 51 MiB
+constexpr uint32_t kNaChunks = 1u << 16;
+constexpr size_t kNaChunkOff = kNaBinsOff + na_align((size_t)kNaBins * sizeof(TileRef));
+constexpr size_t kNaBytes = kNaChunkOff + na_align((size_t)kNaChunks * sizeof(uint2));   // about 29 MiB
 
 // The scratch.  In host code this name is only a host-side stand-in: its
 // device address is taken with cudaGetSymbolAddress below.
@@ -2425,7 +2468,8 @@ extern "C" tgx_status tgx_vis_render_noalloc(void* stream, const tgx_object* d_o
     uint32_t* cta_aux = (uint32_t*)(base + kNaScanAux);
     uint32_t* tile_off = (uint32_t*)(base + kNaTileOff);
     uint4* slot_info = (uint4*)(base + kNaSlotInfo);
-    TileEntry* entries = (TileEntry*)(base + kNaBinsOff);
+    TileRef* refs = (TileRef*)(base + kNaBinsOff);
+    uint2* chunks = (uint2*)(base + kNaChunkOff);
 
     int sms = 0;
     TGX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
@@ -2436,9 +2480,10 @@ extern "C" tgx_status tgx_vis_render_noalloc(void* stream, const tgx_object* d_o
               counters, status, d_objects, n_objects, inv_rot);
     NA_LAUNCH((n_cluster_pointers + 255) / 256, 256, k_vis_cluster_setup<false>, d_objects, d_cluster_pointers,
               d_cluster_idx_to_object_idx, d_voxel_bits, (const uint32_t*)nullptr, n_cluster_pointers, d_vc, 1u,
-              records, rects, kNaMaxClusterPointers, counters, bucket_cnt, n_tiles * kNaBuckets, status);
+              records, rects, kNaMaxClusterPointers, counters, bucket_cnt, n_tiles * kNaBuckets, chunks, kNaChunks,
+              status);
     NA_LAUNCH(warp_grid, 256, k_vis_count, records, rects, counters, kNaMaxClusterPointers, d_objects, d_vc, bucket_cnt,
-              n_tiles, 1u);
+              n_tiles, 1u, chunks, kNaChunks);
     const uint32_t n_scan_ctas = (n_tiles + kScanTiles - 1) / kScanTiles;
     NA_LAUNCH(n_scan_ctas, kScanTiles, k_vis_prefix<kNaBuckets>, bucket_cnt, bucket_off, tile_total, n_tiles, cta_aux);
     if (n_scan_ctas <= kDirectGroups) {
@@ -2448,12 +2493,12 @@ extern "C" tgx_status tgx_vis_render_noalloc(void* stream, const tgx_object* d_o
         NA_LAUNCH(1, 1024, k_vis_scan, cta_aux, n_tiles, tile_off, kNaBins, counters);
         NA_LAUNCH(n_scan_ctas, kScanTiles, k_vis_finalize, tile_total, n_tiles, cta_aux, tile_off, slot_info);
     }
-    NA_LAUNCH(warp_grid, 256, k_vis_bin_fill, records, rects, counters, d_vc, tile_off, bucket_off, bucket_cnt, entries,
-              d_voxel_bits, n_tiles, kNaBins, 1u, status);
+    NA_LAUNCH(warp_grid, 256, k_vis_bin_fill, records, rects, counters, d_vc, tile_off, bucket_off, bucket_cnt, refs,
+              n_tiles, kNaBins, 1u, chunks, kNaChunks, status);
     TileJob J;
     J.records = records;
     J.rects = rects;
-    J.entries = entries;
+    J.refs = refs;
     J.tile_off = tile_off;
     J.slot_info = slot_info;
     J.views = d_vc;
