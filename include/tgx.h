@@ -244,7 +244,7 @@ tgx_status  tgx_vis_host_wait(tgx_ctx* ctx, uint32_t max_in_flight);
  * (objects, cluster pointers, cluster->object map, voxel bits; indices are
  * trusted, not validated), the view on the host, and a DEVICE output of
  * width*height u64.  The result equals tgx_vis_render's bit for bit.  All
- * scratch lives in one fixed device array of about 29 MiB inside the library,
+ * scratch lives in one fixed device array of about 28 MiB inside the library,
  * which every GPU that loads the library holds until the process exits.
  * Limits: at most 65,536 objects, 524,288 cluster pointers and 32,768 screen
  * tiles of 16x16 pixels (3840x2160 fits); larger inputs are rejected with

@@ -370,6 +370,7 @@ struct ViewConst
     float inv_basis[9];        // row-major
     float fwd[3];              // unit view axis
     float planes[12];          // inward unit normals of the 4 side planes of the frustum
+    uint32_t tile_w_rcp;       // ceil(2^20 / tile_w)
 };
 
 void trace_begin(tgx_ctx* ctx, int slot);

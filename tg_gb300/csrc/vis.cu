@@ -12,17 +12,16 @@
 //   2. k_vis_count          per record: the ws2ms matrix and the camera
 //      position in cluster space exactly as the shader does (one thread per
 //      record), and its counts per (tile, depth bucket) (a half-warp per record).
-//   3. k_vis_prefix         per tile: offsets of its 16 depth buckets; per
-//                           256 tiles: their sum and class histogram.
-//   4. k_vis_scan           one CTA: bases of the 256-tile groups and the
-//      k_vis_finalize       cursors of the launch order (heaviest class
-//                           first); then per group: tile offsets and order.
-//                           Up to 512 groups, k_vis_finalize_direct does both:
-//                           each CTA reads all groups' sums and histograms.
+//   3. k_vis_prefix         per tile: offsets of its depth buckets; per 256
+//                           tiles: their sum and class histogram, also added
+//                           up over 64 such groups.
+//   4. k_vis_finalize       per 256 tiles: the tiles' offsets and places in the
+//                           launch order (heaviest class first), from those sums.
 //   5. k_vis_bin_fill       a half-warp per record, a warp per 256 tiles of the
 //                           records of many: an 8-byte reference into each of
 //                           its (tile, bucket) bins, so every tile's references
-//                           are contiguous and run near to far.
+//                           are contiguous and run near to far; tiles without
+//                           entries are cleared.
 //   6. k_vis_tiles          one CTA per tile (heaviest first), one thread per
 //      pixel (k_vis_tiles_groups: several, for frames of few tiles): batches of
 //      the tile's entries (record and 64-byte bitmask) are gathered by cp.async
@@ -33,7 +32,7 @@
 //      surviving (pixel, cluster) pairs are compacted by warp ballot and run
 //      the shader's exact ray/box test and DDA on full warps, keeping each
 //      pixel's minimum packed depth|pointer|voxel word (shared atomicMin);
-//      every pixel is written once (fused clear).
+//      every pixel is written once.
 //      k_vis_tiles_queue is the persistent form over many jobs' tiles.
 //
 // Every pair evaluates the same binary32 operations in the same order as the
@@ -125,6 +124,17 @@ __device__ __forceinline__ uint32_t bucket_lo(uint32_t b, uint32_t bshift)
 {
     const uint32_t f = b << bshift;
     return f == 0u ? 0u : (f & 1u) ? (3u << ((f >> 1) + 7u)) : (1u << ((f >> 1) + 8u));
+}
+
+// p / tile_w for a pixel p < 512 of a tile (make_view_const: ceil(2^20 / tile_w))
+__device__ __forceinline__ uint32_t tile_row(const ViewConst& vc, uint32_t p) { return (p * vc.tile_w_rcp) >> 20; }
+
+// pixel `pix` of the tile at `place` (tile x | y << 16)
+__device__ __forceinline__ void tile_pixel_place(const ViewConst& vc, uint32_t place, uint32_t pix, uint32_t& px, uint32_t& py)
+{
+    const uint32_t row = tile_row(vc, pix);
+    px = (place & 0xffffu) * vc.tile_w + pix - row * vc.tile_w;
+    py = (place >> 16) * vc.tile_h + row;
 }
 
 __device__ __forceinline__ uint32_t warp_append(uint32_t* counter, bool pred)
@@ -368,18 +378,26 @@ __global__ void __launch_bounds__(256) k_vis_count(VisRecord* __restrict__ recor
 // ---------------------------------------------------------------------------
 // 3. per-tile bucket offsets (one thread per tile, bucket-major = coalesced),
 //    and per CTA of 256 tiles: the sum of the tile totals and the histogram
-//    of tile classes (cta_aux = [n_ctas sums][n_ctas x kOrderClasses])
+//    of tile classes (groups = [n_ctas][kGroupWords]: the sum, then the classes),
+//    added to those of its 64 CTAs (supers, zero before, the same layout)
 // ---------------------------------------------------------------------------
 
 constexpr uint32_t kScanTiles = 256;   // tiles per CTA of the prefix and finalize kernels
+constexpr uint32_t kSuperGroups = 64;  // CTAs whose sums are added up
+constexpr uint32_t kGroupWords = 1 + kOrderClasses;
+
+__host__ __device__ constexpr uint32_t scan_groups(uint32_t n_tiles) { return (n_tiles + kScanTiles - 1) / kScanTiles; }
+__host__ __device__ constexpr uint32_t scan_supers(uint32_t n_tiles)
+{
+    return (scan_groups(n_tiles) + kSuperGroups - 1) / kSuperGroups;
+}
 
 __device__ __forceinline__ uint32_t tile_class(uint32_t total) { return total ? 32u - __clz(total) : 0u; }
 
 template <uint32_t kBuckets>
 __global__ void __launch_bounds__(kScanTiles) k_vis_prefix(uint32_t* __restrict__ bucket_cnt,
-                                                          uint32_t* __restrict__ bucket_off,
                                                           uint32_t* __restrict__ tile_total, uint32_t n_tiles,
-                                                          uint32_t* __restrict__ cta_aux)
+                                                          uint32_t* __restrict__ groups, uint32_t* __restrict__ supers)
 {
     __shared__ uint32_t cls[kOrderClasses];
     __shared__ uint32_t wsum[kScanTiles / 32];
@@ -390,13 +408,12 @@ __global__ void __launch_bounds__(kScanTiles) k_vis_prefix(uint32_t* __restrict_
     const uint32_t t = blockIdx.x * kScanTiles + threadIdx.x;
     uint32_t run = 0;
     if (t < n_tiles) {
-        uint32_t c[kBuckets];   // all loads first: the cursor reset below must not wait on them one by one
+        uint32_t c[kBuckets];   // all loads first: the stores below must not wait on them one by one
 #pragma unroll
         for (uint32_t b = 0; b < kBuckets; b++) c[b] = bucket_cnt[b * n_tiles + t];
 #pragma unroll
         for (uint32_t b = 0; b < kBuckets; b++) {
-            bucket_off[b * n_tiles + t] = run;
-            bucket_cnt[b * n_tiles + t] = 0;   // becomes the fill cursor
+            bucket_cnt[b * n_tiles + t] = run;   // becomes the fill cursor
             run += c[b];
         }
         tile_total[t] = run;
@@ -407,183 +424,72 @@ __global__ void __launch_bounds__(kScanTiles) k_vis_prefix(uint32_t* __restrict_
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     if ((threadIdx.x & 31u) == 0) wsum[threadIdx.x >> 5] = sum;
     __syncthreads();
-    const uint32_t n_ctas = (n_tiles + kScanTiles - 1) / kScanTiles;
-    if (threadIdx.x == 0) {
-        uint32_t tot = 0;
+    if (threadIdx.x < kGroupWords) {
+        uint32_t v = 0;
+        if (threadIdx.x == 0)
 #pragma unroll
-        for (uint32_t w = 0; w < kScanTiles / 32; w++) tot += wsum[w];
-        cta_aux[blockIdx.x] = tot;
-    }
-    if (threadIdx.x < kOrderClasses) cta_aux[n_ctas + blockIdx.x * kOrderClasses + threadIdx.x] = cls[threadIdx.x];
-}
-
-// ---------------------------------------------------------------------------
-// 4. one CTA: exclusive scan of the per-CTA sums (-> CTA bases) and, per
-//    tile class (heaviest first), the exclusive scan over CTAs of the class
-//    counts (-> per-(CTA, class) cursors of the launch order)
-// ---------------------------------------------------------------------------
-
-__global__ void __launch_bounds__(1024) k_vis_scan(uint32_t* __restrict__ cta_aux, uint32_t n_tiles,
-                                                   uint32_t* __restrict__ tile_off, uint32_t bin_capacity,
-                                                   uint32_t* __restrict__ counters)
-{
-    __shared__ uint32_t warp_sums[32];
-    __shared__ uint32_t cls_tot[kOrderClasses];
-    __shared__ uint32_t cls_base[kOrderClasses];
-    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
-    const uint32_t n_ctas = (n_tiles + kScanTiles - 1) / kScanTiles;
-    uint32_t* cls_cnt = cta_aux + n_ctas;
-    pdl_wait();
-    pdl_trigger();
-    // CTA bases
-    uint32_t carry = 0;
-    for (uint32_t base = 0; base < n_ctas; base += 1024) {
-        const uint32_t i = base + threadIdx.x;
-        const uint32_t x = i < n_ctas ? cta_aux[i] : 0u;
-        uint32_t incl = x;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-            if ((int)lane >= o) incl += y;
-        }
-        if (lane == 31) warp_sums[wid] = incl;
-        __syncthreads();
-        if (wid == 0) {
-            uint32_t w = warp_sums[lane];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
-                if ((int)lane >= o) w += y;
-            }
-            warp_sums[lane] = w;
-        }
-        __syncthreads();
-        if (i < n_ctas) cta_aux[i] = carry + (wid ? warp_sums[wid - 1] : 0u) + incl - x;
-        carry += warp_sums[31];
-        __syncthreads();
-    }
-    // class totals (warp c sums class c over the CTAs)
-    uint32_t tot = 0;
-#pragma unroll 4
-    for (uint32_t b = lane; b < n_ctas; b += 32) tot += cls_cnt[b * kOrderClasses + wid];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-    if (lane == 0) cls_tot[wid] = tot;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        tile_off[n_tiles] = carry;
-        counters[C_ENTRIES] = carry;
-        counters[C_OVERFLOW] = carry > bin_capacity ? 1u : 0u;
-        counters[C_NONEMPTY] = n_tiles - cls_tot[0];   // class 0: the tiles without entries
-        uint32_t run = 0;   // heaviest class first
-        for (int c = (int)kOrderClasses - 1; c >= 0; c--) {
-            cls_base[c] = run;
-            run += cls_tot[c];
-        }
-    }
-    __syncthreads();
-    // per-(CTA, class) cursors: warp c scans class c over the CTAs
-    uint32_t run = cls_base[wid];
-    for (uint32_t b0 = 0; b0 < n_ctas; b0 += 128) {   // four chunks of 32 CTAs: loads first
-        uint32_t x[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const uint32_t b = b0 + 32u * j + lane;
-            x[j] = b < n_ctas ? cls_cnt[b * kOrderClasses + wid] : 0u;
-        }
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const uint32_t b = b0 + 32u * j + lane;
-            uint32_t incl = x[j];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-                if ((int)lane >= o) incl += y;
-            }
-            if (b < n_ctas) cls_cnt[b * kOrderClasses + wid] = run + incl - x[j];
-            run += __shfl_sync(0xffffffffu, incl, 31);
-        }
+            for (uint32_t w = 0; w < kScanTiles / 32; w++) v += wsum[w];
+        else v = cls[threadIdx.x - 1];
+        groups[blockIdx.x * kGroupWords + threadIdx.x] = v;
+        if (v) atomicAdd(&supers[blockIdx.x / kSuperGroups * kGroupWords + threadIdx.x], v);
     }
 }
 
 // ---------------------------------------------------------------------------
-// 4b. per CTA of 256 tiles: tile offsets (CTA base + scan of the totals) and
-//     each tile's place in the launch order
+// 4. per CTA of 256 tiles: every tile's offset and place in the launch order
+//    (heaviest class first).  Its base and class cursors come from the sums of
+//    all supers and of the groups before it in its own.
+//    (One CTA that scanned all groups' sums first took 104 us at 3488 groups;
+//    reading every group's sums in every CTA 10 us at 507, 7 at 127.)
 // ---------------------------------------------------------------------------
 
 __global__ void __launch_bounds__(kScanTiles) k_vis_finalize(const uint32_t* __restrict__ tile_total, uint32_t n_tiles,
-                                                            const uint32_t* __restrict__ cta_aux,
+                                                            const uint32_t* __restrict__ groups,
+                                                            const uint32_t* __restrict__ supers,
                                                             uint32_t* __restrict__ tile_off,
-                                                            uint4* __restrict__ slot_info)
-{
-    __shared__ uint32_t cur[kOrderClasses];
-    __shared__ uint32_t wsum[kScanTiles / 32];
-    const uint32_t n_ctas = (n_tiles + kScanTiles - 1) / kScanTiles;
-    pdl_wait();
-    pdl_trigger();
-    if (threadIdx.x < kOrderClasses) cur[threadIdx.x] = cta_aux[n_ctas + blockIdx.x * kOrderClasses + threadIdx.x];
-    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
-    const uint32_t t = blockIdx.x * kScanTiles + threadIdx.x;
-    const bool valid = t < n_tiles;
-    const uint32_t x = valid ? tile_total[t] : 0u;
-    uint32_t incl = x;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-        if ((int)lane >= o) incl += y;
-    }
-    if (lane == 31) wsum[wid] = incl;
-    __syncthreads();
-    uint32_t before = cta_aux[blockIdx.x];
-    for (uint32_t w = 0; w < wid; w++) before += wsum[w];
-    if (valid) {
-        const uint32_t off = before + incl - x;
-        tile_off[t] = off;
-        slot_info[atomicAdd(&cur[tile_class(x)], 1u)] = make_uint4(t, off, x, 0u);
-    }
-}
-
-// ---------------------------------------------------------------------------
-// 4'. frames of at most kDirectGroups groups skip the one-CTA scan: every
-//     CTA of the finalize derives its own group base and class cursors from
-//     all groups' sums and class histograms (read from L2; 127 x 33 words at
-//     1080p), then places its tiles as k_vis_finalize does.  Same offsets,
-//     order and counters as k_vis_scan + k_vis_finalize.
-// ---------------------------------------------------------------------------
-
-constexpr uint32_t kDirectGroups = 512;
-
-__global__ void __launch_bounds__(kScanTiles) k_vis_finalize_direct(const uint32_t* __restrict__ tile_total,
-                                                                   uint32_t n_tiles,
-                                                                   const uint32_t* __restrict__ cta_aux,
-                                                                   uint32_t* __restrict__ tile_off,
-                                                                   uint4* __restrict__ slot_info,
-                                                                   uint32_t bin_capacity,
-                                                                   uint32_t* __restrict__ counters)
+                                                            uint4* __restrict__ slot_info, uint32_t bin_capacity,
+                                                            uint32_t* __restrict__ counters,
+                                                            const ViewConst* __restrict__ views, uint32_t n_views)
 {
     constexpr uint32_t kWarps = kScanTiles / 32;
     __shared__ uint32_t cur[kOrderClasses];
     __shared__ uint32_t part_tot[kWarps][kOrderClasses], part_pre[kWarps][kOrderClasses];
     __shared__ uint32_t red_pre[kWarps], red_all[kWarps], wsum[kWarps];
-    const uint32_t n_ctas = (n_tiles + kScanTiles - 1) / kScanTiles;
     const uint32_t g = blockIdx.x, lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    const uint32_t sg = g / kSuperGroups, n_supers = scan_supers(n_tiles);
+    const uint32_t t = g * kScanTiles + threadIdx.x;
+    const bool valid = t < n_tiles;
+    // the tile's view and place in it; the view table is older than the kernels
+    // before, whose end need not be awaited for it
+    uint32_t view = 0, place = 0;
+    if (valid) {
+        uint32_t hi = n_views - 1;   // the last view whose first tile is <= t
+        while (view < hi) {
+            const uint32_t mid = (view + hi + 1) >> 1;
+            if (views[mid].tile_base <= t) view = mid; else hi = mid - 1;
+        }
+        const uint32_t lt = t - views[view].tile_base, tiles_x = views[view].tiles_x;
+        place = lt % tiles_x | (lt / tiles_x) << 16;
+    }
     pdl_wait();
     pdl_trigger();
-    // this group's base (the sums of the groups before it) and the frame's total
+    // this group's base (the sums before it) and the frame's total
     uint32_t pre = 0, all = 0;
-    for (uint32_t i = threadIdx.x; i < n_ctas; i += kScanTiles) {
-        const uint32_t v = cta_aux[i];
+    for (uint32_t i = threadIdx.x; i < n_supers; i += kScanTiles) {
+        const uint32_t v = supers[i * kGroupWords];
         all += v;
-        pre += i < g ? v : 0u;
+        pre += i < sg ? v : 0u;
     }
+    const uint32_t own = sg * kSuperGroups + threadIdx.x;   // kSuperGroups <= kScanTiles
+    if (own < g) pre += groups[own * kGroupWords];
     // per class (lane): its count over all groups and over the groups before this one
-    const uint32_t* cls_cnt = cta_aux + n_ctas;
     uint32_t ct = 0, cp = 0;
-    for (uint32_t b = wid; b < n_ctas; b += kWarps) {
-        const uint32_t v = cls_cnt[b * kOrderClasses + lane];
+    for (uint32_t b = wid; b < n_supers; b += kWarps) {
+        const uint32_t v = supers[b * kGroupWords + 1u + lane];
         ct += v;
-        cp += b < g ? v : 0u;
+        cp += b < sg ? v : 0u;
     }
+    for (uint32_t b = sg * kSuperGroups + wid; b < g; b += kWarps) cp += groups[b * kGroupWords + 1u + lane];
     part_tot[wid][lane] = ct;
     part_pre[wid][lane] = cp;
 #pragma unroll
@@ -593,8 +499,6 @@ __global__ void __launch_bounds__(kScanTiles) k_vis_finalize_direct(const uint32
     }
     if (lane == 0) { red_pre[wid] = pre; red_all[wid] = all; }
     // the tiles' totals, scanned within each warp
-    const uint32_t t = g * kScanTiles + threadIdx.x;
-    const bool valid = t < n_tiles;
     const uint32_t x = valid ? tile_total[t] : 0u;
     uint32_t incl = x;
 #pragma unroll
@@ -622,7 +526,6 @@ __global__ void __launch_bounds__(kScanTiles) k_vis_finalize_direct(const uint32
 #pragma unroll
     for (uint32_t w = 0; w < kWarps; w++) { base += red_pre[w]; total += red_all[w]; }
     if (g == 0 && threadIdx.x == 0) {
-        tile_off[n_tiles] = total;
         counters[C_ENTRIES] = total;
         counters[C_OVERFLOW] = total > bin_capacity ? 1u : 0u;
     }
@@ -630,7 +533,7 @@ __global__ void __launch_bounds__(kScanTiles) k_vis_finalize_direct(const uint32
     if (valid) {
         const uint32_t off = base + incl - x;
         tile_off[t] = off;
-        slot_info[atomicAdd(&cur[tile_class(x)], 1u)] = make_uint4(t, off, x, 0u);
+        slot_info[atomicAdd(&cur[tile_class(x)], 1u)] = make_uint4(view, off, x, place);
     }
 }
 
@@ -640,6 +543,8 @@ __global__ void __launch_bounds__(kScanTiles) k_vis_finalize_direct(const uint32
 //    bucket and writes the 8-byte reference there.  (Writing the 96-byte entry
 //    itself took 26 us at 1080p, 512 objects, and 210 us for 7.3 M entries;
 //    the tile kernel gathers it as quickly from the record as from a copy.)
+//    Then a warp per tile without entries clears it, unless that is left to the
+//    tile kernel, which spreads writes to host memory over its time.
 // ---------------------------------------------------------------------------
 
 __global__ void __launch_bounds__(256) k_vis_bin_fill(const VisRecord* __restrict__ records,
@@ -647,16 +552,17 @@ __global__ void __launch_bounds__(256) k_vis_bin_fill(const VisRecord* __restric
                                                      const uint32_t* __restrict__ counters,
                                                      const ViewConst* __restrict__ views,
                                                      const uint32_t* __restrict__ tile_off,
-                                                     const uint32_t* __restrict__ bucket_off,
                                                      uint32_t* __restrict__ cursor, TileRef* __restrict__ refs,
                                                      uint32_t n_tiles, uint32_t bin_capacity, uint32_t bshift,
                                                      const uint2* __restrict__ chunks, uint32_t chunk_cap,
+                                                     const uint4* __restrict__ slot_info,
+                                                     unsigned long long* const* __restrict__ outs, uint32_t clear,
                                                      tgx_dev_status* __restrict__ status)
 {
     pdl_wait();
     pdl_trigger();
-    if (counters[C_OVERFLOW]) return;   // the tile kernel scans all records instead
-    const uint32_t n = counters[C_RECORDS];
+    // after an overflow the tile kernel scans all records instead
+    const uint32_t n = counters[C_OVERFLOW] ? 0u : counters[C_RECORDS];
     // tiles k, k + step, ... below end of record i, four at a time so that their atomics are in flight together
     auto fill = [&](uint32_t i, const TileRect& t, uint32_t k, uint32_t end, uint32_t step) {
         const VisRecord& rec = records[i];
@@ -671,7 +577,7 @@ __global__ void __launch_bounds__(256) k_vis_bin_fill(const VisRecord* __restric
                 const uint32_t kj = k + j * step;
                 if (kj >= end) continue;
                 const uint32_t tile = base + (kj / t.w) * vc.tiles_x + kj % t.w;
-                pos[j] = tile_off[tile] + bucket_off[row + tile] + atomicAdd(&cursor[row + tile], 1u);
+                pos[j] = tile_off[tile] + atomicAdd(&cursor[row + tile], 1u);
             }
 #pragma unroll
             for (uint32_t j = 0; j < 4u; j++) {
@@ -693,6 +599,18 @@ __global__ void __launch_bounds__(256) k_vis_bin_fill(const VisRecord* __restric
         if (r.y & kListed) continue;
         const TileRect t = tile_rect(r);
         fill(i, t, threadIdx.x & 15u, t.n, 16u);
+    }
+    if (!clear) return;
+    for (uint32_t slot = counters[C_NONEMPTY] + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); slot < n_tiles;
+         slot += (gridDim.x * blockDim.x) >> 5) {
+        const uint4 si = slot_info[slot];
+        const ViewConst& vc = views[si.x];
+        unsigned long long* const out = outs[si.x];
+        for (uint32_t p = threadIdx.x & 31u; p < vc.tile_w * vc.tile_h; p += 32u) {
+            uint32_t px, py;
+            tile_pixel_place(vc, si.w, p, px, py);
+            if (px < vc.width && py < vc.height) out[(size_t)py * vc.width + px] = ULLONG_MAX;
+        }
     }
 }
 
@@ -885,14 +803,14 @@ struct TileJob
     const VisRecord* records;
     const uint2* rects;
     const TileRef* refs;         // the bins, tile after tile
-    const uint32_t* tile_off;
-    const uint4* slot_info;      // per launch slot (heavy first): tile, first entry, entry count
+    const uint4* slot_info;      // per launch slot (heavy first): view, first entry, entry count, tile x | y << 16
     const ViewConst* views;
     const uint32_t* bits;
     const float* inv_rot;
     unsigned long long* const* outs;
     uint32_t* counters;
-    uint32_t n_views, n_tiles;
+    uint32_t n_tiles;
+    uint32_t cleared;            // tiles without entries are done (k_vis_bin_fill)
     uint32_t first;              // the job's first item in a multi-job work queue
     unsigned long long* work;    // W_COUNT work counters (counting variant of the tile kernel only)
     uint32_t bshift;             // depth buckets: 32 >> bshift
@@ -905,7 +823,7 @@ struct TileJob
 };
 
 // Shared memory of a tile CTA (dynamic, tile_smem_bytes(threads)):
-//   the mbarrier of the copies, the tile's view and a gather count;
+//   the mbarrier of the copies and a gather count;
 //   the staged batch: up to kBatch of the tile's 96-byte entries;
 //   every pixel's best packed word so far (the pair lanes' atomicMin target);
 //   per warp, a ring of kQueue live (pixel, entry) pairs waiting for a lane:
@@ -915,7 +833,7 @@ constexpr uint32_t kBatch = 48;                      // entries per staged batch
 constexpr uint32_t kQueue = 64;                      // ring entries per warp (an entry adds at most 32)
 constexpr uint32_t kWarpRays = 7 * kQueue;           // then the bounds of the warp's rays (warp_rays): 6 floats
 constexpr uint32_t kQueueWords = kWarpRays + 8;      // the ring: 6 float arrays + the packed word
-constexpr uint32_t kSmBar = 0, kSmView = 8, kSmN = 12, kSmLost = 16, kSmBars = 24;   // kSmBars: kStages - 1 more mbarriers
+constexpr uint32_t kSmBar = 0, kSmN = 12, kSmLost = 16, kSmBars = 24;   // kSmBars: kStages - 1 more mbarriers
 constexpr uint32_t kSmStage = 128;                   // 16-byte aligned copy target
 constexpr uint32_t kStages = 2;                      // stages of a tile with several groups of threads (vis_tile_groups)
 __host__ __device__ constexpr uint32_t tile_best_off(uint32_t groups)
@@ -935,7 +853,6 @@ struct TileSm
     // mbarrier of stage i (stage 0's is that of the single-stage tiles)
     __device__ __forceinline__ uint32_t bar(uint32_t i) const { return smem_addr(p + (i ? kSmBars + 8u * (i - 1u) : kSmBar)); }
     __device__ __forceinline__ volatile uint32_t& lost() const { return *(volatile uint32_t*)(p + kSmLost); }
-    __device__ __forceinline__ uint32_t& view() const { return *(uint32_t*)(p + kSmView); }
     __device__ __forceinline__ uint32_t& n() const { return *(uint32_t*)(p + kSmN); }
     __device__ __forceinline__ TileEntry* stage() const { return (TileEntry*)(p + kSmStage); }
     __device__ __forceinline__ unsigned long long* best() const { return (unsigned long long*)(p + best_off); }
@@ -1004,11 +921,9 @@ struct TilePixel
     uint32_t qh;                 // the warp's ring: first pending entry (warp-uniform)
 };
 
-__device__ __forceinline__ void tile_pixel(const ViewConst& vc, uint32_t tile, uint32_t pix, TilePixel& P)
+__device__ __forceinline__ void tile_pixel(const ViewConst& vc, uint32_t place, uint32_t pix, TilePixel& P)
 {
-    const uint32_t lt = tile - vc.tile_base;
-    P.px = (lt % vc.tiles_x) * vc.tile_w + pix % vc.tile_w;
-    P.py = (lt / vc.tiles_x) * vc.tile_h + pix / vc.tile_w;
+    tile_pixel_place(vc, place, pix, P.px, P.py);
     P.valid = P.px < vc.width && P.py < vc.height;
     P.far_plane = vc.far_plane;
     P.far_rcp = pow2_reciprocal(vc.far_plane);
@@ -1027,11 +942,18 @@ __device__ __forceinline__ void tile_pixel(const ViewConst& vc, uint32_t tile, u
     P.qh = 0u;
 }
 
+// the warp's minimum and maximum, NaN when some lane holds one
 __device__ __forceinline__ float warp_min(float x)
 {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x = fminf(x, __shfl_xor_sync(0xffffffffu, x, o));
-    return x;
+    float r;
+    asm volatile("redux.sync.min.NaN.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float warp_max(float x)
+{
+    float r;
+    asm volatile("redux.sync.max.NaN.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+    return r;
 }
 
 // Bounds of the warp's world rays (its pixels inside the view) for warp_may_hit:
@@ -1040,17 +962,15 @@ __device__ __forceinline__ float warp_min(float x)
 __device__ __forceinline__ void warp_rays(const TilePixel& P, float* __restrict__ bounds)
 {
     const float inf = __int_as_float(0x7f800000);
-    bool nan = false;
 #pragma unroll
     for (int i = 0; i < 3; i++) {
-        nan |= P.valid && P.dws[i] != P.dws[i];
-        const float lo = warp_min(P.valid ? P.dws[i] : inf), hi = -warp_min(P.valid ? -P.dws[i] : inf);
+        const float lo = warp_min(P.valid ? P.dws[i] : inf), hi = warp_max(P.valid ? P.dws[i] : -inf);
+        const float mid = 0.5f * (lo + hi);
         if ((threadIdx.x & 31u) == 0u) {
-            bounds[i] = 0.5f * (lo + hi);
-            bounds[4 + i] = 0.5f * (hi - lo) * 1.00001f + 2e-6f * fabsf(0.5f * (lo + hi));
+            bounds[i] = mid;
+            bounds[4 + i] = 0.5f * (hi - lo) * 1.00001f + 2e-6f * fabsf(mid);
         }
     }
-    if (__any_sync(0xffffffffu, nan) && (threadIdx.x & 31u) == 0u) bounds[0] = __int_as_float(0x7fffffff);
     __syncwarp();
 }
 
@@ -1209,11 +1129,20 @@ __device__ __forceinline__ void tile_batch(const TileJob& J, const TileEntry* co
     }
 }
 
-__device__ __forceinline__ uint32_t tile_view(const TileJob& J, uint32_t tile)
+// the index of a slot's tile among all views' (what an error names)
+__device__ __forceinline__ uint32_t tile_index(const ViewConst& vc, uint32_t place)
 {
-    uint32_t v = 0;
-    while (v + 1 < J.n_views && J.views[v + 1].tile_base <= tile) v++;
-    return v;
+    return vc.tile_base + (place >> 16) * vc.tiles_x + (place & 0xffffu);
+}
+
+// A tile without entries: only cleared (no ray set-up, no barrier), unless it is already.
+__device__ __forceinline__ void clear_tile(const TileJob& J, const uint4& si, uint32_t pix)
+{
+    if (J.cleared) return;
+    const ViewConst& vc = J.views[si.x];
+    uint32_t px, py;
+    tile_pixel_place(vc, si.w, pix, px, py);
+    if (px < vc.width && py < vc.height) J.outs[si.x][(size_t)py * vc.width + px] = ULLONG_MAX;
 }
 
 // Of records base .. base + m - 1, those of the view whose tile rectangle holds
@@ -1264,31 +1193,22 @@ __device__ __forceinline__ bool vis_tile(const TileJob& J, uint32_t slot, const 
     }
     __syncthreads();   // the CTA's previous tile is done with the shared state
     const uint4 si = J.slot_info[slot];   // one load: the tile and its entry range
-    const uint32_t tile = si.x;
     // bins overflowed this frame: gather every record whose tile rectangle holds the tile (slow, exact)
     const bool scan_all = J.counters[C_OVERFLOW] != 0u;
     const uint32_t begin = scan_all ? 0u : si.y;
     const uint32_t end = scan_all ? J.counters[C_RECORDS] : si.y + si.z;
-    if (!scan_all && si.z == 0u) {
-        // no entry: the tile is only cleared (no ray set-up, no barrier; the same in every thread)
-        const uint32_t v = tile_view(J, tile);
-        const ViewConst& vc = J.views[v];
-        const uint32_t lt = tile - vc.tile_base;
-        const uint32_t px = (lt % vc.tiles_x) * vc.tile_w + threadIdx.x % vc.tile_w;
-        const uint32_t py = (lt / vc.tiles_x) * vc.tile_h + threadIdx.x / vc.tile_w;
-        if (px < vc.width && py < vc.height) J.outs[v][(size_t)py * vc.width + px] = ULLONG_MAX;
+    if (si.z == 0u) {   // the same in every thread
+        clear_tile(J, si, threadIdx.x);
         return true;
     }
     const TileEntry* const E = sm.stage();
-    if (!scan_all && end > begin) stage_entries(J, sm.bar(), E, begin, min(J.batch, end - begin), J.extra_tx);
-    if (threadIdx.x == 0) sm.view() = tile_view(J, tile);
-    sm.best()[threadIdx.x] = ULLONG_MAX;
-    __syncthreads();
-    const uint32_t view = sm.view();
+    if (!scan_all) stage_entries(J, sm.bar(), E, begin, min(J.batch, end - begin), J.extra_tx);
+    sm.best()[threadIdx.x] = ULLONG_MAX;   // read by the thread's own warp, after warp_rays' barrier
+    const uint32_t view = si.x;
     const ViewConst& vc = J.views[view];
     TilePixel P;
-    tile_pixel(vc, tile, threadIdx.x, P);
-    const uint32_t tx = (tile - vc.tile_base) % vc.tiles_x, ty = (tile - vc.tile_base) / vc.tiles_x;
+    tile_pixel(vc, si.w, threadIdx.x, P);
+    const uint32_t tx = si.w & 0xffffu, ty = si.w >> 16;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     uint32_t* const q = sm.queue(warp);
     unsigned long long* const best0 = sm.best() + (warp << 5);
@@ -1332,7 +1252,7 @@ __device__ __forceinline__ bool vis_tile(const TileJob& J, uint32_t slot, const 
     if (__syncthreads_or(lost)) {
         // a batch's copies did not complete: report it, let this thread's own
         // land before the CTA is gone, and write the words found so far
-        if (threadIdx.x == 0) dev_error(status, TGX_ERR_TIMEOUT, 5, tile);
+        if (threadIdx.x == 0) dev_error(status, TGX_ERR_TIMEOUT, 5, tile_index(vc, si.w));
         own_copies_wait();
         if (P.valid) J.outs[view][(size_t)P.py * vc.width + P.px] = best;
         return false;
@@ -1366,16 +1286,10 @@ __device__ __forceinline__ void vis_tile_groups(const TileJob& J, uint32_t slot,
     const uint32_t n_pix = blockDim.x / kGroups;
     const uint32_t grp = threadIdx.x / n_pix, pix = threadIdx.x - grp * n_pix;
     const uint4 si = J.slot_info[slot];
-    const uint32_t tile = si.x;
     // bins overflowed this frame: gather every record whose tile rectangle holds the tile (slow, exact)
     const bool scan_all = J.counters[C_OVERFLOW] != 0u;
-    if (!scan_all && si.z == 0u) {   // no entry: the tile is only cleared
-        const uint32_t v = tile_view(J, tile);
-        const ViewConst& vc = J.views[v];
-        const uint32_t lt = tile - vc.tile_base;
-        const uint32_t px = (lt % vc.tiles_x) * vc.tile_w + pix % vc.tile_w;
-        const uint32_t py = (lt / vc.tiles_x) * vc.tile_h + pix / vc.tile_w;
-        if (grp == 0u && px < vc.width && py < vc.height) J.outs[v][(size_t)py * vc.width + px] = ULLONG_MAX;
+    if (si.z == 0u) {
+        if (grp == 0u) clear_tile(J, si, pix);
         return;
     }
     const uint32_t n_batches = scan_all ? 0u : (si.z + J.batch - 1u) / J.batch;
@@ -1385,16 +1299,13 @@ __device__ __forceinline__ void vis_tile_groups(const TileJob& J, uint32_t slot,
                       j == 0u ? J.extra_tx : 0u);
     };
     for (uint32_t j = 0; j < min(n_batches, kStages); j++) stage(j);
-    if (threadIdx.x == 0) {
-        sm.view() = tile_view(J, tile);
-        sm.lost() = 0u;
-    }
+    if (threadIdx.x == 0) sm.lost() = 0u;
     if (grp == 0u) sm.best()[pix] = ULLONG_MAX;
     __syncthreads();
-    const uint32_t view = sm.view();
+    const uint32_t view = si.x;
     const ViewConst& vc = J.views[view];
     TilePixel P;
-    tile_pixel(vc, tile, pix, P);
+    tile_pixel(vc, si.w, pix, P);
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t* const q = sm.queue(threadIdx.x >> 5);
     unsigned long long* const best0 = sm.best() + (pix & ~31u);
@@ -1419,9 +1330,9 @@ __device__ __forceinline__ void vis_tile_groups(const TileJob& J, uint32_t slot,
         if (j + kStages - 1u < n_batches) stage(j + kStages - 1u);
     }
     own_copies_wait();   // none may land after the CTA is gone
-    if (threadIdx.x == 0 && sm.lost()) dev_error(status, TGX_ERR_TIMEOUT, 5, tile);
+    if (threadIdx.x == 0 && sm.lost()) dev_error(status, TGX_ERR_TIMEOUT, 5, tile_index(vc, si.w));
     if (scan_all) {
-        const uint32_t tx = (tile - vc.tile_base) % vc.tiles_x, ty = (tile - vc.tile_base) / vc.tiles_x;
+        const uint32_t tx = si.w & 0xffffu, ty = si.w >> 16;
         const uint32_t n_rec = J.counters[C_RECORDS];
         for (uint32_t base = 0; base < n_rec; base += J.batch) {
             __syncthreads();
@@ -1481,8 +1392,8 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_vis_tiles_groups(
 }
 
 // Persistent form over several jobs (scenes, each with its views): CTAs take
-// tiles from one work queue in job order, each job's tiles heavy-first, until
-// all jobs' tiles are done.
+// tiles from one work queue in job order, each job's tiles heavy-first and those
+// without entries passed over, until all jobs' tiles are done.
 template <int kThreads, int kMinBlocks>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) k_vis_tiles_queue(const TileJob* __restrict__ jobs,
                                                                           uint32_t n_jobs, uint32_t total,
@@ -1491,23 +1402,34 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_vis_tiles_queue(const 
 {
     const TileSm sm = tile_sm();
     __shared__ TileJob s_job;
-    __shared__ uint32_t s_slot, s_jobidx;
+    __shared__ uint32_t s_slot;
     tile_smem_init(sm);
-    if (threadIdx.x == 0) s_jobidx = 0xffffffffu;
     uint32_t phase = 0;
+    // thread 0: the next item, drawn while the tile before it runs; the current job and its tiles with entries
+    uint32_t item = threadIdx.x == 0 ? atomicAdd(queue, 1u) : 0u, job = 0xffffffffu, with_entries = 0;
     for (;;) {
         __syncthreads();   // the previous tile is done with s_job
         if (threadIdx.x == 0) {
-            const uint32_t item = atomicAdd(queue, 1u);
             s_slot = 0xffffffffu;
-            if (item < total) {
+            while (item < total) {
                 uint32_t lo = 0, hi = n_jobs - 1;   // the last job whose first item is <= item
                 while (lo < hi) {
                     const uint32_t mid = (lo + hi + 1) >> 1;
                     if (jobs[mid].first <= item) lo = mid; else hi = mid - 1;
                 }
-                if (lo != s_jobidx) { s_job = jobs[lo]; s_jobidx = lo; }
-                s_slot = item - s_job.first;
+                if (lo != job) {
+                    job = lo;
+                    s_job = jobs[lo];
+                    with_entries = s_job.counters[C_NONEMPTY];
+                }
+                const uint32_t slot = item - s_job.first;
+                // the job's other tiles are cleared: on to the next job's
+                if (slot >= with_entries) atomicMax(queue, s_job.first + s_job.n_tiles);
+                item = atomicAdd(queue, 1u);
+                if (slot < with_entries) {
+                    s_slot = slot;
+                    break;
+                }
             }
         }
         __syncthreads();
@@ -1534,6 +1456,7 @@ static void make_view_const(const tgx_view& v, uint32_t tile_w, uint32_t tile_h,
     c.height = v.height;
     c.tile_w = tile_w;
     c.tile_h = tile_h;
+    c.tile_w_rcp = ((1u << 20) + tile_w - 1) / tile_w;
     c.tiles_x = (v.width + tile_w - 1) / tile_w;
     c.tiles_y = (v.height + tile_h - 1) / tile_h;
     c.tile_base = tile_base;
@@ -1595,10 +1518,10 @@ struct VisScratch
     uint2* rects;
     uint32_t rec_cap;
     uint32_t* counters;
+    uint32_t* supers;          // directly before bucket_cnt: both start at zero
     uint32_t* bucket_cnt;
-    uint32_t* bucket_off;
     uint32_t* tile_total;
-    uint32_t* cta_aux;
+    uint32_t* groups;
     uint32_t* tile_off;
     uint4* slot_info;
     TileRef* refs;
@@ -1614,9 +1537,8 @@ static uint32_t vis_chunk_cap(uint32_t n_tiles) { return std::max<uint32_t>(1u <
 // (the bucket arrays are sized for the finest setting, kMaxBuckets per tile)
 static size_t vis_tile_bytes(uint32_t n_tiles)
 {
-    const uint32_t n_scan_ctas = (n_tiles + kScanTiles - 1) / kScanTiles;
-    return (size_t)n_tiles * kMaxBuckets * 4 * 2 + (size_t)n_tiles * 4 + (size_t)n_scan_ctas * (1 + kOrderClasses) * 4 + 8 +
-           (size_t)vis_chunk_cap(n_tiles) * sizeof(uint2);
+    return ((size_t)scan_supers(n_tiles) * kGroupWords + (size_t)n_tiles * (kMaxBuckets + 1) + (size_t)scan_groups(n_tiles) * kGroupWords) * 4 +
+           8 + (size_t)vis_chunk_cap(n_tiles) * sizeof(uint2);
 }
 
 // bytes of the tile offsets (n_tiles + 1 words, padded to 16 bytes) and the slot records
@@ -1627,11 +1549,11 @@ static size_t vis_off_bytes(uint32_t n_tiles)
 
 static void vis_carve_tiles(VisScratch& w, uint32_t* tile_cnt, uint32_t* tile_off, uint32_t n_tiles)
 {
-    w.bucket_cnt = tile_cnt;
-    w.bucket_off = w.bucket_cnt + (size_t)n_tiles * kMaxBuckets;
-    w.tile_total = w.bucket_off + (size_t)n_tiles * kMaxBuckets;
-    w.cta_aux = w.tile_total + n_tiles;
-    const size_t words = (size_t)n_tiles * (2 * kMaxBuckets + 1) + (size_t)((n_tiles + kScanTiles - 1) / kScanTiles) * (1 + kOrderClasses);
+    w.supers = tile_cnt;
+    w.bucket_cnt = w.supers + (size_t)scan_supers(n_tiles) * kGroupWords;
+    w.tile_total = w.bucket_cnt + (size_t)n_tiles * kMaxBuckets;
+    w.groups = w.tile_total + n_tiles;
+    const size_t words = (size_t)(w.groups - tile_cnt) + (size_t)scan_groups(n_tiles) * kGroupWords;
     w.chunks = reinterpret_cast<uint2*>(tile_cnt + ((words + 1) & ~(size_t)1));
     w.chunk_cap = vis_chunk_cap(n_tiles);
     w.tile_off = tile_off;
@@ -1650,15 +1572,14 @@ static TileJob tile_job(const tgx_ctx* c, const tgx_scene* s, const ViewConst* d
     J.records = w.records;
     J.rects = w.rects;
     J.refs = w.refs;
-    J.tile_off = w.tile_off;
     J.slot_info = w.slot_info;
     J.views = d_vc;
     J.bits = s->d_bits;
     J.inv_rot = s->d_inv_rot;
     J.outs = d_outs;
     J.counters = w.counters;
-    J.n_views = n_views;
     J.n_tiles = n_tiles;
+    J.cleared = 1;
     J.first = 0;
     J.work = nullptr;
     J.extra_tx = 0;
@@ -1690,7 +1611,7 @@ static tgx_status vis_launch(tgx_ctx* c, const tgx_scene* s, const ViewConst* d_
                              bool interleave = false)
 {
     const uint64_t n_pairs = (uint64_t)s->n_cluster_pointers * n_views;
-    const uint32_t n_scan_ctas = (n_tiles + kScanTiles - 1) / kScanTiles;
+    const uint32_t n_scan_ctas = scan_groups(n_tiles);
     const uint32_t warp_grid = (uint32_t)c->num_sms * 8;
     const uint32_t bshift = c->vis_bshift;
     if (phase != VIS_FROM_BINS) {
@@ -1698,37 +1619,27 @@ static tgx_status vis_launch(tgx_ctx* c, const tgx_scene* s, const ViewConst* d_
         const uint32_t setup_blocks = (uint32_t)((n_pairs + 255) / 256);
         TGX_LAUNCH(c, TR_VIS_SETUP, setup_blocks, 256, 0, k_vis_cluster_setup<true>,
                    s->d_objects, s->d_cluster_pointers, s->d_c2o, s->d_bits, s->d_cp_obj, s->n_cluster_pointers,
-                   d_vc, n_views, w.records, w.rects, w.rec_cap, w.counters, w.bucket_cnt,
-                   n_tiles * (kMaxBuckets >> bshift), w.chunks, w.chunk_cap, c->d_status);
+                   d_vc, n_views, w.records, w.rects, w.rec_cap, w.counters, w.supers,
+                   scan_supers(n_tiles) * kGroupWords + n_tiles * (kMaxBuckets >> bshift), w.chunks, w.chunk_cap, c->d_status);
         // each later pass is a programmatic dependent of the one before
         TGX_LAUNCH_PDL(c, TR_VIS_COUNT, warp_grid, 256, 0, k_vis_count, w.records, w.rects, w.counters, w.rec_cap,
                        s->d_objects, d_vc, w.bucket_cnt, n_tiles, bshift, w.chunks, w.chunk_cap);
-        if (bshift == 0)
-            TGX_LAUNCH_PDL(c, TR_VIS_PREFIX, n_scan_ctas, kScanTiles, 0, k_vis_prefix<32>, w.bucket_cnt, w.bucket_off,
-                           w.tile_total, n_tiles, w.cta_aux);
-        else if (bshift == 1)
-            TGX_LAUNCH_PDL(c, TR_VIS_PREFIX, n_scan_ctas, kScanTiles, 0, k_vis_prefix<16>, w.bucket_cnt, w.bucket_off,
-                           w.tile_total, n_tiles, w.cta_aux);
-        else
-            TGX_LAUNCH_PDL(c, TR_VIS_PREFIX, n_scan_ctas, kScanTiles, 0, k_vis_prefix<8>, w.bucket_cnt, w.bucket_off,
-                           w.tile_total, n_tiles, w.cta_aux);
-        if (n_scan_ctas <= kDirectGroups) {
-            TGX_LAUNCH_PDL(c, TR_VIS_SCAN, n_scan_ctas, kScanTiles, 0, k_vis_finalize_direct, w.tile_total, n_tiles,
-                           w.cta_aux, w.tile_off, w.slot_info, w.bin_capacity, w.counters);
-        } else {
-            TGX_LAUNCH_PDL(c, TR_VIS_SCAN, 1, 1024, 0, k_vis_scan, w.cta_aux, n_tiles, w.tile_off, w.bin_capacity,
-                           w.counters);
-            TGX_LAUNCH_PDL(c, TR_VIS_SCAN, n_scan_ctas, kScanTiles, 0, k_vis_finalize, w.tile_total, n_tiles,
-                           w.cta_aux, w.tile_off, w.slot_info);
-        }
+#define PREFIX_ARGS w.bucket_cnt, w.tile_total, n_tiles, w.groups, w.supers
+        if (bshift == 0) TGX_LAUNCH_PDL(c, TR_VIS_PREFIX, n_scan_ctas, kScanTiles, 0, k_vis_prefix<32>, PREFIX_ARGS);
+        else if (bshift == 1) TGX_LAUNCH_PDL(c, TR_VIS_PREFIX, n_scan_ctas, kScanTiles, 0, k_vis_prefix<16>, PREFIX_ARGS);
+        else TGX_LAUNCH_PDL(c, TR_VIS_PREFIX, n_scan_ctas, kScanTiles, 0, k_vis_prefix<8>, PREFIX_ARGS);
+#undef PREFIX_ARGS
+        TGX_LAUNCH_PDL(c, TR_VIS_SCAN, n_scan_ctas, kScanTiles, 0, k_vis_finalize, w.tile_total, n_tiles, w.groups, w.supers,
+                       w.tile_off, w.slot_info, w.bin_capacity, w.counters, d_vc, n_views);
     }
     if (phase == VIS_TO_SCAN) return TGX_OK;
     TGX_LAUNCH_PDL(c, TR_VIS_BIN, warp_grid, 256, 0, k_vis_bin_fill,
-                   w.records, w.rects, w.counters, d_vc, w.tile_off, w.bucket_off, w.bucket_cnt, w.refs,
-                   n_tiles, w.bin_capacity, bshift, w.chunks, w.chunk_cap, c->d_status);
+                   w.records, w.rects, w.counters, d_vc, w.tile_off, w.bucket_cnt, w.refs,
+                   n_tiles, w.bin_capacity, bshift, w.chunks, w.chunk_cap, w.slot_info, d_outs, interleave ? 0u : 1u, c->d_status);
     if (phase == VIS_NO_TILES) return TGX_OK;
     TileJob J = tile_job(c, s, d_vc, d_outs, n_views, n_tiles, w);
     J.interleave = interleave ? 1u : 0u;
+    J.cleared = interleave ? 0u : 1u;
     if (c->flags & TGX_FLAG_TEST_LOST_COPY) J.extra_tx = 64u;
     const uint32_t threads = c->tile_w * c->tile_h, smem = tile_smem_bytes(threads);
     if (c->vis_count_work) {
@@ -2332,17 +2243,17 @@ constexpr size_t kNaViews = kNaStatus + 256;
 constexpr size_t kNaInvRot = kNaViews + na_align(sizeof(ViewConst) + 16);
 constexpr size_t kNaRecords = kNaInvRot + na_align((size_t)kNaMaxObjects * 9 * 4);
 constexpr size_t kNaRects = kNaRecords + na_align((size_t)kNaMaxClusterPointers * sizeof(VisRecord));
-constexpr size_t kNaBucketCnt = kNaRects + na_align((size_t)kNaMaxClusterPointers * 8);
+constexpr size_t kNaSupers = kNaRects + na_align((size_t)kNaMaxClusterPointers * 8);   // the last words before the counts
+constexpr size_t kNaBucketCnt = kNaSupers + na_align((size_t)scan_supers(kNaMaxTiles) * kGroupWords * 4);
 constexpr uint32_t kNaBuckets = 16;          // depth buckets per tile (bucket shift 1)
-constexpr size_t kNaBucketOff = kNaBucketCnt + na_align((size_t)kNaMaxTiles * kNaBuckets * 4);
-constexpr size_t kNaTileTotal = kNaBucketOff + na_align((size_t)kNaMaxTiles * kNaBuckets * 4);
-constexpr size_t kNaScanAux = kNaTileTotal + na_align((size_t)kNaMaxTiles * 4);
-constexpr size_t kNaTileOff = kNaScanAux + na_align(((size_t)kNaMaxTiles / kScanTiles + 1) * (1 + kOrderClasses) * 4);
+constexpr size_t kNaTileTotal = kNaBucketCnt + na_align((size_t)kNaMaxTiles * kNaBuckets * 4);
+constexpr size_t kNaGroups = kNaTileTotal + na_align((size_t)kNaMaxTiles * 4);
+constexpr size_t kNaTileOff = kNaGroups + na_align((size_t)scan_groups(kNaMaxTiles) * kGroupWords * 4);
 constexpr size_t kNaSlotInfo = kNaTileOff + na_align(((size_t)kNaMaxTiles + 4) * 4);
 constexpr size_t kNaBinsOff = kNaSlotInfo + na_align((size_t)kNaMaxTiles * 16);
 constexpr uint32_t kNaChunks = 1u << 16;
 constexpr size_t kNaChunkOff = kNaBinsOff + na_align((size_t)kNaBins * sizeof(TileRef));
-constexpr size_t kNaBytes = kNaChunkOff + na_align((size_t)kNaChunks * sizeof(uint2));   // about 29 MiB
+constexpr size_t kNaBytes = kNaChunkOff + na_align((size_t)kNaChunks * sizeof(uint2));   // about 28 MiB
 
 // The scratch.  In host code this name is only a host-side stand-in: its
 // device address is taken with cudaGetSymbolAddress below.
@@ -2463,9 +2374,9 @@ extern "C" tgx_status tgx_vis_render_noalloc(void* stream, const tgx_object* d_o
     VisRecord* records = (VisRecord*)(base + kNaRecords);
     uint2* rects = (uint2*)(base + kNaRects);
     uint32_t* bucket_cnt = (uint32_t*)(base + kNaBucketCnt);
-    uint32_t* bucket_off = (uint32_t*)(base + kNaBucketOff);
+    uint32_t* supers = bucket_cnt - scan_supers(n_tiles) * kGroupWords;
     uint32_t* tile_total = (uint32_t*)(base + kNaTileTotal);
-    uint32_t* cta_aux = (uint32_t*)(base + kNaScanAux);
+    uint32_t* groups = (uint32_t*)(base + kNaGroups);
     uint32_t* tile_off = (uint32_t*)(base + kNaTileOff);
     uint4* slot_info = (uint4*)(base + kNaSlotInfo);
     TileRef* refs = (TileRef*)(base + kNaBinsOff);
@@ -2480,34 +2391,29 @@ extern "C" tgx_status tgx_vis_render_noalloc(void* stream, const tgx_object* d_o
               counters, status, d_objects, n_objects, inv_rot);
     NA_LAUNCH((n_cluster_pointers + 255) / 256, 256, k_vis_cluster_setup<false>, d_objects, d_cluster_pointers,
               d_cluster_idx_to_object_idx, d_voxel_bits, (const uint32_t*)nullptr, n_cluster_pointers, d_vc, 1u,
-              records, rects, kNaMaxClusterPointers, counters, bucket_cnt, n_tiles * kNaBuckets, chunks, kNaChunks,
+              records, rects, kNaMaxClusterPointers, counters, supers,
+              scan_supers(n_tiles) * kGroupWords + n_tiles * kNaBuckets, chunks, kNaChunks,
               status);
     NA_LAUNCH(warp_grid, 256, k_vis_count, records, rects, counters, kNaMaxClusterPointers, d_objects, d_vc, bucket_cnt,
               n_tiles, 1u, chunks, kNaChunks);
-    const uint32_t n_scan_ctas = (n_tiles + kScanTiles - 1) / kScanTiles;
-    NA_LAUNCH(n_scan_ctas, kScanTiles, k_vis_prefix<kNaBuckets>, bucket_cnt, bucket_off, tile_total, n_tiles, cta_aux);
-    if (n_scan_ctas <= kDirectGroups) {
-        NA_LAUNCH(n_scan_ctas, kScanTiles, k_vis_finalize_direct, tile_total, n_tiles, cta_aux, tile_off, slot_info,
-                  kNaBins, counters);
-    } else {
-        NA_LAUNCH(1, 1024, k_vis_scan, cta_aux, n_tiles, tile_off, kNaBins, counters);
-        NA_LAUNCH(n_scan_ctas, kScanTiles, k_vis_finalize, tile_total, n_tiles, cta_aux, tile_off, slot_info);
-    }
-    NA_LAUNCH(warp_grid, 256, k_vis_bin_fill, records, rects, counters, d_vc, tile_off, bucket_off, bucket_cnt, refs,
-              n_tiles, kNaBins, 1u, chunks, kNaChunks, status);
+    const uint32_t n_scan_ctas = scan_groups(n_tiles);
+    NA_LAUNCH(n_scan_ctas, kScanTiles, k_vis_prefix<kNaBuckets>, bucket_cnt, tile_total, n_tiles, groups, supers);
+    NA_LAUNCH(n_scan_ctas, kScanTiles, k_vis_finalize, tile_total, n_tiles, groups, supers, tile_off, slot_info, kNaBins,
+              counters, d_vc, 1u);
+    NA_LAUNCH(warp_grid, 256, k_vis_bin_fill, records, rects, counters, d_vc, tile_off, bucket_cnt, refs,
+              n_tiles, kNaBins, 1u, chunks, kNaChunks, slot_info, d_outs, 1u, status);
     TileJob J;
     J.records = records;
     J.rects = rects;
     J.refs = refs;
-    J.tile_off = tile_off;
     J.slot_info = slot_info;
     J.views = d_vc;
     J.bits = d_voxel_bits;
     J.inv_rot = inv_rot;
     J.outs = d_outs;
     J.counters = counters;
-    J.n_views = 1;
     J.n_tiles = n_tiles;
+    J.cleared = 1;
     J.first = 0;
     J.work = nullptr;
     J.extra_tx = 0;
