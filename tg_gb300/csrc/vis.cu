@@ -1592,10 +1592,10 @@ static TileJob tile_job(const tgx_ctx* c, const tgx_scene* s, const ViewConst* d
 // holds (1024 per SM at the kernels' 64 registers).  Below that the time is the
 // heaviest tile's chain of batches, above it the sum of all tiles' work, which
 // grows with the threads.  Tile kernel over the 512-object scene, 8x8 tiles,
-// 1 / 2 / 4 / 8 threads per pixel: 480x270 239 / 141 / 99 / 76 us, 640x480 133 /
-// 87 / 71 / 100, 960x540 124 / 83 / 99 / 151, 1280x720 107 / 107 / 145 / 231,
-// 1920x1080 146 / 186 / 272 / 447; 16x16 tiles, 1 / 2 / 4: 480x270 554 / 318 / 234,
-// 1280x720 175 / 154 / 216, 1920x1080 181 / 249 / 376.
+// 1 / 2 / 4 / 8 threads per pixel: 480x270 128 / 85 / 67 / 62 us, 640x480 78 /
+// 57 / 54 / 85, 960x540 75 / 57 / 78 / 129, 1280x720 68 / 77 / 116 / 197,
+// 1920x1080 102 / 141 / 220 / 385; 16x16 tiles, 1 / 2 / 4: 480x270 273 / 174 / 153,
+// 1280x720 102 / 106 / 168, 1920x1080 124 / 180 / 299.
 static uint32_t vis_groups(const tgx_ctx* c, uint32_t pixels, uint32_t n_tiles)
 {
     const uint64_t limit = 12ull * 1024ull * (uint64_t)c->num_sms;
