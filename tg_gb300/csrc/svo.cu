@@ -923,6 +923,33 @@ static void svo_free(tgx_svo* s)
     delete s;
 }
 
+// An SVO's arrays come from a memory pool of the context that builds it, which
+// keeps up to kSvoPoolKeep bytes of freed arrays for the next build and gives the
+// rest back; the pool goes with the context (an array still in use keeps its
+// part alive).  A build of 18.4k blocks with materials (1.3 GB) and its free took
+// 1.1 ms in the driver's allocator beside 1.9 ms of GPU work.  Arrays are freed
+// by cudaFree, which waits for all streams that may still read them.
+constexpr uint64_t kSvoPoolKeep = 4ull << 30;
+
+static cudaError_t svo_malloc(tgx_ctx* c, void** p, uint64_t bytes)
+{
+    if (!c->svo_pool) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = c->device;
+        cudaMemPool_t pool = nullptr;
+        if (const cudaError_t e = cudaMemPoolCreate(&pool, &props); e != cudaSuccess) return e;
+        uint64_t keep = kSvoPoolKeep;
+        if (const cudaError_t e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep); e != cudaSuccess) {
+            cudaMemPoolDestroy(pool);
+            return e;
+        }
+        c->svo_pool = pool;
+    }
+    return cudaMallocFromPoolAsync(p, std::max<uint64_t>(bytes, 1), c->svo_pool, c->stream);
+}
+
 // The pair storage: pairs, then as many words for the list of the marked blocks.
 constexpr uint64_t kPairBytes = sizeof(SvoPair) + 4;
 static uint32_t* svo_marked(tgx_ctx* c)
@@ -950,7 +977,7 @@ static tgx_status svo_resize_slots(tgx_ctx* c, tgx_svo* s, uint32_t cap, uint32_
     const int n_arr = materials ? 6 : 5;
     void* fresh[6] = {};
     for (int a = 0; a < n_arr; a++)
-        if (cudaMalloc(&fresh[a], (uint64_t)cap * arrs[a].per_slot) != cudaSuccess) {
+        if (svo_malloc(c, &fresh[a], (uint64_t)cap * arrs[a].per_slot) != cudaSuccess) {
             for (int k = 0; k < a; k++) cudaFree(fresh[k]);
             cudaGetLastError();
             tgx_set_error("tgx_svo: out of device memory for %u blocks", cap);
@@ -961,7 +988,7 @@ static tgx_status svo_resize_slots(tgx_ctx* c, tgx_svo* s, uint32_t cap, uint32_
         if (kept) TGX_CUDA(cudaMemcpyAsync(fresh[a], *arrs[a].p, kept, cudaMemcpyDeviceToDevice, c->stream));
         if (a != 0 && a != 5) TGX_CUDA(cudaMemsetAsync((char*)fresh[a] + kept, a == 4 ? 0xff : 0, total - kept, c->stream));
     }
-    TGX_CUDA(cudaStreamSynchronize(c->stream));
+    if (s->d_pool) TGX_CUDA(cudaStreamSynchronize(c->stream));
     for (int a = 0; a < n_arr; a++) {
         cudaFree(*arrs[a].p);
         *arrs[a].p = fresh[a];
@@ -1100,9 +1127,10 @@ extern "C" tgx_status tgx_svo_build_flags(tgx_ctx* c, const tgx_scene* sc, const
     s->occ_words = occ_words;
 
     auto fail = [&](tgx_status st) { cudaStreamSynchronize(c->stream); svo_free(s); return st; };
-    if (cudaMalloc(&s->d_table, n_table * 4) != cudaSuccess || cudaMalloc(&s->d_occ, occ_words * 4 + 128) != cudaSuccess ||
-        cudaMalloc(&s->d_counters, S_COUNT * 4) != cudaSuccess ||
-        cudaMalloc(&s->d_objs, std::max<uint64_t>(1, (uint64_t)sc->n_objects) * sizeof(tgx_object)) != cudaSuccess) {
+    if (svo_malloc(c, (void**)&s->d_table, n_table * 4) != cudaSuccess ||
+        svo_malloc(c, (void**)&s->d_occ, occ_words * 4 + 128) != cudaSuccess ||
+        svo_malloc(c, (void**)&s->d_counters, S_COUNT * 4) != cudaSuccess ||
+        svo_malloc(c, (void**)&s->d_objs, std::max<uint64_t>(1, (uint64_t)sc->n_objects) * sizeof(tgx_object)) != cudaSuccess) {
         cudaGetLastError();
         tgx_set_error("tgx_svo_build: out of device memory for the block table");
         return fail(TGX_ERR_OUT_OF_MEMORY);

@@ -133,6 +133,7 @@ extern "C" void tgx_destroy(tgx_ctx* c)
     devbuf_free(c->vis_bins);
     devbuf_free(c->vis_views);
     devbuf_free(c->svo_counters);
+    if (c->svo_pool) cudaMemPoolDestroy(c->svo_pool);
     devbuf_free(c->svo_pairs);
     devbuf_free(c->svo_scratch);
     devbuf_free(c->svo_sort);

@@ -126,6 +126,7 @@ struct tgx_ctx
     DevBuf vis_bins;       // tile -> record indices
     DevBuf vis_views;      // device copies of the views
     DevBuf svo_counters;   // SVO build counters
+    cudaMemPool_t svo_pool = nullptr;   // where SVOs built by the context keep their arrays (svo_malloc)
     DevBuf svo_pairs;      // (cluster, block) voxelisation pairs
     DevBuf gi_scratch;     // learned-cache GI queries, hits, training batch
     DevBuf svo_scratch;    // SVO update: dirty-block marks
