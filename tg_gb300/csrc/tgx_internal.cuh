@@ -142,8 +142,10 @@ struct tgx_ctx
     uint32_t vis_drain = 32;           // live pairs a warp collects before running their DDAs
     uint32_t vis_last_tiles = 0;
     uint64_t vis_last_pairs = 0;
-    void*  h_vis_counters = nullptr;   // pinned copy of the last frame's counters
-    cudaEvent_t vis_done = nullptr;    // recorded after that copy
+    void*  h_vis_counters = nullptr;   // pinned: the last frame's entry count and overflow flag
+    cudaEvent_t vis_done = nullptr;    // recorded after the frame
+    uint32_t vis_counter_set = 0;      // which set of counters the last frame used
+    bool   vis_counters_clear[2] = {false, false};
     DevBuf host_stage;     // pinned host staging (views)
     void*  h_pinned = nullptr;
     size_t h_pinned_bytes = 0;

@@ -42,6 +42,7 @@
 
 #include <climits>
 #include <cmath>
+#include <type_traits>
 #include <mutex>
 #include <vector>
 
@@ -158,12 +159,22 @@ __device__ __forceinline__ uint32_t warp_append(uint32_t* counter, bool pred)
 // whether its cluster is empty (one load beside the pointer's own, instead of
 // the chain pointer -> owner -> bitmask); without it (the entry point that
 // allocates nothing) the owner and the bitmask are read.
-template <bool kPacked>
+// kInline: the views and outputs of a frame of few views come as an argument;
+// the first CTA stores them in the tables the later passes read.
+constexpr uint32_t kInlineViews = 8;
+struct InlineViews
+{
+    ViewConst views[kInlineViews];
+    unsigned long long* outs[kInlineViews];
+};
+struct NoViews {};
+
+template <bool kPacked, class Inline>
 __global__ void __launch_bounds__(256, 4) k_vis_cluster_setup(
     const tgx_object* __restrict__ objects, const uint32_t* __restrict__ cluster_pointers,
     const uint32_t* __restrict__ c2o, const uint32_t* __restrict__ bits, const uint32_t* __restrict__ cp_obj,
-    uint32_t n_cp, const ViewConst* __restrict__ views, uint32_t n_views, VisRecord* __restrict__ records,
-    uint2* __restrict__ rects, uint32_t record_capacity, uint32_t* __restrict__ counters,
+    uint32_t n_cp, const __grid_constant__ Inline inl, ViewConst* views, unsigned long long** outs, uint32_t n_views,
+    VisRecord* __restrict__ records, uint2* __restrict__ rects, uint32_t record_capacity, uint32_t* __restrict__ counters,
     uint32_t* __restrict__ zero, uint32_t n_zero, uint2* __restrict__ chunks, uint32_t chunk_cap,
     tgx_dev_status* __restrict__ status)
 {
@@ -172,13 +183,24 @@ __global__ void __launch_bounds__(256, 4) k_vis_cluster_setup(
     const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     // the (tile, bucket) counts start at zero; k_vis_count runs after this kernel
     for (uint64_t i = gid; i < n_zero; i += (uint64_t)gridDim.x * blockDim.x) zero[i] = 0u;
+    constexpr bool kInline = !std::is_same<Inline, NoViews>::value;
+    if constexpr (kInline) {
+        if (blockIdx.x == 0) {
+            constexpr uint32_t kWords = sizeof(ViewConst) / 4u;
+            for (uint32_t i = threadIdx.x; i < n_views * kWords; i += blockDim.x)
+                reinterpret_cast<uint32_t*>(views)[i] = reinterpret_cast<const uint32_t*>(inl.views)[i];
+            if (threadIdx.x < n_views) outs[threadIdx.x] = inl.outs[threadIdx.x];
+        }
+    }
     const uint32_t v = (uint32_t)(gid / n_cp);
     const uint32_t cp = (uint32_t)(gid % n_cp);
     bool keep = false;
     VisRecord rec = {};
     uint32_t tx0 = 0, ty0 = 0, tx1 = 0, ty1 = 0;
     if (v < n_views) {
-        const ViewConst& vc = views[v];
+        const ViewConst* table = views;
+        if constexpr (kInline) table = inl.views;
+        const ViewConst& vc = table[v];
         const uint32_t ci = cluster_pointers[cp];
         const uint32_t po = kPacked ? cp_obj[cp] : 0u;
         if (!kPacked || !(po >> 31)) {   // bit 31: the cluster has no set voxel
@@ -449,6 +471,7 @@ __global__ void __launch_bounds__(kScanTiles) k_vis_finalize(const uint32_t* __r
                                                             uint32_t* __restrict__ tile_off,
                                                             uint4* __restrict__ slot_info, uint32_t bin_capacity,
                                                             uint32_t* __restrict__ counters,
+                                                            uint32_t* __restrict__ next_counters,
                                                             const ViewConst* __restrict__ views, uint32_t n_views)
 {
     constexpr uint32_t kWarps = kScanTiles / 32;
@@ -529,6 +552,7 @@ __global__ void __launch_bounds__(kScanTiles) k_vis_finalize(const uint32_t* __r
         counters[C_ENTRIES] = total;
         counters[C_OVERFLOW] = total > bin_capacity ? 1u : 0u;
     }
+    if (g == 0 && next_counters && threadIdx.x < C_COUNT) next_counters[threadIdx.x] = 0u;   // the next frame's
     for (uint32_t w = 0; w < wid; w++) base += wsum[w];
     if (valid) {
         const uint32_t off = base + incl - x;
@@ -809,6 +833,7 @@ struct TileJob
     const float* inv_rot;
     unsigned long long* const* outs;
     uint32_t* counters;
+    uint32_t* host_counters;     // pinned host memory for the frame's entry count and overflow flag, or null
     uint32_t n_tiles;
     uint32_t cleared;            // tiles without entries are done (k_vis_bin_fill)
     uint32_t first;              // the job's first item in a multi-job work queue
@@ -1362,12 +1387,22 @@ __device__ __forceinline__ uint32_t tile_slot(uint32_t b, uint32_t t, uint32_t n
     return c1 > c0 ? c0 : n + (b - c0);
 }
 
+// The totals the host sizes the next frame by, written while the frame's first tile starts.
+__device__ __forceinline__ void publish_totals(const TileJob& J)
+{
+    if (blockIdx.x == 0 && threadIdx.x == 0 && J.host_counters) {
+        J.host_counters[C_ENTRIES] = J.counters[C_ENTRIES];
+        J.host_counters[C_OVERFLOW] = J.counters[C_OVERFLOW];
+    }
+}
+
 template <int kThreads, int kMinBlocks, bool kCount = false>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) k_vis_tiles(TileJob J, tgx_dev_status* __restrict__ status)
 {
     const TileSm sm = tile_sm();
     tile_smem_init(sm);
     pdl_wait();
+    publish_totals(J);
     uint32_t phase = 0;
     const uint32_t slot = J.interleave ? tile_slot(blockIdx.x, J.n_tiles, J.counters[C_NONEMPTY], true) : blockIdx.x;
     vis_tile<kCount>(J, slot, sm, phase, status);
@@ -1386,6 +1421,7 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_vis_tiles_groups(
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     pdl_wait();
+    publish_totals(J);
     __syncthreads();   // every thread arrives on the mbarriers
     const uint32_t slot = J.interleave ? tile_slot(blockIdx.x, J.n_tiles, J.counters[C_NONEMPTY], true) : blockIdx.x;
     vis_tile_groups<kGroups>(J, slot, sm, status);
@@ -1518,6 +1554,8 @@ struct VisScratch
     uint2* rects;
     uint32_t rec_cap;
     uint32_t* counters;
+    uint32_t* next_counters = nullptr;   // cleared on the way, for the next frame (null: `counters` are cleared first)
+    uint32_t* host_counters = nullptr;
     uint32_t* supers;          // directly before bucket_cnt: both start at zero
     uint32_t* bucket_cnt;
     uint32_t* tile_total;
@@ -1578,6 +1616,7 @@ static TileJob tile_job(const tgx_ctx* c, const tgx_scene* s, const ViewConst* d
     J.inv_rot = s->d_inv_rot;
     J.outs = d_outs;
     J.counters = w.counters;
+    J.host_counters = w.host_counters;
     J.n_tiles = n_tiles;
     J.cleared = 1;
     J.first = 0;
@@ -1606,21 +1645,25 @@ static uint32_t vis_groups(const tgx_ctx* c, uint32_t pixels, uint32_t n_tiles)
 
 // The launches of one frame (n_views views of scene s, view table d_vc / d_outs
 // on the device): all of them, or the part up to the tile scan, or the rest.
-static tgx_status vis_launch(tgx_ctx* c, const tgx_scene* s, const ViewConst* d_vc, unsigned long long* const* d_outs,
+static tgx_status vis_launch(tgx_ctx* c, const tgx_scene* s, ViewConst* d_vc, unsigned long long** d_outs,
                              uint32_t n_views, uint32_t n_tiles, const VisScratch& w, int phase = VIS_ALL,
-                             bool interleave = false)
+                             bool interleave = false, const InlineViews* views = nullptr)
 {
     const uint64_t n_pairs = (uint64_t)s->n_cluster_pointers * n_views;
     const uint32_t n_scan_ctas = scan_groups(n_tiles);
     const uint32_t warp_grid = (uint32_t)c->num_sms * 8;
     const uint32_t bshift = c->vis_bshift;
     if (phase != VIS_FROM_BINS) {
-        TGX_CUDA(cudaMemsetAsync(w.counters, 0, C_COUNT * sizeof(uint32_t), c->stream));
+        if (!w.next_counters) TGX_CUDA(cudaMemsetAsync(w.counters, 0, C_COUNT * sizeof(uint32_t), c->stream));
         const uint32_t setup_blocks = (uint32_t)((n_pairs + 255) / 256);
-        TGX_LAUNCH(c, TR_VIS_SETUP, setup_blocks, 256, 0, k_vis_cluster_setup<true>,
-                   s->d_objects, s->d_cluster_pointers, s->d_c2o, s->d_bits, s->d_cp_obj, s->n_cluster_pointers,
-                   d_vc, n_views, w.records, w.rects, w.rec_cap, w.counters, w.supers,
-                   scan_supers(n_tiles) * kGroupWords + n_tiles * (kMaxBuckets >> bshift), w.chunks, w.chunk_cap, c->d_status);
+#define SETUP(type, inl)                                                                                               \
+        TGX_LAUNCH(c, TR_VIS_SETUP, setup_blocks, 256, 0, (k_vis_cluster_setup<true, type>),                           \
+                   s->d_objects, s->d_cluster_pointers, s->d_c2o, s->d_bits, s->d_cp_obj, s->n_cluster_pointers, inl,  \
+                   d_vc, d_outs, n_views, w.records, w.rects, w.rec_cap, w.counters, w.supers,                         \
+                   scan_supers(n_tiles) * kGroupWords + n_tiles * (kMaxBuckets >> bshift), w.chunks, w.chunk_cap, c->d_status)
+        if (views) SETUP(InlineViews, *views);
+        else SETUP(NoViews, NoViews{});
+#undef SETUP
         // each later pass is a programmatic dependent of the one before
         TGX_LAUNCH_PDL(c, TR_VIS_COUNT, warp_grid, 256, 0, k_vis_count, w.records, w.rects, w.counters, w.rec_cap,
                        s->d_objects, d_vc, w.bucket_cnt, n_tiles, bshift, w.chunks, w.chunk_cap);
@@ -1630,7 +1673,7 @@ static tgx_status vis_launch(tgx_ctx* c, const tgx_scene* s, const ViewConst* d_
         else TGX_LAUNCH_PDL(c, TR_VIS_PREFIX, n_scan_ctas, kScanTiles, 0, k_vis_prefix<8>, PREFIX_ARGS);
 #undef PREFIX_ARGS
         TGX_LAUNCH_PDL(c, TR_VIS_SCAN, n_scan_ctas, kScanTiles, 0, k_vis_finalize, w.tile_total, n_tiles, w.groups, w.supers,
-                       w.tile_off, w.slot_info, w.bin_capacity, w.counters, d_vc, n_views);
+                       w.tile_off, w.slot_info, w.bin_capacity, w.counters, w.next_counters, d_vc, n_views);
     }
     if (phase == VIS_TO_SCAN) return TGX_OK;
     TGX_LAUNCH_PDL(c, TR_VIS_BIN, warp_grid, 256, 0, k_vis_bin_fill,
@@ -1747,14 +1790,26 @@ tgx_status vis_render_device(tgx_ctx* c, const tgx_scene* s, const tgx_view* vie
         if (!d_visbuf[i]) { tgx_set_error("tgx_vis_render: output %u is NULL", i); return TGX_ERR_INVALID_ARGUMENT; }
     TGX_CUDA(cudaSetDevice(c->device));
 
-    // view constants + output pointer table, copied from pageable memory (staged by the driver, no sync)
+    // View constants and output pointers: up to kInlineViews go with the first
+    // kernel as its argument, more are copied from pageable memory (staged by
+    // the driver, no sync).  A small frame is a chain of short dependent kernels;
+    // a copy or a memset in it costs as much as one of them (256x256 frame of a
+    // small scene 37.3 us with a copy, a memset and the counters' copy back, 31.4
+    // without; 512 objects at 1920x1080 with shading 148.6 and 137.9).
     uint32_t n_tiles = 0;
     size_t ptr_off = 0;
     const std::vector<unsigned char> stage = vis_view_table(c, views, n_views, d_visbuf, n_tiles, ptr_off);
     TGX_TRY(devbuf_reserve(c->vis_views, stage.size()));
-    TGX_CUDA(cudaMemcpyAsync(c->vis_views.ptr, stage.data(), stage.size(), cudaMemcpyHostToDevice, c->stream));
-    const ViewConst* d_vc = (const ViewConst*)c->vis_views.ptr;
-    unsigned long long* const* d_outs = (unsigned long long* const*)((char*)c->vis_views.ptr + ptr_off);
+    ViewConst* d_vc = (ViewConst*)c->vis_views.ptr;
+    unsigned long long** d_outs = (unsigned long long**)((char*)c->vis_views.ptr + ptr_off);
+    InlineViews inl;
+    const bool few = n_views <= kInlineViews;
+    if (few) {
+        memcpy(inl.views, stage.data(), n_views * sizeof(ViewConst));
+        memcpy(inl.outs, stage.data() + ptr_off, n_views * sizeof(void*));
+    } else {
+        TGX_CUDA(cudaMemcpyAsync(c->vis_views.ptr, stage.data(), stage.size(), cudaMemcpyHostToDevice, c->stream));
+    }
 
     // bin capacity: grown from earlier frames' totals (read back without waiting); a frame
     // that still overflows is rendered correctly by the tile kernel's record scan
@@ -1786,18 +1841,35 @@ tgx_status vis_render_device(tgx_ctx* c, const tgx_scene* s, const tgx_view* vie
     }
     w.rec_cap = (uint32_t)n_pairs;
     TGX_TRY(devbuf_reserve(c->vis_records, (size_t)w.rec_cap * (sizeof(VisRecord) + sizeof(uint2))));
-    TGX_TRY(devbuf_reserve(c->vis_counters, C_COUNT * sizeof(uint32_t)));
+    // Two sets of counters take turns: each frame's finalize kernel clears the
+    // other set.  A set that may not be clear (the first frames, or a frame that
+    // was not launched whole) is cleared by a memset.  So is the third set, which
+    // frames use that a caller captures: their graph may run between any others.
+    TGX_TRY(devbuf_reserve(c->vis_counters, 3 * C_COUNT * sizeof(uint32_t)));
     TGX_TRY(devbuf_reserve(c->vis_tile_cnt, vis_tile_bytes(n_tiles)));
     TGX_TRY(devbuf_reserve(c->vis_tile_off, vis_off_bytes(n_tiles)));
     w.records = (VisRecord*)c->vis_records.ptr;
     w.rects = (uint2*)(w.records + w.rec_cap);
-    w.counters = (uint32_t*)c->vis_counters.ptr;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    TGX_CUDA(cudaStreamIsCapturing(c->stream, &capture));
+    const bool captured = capture != cudaStreamCaptureStatusNone;
+    const uint32_t set = captured ? 2u : c->vis_counter_set == 0u ? 1u : 0u;
+    uint32_t* const sets = (uint32_t*)c->vis_counters.ptr;
+    w.counters = sets + set * C_COUNT;
+    w.host_counters = (uint32_t*)c->h_vis_counters;
+    if (!captured) {
+        w.next_counters = sets + (set ^ 1u) * C_COUNT;
+        if (!c->vis_counters_clear[set])
+            TGX_CUDA(cudaMemsetAsync(w.counters, 0, C_COUNT * sizeof(uint32_t), c->stream));
+        c->vis_counters_clear[0] = c->vis_counters_clear[1] = false;
+    }
+    c->vis_counter_set = set;
     w.refs = (TileRef*)c->vis_bins.ptr;
     vis_carve_tiles(w, (uint32_t*)c->vis_tile_cnt.ptr, (uint32_t*)c->vis_tile_off.ptr, n_tiles);
     if (!exact) {
-        TGX_TRY(vis_launch(c, s, d_vc, d_outs, n_views, n_tiles, w, VIS_ALL, host_out));
+        TGX_TRY(vis_launch(c, s, d_vc, d_outs, n_views, n_tiles, w, VIS_ALL, host_out, few ? &inl : nullptr));
     } else {
-        TGX_TRY(vis_launch(c, s, d_vc, d_outs, n_views, n_tiles, w, VIS_TO_SCAN, host_out));
+        TGX_TRY(vis_launch(c, s, d_vc, d_outs, n_views, n_tiles, w, VIS_TO_SCAN, host_out, few ? &inl : nullptr));
         TGX_CUDA(cudaMemcpyAsync(c->h_vis_counters, w.counters, C_COUNT * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
         TGX_CUDA(cudaStreamSynchronize(c->stream));
         const uint32_t entries = ((const uint32_t*)c->h_vis_counters)[C_ENTRIES];
@@ -1811,8 +1883,8 @@ tgx_status vis_render_device(tgx_ctx* c, const tgx_scene* s, const tgx_view* vie
     }
     c->vis_last_tiles = n_tiles;
     c->vis_last_pairs = n_pairs;
-    // counters of this frame to pinned memory, read by the next call without waiting
-    TGX_CUDA(cudaMemcpyAsync(c->h_vis_counters, w.counters, C_COUNT * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
+    if (!captured) c->vis_counters_clear[set ^ 1u] = true;
+    // the tile kernel wrote this frame's totals to pinned memory, read by the next call without waiting
     if (!c->vis_done) TGX_CUDA(cudaEventCreateWithFlags(&c->vis_done, cudaEventDisableTiming));
     TGX_CUDA(cudaEventRecord(c->vis_done, c->stream));
     return TGX_OK;
@@ -1929,8 +2001,8 @@ extern "C" tgx_status tgx_frame_graph_create(tgx_ctx* c, const tgx_vis_job* jobs
         w.refs = (TileRef*)p;
         w.bin_capacity = (uint32_t)job.bin_cap;
         vis_carve_tiles(w, tile_cnt, tile_off, job.n_tiles);
-        const ViewConst* d_vc = (const ViewConst*)(base + job.table_off);
-        unsigned long long* const* d_outs = (unsigned long long* const*)(base + job.table_off + job.ptr_off);
+        ViewConst* d_vc = (ViewConst*)(base + job.table_off);
+        unsigned long long** d_outs = (unsigned long long**)(base + job.table_off + job.ptr_off);
         tjobs[j] = tile_job(c, job.scene, d_vc, d_outs, (uint32_t)job.views.size(), job.n_tiles, w);
         tjobs[j].first = j ? tjobs[j - 1].first + g->jobs[j - 1].n_tiles : 0u;
     }
@@ -1974,8 +2046,8 @@ extern "C" tgx_status tgx_frame_graph_create(tgx_ctx* c, const tgx_vis_job* jobs
     if (n_jobs == 1) {
         // one job: its passes and its own tile launch, no fork
         const tgx_frame_graph::Job& job = g->jobs[0];
-        const ViewConst* d_vc = (const ViewConst*)(base + job.table_off);
-        unsigned long long* const* d_outs = (unsigned long long* const*)(base + job.table_off + job.ptr_off);
+        ViewConst* d_vc = (ViewConst*)(base + job.table_off);
+        unsigned long long** d_outs = (unsigned long long**)(base + job.table_off + job.ptr_off);
         st = vis_launch(c, job.scene, d_vc, d_outs, (uint32_t)job.views.size(), job.n_tiles, ws[0], VIS_ALL);
         goto captured;
     }
@@ -1985,8 +2057,8 @@ extern "C" tgx_status tgx_frame_graph_create(tgx_ctx* c, const tgx_vis_job* jobs
     for (uint32_t j = 0; j < n_jobs && st == TGX_OK; j++) {
         const tgx_frame_graph::Job& job = g->jobs[j];
         c->stream = side[j % n_side];
-        const ViewConst* d_vc = (const ViewConst*)(base + job.table_off);
-        unsigned long long* const* d_outs = (unsigned long long* const*)(base + job.table_off + job.ptr_off);
+        ViewConst* d_vc = (ViewConst*)(base + job.table_off);
+        unsigned long long** d_outs = (unsigned long long**)(base + job.table_off + job.ptr_off);
         st = vis_launch(c, job.scene, d_vc, d_outs, (uint32_t)job.views.size(), job.n_tiles, ws[j], VIS_NO_TILES);
         if (st == TGX_OK && cudaEventRecord(done[j], c->stream) != cudaSuccess) st = TGX_ERR_CUDA;
     }
@@ -2172,7 +2244,7 @@ extern "C" tgx_status tgx_vis_get_stats(tgx_ctx* c, tgx_vis_stats* out)
     memset(out, 0, sizeof(*out));
     if (!c->vis_counters.ptr) return TGX_OK;
     uint32_t h[C_COUNT];
-    TGX_CUDA(cudaMemcpyAsync(c->h_counter, c->vis_counters.ptr, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
+    TGX_CUDA(cudaMemcpyAsync(c->h_counter, (uint32_t*)c->vis_counters.ptr + c->vis_counter_set * C_COUNT, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
     TGX_CUDA(cudaStreamSynchronize(c->stream));
     memcpy(h, c->h_counter, sizeof(h));
     out->visible_clusters = h[C_RECORDS];
@@ -2389,9 +2461,9 @@ extern "C" tgx_status tgx_vis_render_noalloc(void* stream, const tgx_object* d_o
     // everything else is written before it is read
     NA_LAUNCH((n_objects + 127) / 128, 128, k_vis_noalloc_setup, vc, (unsigned long long*)d_visbuf, d_vc, d_outs,
               counters, status, d_objects, n_objects, inv_rot);
-    NA_LAUNCH((n_cluster_pointers + 255) / 256, 256, k_vis_cluster_setup<false>, d_objects, d_cluster_pointers,
-              d_cluster_idx_to_object_idx, d_voxel_bits, (const uint32_t*)nullptr, n_cluster_pointers, d_vc, 1u,
-              records, rects, kNaMaxClusterPointers, counters, supers,
+    NA_LAUNCH((n_cluster_pointers + 255) / 256, 256, (k_vis_cluster_setup<false, NoViews>), d_objects, d_cluster_pointers,
+              d_cluster_idx_to_object_idx, d_voxel_bits, (const uint32_t*)nullptr, n_cluster_pointers, NoViews{}, d_vc,
+              d_outs, 1u, records, rects, kNaMaxClusterPointers, counters, supers,
               scan_supers(n_tiles) * kGroupWords + n_tiles * kNaBuckets, chunks, kNaChunks,
               status);
     NA_LAUNCH(warp_grid, 256, k_vis_count, records, rects, counters, kNaMaxClusterPointers, d_objects, d_vc, bucket_cnt,
@@ -2399,7 +2471,7 @@ extern "C" tgx_status tgx_vis_render_noalloc(void* stream, const tgx_object* d_o
     const uint32_t n_scan_ctas = scan_groups(n_tiles);
     NA_LAUNCH(n_scan_ctas, kScanTiles, k_vis_prefix<kNaBuckets>, bucket_cnt, tile_total, n_tiles, groups, supers);
     NA_LAUNCH(n_scan_ctas, kScanTiles, k_vis_finalize, tile_total, n_tiles, groups, supers, tile_off, slot_info, kNaBins,
-              counters, d_vc, 1u);
+              counters, (uint32_t*)nullptr, d_vc, 1u);
     NA_LAUNCH(warp_grid, 256, k_vis_bin_fill, records, rects, counters, d_vc, tile_off, bucket_cnt, refs,
               n_tiles, kNaBins, 1u, chunks, kNaChunks, slot_info, d_outs, 1u, status);
     TileJob J;
@@ -2412,6 +2484,7 @@ extern "C" tgx_status tgx_vis_render_noalloc(void* stream, const tgx_object* d_o
     J.inv_rot = inv_rot;
     J.outs = d_outs;
     J.counters = counters;
+    J.host_counters = nullptr;
     J.n_tiles = n_tiles;
     J.cleared = 1;
     J.first = 0;
