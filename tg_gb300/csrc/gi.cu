@@ -291,6 +291,7 @@ __global__ void __launch_bounds__(32 * kTraceWarps, kTraceCtas) k_trace_queue(
     const uint32_t* __restrict__ n_dev, uint32_t steps_per_round, uint32_t* __restrict__ queue,
     uint32_t* __restrict__ exhausted, unsigned long long* __restrict__ work)
 {
+    pdl_wait();
     const uint32_t n = *n_dev;
     const RayLists io = {ra, ha, rb, hb, n * mul_a, {p.sun_dir[0], p.sun_dir[1], p.sun_dir[2]}};
     svo_trace_queue(s, io, n * mul_a + n * mul_b, p.max_steps, steps_per_round, queue, exhausted, work);
@@ -304,6 +305,7 @@ __global__ void __launch_bounds__(128, 10) k_gi_roots(const tgx_object* __restri
                                                   const unsigned long long* __restrict__ visbuf, float* __restrict__ out,
                                                   PathRoot* __restrict__ roots, uint32_t* __restrict__ n_roots)
 {
+    pdl_wait();
     const uint32_t px = blockIdx.x * 16 + (threadIdx.x & 15u);
     const uint32_t py = blockIdx.y * 8 + (threadIdx.x >> 4);
     if (px >= cam.width || py >= cam.height) return;
@@ -334,8 +336,10 @@ __global__ void __launch_bounds__(128, 10) k_gi_roots(const tgx_object* __restri
 // samples; with root_rays, also the shadow ray of every root.
 __global__ void __launch_bounds__(256) k_gi_emit(const PathRoot* __restrict__ roots, const uint32_t* __restrict__ n_dev,
                                                  uint32_t cs, uint32_t s0, GiParams p, Ray* __restrict__ rays,
-                                                 float4* __restrict__ root_rays)
+                                                 float4* __restrict__ root_rays, uint32_t* __restrict__ queue)
 {
+    pdl_wait();
+    if (blockIdx.x == 0 && threadIdx.x == 0) *queue = 0u;   // of the traversal that follows
     const uint32_t n = *n_dev;
     const uint64_t n_paths = (uint64_t)n * cs;
     const uint64_t n_items = n_paths + (root_rays ? n : 0u);
@@ -365,8 +369,11 @@ __global__ void __launch_bounds__(256) k_gi_shade(SvoDev s, const tgx_material* 
                                                   uint32_t cs, uint32_t s0, uint32_t k, GiParams p,
                                                   Ray* __restrict__ rb, const RayHit* __restrict__ hb,
                                                   float4* __restrict__ rs, const uint32_t* __restrict__ hs,
-                                                  PathSum* __restrict__ sums, float4* __restrict__ through)
+                                                  PathSum* __restrict__ sums, float4* __restrict__ through,
+                                                  uint32_t* __restrict__ queue)
 {
+    pdl_wait();
+    if (blockIdx.x == 0 && threadIdx.x == 0) *queue = 0u;   // of the traversal that follows
     const uint64_t n_paths = (uint64_t)(*n_dev) * cs;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_paths; i += (uint64_t)gridDim.x * blockDim.x) {
         float v[3] = {0.0f, 0.0f, 0.0f}, T[3] = {1.0f, 1.0f, 1.0f};
@@ -433,6 +440,7 @@ __global__ void __launch_bounds__(256) k_gi_finish(const PathRoot* __restrict__ 
                                                    float* __restrict__ acc_buf, bool first, bool last, uint32_t spp,
                                                    float* __restrict__ out)
 {
+    pdl_wait();
     const uint32_t n = *n_dev;
     for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
         float acc[3] = {0.0f, 0.0f, 0.0f};
@@ -507,6 +515,7 @@ __global__ void __launch_bounds__(256) k_gi_query_shade(SvoDev s, const tgx_mate
                                                         float* __restrict__ qx, CacheHit* __restrict__ hits,
                                                         uint32_t* __restrict__ counters, uint32_t capacity)
 {
+    pdl_wait();
     const uint64_t n_paths = (uint64_t)(*n_dev) * cs;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_paths; i += (uint64_t)gridDim.x * blockDim.x) {
         const RayHit h = hb[i];
@@ -539,6 +548,7 @@ __global__ void __launch_bounds__(256) k_gi_primary_queries(const PathRoot* __re
                                                             CacheGiConst q, float cam_x, float cam_y, float cam_z,
                                                             float* __restrict__ qx)
 {
+    pdl_wait();
     const uint32_t n = *n_dev;
     for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
         const PathRoot& rt = roots[r];
@@ -563,6 +573,7 @@ __global__ void __launch_bounds__(256) k_gi_primary_batch(GiParams p, CacheGiCon
                                                           const float* __restrict__ pqx, const float* __restrict__ pmean,
                                                           float* __restrict__ tx, float* __restrict__ tt)
 {
+    pdl_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= q.n_train_primary) return;
     const uint32_t n = *n_dev;
@@ -594,6 +605,7 @@ __global__ void __launch_bounds__(256) k_gi_cache_resolve(const PathRoot* __rest
                                                          float* __restrict__ pmean, float2* __restrict__ pstat,
                                                          float* __restrict__ out)
 {
+    pdl_wait();
     const uint32_t n = *n_dev;
     for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
         const PathRoot& rt = roots[r];
@@ -663,6 +675,7 @@ __global__ void __launch_bounds__(256) k_gi_cache_blend(const PathRoot* __restri
                                                        float primary_weight, float variance_scale,
                                                        float* __restrict__ out)
 {
+    pdl_wait();
     const uint32_t n = *n_dev;
     const float a = (float)(p.spp - 1) / ((float)p.spp - 0.5f);
     for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
@@ -706,6 +719,7 @@ __global__ void __launch_bounds__(256) k_gi_target_roots(GiParams p, CacheGiCons
                                                         PathRoot* __restrict__ roots, float* __restrict__ tx,
                                                         float* __restrict__ tt)
 {
+    pdl_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= q.n_train) return;
     const uint32_t per = steps ? q.n_train / steps : 0u;
@@ -814,13 +828,12 @@ __host__ __device__ inline unsigned long long* trace_work(uint32_t* counters)
     return reinterpret_cast<unsigned long long*>(counters + 32);
 }
 
-// queue = &counters[CC_QUEUE] of the frame's counters
+// queue = &counters[CC_QUEUE] of the frame's counters, zeroed by the kernel that wrote the lists
 tgx_status trace_lists(tgx_ctx* c, const SvoDev& s, const GiParams& p, const Ray* ra, RayHit* ha, uint32_t mul_a,
                        const float4* rb, uint32_t* hb, uint32_t mul_b, const uint32_t* n_dev, uint32_t* queue,
                        uint32_t* exhausted)
 {
-    TGX_CUDA(cudaMemsetAsync(queue, 0, 4, c->stream));
-    TGX_LAUNCH(c, TR_GI_TRACE, trace_grid(c), 128, 0, k_trace_queue, s, ra, ha, mul_a, rb, hb, mul_b, p, n_dev,
+    TGX_LAUNCH_PDL(c, TR_GI_TRACE, trace_grid(c), 128, 0, k_trace_queue, s, ra, ha, mul_a, rb, hb, mul_b, p, n_dev,
                c->trace_steps_per_round, queue, exhausted, trace_work(queue - CC_QUEUE));
     return TGX_OK;
 }
@@ -833,9 +846,9 @@ tgx_status run_paths(tgx_ctx* c, const SvoDev& s, const tgx_material* luts, cons
     const uint32_t cs = chunk_samples(spp, max_roots);
     const uint32_t rg = stride_grid(c, max_roots, 256);
     if (spp == 0 || p.bounces == 0) {   // direct term only
-        TGX_LAUNCH(c, TR_GI, rg, 256, 0, k_gi_emit, b.roots, n_dev, 0u, 0u, p, b.rb, b.root_rays);
+        TGX_LAUNCH_PDL(c, TR_GI, rg, 256, 0, k_gi_emit, b.roots, n_dev, 0u, 0u, p, b.rb, b.root_rays, queue);
         TGX_TRY(trace_lists(c, s, p, nullptr, nullptr, 0u, b.root_rays, b.root_hits, 1u, n_dev, queue, exhausted));
-        TGX_LAUNCH(c, TR_GI, rg, 256, 0, k_gi_finish, b.roots, n_dev, 0u, p, b.hs, b.sums, b.root_hits, b.acc, true, true,
+        TGX_LAUNCH_PDL(c, TR_GI, rg, 256, 0, k_gi_finish, b.roots, n_dev, 0u, p, b.hs, b.sums, b.root_hits, b.acc, true, true,
                    spp, out);
         return TGX_OK;
     }
@@ -843,12 +856,13 @@ tgx_status run_paths(tgx_ctx* c, const SvoDev& s, const tgx_material* luts, cons
     for (uint32_t s0 = 0; s0 < spp; s0 += cs) {
         const uint32_t n = std::min(cs, spp - s0);
         const bool first = s0 == 0, last = s0 + n >= spp;
-        TGX_LAUNCH(c, TR_GI, eg, 256, 0, k_gi_emit, b.roots, n_dev, n, s0, p, b.rb, first ? b.root_rays : nullptr);
+        TGX_LAUNCH_PDL(c, TR_GI, eg, 256, 0, k_gi_emit, b.roots, n_dev, n, s0, p, b.rb, first ? b.root_rays : nullptr,
+                       queue);
         TGX_TRY(trace_lists(c, s, p, b.rb, b.hb, n, b.root_rays, b.root_hits, first ? 1u : 0u, n_dev, queue, exhausted));
         for (uint32_t k = 0; k < p.bounces; k++) {
             const bool more = k + 1 < p.bounces;
-#define SHADE(f, l) TGX_LAUNCH(c, TR_GI, eg, 256, 0, (k_gi_shade<f, l>), s, luts, b.roots, n_dev, n, s0, k, p, b.rb, b.hb, \
-                               b.rs, b.hs, b.sums, b.through)
+#define SHADE(f, l) TGX_LAUNCH_PDL(c, TR_GI, eg, 256, 0, (k_gi_shade<f, l>), s, luts, b.roots, n_dev, n, s0, k, p, b.rb, b.hb, \
+                               b.rs, b.hs, b.sums, b.through, queue)
             if (k == 0 && more) SHADE(true, false);
             else if (k == 0) SHADE(true, true);
             else if (more) SHADE(false, false);
@@ -856,7 +870,7 @@ tgx_status run_paths(tgx_ctx* c, const SvoDev& s, const tgx_material* luts, cons
 #undef SHADE
             TGX_TRY(trace_lists(c, s, p, b.rb, b.hb, more ? n : 0u, b.rs, b.hs, n, n_dev, queue, exhausted));
         }
-        TGX_LAUNCH(c, TR_GI, rg, 256, 0, k_gi_finish, b.roots, n_dev, n, p, b.hs, b.sums, b.root_hits, b.acc, first, last,
+        TGX_LAUNCH_PDL(c, TR_GI, rg, 256, 0, k_gi_finish, b.roots, n_dev, n, p, b.hs, b.sums, b.root_hits, b.acc, first, last,
                    spp, out);
     }
     return TGX_OK;
@@ -893,7 +907,7 @@ extern "C" tgx_status tgx_gi_render(tgx_ctx* c, const tgx_scene* sc, const tgx_s
     uint32_t* exhausted = (uint32_t*)c->svo_counters.ptr + 8;
     TGX_CUDA(cudaMemsetAsync(counters, 0, 64 * 4, c->stream));
     const dim3 grid((view->width + 15) / 16, (view->height + 7) / 8);
-    TGX_LAUNCH(c, TR_GI, grid, 128, 0, k_gi_roots, sc->d_objects, sc->d_cluster_pointers, sc->d_cp_obj, sc->d_inv, sc->d_material,
+    TGX_LAUNCH_PDL(c, TR_GI, grid, 128, 0, k_gi_roots, sc->d_objects, sc->d_cluster_pointers, sc->d_cp_obj, sc->d_inv, sc->d_material,
                sc->d_luts, *view, p, (const unsigned long long*)d_visbuf, d_rgb, b.roots, &counters[CC_ROOTS]);
     return run_paths(c, svo_dev(svo), sc->d_luts, p, b, &counters[CC_ROOTS], (uint32_t)n_pix, p.spp,
                      &counters[CC_QUEUE], exhausted, d_rgb);
@@ -982,42 +996,42 @@ extern "C" tgx_status tgx_gi_render_cached(tgx_ctx* c, const tgx_scene* sc, cons
 
     // primary hits, then the first bounce of every (pixel, sample) in chunks
     const dim3 grid((view->width + 15) / 16, (view->height + 7) / 8);
-    TGX_LAUNCH(c, TR_GI, grid, 128, 0, k_gi_roots, sc->d_objects, sc->d_cluster_pointers, sc->d_cp_obj, sc->d_inv, sc->d_material,
+    TGX_LAUNCH_PDL(c, TR_GI, grid, 128, 0, k_gi_roots, sc->d_objects, sc->d_cluster_pointers, sc->d_cp_obj, sc->d_inv, sc->d_material,
                sc->d_luts, *view, p, (const unsigned long long*)d_visbuf, d_rgb, b.roots, &counters[CC_ROOTS]);
     const uint32_t eg = stride_grid(c, n_pix * cs + n_pix, 256);
     for (uint32_t s0 = 0; s0 < p.spp; s0 += cs) {
         const uint32_t n = std::min(cs, p.spp - s0);
         const bool first = s0 == 0;
-        TGX_LAUNCH(c, TR_GI, eg, 256, 0, k_gi_emit, b.roots, &counters[CC_ROOTS], n, s0, p, b.rb,
-                   first ? b.root_rays : nullptr);
+        TGX_LAUNCH_PDL(c, TR_GI, eg, 256, 0, k_gi_emit, b.roots, &counters[CC_ROOTS], n, s0, p, b.rb,
+                   first ? b.root_rays : nullptr, &counters[CC_QUEUE]);
         TGX_TRY(trace_lists(c, s, p, b.rb, b.hb, n, b.root_rays, b.root_hits, first ? 1u : 0u, &counters[CC_ROOTS],
                             &counters[CC_QUEUE], exhausted));
-        TGX_LAUNCH(c, TR_GI, eg, 256, 0, k_gi_query_shade, s, sc->d_luts, q, &counters[CC_ROOTS], n, s0, p.spp, b.rb,
+        TGX_LAUNCH_PDL(c, TR_GI, eg, 256, 0, k_gi_query_shade, s, sc->d_luts, q, &counters[CC_ROOTS], n, s0, p.spp, b.rb,
                    b.hb, qidx, qx, hits, counters, (uint32_t)capacity);
     }
     // inference over all potential queries: slots past the hit count are never read
     TGX_TRY(cache_infer_counted(c, cache, &counters[CC_QUERIES], (uint32_t)capacity, qx, qrgb));
     if (primary) {
-        TGX_LAUNCH(c, TR_GI, stride_grid(c, n_pix, 256), 256, 0, k_gi_primary_queries, b.roots, &counters[CC_ROOTS], p,
+        TGX_LAUNCH_PDL(c, TR_GI, stride_grid(c, n_pix, 256), 256, 0, k_gi_primary_queries, b.roots, &counters[CC_ROOTS], p,
                    q, view->camera[0], view->camera[1], view->camera[2], pqx);
         if (q.primary_weight > 0.0f)
             TGX_TRY(cache_infer_counted(c, pnet, &counters[CC_ROOTS], (uint32_t)n_pix, pqx, pqrgb));
     }
     // pixels without geometry keep NaN statistics (all bytes 0xff)
     if (blend) TGX_CUDA(cudaMemsetAsync(pstat, 0xff, n_pix * sizeof(float2), c->stream));
-    TGX_LAUNCH(c, TR_GI, stride_grid(c, n_pix, 256), 256, 0, k_gi_cache_resolve, b.roots, &counters[CC_ROOTS], p,
+    TGX_LAUNCH_PDL(c, TR_GI, stride_grid(c, n_pix, 256), 256, 0, k_gi_cache_resolve, b.roots, &counters[CC_ROOTS], p,
                b.root_hits, qidx, qrgb, hits, q.primary_weight > 0.0f ? pqrgb : nullptr, q.primary_weight,
                primary ? pmean : nullptr, blend ? pstat : nullptr, d_rgb);
     if (blend)
-        TGX_LAUNCH(c, TR_GI, stride_grid(c, n_pix, 256), 256, 0, k_gi_cache_blend, b.roots, &counters[CC_ROOTS], p,
+        TGX_LAUNCH_PDL(c, TR_GI, stride_grid(c, n_pix, 256), 256, 0, k_gi_cache_blend, b.roots, &counters[CC_ROOTS], p,
                    b.root_hits, pmean, pqrgb, pstat, view->width, view->height, q.primary_weight,
                    q.primary_variance_scale, d_rgb);
     const bool train_primary = primary && q.n_train_primary && cp->train_steps;
     if (train_primary)
-        TGX_LAUNCH(c, TR_GI, (q.n_train_primary + 255) / 256, 256, 0, k_gi_primary_batch, p, q, &counters[CC_ROOTS], pqx,
+        TGX_LAUNCH_PDL(c, TR_GI, (q.n_train_primary + 255) / 256, 256, 0, k_gi_primary_batch, p, q, &counters[CC_ROOTS], pqx,
                    pmean, ptx, ptt);
     if (train) {
-        TGX_LAUNCH(c, TR_GI, (q.n_train + 255) / 256, 256, 0, k_gi_target_roots, p, q, cp->train_steps, hits,
+        TGX_LAUNCH_PDL(c, TR_GI, (q.n_train + 255) / 256, 256, 0, k_gi_target_roots, p, q, cp->train_steps, hits,
                    counters, (uint32_t)capacity, b.roots, tx, tt);
         GiParams pp = p;
         pp.bounces = p.bounces - 1;

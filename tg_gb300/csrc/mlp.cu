@@ -250,6 +250,7 @@ __global__ void __launch_bounds__(tc::THREADS, 1) k_mlp_forward_tc(const __nv_bf
                                                                   const float* __restrict__ x, float* __restrict__ y,
                                                                   tgx_dev_status* __restrict__ status)
 {
+    pdl_wait();
     extern __shared__ __align__(1024) unsigned char sm[];
     using namespace tc;
     const uint32_t tid = threadIdx.x, warp = tid >> 5;
@@ -973,7 +974,7 @@ static tgx_status cache_forward(tgx_ctx* c, tgx_cache* k, const uint32_t* d_n, u
     }
     const uint32_t tiles = (n + tc::M - 1) / tc::M;
     const uint32_t grid = std::max(1u, std::min<uint32_t>(tiles, (uint32_t)c->num_sms));
-    TGX_LAUNCH(c, TR_MLP, grid, tc::THREADS, tc::SMEM, k_mlp_forward_tc, k->img, n, d_n, d_x, d_rgb, c->d_status);
+    TGX_LAUNCH_PDL(c, TR_MLP, grid, tc::THREADS, tc::SMEM, k_mlp_forward_tc, k->img, n, d_n, d_x, d_rgb, c->d_status);
     return TGX_OK;
 }
 

@@ -109,6 +109,7 @@ __global__ void __launch_bounds__(128, 10) k_shade(const tgx_object* __restrict_
                                               const unsigned long long* __restrict__ visbuf, uint32_t mode,
                                               float4* __restrict__ out)
 {
+    pdl_wait();
     const uint32_t px = blockIdx.x * 16 + (threadIdx.x & 15u);
     const uint32_t py = blockIdx.y * 8 + (threadIdx.x >> 4);
     if (px >= cam.width || py >= cam.height) return;
@@ -163,7 +164,7 @@ extern "C" tgx_status tgx_shade(tgx_ctx* c, const tgx_scene* sc, const tgx_view*
         return TGX_ERR_INVALID_ARGUMENT;
     }
     const dim3 grid((view->width + 15) / 16, (view->height + 7) / 8);
-    TGX_LAUNCH(c, TR_GI, grid, 128, 0, k_shade, sc->d_objects, sc->d_cluster_pointers, sc->d_cp_obj, sc->d_inv, sc->d_material,
+    TGX_LAUNCH_PDL(c, TR_GI, grid, 128, 0, k_shade, sc->d_objects, sc->d_cluster_pointers, sc->d_cp_obj, sc->d_inv, sc->d_material,
                sc->d_luts, *view, (const unsigned long long*)d_visbuf, mode, (float4*)d_rgba);
     return TGX_OK;
 }

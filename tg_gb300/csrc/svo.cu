@@ -219,6 +219,7 @@ __global__ void __launch_bounds__(128) k_svo_candidates(const tgx_object* __rest
                                                        tgx_dev_status* __restrict__ status,
                                                        const uint32_t* __restrict__ dirty /* null: every block; else a bit per block */)
 {
+    pdl_wait();
     const uint32_t cp = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
     const float mn[3] = {mnx, mny, mnz};
     float lo[3], hi[3];
@@ -278,6 +279,7 @@ __global__ void __launch_bounds__(128) k_svo_test_pairs(
     float mny, float mnz, uint32_t L, uint32_t B, uint32_t* __restrict__ table, SvoPair* __restrict__ pairs,
     uint32_t* __restrict__ marked, uint32_t pair_capacity, uint32_t* __restrict__ counters)
 {
+    pdl_wait();
     const uint32_t n = min(counters[S_CAND], pair_capacity), lane = threadIdx.x & 31u;
     const float mn[3] = {mnx, mny, mnz};
     const float ext = (float)(1u << L);
@@ -366,6 +368,7 @@ __global__ void __launch_bounds__(256) k_svo_alloc(uint32_t* __restrict__ table,
                                                   uint32_t* __restrict__ slot_block, uint32_t* __restrict__ nonempty,
                                                   uint32_t* __restrict__ cnt)
 {
+    pdl_wait();
     const uint32_t m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= n) return;
     const uint32_t blk = marked[m];
@@ -405,6 +408,7 @@ __device__ __forceinline__ void smem_max_u16(uint32_t* words, uint32_t idx, uint
 __global__ void __launch_bounds__(256) k_svo_pair_count(const SvoPair* __restrict__ pairs, uint32_t n,
                                                        const uint32_t* __restrict__ table, uint32_t* __restrict__ cnt)
 {
+    pdl_wait();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t blk = pairs[i].block;
         if (blk != kNoBlock) atomicAdd(&cnt[table[blk] - 1u], 1u);
@@ -415,6 +419,7 @@ __global__ void __launch_bounds__(256) k_svo_pair_ranges(const uint32_t* __restr
                                                         uint32_t* __restrict__ total, uint32_t* __restrict__ off,
                                                         uint32_t* __restrict__ cursor)
 {
+    pdl_wait();
     const uint32_t m = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
     const uint32_t c = m < n ? cnt[m] : 0u;
     uint32_t incl = c;
@@ -433,6 +438,7 @@ __global__ void __launch_bounds__(256) k_svo_pair_fill(const SvoPair* __restrict
                                                       const uint32_t* __restrict__ table, uint32_t* __restrict__ cursor,
                                                       SvoPair* __restrict__ sorted)
 {
+    pdl_wait();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const SvoPair pr = pairs[i];
         if (pr.block != kNoBlock) sorted[atomicAdd(&cursor[table[pr.block] - 1u], 1u)] = pr;
@@ -626,6 +632,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerVoxCta, 2) k_svo_voxelize(
     uint32_t* __restrict__ pool, uint32_t* __restrict__ sub, uint32_t* __restrict__ nonempty,
     const uint8_t* __restrict__ material, uint16_t* __restrict__ mat_pool, float mnx, float mny, float mnz, uint32_t B)
 {
+    pdl_wait();
     constexpr uint32_t kLayers = 32u / kSlabs, kWords = kBlockWords / kSlabs;
     extern __shared__ __align__(16) uint32_t s_blk[];   // the slab's bit words, then 16 words of u16 codes for each
     __shared__ PairRec s_rec[kVoxRound];
@@ -781,6 +788,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerVoxCta, 2) k_svo_voxelize(
 __global__ void __launch_bounds__(256) k_svo_publish(uint32_t* __restrict__ table, const uint32_t* __restrict__ marked,
                                                     const uint32_t* __restrict__ slots, uint32_t n)
 {
+    pdl_wait();
     const uint32_t m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m < n) table[marked[m]] = slots[m] + 1u;
 }
@@ -794,6 +802,7 @@ __global__ void __launch_bounds__(256) k_svo_pyramid(const uint32_t* __restrict_
                                                     const uint64_t* __restrict__ occ_off, uint32_t n_levels, uint32_t B,
                                                     uint32_t* __restrict__ counters)
 {
+    pdl_wait();
     const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t i = slot < n_slots ? slot_block[slot] : 0xffffffffu;
     const bool any = i != 0xffffffffu && nonempty[slot] != 0u;
@@ -853,6 +862,7 @@ __global__ void __launch_bounds__(128) k_svo_mark_dirty(const tgx_object* __rest
                                                        const uint32_t* __restrict__ cp_obj, float mnx, float mny,
                                                        float mnz, uint32_t B, uint32_t* __restrict__ dirty)
 {
+    pdl_wait();
     const tgx_object now = cur[blockIdx.x], was = built[blockIdx.x];
     if (same_record(now, was)) return;
     const float mn[3] = {mnx, mny, mnz};
@@ -872,6 +882,7 @@ __global__ void __launch_bounds__(256) k_svo_release_dirty(uint32_t* __restrict_
                                                           const tgx_object* __restrict__ cur, tgx_object* __restrict__ built,
                                                           uint32_t n_objects, uint32_t* __restrict__ counters)
 {
+    pdl_wait();
     const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t w = t; w < n_words; w += stride) {
         uint32_t m = dirty[w];
@@ -897,6 +908,7 @@ __global__ void __launch_bounds__(256) k_svo_release_dirty(uint32_t* __restrict_
 // Table entries still marked after an overflowed candidate pass go back to empty.
 __global__ void __launch_bounds__(256) k_svo_unmark(uint32_t* __restrict__ table, uint64_t n_table)
 {
+    pdl_wait();
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_table; i += (uint64_t)gridDim.x * blockDim.x)
         if (table[i] == kMark) table[i] = 0u;
 }
@@ -1013,10 +1025,10 @@ static tgx_status svo_candidates(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc, co
         TGX_CUDA(cudaMemsetAsync(counters + S_CAND, 0, 4, c->stream));
         if (sc->n_cluster_pointers) {
             const uint32_t cap32 = (uint32_t)std::min<uint64_t>(cap, 0xffffffffu);
-            TGX_LAUNCH(c, TR_SVO_CANDIDATES, (sc->n_cluster_pointers + 127) / 128, 128, 0, k_svo_candidates, sc->d_objects,
+            TGX_LAUNCH_PDL(c, TR_SVO_CANDIDATES, (sc->n_cluster_pointers + 127) / 128, 128, 0, k_svo_candidates, sc->d_objects,
                        sc->d_cp_obj, sc->n_cluster_pointers, s->mn[0], s->mn[1], s->mn[2], s->B, (SvoPair*)c->svo_pairs.ptr,
                        cap32, counters, c->d_status, dirty);
-            TGX_LAUNCH(c, TR_SVO_CANDIDATES, (uint32_t)c->num_sms * 16, 128, 0, k_svo_test_pairs, sc->d_objects, sc->d_inv,
+            TGX_LAUNCH_PDL(c, TR_SVO_CANDIDATES, (uint32_t)c->num_sms * 16, 128, 0, k_svo_test_pairs, sc->d_objects, sc->d_inv,
                        sc->d_cp_obj, s->mn[0], s->mn[1], s->mn[2], s->L, s->B, s->d_table, (SvoPair*)c->svo_pairs.ptr,
                        svo_marked(c), cap32, counters);
         }
@@ -1030,7 +1042,7 @@ static tgx_status svo_candidates(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc, co
         // the capacity error recorded by the first attempt is expected; clear it and the marks it left
         TGX_CUDA(cudaMemsetAsync(c->d_status, 0, sizeof(tgx_dev_status), c->stream));
         const uint32_t grid = (uint32_t)std::min<uint64_t>((n_table + 255) / 256, (uint64_t)c->num_sms * 32);
-        TGX_LAUNCH(c, TR_SVO_ALLOC, grid, 256, 0, k_svo_unmark, s->d_table, n_table);
+        TGX_LAUNCH_PDL(c, TR_SVO_ALLOC, grid, 256, 0, k_svo_unmark, s->d_table, n_table);
         cap = (uint64_t)n_cand + 1024;
     }
     tgx_set_error("tgx_svo: pair count grew between two identical passes");
@@ -1055,12 +1067,12 @@ static tgx_status svo_fill(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc, uint32_t
         SvoPair* sorted = (SvoPair*)(((uintptr_t)(slots + n_marked) + 15) & ~(uintptr_t)15);
         const uint32_t mgrid = (n_marked + 255) / 256;
         const uint32_t pgrid = (uint32_t)std::min<uint64_t>(((uint64_t)n_cand + 255) / 256, (uint64_t)c->num_sms * 16);
-        TGX_LAUNCH(c, TR_SVO_ALLOC, mgrid, 256, 0, k_svo_alloc, s->d_table, marked, n_marked, s->d_free, n_free, next_slot,
+        TGX_LAUNCH_PDL(c, TR_SVO_ALLOC, mgrid, 256, 0, k_svo_alloc, s->d_table, marked, n_marked, s->d_free, n_free, next_slot,
                    slots, s->d_slot_block, s->d_nonempty, cnt);
-        TGX_LAUNCH(c, TR_SVO_VOXELIZE, pgrid, 256, 0, k_svo_pair_count, (const SvoPair*)c->svo_pairs.ptr, n_cand,
+        TGX_LAUNCH_PDL(c, TR_SVO_VOXELIZE, pgrid, 256, 0, k_svo_pair_count, (const SvoPair*)c->svo_pairs.ptr, n_cand,
                    s->d_table, cnt);
-        TGX_LAUNCH(c, TR_SVO_VOXELIZE, mgrid, 256, 0, k_svo_pair_ranges, cnt, n_marked, counters + S_SLOTS, off, cursor);
-        TGX_LAUNCH(c, TR_SVO_VOXELIZE, pgrid, 256, 0, k_svo_pair_fill, (const SvoPair*)c->svo_pairs.ptr, n_cand,
+        TGX_LAUNCH_PDL(c, TR_SVO_VOXELIZE, mgrid, 256, 0, k_svo_pair_ranges, cnt, n_marked, counters + S_SLOTS, off, cursor);
+        TGX_LAUNCH_PDL(c, TR_SVO_VOXELIZE, pgrid, 256, 0, k_svo_pair_fill, (const SvoPair*)c->svo_pairs.ptr, n_cand,
                    s->d_table, cursor, sorted);
         // one CTA per marked block, or four (8 layers each) when there are so few blocks
         // that the heaviest ones (up to 190 pairs against 30 on average) would decide the
@@ -1073,7 +1085,7 @@ static tgx_status svo_fill(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc, uint32_t
             const uint32_t smem = kBlockWords / (slabs) * ((mat) ? 17u : 1u) * 4u;                                     \
             TGX_CUDA(cudaFuncSetAttribute(k_svo_voxelize<mat, slabs>, cudaFuncAttributeMaxDynamicSharedMemorySize,     \
                                           (int)smem));                                                                \
-            TGX_LAUNCH(c, TR_SVO_VOXELIZE, n_marked * (slabs), 32 * kWarpsPerVoxCta, smem, (k_svo_voxelize<mat, slabs>), \
+            TGX_LAUNCH_PDL(c, TR_SVO_VOXELIZE, n_marked * (slabs), 32 * kWarpsPerVoxCta, smem, (k_svo_voxelize<mat, slabs>), \
                        sc->d_objects, sc->d_cluster_pointers, sc->d_c2o, sc->d_bits, sorted, off, cnt, slots, s->d_pool, \
                        s->d_sub, s->d_nonempty, sc->d_material, s->d_mat, s->mn[0], s->mn[1], s->mn[2], s->B);         \
         } while (0)
@@ -1082,10 +1094,10 @@ static tgx_status svo_fill(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc, uint32_t
         else if (split) VOXELIZE(false, 4);
         else VOXELIZE(false, 1);
 #undef VOXELIZE
-        TGX_LAUNCH(c, TR_SVO_PYRAMID, mgrid, 256, 0, k_svo_publish, s->d_table, marked, slots, n_marked);
+        TGX_LAUNCH_PDL(c, TR_SVO_PYRAMID, mgrid, 256, 0, k_svo_publish, s->d_table, marked, slots, n_marked);
     }
     if (n_slots)
-        TGX_LAUNCH(c, TR_SVO_PYRAMID, (n_slots + 255) / 256, 256, 0, k_svo_pyramid, s->d_slot_block, n_slots, s->d_nonempty,
+        TGX_LAUNCH_PDL(c, TR_SVO_PYRAMID, (n_slots + 255) / 256, 256, 0, k_svo_pyramid, s->d_slot_block, n_slots, s->d_nonempty,
                    s->d_occ, (const uint64_t*)((char*)s->d_occ + svo_occ_off_bytes(s->occ_words)), s->n_levels, s->B,
                    counters);
     return TGX_OK;
@@ -1179,11 +1191,11 @@ extern "C" tgx_status tgx_svo_update(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc
     uint32_t* counters = s->d_counters;
     TGX_CUDA(cudaMemsetAsync(dirty, 0, n_words * 4, c->stream));
     TGX_CUDA(cudaMemsetAsync(counters + S_FREED, 0, 2 * 4, c->stream));   // freed, moved
-    TGX_LAUNCH(c, TR_SVO_CANDIDATES, dim3(sc->n_objects, 8), 128, 0, k_svo_mark_dirty, sc->d_objects, s->d_objs,
+    TGX_LAUNCH_PDL(c, TR_SVO_CANDIDATES, dim3(sc->n_objects, 8), 128, 0, k_svo_mark_dirty, sc->d_objects, s->d_objs,
                sc->d_cp_obj, s->mn[0], s->mn[1], s->mn[2], s->B, dirty);
     const uint64_t items = std::max<uint64_t>(n_words, sc->n_objects);
     const uint32_t wgrid = (uint32_t)std::min<uint64_t>((items + 255) / 256, (uint64_t)c->num_sms * 16);
-    TGX_LAUNCH(c, TR_SVO_ALLOC, wgrid, 256, 0, k_svo_release_dirty, s->d_table, n_words, dirty, n_table, s->d_nonempty,
+    TGX_LAUNCH_PDL(c, TR_SVO_ALLOC, wgrid, 256, 0, k_svo_release_dirty, s->d_table, n_words, dirty, n_table, s->d_nonempty,
                s->d_slot_block, s->d_free + s->n_free, sc->d_objects, s->d_objs, sc->n_objects, counters);
     // pairs of the dirty blocks, into the pair storage the last build left (grown when short)
     TGX_TRY(svo_candidates(c, s, sc, dirty, std::max<uint64_t>(1024, c->svo_pairs.bytes / kPairBytes)));
@@ -1200,7 +1212,7 @@ extern "C" tgx_status tgx_svo_update(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc
     if (st == TGX_OK) st = svo_fill(c, s, sc, n_cand, n_marked, n_free, s->n_slots, need);
     if (st != TGX_OK) {   // no mark stays in the table: a traversal would take it for a slot
         const uint32_t grid = (uint32_t)std::min<uint64_t>((n_table + 255) / 256, (uint64_t)c->num_sms * 32);
-        TGX_LAUNCH(c, TR_SVO_ALLOC, grid, 256, 0, k_svo_unmark, s->d_table, n_table);
+        TGX_LAUNCH_PDL(c, TR_SVO_ALLOC, grid, 256, 0, k_svo_unmark, s->d_table, n_table);
         return st;
     }
     s->n_free = n_free - (n_marked - fresh);

@@ -179,7 +179,6 @@ __global__ void __launch_bounds__(256, 4) k_vis_cluster_setup(
     tgx_dev_status* __restrict__ status)
 {
     pdl_wait();
-    pdl_trigger();
     const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     // the (tile, bucket) counts start at zero; k_vis_count runs after this kernel
     for (uint64_t i = gid; i < n_zero; i += (uint64_t)gridDim.x * blockDim.x) zero[i] = 0u;
@@ -350,7 +349,6 @@ __global__ void __launch_bounds__(256) k_vis_count(VisRecord* __restrict__ recor
                                                   uint32_t bshift, const uint2* __restrict__ chunks, uint32_t chunk_cap)
 {
     pdl_wait();
-    pdl_trigger();
     const uint32_t n = min(counters[C_RECORDS], record_capacity);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         VisRecord& rec = records[i];
@@ -425,7 +423,6 @@ __global__ void __launch_bounds__(kScanTiles) k_vis_prefix(uint32_t* __restrict_
     __shared__ uint32_t wsum[kScanTiles / 32];
     if (threadIdx.x < kOrderClasses) cls[threadIdx.x] = 0;
     pdl_wait();
-    pdl_trigger();
     __syncthreads();
     const uint32_t t = blockIdx.x * kScanTiles + threadIdx.x;
     uint32_t run = 0;
@@ -489,13 +486,12 @@ __global__ void __launch_bounds__(kScanTiles) k_vis_finalize(const uint32_t* __r
         uint32_t hi = n_views - 1;   // the last view whose first tile is <= t
         while (view < hi) {
             const uint32_t mid = (view + hi + 1) >> 1;
-            if (views[mid].tile_base <= t) view = mid; else hi = mid - 1;
+            if (__ldcg(&views[mid].tile_base) <= t) view = mid; else hi = mid - 1;
         }
-        const uint32_t lt = t - views[view].tile_base, tiles_x = views[view].tiles_x;
+        const uint32_t lt = t - __ldcg(&views[view].tile_base), tiles_x = __ldcg(&views[view].tiles_x);
         place = lt % tiles_x | (lt / tiles_x) << 16;
     }
     pdl_wait();
-    pdl_trigger();
     // this group's base (the sums before it) and the frame's total
     uint32_t pre = 0, all = 0;
     for (uint32_t i = threadIdx.x; i < n_supers; i += kScanTiles) {
@@ -584,7 +580,6 @@ __global__ void __launch_bounds__(256) k_vis_bin_fill(const VisRecord* __restric
                                                      tgx_dev_status* __restrict__ status)
 {
     pdl_wait();
-    pdl_trigger();
     // after an overflow the tile kernel scans all records instead
     const uint32_t n = counters[C_OVERFLOW] ? 0u : counters[C_RECORDS];
     // tiles k, k + step, ... below end of record i, four at a time so that their atomics are in flight together
@@ -1657,14 +1652,14 @@ static tgx_status vis_launch(tgx_ctx* c, const tgx_scene* s, ViewConst* d_vc, un
         if (!w.next_counters) TGX_CUDA(cudaMemsetAsync(w.counters, 0, C_COUNT * sizeof(uint32_t), c->stream));
         const uint32_t setup_blocks = (uint32_t)((n_pairs + 255) / 256);
 #define SETUP(type, inl)                                                                                               \
-        TGX_LAUNCH(c, TR_VIS_SETUP, setup_blocks, 256, 0, (k_vis_cluster_setup<true, type>),                           \
+        TGX_LAUNCH_PDL(c, TR_VIS_SETUP, setup_blocks, 256, 0, (k_vis_cluster_setup<true, type>),                           \
                    s->d_objects, s->d_cluster_pointers, s->d_c2o, s->d_bits, s->d_cp_obj, s->n_cluster_pointers, inl,  \
                    d_vc, d_outs, n_views, w.records, w.rects, w.rec_cap, w.counters, w.supers,                         \
                    scan_supers(n_tiles) * kGroupWords + n_tiles * (kMaxBuckets >> bshift), w.chunks, w.chunk_cap, c->d_status)
         if (views) SETUP(InlineViews, *views);
         else SETUP(NoViews, NoViews{});
 #undef SETUP
-        // each later pass is a programmatic dependent of the one before
+        // each pass is a programmatic dependent of the one before
         TGX_LAUNCH_PDL(c, TR_VIS_COUNT, warp_grid, 256, 0, k_vis_count, w.records, w.rects, w.counters, w.rec_cap,
                        s->d_objects, d_vc, w.bucket_cnt, n_tiles, bshift, w.chunks, w.chunk_cap);
 #define PREFIX_ARGS w.bucket_cnt, w.tile_total, n_tiles, w.groups, w.supers
