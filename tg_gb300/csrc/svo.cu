@@ -12,8 +12,8 @@
 //      whose whole path passes becomes a (cluster, block) pair; the block is
 //      marked in the dense block table.
 //   2. k_svo_alloc       gives every marked block a slot in the block pool.
-//   3. k_svo_voxelize    the pairs grouped by block (count, ranges, place),
-//      then one CTA per marked block, one warp per pair: the leaf voxelisation
+//   3. k_svo_voxelize    the pairs grouped by block (count, ranges, place; a
+//      record of its corners and range for each), then one CTA per marked block, one warp per pair: the leaf voxelisation
 //      of tg__construct_leaf_node (:102-317) -- corner lerp, [0,8)^3 test, bit
 //      fetch -- into the block's image (and material grid) in shared memory,
 //      written out whole and coalesced, with no global atomics; and inside each
@@ -434,17 +434,6 @@ __global__ void __launch_bounds__(256) k_svo_pair_ranges(const uint32_t* __restr
     if (m < n) off[m] = cursor[m] = base + incl - c;
 }
 
-__global__ void __launch_bounds__(256) k_svo_pair_fill(const SvoPair* __restrict__ pairs, uint32_t n,
-                                                      const uint32_t* __restrict__ table, uint32_t* __restrict__ cursor,
-                                                      SvoPair* __restrict__ sorted)
-{
-    pdl_wait();
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const SvoPair pr = pairs[i];
-        if (pr.block != kNoBlock) sorted[atomicAdd(&cursor[table[pr.block] - 1u], 1u)] = pr;
-    }
-}
-
 // 3b. voxelisation: one CTA per marked block.  Its warps take the block's
 // (cluster, block) pairs; every set voxel goes into the CTA's shared image of
 // the block and its material code into the shared material grid, then the
@@ -461,14 +450,13 @@ struct alignas(16) PairRec
 };
 static_assert(sizeof(PairRec) == 112, "seven 16-byte shared loads");
 
-// Returns the pair's trimmed voxel count in the `layers` layers from slab0 on (the
-// record is written only when there are any).  `plain`: the block side is exactly 32
-// (min not so large that min + extent rounds) and no corner coordinate is NaN or
-// beyond 10^6, which the row loop's arithmetic needs.
-__device__ __forceinline__ uint32_t pair_setup(const tgx_object* __restrict__ objects,
-                                               const uint32_t* __restrict__ cluster_pointers,
-                                               const uint32_t* __restrict__ c2o, const SvoPair& pr, float mnx, float mny,
-                                               float mnz, uint32_t B, uint32_t slab0, uint32_t layers, PairRec* out)
+// `plain`: the block side is exactly 32 (min not so large that min + extent rounds)
+// and no corner coordinate is NaN or beyond 10^6, which the row loop's arithmetic
+// needs.  A pair whose trimmed range is empty has lo = hi = 0.
+__device__ __forceinline__ void pair_setup(const tgx_object* __restrict__ objects,
+                                           const uint32_t* __restrict__ cluster_pointers,
+                                           const uint32_t* __restrict__ c2o, const SvoPair& pr, float mnx, float mny,
+                                           float mnz, uint32_t B, PairRec* __restrict__ out)
 {
     const uint32_t cp = pr.cluster_pointer;
     const uint32_t ci = cluster_pointers[cp];
@@ -495,22 +483,41 @@ __device__ __forceinline__ uint32_t pair_setup(const tgx_object* __restrict__ ob
     const dv3 tmax = vmin(pmax, dv3{ceilf(max_c.x), ceilf(max_c.y), ceilf(max_c.z)});
     const uint32_t x0 = trim_u32(xsub(tmin.x, pmin.x)), y0 = trim_u32(xsub(tmin.y, pmin.y));
     const uint32_t x1 = trim_u32(xsub(tmax.x, pmin.x)), y1 = trim_u32(xsub(tmax.y, pmin.y));
-    const uint32_t z0 = max(trim_u32(xsub(tmin.z, pmin.z)), slab0);
-    const uint32_t z1 = layers == 32u ? trim_u32(xsub(tmax.z, pmin.z)) : min(trim_u32(xsub(tmax.z, pmin.z)), slab0 + layers);
-    if (x0 >= x1 || y0 >= y1 || z0 >= z1) return 0u;
+    const uint32_t z0 = trim_u32(xsub(tmin.z, pmin.z)), z1 = trim_u32(xsub(tmax.z, pmin.z));
+    float4* const q4 = reinterpret_cast<float4*>(out);
+    if (x0 >= x1 || y0 >= y1 || z0 >= z1) {
+        q4[6] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        return;
+    }
     dm4_inverse(cs2ws, ws2cs);
+    float bc[24];
     bool plain = pext.x == 32.0f && pext.y == 32.0f && pext.z == 32.0f;
 #pragma unroll
     for (int q = 0; q < 8; q++) {
         const dv3 c = mulv4p(ws2cs, (q & 1) ? pmax.x : pmin.x, (q & 2) ? pmax.y : pmin.y, (q & 4) ? pmax.z : pmin.z);
-        out->bc[3 * q] = c.x; out->bc[3 * q + 1] = c.y; out->bc[3 * q + 2] = c.z;
+        bc[3 * q] = c.x; bc[3 * q + 1] = c.y; bc[3 * q + 2] = c.z;
         plain = plain && fabsf(c.x) <= 1e6f && fabsf(c.y) <= 1e6f && fabsf(c.z) <= 1e6f;
     }
-    out->lo = x0 | y0 << 8 | z0 << 16;
-    out->hi = x1 | y1 << 8 | z1 << 16;
-    out->ci = ci;
-    out->lut = ((od.lut_idx << 8) & 0x7fffffffu) | (plain ? 0u : 0x80000000u);
-    return (x1 - x0) * (y1 - y0) * (z1 - z0);
+#pragma unroll
+    for (int q = 0; q < 6; q++) q4[q] = make_float4(bc[4 * q], bc[4 * q + 1], bc[4 * q + 2], bc[4 * q + 3]);
+    reinterpret_cast<uint4*>(out)[6] = make_uint4(x0 | y0 << 8 | z0 << 16, x1 | y1 << 8 | z1 << 16, ci,
+                                                  ((od.lut_idx << 8) & 0x7fffffffu) | (plain ? 0u : 0x80000000u));
+}
+
+// The pairs' records, those of a block side by side: a thread per pair.
+__global__ void __launch_bounds__(128) k_svo_pair_fill(const SvoPair* __restrict__ pairs, uint32_t n,
+                                                      const uint32_t* __restrict__ table, uint32_t* __restrict__ cursor,
+                                                      const tgx_object* __restrict__ objects,
+                                                      const uint32_t* __restrict__ cluster_pointers,
+                                                      const uint32_t* __restrict__ c2o, float mnx, float mny, float mnz,
+                                                      uint32_t B, PairRec* __restrict__ recs)
+{
+    pdl_wait();
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const SvoPair pr = pairs[i];
+        if (pr.block == kNoBlock) continue;
+        pair_setup(objects, cluster_pointers, c2o, pr, mnx, mny, mnz, B, recs + atomicAdd(&cursor[table[pr.block] - 1u], 1u));
+    }
 }
 
 // The z- and y-lerps of tg__construct_leaf_node for row (iy, iz) of a block:
@@ -608,27 +615,30 @@ __device__ __forceinline__ void layer_masks(const uint32_t* rows, uint32_t u, ui
     if (lane == 0) reinterpret_cast<uint16_t*>(sb + 16)[u] = (uint16_t)w8;
 }
 
-// Bound by instruction issue.  The pairs are taken kVoxRound at a time.  First a
-// lane per pair computes its matrices, trimmed range and corners (with a warp
-// per pair that set-up was half of all instructions) and the ranges' voxel
-// counts are sorted by a warp bitonic sort per 32, heaviest first; then the
-// warps take pairs in that order from a shared counter, the next one whenever
-// they finish one.  Within a pair, a lane takes a row (iy, iz) of the range: the
-// z- and y-lerps once per row; the x-lerp, the [0, 8)^3 test and the bit fetch
-// per voxel, floor and range test in the bits of c + 1.5 * 2^23 rounded down
-// (no conversion); the row's bits in one atomicOr on its word of the image.
-// Material codes are stored plainly.  A voxel that two pairs set (objects that
-// overlap) needs the larger code: the second atomicOr finds its bit, marks it
-// in s_conf, and blocks with marks go over their pairs once more for those
-// voxels alone, with a 16-bit max.  The order of the pairs changes no bit.
-// 512 objects, 4096^3, 565k pairs in 18.4k blocks: 2350 -> 1520 us.
-constexpr uint32_t kVoxRound = 128;     // pairs set up at a time
+// Bound by instruction issue.  The pairs are taken kVoxRound at a time: their
+// records (k_svo_pair_fill: matrices, trimmed range, corners) are copied to
+// shared memory, their voxel counts sorted by a warp bitonic sort per 32,
+// heaviest first; then the warps take pairs in that order from a shared counter,
+// the next one whenever they finish one.  Within a pair, a lane takes a row
+// (iy, iz) of the range: the z- and y-lerps once per row; the x-lerp, the
+// [0, 8)^3 test and the bit fetch per voxel, floor and range test in the bits of
+// c + 1.5 * 2^23 rounded down (no conversion); the row's bits in one atomicOr on
+// its word of the image.  Material codes are stored plainly.  A voxel that two
+// pairs set (objects that overlap) needs the larger code: the second atomicOr
+// finds its bit, marks it in s_conf, and blocks with marks go over their pairs
+// once more for those voxels alone, with a 16-bit max.  The order of the pairs
+// changes no bit.
+// 512 objects, 4096^3, 565k pairs in 18.4k blocks: 2350 us with a warp per pair
+// doing its set-up, 1430 with a lane per pair in the CTA's first warp (the
+// others waited for it), 1245 with the records made by the pass that groups the
+// pairs (29 us, 13 before).  Loading the next pair's bits ahead into registers:
+// 1460 (spills); into L1: no change.
+constexpr uint32_t kVoxRound = 128;     // pairs in shared memory at a time
 
 template <bool kMat, uint32_t kSlabs>
 __global__ void __launch_bounds__(32 * kWarpsPerVoxCta, 2) k_svo_voxelize(
-    const tgx_object* __restrict__ objects, const uint32_t* __restrict__ cluster_pointers,
-    const uint32_t* __restrict__ c2o, const uint32_t* __restrict__ bits, const SvoPair* __restrict__ sorted,
-    const uint32_t* __restrict__ off, const uint32_t* __restrict__ cnt, const uint32_t* __restrict__ slots,
+    const uint32_t* __restrict__ bits, const PairRec* __restrict__ recs, const uint32_t* __restrict__ off,
+    const uint32_t* __restrict__ cnt, const uint32_t* __restrict__ marked, const uint32_t* __restrict__ slots,
     uint32_t* __restrict__ pool, uint32_t* __restrict__ sub, uint32_t* __restrict__ nonempty,
     const uint8_t* __restrict__ material, uint16_t* __restrict__ mat_pool, float mnx, float mny, float mnz, uint32_t B)
 {
@@ -647,6 +657,8 @@ __global__ void __launch_bounds__(32 * kWarpsPerVoxCta, 2) k_svo_voxelize(
     const uint32_t slot = slots[m];
     const uint32_t pb = off[m], pe = pb + cnt[m];   // at least one pair
     const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    // the end of a pair's layers inside the slab (whole blocks: as the record has it)
+    auto slab_end = [&](uint32_t z1) { return kSlabs == 1u ? z1 : min(z1, slab0 + kLayers); };
     bool again = false;                  // the pass over the doubly set voxels (the same in every thread)
     for (;;) {
         bool conflict = false;           // this thread met a doubly set voxel
@@ -656,11 +668,15 @@ __global__ void __launch_bounds__(32 * kWarpsPerVoxCta, 2) k_svo_voxelize(
             __syncthreads();   // the previous round's records are consumed
             if (wid < n_chunks) {
                 const uint32_t i = wid * 32u + lane;
-                // key: voxel count (pairs past the end sort last); value: pair in the round
+                // key: voxel count in the slab (pairs past the end sort last); value: pair in the round
                 int32_t key = -1;
                 uint32_t idx = i;
-                if (i < np)
-                    key = (int32_t)pair_setup(objects, cluster_pointers, c2o, sorted[r0 + i], mnx, mny, mnz, B, slab0, kLayers, &s_rec[i]);
+                if (i < np) {
+                    const uint2 range = *reinterpret_cast<const uint2*>(&recs[r0 + i].lo);
+                    const uint32_t x = (range.y & 255u) - (range.x & 255u), y = ((range.y >> 8) & 255u) - ((range.x >> 8) & 255u);
+                    const uint32_t z0 = max(range.x >> 16, slab0), z1 = slab_end(range.y >> 16);
+                    key = z0 < z1 ? (int32_t)(x * y * (z1 - z0)) : 0;
+                }
                 // ascending bitonic sort over the warp's 32 lanes
 #pragma unroll
                 for (uint32_t k = 2; k <= 32; k <<= 1) {
@@ -675,12 +691,14 @@ __global__ void __launch_bounds__(32 * kWarpsPerVoxCta, 2) k_svo_voxelize(
                 }
                 // descending rank 31 - lane; pairs without voxels are left out
                 s_order[wid * 32u + (31u - lane)] = (uint8_t)(key > 0 ? idx : 255u);
-            } else if (r0 == pb && !again) {   // the other warps clear the block
-                const uint32_t words = kWords * (kMat ? 17u : 1u), first = n_chunks * 32u;
-                for (uint32_t k = threadIdx.x - first; k < words / 4u; k += blockDim.x - first)
+            }
+            for (uint32_t k = threadIdx.x; k < np * 7u; k += blockDim.x)
+                reinterpret_cast<uint4*>(s_rec)[k] = reinterpret_cast<const uint4*>(recs + r0)[k];
+            if (r0 == pb && !again) {   // clear the block
+                for (uint32_t k = threadIdx.x; k < kWords * (kMat ? 17u : 1u) / 4u; k += blockDim.x)
                     reinterpret_cast<uint4*>(s_blk)[k] = make_uint4(0u, 0u, 0u, 0u);
                 if (kMat)
-                    for (uint32_t k = threadIdx.x - first; k < kWords; k += blockDim.x - first) s_conf[k] = 0u;
+                    for (uint32_t k = threadIdx.x; k < kWords; k += blockDim.x) s_conf[k] = 0u;
             }
             if (threadIdx.x == 0) s_next = 0u;
             __syncthreads();
@@ -699,8 +717,8 @@ __global__ void __launch_bounds__(32 * kWarpsPerVoxCta, 2) k_svo_voxelize(
                     bc[4 * q] = t.x; bc[4 * q + 1] = t.y; bc[4 * q + 2] = t.z; bc[4 * q + 3] = t.w;
                 }
                 const uint4 rm = *reinterpret_cast<const uint4*>(&s_rec[k].lo);
-                const uint32_t x0 = rm.x & 255u, y0 = (rm.x >> 8) & 255u, z0 = rm.x >> 16;
-                const uint32_t x1 = rm.y & 255u, ny = ((rm.y >> 8) & 255u) - y0, nz = (rm.y >> 16) - z0;
+                const uint32_t x0 = rm.x & 255u, y0 = (rm.x >> 8) & 255u, z0 = max(rm.x >> 16, slab0);
+                const uint32_t x1 = rm.y & 255u, ny = ((rm.y >> 8) & 255u) - y0, nz = slab_end(rm.y >> 16) - z0;
                 const uint32_t lut = rm.w & 0x7fffffffu;   // << 8 already
                 // the cluster's 16 bit words and 512 material bytes
                 __syncwarp();
@@ -717,7 +735,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerVoxCta, 2) k_svo_voxelize(
                 if (rm.w >> 31) {
                     // (again as well: it only takes maxima)
                     voxelize_any<kMat>(bc, x0, x1, y0, z0, ny, rows, rny, lut, cw, cm, mnx, mny, mnz, B,
-                                       sorted[r0 + k].block, slab0 * 32u, kWords, img, s_blk + kWords);
+                                       marked[m], slab0 * 32u, kWords, img, s_blk + kWords);
                     continue;
                 }
                 for (uint32_t row = lane; row < rows; row += 32) {
@@ -1055,7 +1073,7 @@ static tgx_status svo_fill(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc, uint32_t
                            uint32_t n_free, uint32_t next_slot, uint32_t n_slots)
 {
     uint32_t* counters = s->d_counters;
-    const size_t sort_bytes = (size_t)n_marked * 4 * 4 + (size_t)s->n_pairs * sizeof(SvoPair) + 64;
+    const size_t sort_bytes = (size_t)n_marked * 4 * 4 + (size_t)s->n_pairs * sizeof(PairRec) + 64;
     TGX_TRY(devbuf_reserve(c->svo_sort, sort_bytes));
     TGX_CUDA(cudaMemsetAsync(counters + S_SLOTS, 0, 2 * 4, c->stream));   // pair ranges handed out, non-empty
     TGX_CUDA(cudaMemsetAsync(s->d_occ, 0, s->occ_words * 4, c->stream));
@@ -1064,7 +1082,7 @@ static tgx_status svo_fill(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc, uint32_t
         const uint32_t* marked = svo_marked(c);
         uint32_t* cnt = (uint32_t*)c->svo_sort.ptr;
         uint32_t *off = cnt + n_marked, *cursor = off + n_marked, *slots = cursor + n_marked;
-        SvoPair* sorted = (SvoPair*)(((uintptr_t)(slots + n_marked) + 15) & ~(uintptr_t)15);
+        PairRec* recs = (PairRec*)(((uintptr_t)(slots + n_marked) + 15) & ~(uintptr_t)15);
         const uint32_t mgrid = (n_marked + 255) / 256;
         const uint32_t pgrid = (uint32_t)std::min<uint64_t>(((uint64_t)n_cand + 255) / 256, (uint64_t)c->num_sms * 16);
         TGX_LAUNCH_PDL(c, TR_SVO_ALLOC, mgrid, 256, 0, k_svo_alloc, s->d_table, marked, n_marked, s->d_free, n_free, next_slot,
@@ -1072,11 +1090,12 @@ static tgx_status svo_fill(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc, uint32_t
         TGX_LAUNCH_PDL(c, TR_SVO_VOXELIZE, pgrid, 256, 0, k_svo_pair_count, (const SvoPair*)c->svo_pairs.ptr, n_cand,
                    s->d_table, cnt);
         TGX_LAUNCH_PDL(c, TR_SVO_VOXELIZE, mgrid, 256, 0, k_svo_pair_ranges, cnt, n_marked, counters + S_SLOTS, off, cursor);
-        TGX_LAUNCH_PDL(c, TR_SVO_VOXELIZE, pgrid, 256, 0, k_svo_pair_fill, (const SvoPair*)c->svo_pairs.ptr, n_cand,
-                   s->d_table, cursor, sorted);
+        TGX_LAUNCH_PDL(c, TR_SVO_VOXELIZE, (uint32_t)std::min<uint64_t>(((uint64_t)n_cand + 127) / 128, (uint64_t)c->num_sms * 32),
+                       128, 0, k_svo_pair_fill, (const SvoPair*)c->svo_pairs.ptr, n_cand, s->d_table, cursor, sc->d_objects,
+                       sc->d_cluster_pointers, sc->d_c2o, s->mn[0], s->mn[1], s->mn[2], s->B, recs);
         // one CTA per marked block, or four (8 layers each) when there are so few blocks
         // that the heaviest ones (up to 190 pairs against 30 on average) would decide the
-        // time: 280 blocks of an update 222 -> 98 us; 18.4k blocks take 1430 us whole and 2560 split
+        // time: 280 blocks of an update 222 -> 98 us; 18.4k blocks took 1430 us whole and 2560 split
         // (and only where every block's side is exactly 32, so that a voxel's index stays in its layers)
         bool split = (uint64_t)n_marked < (uint64_t)c->num_sms * 16u;
         for (int i = 0; i < 3; i++) split = split && fabsf(s->mn[i]) + (float)(1u << s->L) <= 16777216.0f;
@@ -1086,7 +1105,7 @@ static tgx_status svo_fill(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc, uint32_t
             TGX_CUDA(cudaFuncSetAttribute(k_svo_voxelize<mat, slabs>, cudaFuncAttributeMaxDynamicSharedMemorySize,     \
                                           (int)smem));                                                                \
             TGX_LAUNCH_PDL(c, TR_SVO_VOXELIZE, n_marked * (slabs), 32 * kWarpsPerVoxCta, smem, (k_svo_voxelize<mat, slabs>), \
-                       sc->d_objects, sc->d_cluster_pointers, sc->d_c2o, sc->d_bits, sorted, off, cnt, slots, s->d_pool, \
+                       sc->d_bits, recs, off, cnt, marked, slots, s->d_pool,                                           \
                        s->d_sub, s->d_nonempty, sc->d_material, s->d_mat, s->mn[0], s->mn[1], s->mn[2], s->B);         \
         } while (0)
         if (s->d_mat && split) VOXELIZE(true, 4);
