@@ -295,7 +295,8 @@ tgx_status  tgx_get_memory(tgx_ctx* ctx, uint64_t* out_budget, uint64_t* out_sce
  *                  tile can stop once every pixel is nearer than what is left;
  *   batch          clusters staged per shared-memory batch, 1..48 (48);
  *   drain          (pixel, cluster) pairs a warp collects before its lanes
- *                  run their DDAs, 1..32 (32).
+ *                  run their DDAs, 1..32 (32); half as many as long as a
+ *                  pixel of the warp has found nothing.
  * The result never depends on them (bit for bit); tg_gb300/autotune.py picks
  * them per workload.  No counterpart in the reference. */
 tgx_status  tgx_set_vis_tuning(tgx_ctx* ctx, uint32_t depth_buckets, uint32_t batch, uint32_t drain);
