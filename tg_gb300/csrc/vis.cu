@@ -1380,15 +1380,21 @@ __device__ __forceinline__ void vis_tile_groups(const TileJob& J, uint32_t slot,
 // Instantiated per block size (= tile pixels) so the register budget can be
 // bounded for the occupancy each size needs.  One CTA per tile of one job.
 // The slot (heavy-first order, the tiles without entries last) that CTA b of
-// t takes.  With interleave, the n non-empty tiles keep their order but are
-// spread over the launch, one every t / n CTAs, and the empty ones fill the
-// CTAs between: CTA b is the c(b)-th non-empty one when c(b + 1) > c(b), with
-// c(b) = floor(b n / t), else the (b - c(b))-th empty one.  Both maps are
-// bijections of [0, t).
+// t takes.  With interleave (outputs in host memory), the n non-empty tiles keep
+// their order but the e = t - n empty ones are spread over the first f = 3/2 e
+// CTAs, two of three: there the heavy tiles write little, and at the end the
+// light ones fill the link by themselves.  Among the first f, CTA b is the
+// c(b)-th non-empty one when c(b + 1) > c(b), with c(b) = floor(b (f - e) / f),
+// else the (b - c(b))-th empty one.  Both maps are bijections of [0, t).  Frame of
+// 512 objects at 1920x1080 to pinned memory: 148.1 us with the empty tiles
+// spread over the whole launch, 145.2 at 2 of 3 (or 3 of 5), 148.4 at 4 of 5,
+// 163 with all of them first.
 __device__ __forceinline__ uint32_t tile_slot(uint32_t b, uint32_t t, uint32_t n, bool interleave)
 {
     if (!interleave || n >= t) return b;
-    const uint32_t c0 = (uint32_t)((uint64_t)b * n / t), c1 = (uint32_t)((uint64_t)(b + 1) * n / t);
+    const uint32_t e = t - n, f = (uint32_t)min((uint64_t)t, (uint64_t)e * 3u / 2u);
+    if (b >= f) return b - e;
+    const uint32_t c0 = (uint32_t)((uint64_t)b * (f - e) / f), c1 = (uint32_t)((uint64_t)(b + 1) * (f - e) / f);
     return c1 > c0 ? c0 : n + (b - c0);
 }
 
