@@ -290,7 +290,7 @@ struct alignas(16) LevelDesc
     uint32_t pad;
 };
 static_assert(sizeof(LevelDesc) == 32, "two 16-byte shared loads");
-constexpr uint32_t kAscend = 16;   // ascend[p]: p = trailing zeros of the coordinate stepped to
+constexpr uint32_t kAscend = 32;   // ascend[p]: p = trailing zeros of the coordinate stepped to (kMagic's end at 22)
 
 // The level a step ascends to and that level's low mask.  p is the highest
 // coordinate bit the step changed (the carry of the increment, i.e. the
@@ -310,11 +310,11 @@ struct TraceTables
     uint2 ascend[kAscend];   // level * sizeof(LevelDesc), low mask
 };
 
-// Fills the tables for SVO s, threads 0 .. 15 of the block; the caller synchronises.
+// Fills the tables for SVO s, the first warp of the block; the caller synchronises.
 __device__ __forceinline__ void svo_level_tables(const SvoDev& s, TraceTables& tb)
 {
     const uint32_t i = threadIdx.x;
-    if (i >= 16u) return;
+    if (i >= kAscend) return;
     LevelDesc d = {};
     if (i < s.NL) {
         const uint32_t g = svo_level_log2(s.L, i);
@@ -334,7 +334,7 @@ __device__ __forceinline__ void svo_level_tables(const SvoDev& s, TraceTables& t
             d.mk = 31u & ~d.low;
         }
     }
-    tb.lv[i] = d;
+    if (i < 16u) tb.lv[i] = d;
     const uint32_t up = svo_ascend_level(s.L, s.NL, i);
     tb.ascend[i] = make_uint2(up * (uint32_t)sizeof(LevelDesc), (1u << svo_level_log2(s.L, up)) - 1u);
 }
@@ -469,6 +469,18 @@ __device__ __forceinline__ int svo_trace_begin(const SvoDev& s, const TraceTable
     return kTraceRunning;
 }
 
+// v = min(a, b) and v = max(v, a) unless `keep`: one predicated instruction each,
+// where a selection would be a second one (GI frame 1355 -> 1334 us, with the four
+// places of the traversal's loop).
+__device__ __forceinline__ void min_unless(bool keep, uint32_t& v, uint32_t a, uint32_t b)
+{
+    asm("{\n .reg .pred p;\n setp.eq.u32 p, %1, 0;\n @p min.s32 %0, %2, %3;\n}" : "+r"(v) : "r"((uint32_t)keep), "r"(a), "r"(b));
+}
+__device__ __forceinline__ void max_unless(bool keep, float& v, float a)
+{
+    asm("{\n .reg .pred p;\n setp.eq.u32 p, %1, 0;\n @p max.f32 %0, %0, %2;\n}" : "+f"(v) : "r"((uint32_t)keep), "f"(a));
+}
+
 // Runs at most n iterations of the DDA of a ray (each is one step of the
 // max_steps budget: one level down into an occupied cell, or one cell on).
 // Returns kTraceRunning, 1 on hit (r.t, r.v real coordinates, r.last_axis), 0
@@ -489,7 +501,7 @@ __device__ __forceinline__ int svo_trace_run(const SvoDev& s, const TraceTables&
             const uint32_t word = svo_level_word(ld, i, r.tv);
             // While the word is on its way: the step that an empty cell takes.  The distance to
             // the next cell on every axis: its first voxel w, less the origin, times 1 / d
-            uint32_t w[3], nv[3];
+            uint32_t w[3], nv[3], hi[3];
             float tn[3];
 #pragma unroll
             for (int a = 0; a < 3; a++) {
@@ -501,21 +513,22 @@ __device__ __forceinline__ int svo_trace_run(const SvoDev& s, const TraceTables&
             const bool a2 = tn[2] < t01;
             const uint32_t ws = a2 ? w[2] : a1 ? w[1] : w[0];
             // a step out of the cube also runs to the end (its level and point are not used)
-            const uint2 up = tb.ascend[__popc(~ws & (ws - 1u)) & (kAscend - 1u)];
-            const float t = fmaxf(r.t, fminf(t01, tn[2]));   // no NaN, and r.t is never -0
+            const uint2 up = tb.ascend[__popc(~ws & (ws - 1u))];
+            const float to = fminf(t01, tn[2]), t = fmaxf(r.t, to);   // no NaN, and r.t is never -0
             // the point in the new cell: located at voxel resolution, clamped to the cell
 #pragma unroll
             for (int a = 0; a < 3; a++) {
                 const bool moved = a == 2 ? a2 : a == 1 ? a1 && !a2 : !a1 && !a2;
-                const int32_t lo = (int32_t)((moved ? w[a] : r.v[a]) & ~up.y), hi = lo | (int32_t)up.y;
+                const int32_t lo = (int32_t)((moved ? w[a] : r.v[a]) & ~up.y);
                 const int32_t at = __float_as_int(__fadd_rd(xadd(r.og[a], xmul(t, r.d[a])), r.off[a]));
-                nv[a] = (uint32_t)min(max(at, lo), hi);
+                nv[a] = (uint32_t)max(at, lo);
+                hi[a] = (uint32_t)lo | up.y;
             }
             const bool set = __funnelshift_r(word, 0u, i) & 1u;   // the shift takes i mod 32
             const uint32_t lo0 = r.lo;
 #pragma unroll
-            for (int a = 0; a < 3; a++) r.v[a] = set ? r.v[a] : nv[a];
-            r.t = set ? r.t : t;
+            for (int a = 0; a < 3; a++) min_unless(set, r.v[a], nv[a], hi[a]);
+            max_unless(set, r.t, to);
             r.last_axis = set ? r.last_axis : a2 ? 2 : a1 ? 1 : 0;
             r.lo = set ? lo0 - (uint32_t)sizeof(LevelDesc) : up.x;
             if (set) {
