@@ -1121,7 +1121,7 @@ def main() -> None:
             # the tile kernel's real ceiling is instruction issue, not HBM: its ncu issue-slot fraction
             limiter = {"kind": "issue", "smsp__issue_active": prof["smsp__issue_active"],
                        "threads_per_warp_instruction": prof.get("threads_per_warp_instruction"),
-                       "what": prof.get("limiter"), "source": "profiles/vis_tiles_1080p_512obj.md"}
+                       "what": prof.get("limiter"), "source": "profiles/hot_kernels_512obj.md"}
     # the pass's FP32 work model (12 ops per DDA step + 60 ops of set-up per evaluated pair), from
     # the kernel's own counts, against one FP32 op per lane per clock at the sampled SM clock
     clk = clocks.summary()
@@ -1143,12 +1143,12 @@ def main() -> None:
     bf16 = peaks.get("bf16_tflops", 1900.0)
     if "gi_trace_work" in gi_report:
         tw = gi_report["gi_trace_work"]
-        tbytes = 4 * tw["dda_steps"] + 48 * tw["rays"]
+        tbytes = 4 * tw["dda_steps"] + 20 * tw["rays"]
         tach = tbytes / (tw["k_trace_queue_ms"] * 1e-3) / 1e9
         rooflines["k_trace_queue"] = {
             "bound": "hbm", "achieved": tach, "peak": hbm_peak, "unit": "GB/s", "frac": tach / hbm_peak,
             "algorithmic_bytes": tbytes, "traffic": None,
-            "bytes_model": "4 B of occupancy per DDA step + 24 B ray read + 24 B hit written per ray, counted by "
+            "bytes_model": "4 B of occupancy per DDA step + at least 16 B ray read + 4 B result written per ray (a shadow ray; a bounce ray has 24 and 16), counted by "
                            "the kernel (tgx_gi_get_work); the SVO working set is L2-resident, so the limiter is "
                            "latency and divergent issue, not DRAM",
             "dda_steps_per_s": tw["dda_steps"] / (tw["k_trace_queue_ms"] * 1e-3)}
