@@ -1847,7 +1847,7 @@ tgx_status vis_render_device(tgx_ctx* c, const tgx_scene* s, const tgx_view* vie
                 TGX_TRY(devbuf_reserve(c->vis_bins, (size_t)hc[C_ENTRIES] * 2 * kEntry));
         }
         cudaGetLastError();
-        TGX_TRY(devbuf_reserve(c->vis_bins, std::max<size_t>((size_t)n_tiles * 16, (size_t)1 << 18) * kEntry));
+        TGX_TRY(devbuf_reserve(c->vis_bins, std::max<size_t>((size_t)n_tiles * 128, (size_t)1 << 20) * kEntry));
         w.bin_capacity = (uint32_t)std::min<size_t>(c->vis_bins.bytes / kEntry, 0xffffffffu);
     }
     w.rec_cap = (uint32_t)n_pairs;
@@ -1969,7 +1969,11 @@ extern "C" tgx_status tgx_frame_graph_create(tgx_ctx* c, const tgx_vis_job* jobs
         job.table_off = table_bytes;
         table_bytes += al(tables[j].size());
         job.rec_cap = (uint64_t)jb.scene->n_cluster_pointers * jb.n_views;
-        job.bin_cap = std::max<uint64_t>(1u << 14, std::max<uint64_t>((uint64_t)job.n_tiles * 4, (uint64_t)entries * 3 / 2));
+        // Room for cameras that meet more than these ones: a replay that overflows scans all
+        // records for every tile (batches of 20 views at random poses, 16 of one scene: with a
+        // twelfth of this room, the same bytes when an entry had 96, 19 of 60 replays with new
+        // cameras overflowed and took 4 to 15 ms; with this room none of 100 does and they take 2).
+        job.bin_cap = std::max<uint64_t>(3u << 16, std::max<uint64_t>((uint64_t)job.n_tiles * 48, (uint64_t)entries * 18));
         if (job.rec_cap > 0xffffffffull || job.bin_cap > 0xffffffffull || (uint64_t)total_tiles + job.n_tiles > 0xffffffffull) {
             tgx_set_error("tgx_frame_graph_create: job %u has too many (view, cluster) pairs or tiles", j);
             return fail(TGX_ERR_CAPACITY);
