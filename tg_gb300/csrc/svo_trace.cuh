@@ -568,6 +568,10 @@ constexpr uint32_t kTraceWarps = 4;     // 128 threads
 // 6 CTAs measured 5 % and 4 % slower on a 1080p GI frame (2.00 and 1.97 ms against 1.90)
 constexpr uint32_t kTraceCtas = 7;
 constexpr uint32_t kRing = 64;          // parked states per warp
+// Rounds once no ray is left to take are longer by this factor: a refill has nothing
+// to give, and the longest rays decide the time (two frames of an update 903 -> 887
+// us, million rays 306 -> 302; 8 the same, 32: 893 and 304).
+constexpr uint32_t kTailFactor = 4;
 
 template <class IO>
 __device__ __forceinline__ void svo_trace_queue(const SvoDev& s, const IO& io, uint32_t n, uint32_t max_steps,
@@ -644,7 +648,8 @@ __device__ __forceinline__ void svo_trace_queue(const SvoDev& s, const IO& io, u
         __syncwarp();
         if (!__any_sync(0xffffffffu, have) && drained && count == 0) break;
         if (have) {
-            const int res = svo_trace_run(s, tb, r, max_steps, steps_per_round);
+            // nothing left to take: the lanes run on by themselves
+            const int res = svo_trace_run(s, tb, r, max_steps, drained && count == 0 ? kTailFactor * steps_per_round : steps_per_round);
             if (res != kTraceRunning) {
                 store(item, res, r);
                 have = false;
