@@ -848,17 +848,23 @@ struct TileJob
 //   every pixel's best packed word so far (the pair lanes' atomicMin target);
 //   per warp, a ring of kQueue live (pixel, entry) pairs waiting for a lane:
 //   the pixel's cluster-space direction and reciprocals and the packed
-//   lane | entry << 5 | sure_hit << 11.
-constexpr uint32_t kBatch = 48;                      // entries per staged batch (k < 64 fits the packed word)
+//   lane | entry << 5 | sure_hit << 13.
+constexpr uint32_t kBatch = 48;                      // entries per staged batch
 constexpr uint32_t kQueue = 64;                      // ring entries per warp (an entry adds at most 32)
 constexpr uint32_t kWarpRays = 7 * kQueue;           // then the bounds of the warp's rays (warp_rays): 6 floats
 constexpr uint32_t kQueueWords = kWarpRays + 8;      // the ring: 6 float arrays + the packed word
 constexpr uint32_t kSmBar = 0, kSmN = 12, kSmLost = 16, kSmBars = 24;   // kSmBars: kStages - 1 more mbarriers
 constexpr uint32_t kSmStage = 128;                   // 16-byte aligned copy target
 constexpr uint32_t kStages = 2;                      // stages of a tile with several groups of threads (vis_tile_groups)
+// With several groups of threads a batch is up to four times as large: a group walks
+// every kGroups-th entry, and the chain of a heavy tile is its batches (8x8 tiles at
+// 480x270, 512 objects, 8 groups: 62 us with batches of 48, 49 with 192, 48 with 384;
+// 16x16, 4 groups: 153 and 103; 2 groups gain 3 % from 96 and lose from 192).
+__host__ __device__ constexpr uint32_t batch_factor(uint32_t groups) { return groups < 4u ? groups : 4u; }
+static_assert(kBatch * 4u <= 256u, "an entry's index is 8 bits of a ring entry's packed word");
 __host__ __device__ constexpr uint32_t tile_best_off(uint32_t groups)
 {
-    return kSmStage + (groups > 1u ? kStages : 1u) * kBatch * (uint32_t)sizeof(TileEntry);
+    return kSmStage + (groups > 1u ? kStages : 1u) * batch_factor(groups) * kBatch * (uint32_t)sizeof(TileEntry);
 }
 __host__ __device__ constexpr uint32_t tile_smem_bytes(uint32_t pixels, uint32_t groups = 1u)
 {
@@ -1125,7 +1131,7 @@ __device__ __forceinline__ void tile_batch(const TileJob& J, const TileEntry* co
                 const uint32_t e = (P.qh + qn + __popc(m & ((1u << lane) - 1u))) & (kQueue - 1u);
                 qf[0 * kQueue + e] = P.dx; qf[1 * kQueue + e] = P.dy; qf[2 * kQueue + e] = P.dz;
                 qf[3 * kQueue + e] = P.ix; qf[4 * kQueue + e] = P.iy; qf[5 * kQueue + e] = P.iz;
-                q[6 * kQueue + e] = lane | (k << 5) | ((uint32_t)sure << 11);
+                q[6 * kQueue + e] = lane | (k << 5) | ((uint32_t)sure << 13);
             }
             qn += __popc(m);
         }
@@ -1137,11 +1143,11 @@ __device__ __forceinline__ void tile_batch(const TileJob& J, const TileEntry* co
         if (lane < take) {
             const uint32_t e = (P.qh + lane) & (kQueue - 1u);
             const uint32_t pk = q[6 * kQueue + e];
-            const TileEntry& te = E[(pk >> 5) & 63u];
+            const TileEntry& te = E[(pk >> 5) & 255u];
             const float4 o = *reinterpret_cast<const float4*>(&te.rec.ox);
             const unsigned long long w = vis_pair<kCount>(
                 o.x, o.y, o.z, qf[0 * kQueue + e], qf[1 * kQueue + e], qf[2 * kQueue + e],
-                qf[3 * kQueue + e], qf[4 * kQueue + e], qf[5 * kQueue + e], (pk >> 11) != 0u, te.bits,
+                qf[3 * kQueue + e], qf[4 * kQueue + e], qf[5 * kQueue + e], (pk >> 13) != 0u, te.bits,
                 te.rec.cluster_pointer, P.far_plane, P.far_rcp, &J.counters[C_DDA_OVERRUN], work);
             // the minimum of 64 bits is a compare-and-swap loop: only where it can lower the word
             unsigned long long* const word = best + (pk & 31u);
@@ -1322,11 +1328,12 @@ __device__ __forceinline__ void vis_tile_groups(const TileJob& J, uint32_t slot,
         if (grp == 0u) clear_tile(J, si, pix);
         return;
     }
-    const uint32_t n_batches = scan_all ? 0u : (si.z + J.batch - 1u) / J.batch;
+    const uint32_t batch = J.batch * batch_factor(kGroups);
+    const uint32_t n_batches = scan_all ? 0u : (si.z + batch - 1u) / batch;
+    auto stage_of = [&](uint32_t j) { return sm.stage() + (j % kStages) * kBatch * batch_factor(kGroups); };
     auto stage = [&](uint32_t j) {   // batch j, in order
-        const uint32_t first = j * J.batch;
-        stage_entries(J, sm.bar(j % kStages), sm.stage() + (j % kStages) * kBatch, si.y + first, min(J.batch, si.z - first),
-                      j == 0u ? J.extra_tx : 0u);
+        const uint32_t first = j * batch;
+        stage_entries(J, sm.bar(j % kStages), stage_of(j), si.y + first, min(batch, si.z - first), j == 0u ? J.extra_tx : 0u);
     };
     for (uint32_t j = 0; j < min(n_batches, kStages); j++) stage(j);
     if (threadIdx.x == 0) sm.lost() = 0u;
@@ -1342,8 +1349,8 @@ __device__ __forceinline__ void vis_tile_groups(const TileJob& J, uint32_t slot,
     warp_rays(P, (float*)q + kWarpRays);
     uint32_t j = 0;
     while (j < n_batches) {
-        const uint32_t n = min(J.batch, si.z - j * J.batch);
-        const TileEntry* const E = sm.stage() + (j % kStages) * kBatch;
+        const uint32_t n = min(batch, si.z - j * batch);
+        const TileEntry* const E = stage_of(j);
         const bool late = __any_sync(0xffffffffu, !mbar_wait_bounded(sm.bar(j % kStages), (j / kStages) & 1u));
         uint32_t lo = 0u;
         if (late) {
@@ -1642,10 +1649,10 @@ static TileJob tile_job(const tgx_ctx* c, const tgx_scene* s, const ViewConst* d
 // holds (1024 per SM at the kernels' 64 registers).  Below that the time is the
 // heaviest tile's chain of batches, above it the sum of all tiles' work, which
 // grows with the threads.  Tile kernel over the 512-object scene, 8x8 tiles,
-// 1 / 2 / 4 / 8 threads per pixel: 480x270 128 / 85 / 67 / 62 us, 640x480 78 /
-// 57 / 54 / 85, 960x540 75 / 57 / 78 / 129, 1280x720 68 / 77 / 116 / 197,
-// 1920x1080 102 / 141 / 220 / 385; 16x16 tiles, 1 / 2 / 4: 480x270 273 / 174 / 153,
-// 1280x720 102 / 106 / 168, 1920x1080 124 / 180 / 299.
+// 1 / 2 / 4 / 8 threads per pixel: 480x270 130 / 72 / 50 / 49 us, 640x480 80 /
+// 51 / 50 / 75, 960x540 73 / 52 / 71 / 117, 1280x720 65 / 70 / 106 / 181,
+// 1920x1080 88 / 123 / 200 / 360; 16x16 tiles, 1 / 2 / 4: 480x270 268 / 145 / 100,
+// 1280x720 101 / 96 / 151, 1920x1080 110 / 161 / 274.
 static uint32_t vis_groups(const tgx_ctx* c, uint32_t pixels, uint32_t n_tiles)
 {
     const uint64_t limit = 12ull * 1024ull * (uint64_t)c->num_sms;
@@ -1748,11 +1755,13 @@ tgx_status vis_prepare_device(tgx_ctx* c)
     const uint32_t per_sm = threads == 64 ? vis_queue_per_sm<64, 16>() : threads == 128 ? vis_queue_per_sm<128, 10>()
                           : threads == 256 ? vis_queue_per_sm<256, 5>() : vis_queue_per_sm<512, 2>();
     c->vis_tile_ctas = (uint32_t)c->num_sms * per_sm;
-    // 1024 threads take more dynamic shared memory than a launch gets by default
+    // several threads per pixel take more dynamic shared memory than a launch gets by default
 #define BIG_SMEM(px, g) \
     TGX_CUDA(cudaFuncSetAttribute(k_vis_tiles_groups<(px) * (g), (g)>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                   (int)tile_smem_bytes((px), (g))))
-    BIG_SMEM(128, 8); BIG_SMEM(256, 4); BIG_SMEM(512, 2);
+    BIG_SMEM(64, 2); BIG_SMEM(64, 4); BIG_SMEM(64, 8);
+    BIG_SMEM(128, 2); BIG_SMEM(128, 4); BIG_SMEM(128, 8);
+    BIG_SMEM(256, 2); BIG_SMEM(256, 4); BIG_SMEM(512, 2);
 #undef BIG_SMEM
     return TGX_OK;
 }
