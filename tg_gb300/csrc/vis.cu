@@ -1645,19 +1645,21 @@ static TileJob tile_job(const tgx_ctx* c, const tgx_scene* s, const ViewConst* d
 }
 
 // Threads per pixel of the tile launch: the largest power of two, up to 8 and
-// 1024 threads a CTA, that keeps the launch within 12 times the threads the GPU
-// holds (1024 per SM at the kernels' 64 registers).  Below that the time is the
-// heaviest tile's chain of batches, above it the sum of all tiles' work, which
-// grows with the threads.  Tile kernel over the 512-object scene, 8x8 tiles,
-// 1 / 2 / 4 / 8 threads per pixel: 480x270 130 / 72 / 50 / 49 us, 640x480 80 /
-// 51 / 50 / 75, 960x540 73 / 52 / 71 / 117, 1280x720 65 / 70 / 106 / 181,
-// 1920x1080 88 / 123 / 200 / 360; 16x16 tiles, 1 / 2 / 4: 480x270 268 / 145 / 100,
-// 1280x720 101 / 96 / 151, 1920x1080 110 / 161 / 274.
+// 1024 threads a CTA, that keeps the launch within 12 (two) or 8 (four, eight)
+// times 1024 threads per SM, as many as the kernels' 64 registers let run.  Below
+// that the time is the heaviest tile's chain of batches, above it the sum of all
+// tiles' work, which grows with the threads.  Tile kernel over the 512-object
+// scene, 8x8 tiles, 1 / 2 / 4 / 8 threads per pixel, on 152 SMs: 480x270 130 / 72 /
+// 50 / 49 us, 560x315 116 / 66 / 47 / 57, 640x480 80 / 51 / 50 / 75, 800x450 81 / 53 /
+// 58 / 89, 1120x630 68 / 61 / 88 / 147, 1280x720 66 / 70 / 107 / 181, 1920x1080 88 /
+// 123 / 200 / 360; 16x16 tiles, 1 / 2 / 4: 640x360 200 / 108 / 76, 800x450 155 / 84 /
+// 88, 1280x720 100 / 97 / 151; 64 objects, 8x8: 640x360 31 / 22 / 18 / 21, 853x479
+// 25 / 20 / 18 / 29.
 static uint32_t vis_groups(const tgx_ctx* c, uint32_t pixels, uint32_t n_tiles)
 {
-    const uint64_t limit = 12ull * 1024ull * (uint64_t)c->num_sms;
+    const uint64_t unit = 1024ull * (uint64_t)c->num_sms;
     uint32_t g = 1;
-    while (g < 8u && pixels * g * 2u <= 1024u && (uint64_t)n_tiles * pixels * g * 2u <= limit) g *= 2u;
+    while (g < 8u && pixels * g * 2u <= 1024u && (uint64_t)n_tiles * pixels * g * 2u <= (g == 1u ? 12u : 8u) * unit) g *= 2u;
     return g;
 }
 
