@@ -13,8 +13,8 @@ from scenes import fuzz_scene
 
 pytestmark = pytest.mark.gpu
 
-# 12 * 1024 threads per SM over the tile's pixels and 2, 4 or 8 threads each, on 152 SMs
-EDGES = [12 * 1024 * 152 // (2 * g) for g in (1, 2, 4)]
+# 12 * 1024 threads per SM over the tile's pixels and 2 threads each, 8 * 1024 with 4 or 8, on 152 SMs
+EDGES = [m * 1024 * 152 // (2 * g) for m, g in ((12, 1), (8, 2), (8, 4))]
 
 
 @pytest.mark.parametrize("tile", [(8, 8), (16, 8), (16, 16), (32, 16), (8, 4), (8, 12)])
