@@ -270,8 +270,12 @@ __global__ void __launch_bounds__(128) k_svo_candidates(const tgx_object* __rest
 // (1 + 2e-5 of the coordinates) is far above the test's rounding.  Most levels of
 // most paths are like that (a cluster's box lies inside its cell of 2^k voxels in
 // all but about 45 / 2^k of the cases), so their tests are left out.  That needs a
-// matrix that is a rotation to 10^-3 and node corners that are exact; other
-// objects run every test.
+// matrix that is a rotation to 10^-5 and node corners that are exact; other
+// objects run every test: it takes a node's edges for the normals of its faces,
+// and where they meet at other angles it separates clusters well inside a large
+// node.  With all products of columns within 10^-5 a face leans by less than
+// 2 x 3 10^-5 x 8192 = 0.5 over a node's side, half the margin (10^-3 leant by 16
+// at 2^14 and kept clusters that the test drops).
 // 386k clusters at 4096^3, both kernels: 90 us, against 385 with every test and a
 // thread per cluster; with a dirty map (8 moved objects) 83 -> 27 us.
 __global__ void __launch_bounds__(128) k_svo_test_pairs(
@@ -316,7 +320,7 @@ __global__ void __launch_bounds__(128) k_svo_test_pairs(
 #pragma unroll
                 for (int j = 0; j <= r; j++) {
                     const float* q = od.rotation + 4 * j;
-                    skip = skip && fabsf(p[0] * q[0] + p[1] * q[1] + p[2] * q[2] - (r == j ? 1.0f : 0.0f)) <= 1e-3f;
+                    skip = skip && fabsf(p[0] * q[0] + p[1] * q[1] + p[2] * q[2] - (r == j ? 1.0f : 0.0f)) <= 1e-5f;
                 }
                 // the last column and row are those of a rotation; node corners below 2^24 are exact
                 skip = skip && p[3] == 0.0f && od.rotation[12 + r] == 0.0f && fabsf(mn[r]) + ext <= 16777216.0f;
