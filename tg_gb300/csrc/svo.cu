@@ -941,9 +941,14 @@ __global__ void __launch_bounds__(256) k_svo_unmark(uint32_t* __restrict__ table
 // host side
 // ---------------------------------------------------------------------------
 
+// The counters are an ordinary allocation, and the first to go: their cudaFree
+// waits for all work on the device (other contexts may still traverse the SVO),
+// which that of a pool array does not.  cudaDeviceSynchronize would wait too, but
+// it fails, and ends the capture, while another thread captures a stream.
 static void svo_free(tgx_svo* s)
 {
     if (!s) return;
+    cudaFree(s->d_counters);
     cudaFree(s->d_table);
     cudaFree(s->d_pool);
     cudaFree(s->d_sub);
@@ -952,7 +957,6 @@ static void svo_free(tgx_svo* s)
     cudaFree(s->d_mat);
     cudaFree(s->d_free);
     cudaFree(s->d_slot_block);
-    cudaFree(s->d_counters);
     cudaFree(s->d_objs);
     delete s;
 }
@@ -961,8 +965,8 @@ static void svo_free(tgx_svo* s)
 // keeps up to kSvoPoolKeep bytes of freed arrays for the next build and gives the
 // rest back; the pool goes with the context (an array still in use keeps its
 // part alive).  A build of 18.4k blocks with materials (1.3 GB) and its free took
-// 1.1 ms in the driver's allocator beside 1.9 ms of GPU work.  Arrays are freed
-// by cudaFree, which waits for all streams that may still read them.
+// 1.1 ms in the driver's allocator beside 1.9 ms of GPU work.  Nothing waits when
+// a pool array is freed: svo_free and svo_resize_slots do before.
 constexpr uint64_t kSvoPoolKeep = 4ull << 30;
 
 static cudaError_t svo_malloc(tgx_ctx* c, void** p, uint64_t bytes)
@@ -1009,10 +1013,12 @@ static tgx_status svo_resize_slots(tgx_ctx* c, tgx_svo* s, uint32_t cap, uint32_
     Arr arrs[6] = {{(void**)&s->d_pool, kBlockWords * 4}, {(void**)&s->d_sub, 128}, {(void**)&s->d_nonempty, 4},
                    {(void**)&s->d_free, 4}, {(void**)&s->d_slot_block, 4}, {&mat, 65536}};
     const int n_arr = materials ? 6 : 5;
-    void* fresh[6] = {};
+    void *fresh[6] = {}, *wait = nullptr;
     for (int a = 0; a < n_arr; a++)
-        if (svo_malloc(c, &fresh[a], (uint64_t)cap * arrs[a].per_slot) != cudaSuccess) {
-            for (int k = 0; k < a; k++) cudaFree(fresh[k]);
+        if (svo_malloc(c, &fresh[a], (uint64_t)cap * arrs[a].per_slot) != cudaSuccess ||
+            (a == 0 && s->d_pool && cudaMalloc(&wait, 256) != cudaSuccess)) {
+            for (int k = 0; k <= a; k++) cudaFree(fresh[k]);
+            cudaFree(wait);
             cudaGetLastError();
             tgx_set_error("tgx_svo: out of device memory for %u blocks", cap);
             return TGX_ERR_OUT_OF_MEMORY;
@@ -1022,7 +1028,10 @@ static tgx_status svo_resize_slots(tgx_ctx* c, tgx_svo* s, uint32_t cap, uint32_
         if (kept) TGX_CUDA(cudaMemcpyAsync(fresh[a], *arrs[a].p, kept, cudaMemcpyDeviceToDevice, c->stream));
         if (a != 0 && a != 5) TGX_CUDA(cudaMemsetAsync((char*)fresh[a] + kept, a == 4 ? 0xff : 0, total - kept, c->stream));
     }
-    if (s->d_pool) TGX_CUDA(cudaStreamSynchronize(c->stream));
+    if (s->d_pool) {
+        TGX_CUDA(cudaStreamSynchronize(c->stream));
+        cudaFree(wait);   // for every stream, as in svo_free
+    }
     for (int a = 0; a < n_arr; a++) {
         cudaFree(*arrs[a].p);
         *arrs[a].p = fresh[a];
@@ -1164,7 +1173,7 @@ extern "C" tgx_status tgx_svo_build_flags(tgx_ctx* c, const tgx_scene* sc, const
     auto fail = [&](tgx_status st) { cudaStreamSynchronize(c->stream); svo_free(s); return st; };
     if (svo_malloc(c, (void**)&s->d_table, n_table * 4) != cudaSuccess ||
         svo_malloc(c, (void**)&s->d_occ, occ_words * 4 + 128) != cudaSuccess ||
-        svo_malloc(c, (void**)&s->d_counters, S_COUNT * 4) != cudaSuccess ||
+        cudaMalloc((void**)&s->d_counters, S_COUNT * 4) != cudaSuccess ||
         svo_malloc(c, (void**)&s->d_objs, std::max<uint64_t>(1, (uint64_t)sc->n_objects) * sizeof(tgx_object)) != cudaSuccess) {
         cudaGetLastError();
         tgx_set_error("tgx_svo_build: out of device memory for the block table");
