@@ -412,7 +412,15 @@ tgx_status  tgx_svo_build(tgx_ctx* ctx, const tgx_scene* scene, const float min[
 /* tgx_svo_build with TGX_SVO_* flags. */
 tgx_status  tgx_svo_build_flags(tgx_ctx* ctx, const tgx_scene* scene, const float min[3], uint32_t extent_log2,
                                 uint32_t flags, tgx_svo** out_svo);
+/* Waits for all work on the device.  The context keeps the memory, up to 4 GiB,
+ * for its next build; tgx_trim gives it back. */
 void        tgx_svo_destroy(tgx_ctx* ctx, tgx_svo* svo);
+/* Gives back the device memory that the context keeps for SVOs to come: that of
+ * closed ones and the scratch of builds and updates.  Blocks until the context's
+ * stream is idle.  For a program that runs its own allocations close to the
+ * device's memory; an allocation of the library that finds no room gives back
+ * the memory of closed SVOs, of all contexts, by itself. */
+tgx_status  tgx_trim(tgx_ctx* ctx);
 
 /*
  * Brings an SVO up to date with the scene's current object records after

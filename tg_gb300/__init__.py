@@ -170,6 +170,7 @@ EXPORTS = [
     "tgx_scene_counts", "tgx_scene_download", "tgx_shade", "tgx_svo_update", "tgx_scene_set_objects",
     "tgx_set_trace_steps", "tgx_vis_render_host_async", "tgx_vis_host_wait", "tgx_vis_count_work",
     "tgx_vis_get_work", "tgx_gi_get_work", "tgx_set_vis_tuning", "tgx_set_memory_budget", "tgx_get_memory",
+    "tgx_trim",
 ]
 
 
@@ -220,6 +221,7 @@ def _load() -> C.CDLL:
         "tgx_set_vis_tuning": (i32, [vp, u32, u32, u32]),
         "tgx_set_memory_budget": (i32, [vp, u64]),
         "tgx_get_memory": (i32, [vp, C.POINTER(C.c_uint64), C.POINTER(C.c_uint64)]),
+        "tgx_trim": (i32, [vp]),
         "tgx_gi_render": (i32, [vp, vp, vp, vp, vp, vp, vp]),
         "tgx_cache_n_params": (u32, []),
         "tgx_gi_render_cached": (i32, [vp, vp, vp, vp, vp, vp, vp, vp, vp]),
@@ -514,6 +516,10 @@ class Context:
         b, u = C.c_uint64(), C.c_uint64()
         check(lib.tgx_get_memory(self.handle, C.byref(b), C.byref(u)), "tgx_get_memory")
         return b.value, u.value
+
+    def trim(self) -> None:
+        """tgx_trim: device memory kept for later SVO builds and updates back to the device."""
+        check(lib.tgx_trim(self.handle), "tgx_trim")
 
     def set_vis_tuning(self, depth_buckets: int = 0, batch: int = 0, drain: int = 0) -> None:
         """tgx_set_vis_tuning: depth buckets per tile (8/16/32), clusters per staged batch (1..48) and pairs per

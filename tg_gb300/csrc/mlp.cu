@@ -901,9 +901,9 @@ extern "C" tgx_status tgx_cache_create(tgx_ctx* c, uint64_t seed, tgx_cache** ou
     tgx_cache* k = new (std::nothrow) tgx_cache();
     if (!k) return TGX_ERR_OUT_OF_MEMORY;
     k->seed = seed;
-    bool ok = cudaMalloc(&k->w, N_PARAMS * 4) == cudaSuccess && cudaMalloc(&k->m, N_PARAMS * 4) == cudaSuccess &&
-              cudaMalloc(&k->v, N_PARAMS * 4) == cudaSuccess && cudaMalloc(&k->g, N_PARAMS * 4) == cudaSuccess &&
-              cudaMalloc(&k->img, B_TOTAL * 2) == cudaSuccess && cudaMalloc(&k->loss, 16) == cudaSuccess;
+    auto alloc = [](auto** p, size_t bytes) { return tgx_malloc((void**)p, bytes) == cudaSuccess; };
+    bool ok = alloc(&k->w, N_PARAMS * 4) && alloc(&k->m, N_PARAMS * 4) && alloc(&k->v, N_PARAMS * 4) &&
+              alloc(&k->g, N_PARAMS * 4) && alloc(&k->img, B_TOTAL * 2) && alloc(&k->loss, 16);
     if (!ok) {
         tgx_cache_destroy(c, k);
         tgx_set_error("tgx_cache_create: out of device memory");

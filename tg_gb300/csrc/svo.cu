@@ -964,7 +964,8 @@ static void svo_free(tgx_svo* s)
 // An SVO's arrays come from a memory pool of the context that builds it, which
 // keeps up to kSvoPoolKeep bytes of freed arrays for the next build and gives the
 // rest back; the pool goes with the context (an array still in use keeps its
-// part alive).  A build of 18.4k blocks with materials (1.3 GB) and its free took
+// part alive), or sooner: on tgx_trim, and when an allocation of any context finds
+// no room (tgx_malloc).  A build of 18.4k blocks with materials (1.3 GB) and its free took
 // 1.1 ms in the driver's allocator beside 1.9 ms of GPU work.  Nothing waits when
 // a pool array is freed: svo_free and svo_resize_slots do before.
 constexpr uint64_t kSvoPoolKeep = 4ull << 30;
@@ -984,8 +985,16 @@ static cudaError_t svo_malloc(tgx_ctx* c, void** p, uint64_t bytes)
             return e;
         }
         c->svo_pool = pool;
+        svo_pool_opened(pool);
     }
-    return cudaMallocFromPoolAsync(p, std::max<uint64_t>(bytes, 1), c->svo_pool, c->stream);
+    const uint64_t n = std::max<uint64_t>(bytes, 1);
+    cudaError_t e = cudaMallocFromPoolAsync(p, n, c->svo_pool, c->stream);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        svo_pools_trim();
+        e = cudaMallocFromPoolAsync(p, n, c->svo_pool, c->stream);
+    }
+    return e;
 }
 
 // The pair storage: pairs, then as many words for the list of the marked blocks.
@@ -1016,7 +1025,7 @@ static tgx_status svo_resize_slots(tgx_ctx* c, tgx_svo* s, uint32_t cap, uint32_
     void *fresh[6] = {}, *wait = nullptr;
     for (int a = 0; a < n_arr; a++)
         if (svo_malloc(c, &fresh[a], (uint64_t)cap * arrs[a].per_slot) != cudaSuccess ||
-            (a == 0 && s->d_pool && cudaMalloc(&wait, 256) != cudaSuccess)) {
+            (a == 0 && s->d_pool && tgx_malloc(&wait, 256) != cudaSuccess)) {
             for (int k = 0; k <= a; k++) cudaFree(fresh[k]);
             cudaFree(wait);
             cudaGetLastError();
@@ -1173,7 +1182,7 @@ extern "C" tgx_status tgx_svo_build_flags(tgx_ctx* c, const tgx_scene* sc, const
     auto fail = [&](tgx_status st) { cudaStreamSynchronize(c->stream); svo_free(s); return st; };
     if (svo_malloc(c, (void**)&s->d_table, n_table * 4) != cudaSuccess ||
         svo_malloc(c, (void**)&s->d_occ, occ_words * 4 + 128) != cudaSuccess ||
-        cudaMalloc((void**)&s->d_counters, S_COUNT * 4) != cudaSuccess ||
+        tgx_malloc((void**)&s->d_counters, S_COUNT * 4) != cudaSuccess ||
         svo_malloc(c, (void**)&s->d_objs, std::max<uint64_t>(1, (uint64_t)sc->n_objects) * sizeof(tgx_object)) != cudaSuccess) {
         cudaGetLastError();
         tgx_set_error("tgx_svo_build: out of device memory for the block table");

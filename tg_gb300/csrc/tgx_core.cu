@@ -11,7 +11,9 @@
 
 #include <cstdarg>
 #include <cstdlib>
+#include <mutex>
 #include <new>
+#include <vector>
 
 static thread_local char g_error[1024];
 
@@ -43,13 +45,51 @@ extern "C" const char* tgx_status_string(tgx_status s)
     return "unknown status";
 }
 
+// The pools of all live contexts: memory that one of them keeps must not fail an
+// allocation of another.
+static std::mutex g_svo_pools_mutex;
+static std::vector<cudaMemPool_t> g_svo_pools;
+
+void svo_pool_opened(cudaMemPool_t pool)
+{
+    std::lock_guard<std::mutex> lock(g_svo_pools_mutex);
+    g_svo_pools.push_back(pool);
+}
+
+void svo_pool_close(cudaMemPool_t pool)
+{
+    std::lock_guard<std::mutex> lock(g_svo_pools_mutex);
+    g_svo_pools.erase(std::remove(g_svo_pools.begin(), g_svo_pools.end(), pool), g_svo_pools.end());
+    cudaMemPoolDestroy(pool);
+}
+
+void svo_pools_trim()
+{
+    std::lock_guard<std::mutex> lock(g_svo_pools_mutex);
+    for (cudaMemPool_t pool : g_svo_pools) cudaMemPoolTrimTo(pool, 0);
+}
+
+cudaError_t tgx_malloc(void** p, size_t bytes)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        svo_pools_trim();
+        e = cudaMalloc(p, bytes);
+    }
+    if (e != cudaSuccess) {
+        *p = nullptr;
+        cudaGetLastError();
+    }
+    return e;
+}
+
 tgx_status devbuf_reserve(DevBuf& b, size_t bytes)
 {
     if (bytes <= b.bytes && b.ptr) return TGX_OK;
     if (b.ptr) { cudaFree(b.ptr); b.ptr = nullptr; b.bytes = 0; }
     size_t want = bytes < 256 ? 256 : bytes;
     want = want + want / 4;   // headroom so slowly growing scenes do not reallocate every frame
-    TGX_CUDA(cudaMalloc(&b.ptr, want));
+    TGX_CUDA(tgx_malloc(&b.ptr, want));
     b.bytes = want;
     return TGX_OK;
 }
@@ -105,7 +145,7 @@ extern "C" tgx_status tgx_create(const tgx_config* cfg, tgx_ctx** out)
         }
         c->own_stream = true;
     }
-    if (cudaMalloc(&c->d_status, sizeof(tgx_dev_status)) != cudaSuccess ||
+    if (tgx_malloc((void**)&c->d_status, sizeof(tgx_dev_status)) != cudaSuccess ||
         cudaMemset(c->d_status, 0, sizeof(tgx_dev_status)) != cudaSuccess ||
         cudaMallocHost(&c->h_counter, 64) != cudaSuccess || cudaMallocHost(&c->h_vis_counters, 64) != cudaSuccess) {
         tgx_set_error("tgx_create: allocation failed");
@@ -133,7 +173,7 @@ extern "C" void tgx_destroy(tgx_ctx* c)
     devbuf_free(c->vis_bins);
     devbuf_free(c->vis_views);
     devbuf_free(c->svo_counters);
-    if (c->svo_pool) cudaMemPoolDestroy(c->svo_pool);
+    if (c->svo_pool) svo_pool_close(c->svo_pool);
     devbuf_free(c->svo_pairs);
     devbuf_free(c->svo_scratch);
     devbuf_free(c->svo_sort);
@@ -361,7 +401,7 @@ tgx_status scene_finish(tgx_ctx* c, tgx_scene* s)
         if (cudaGetLastError() == cudaSuccess) c->launches++;
     }
     if (!s->d_inv) {
-        const cudaError_t e = cudaMalloc((void**)&s->d_inv, (size_t)s->n_objects * 4 * sizeof(float4));
+        const cudaError_t e = tgx_malloc((void**)&s->d_inv, (size_t)s->n_objects * 4 * sizeof(float4));
         if (e != cudaSuccess) {
             cudaGetLastError();
             tgx_set_error("scene setup: out of device memory (%u object matrices)", s->n_objects);
@@ -386,7 +426,7 @@ tgx_status scene_finish(tgx_ctx* c, tgx_scene* s)
 cudaError_t scene_malloc(tgx_ctx* c, tgx_scene* s, void** p, size_t bytes)
 {
     if (c->mem_budget && c->mem_scenes + bytes > c->mem_budget) return cudaErrorMemoryAllocation;
-    const cudaError_t e = cudaMalloc(p, bytes);
+    const cudaError_t e = tgx_malloc(p, bytes);
     if (e == cudaSuccess) {
         c->mem_scenes += bytes;
         s->bytes += bytes;
@@ -398,6 +438,17 @@ extern "C" tgx_status tgx_set_memory_budget(tgx_ctx* c, uint64_t bytes)
 {
     if (!c) return TGX_ERR_INVALID_ARGUMENT;
     c->mem_budget = bytes;
+    return TGX_OK;
+}
+
+extern "C" tgx_status tgx_trim(tgx_ctx* c)
+{
+    if (!c) return TGX_ERR_INVALID_ARGUMENT;
+    TGX_CUDA(cudaStreamSynchronize(c->stream));
+    devbuf_free(c->svo_pairs);
+    devbuf_free(c->svo_scratch);
+    devbuf_free(c->svo_sort);
+    if (c->svo_pool) TGX_CUDA(cudaMemPoolTrimTo(c->svo_pool, 0));
     return TGX_OK;
 }
 

@@ -63,6 +63,15 @@ struct DevBuf
     size_t bytes = 0;
 };
 
+// cudaMalloc that, when the device has no room, first gives back what the contexts'
+// SVO pools keep for later builds (svo_malloc)
+cudaError_t tgx_malloc(void** p, size_t bytes);
+// a context's SVO pool, from its creation to its end among those
+void svo_pool_opened(cudaMemPool_t pool);
+void svo_pool_close(cudaMemPool_t pool);
+// the unused memory of every such pool back to the device
+void svo_pools_trim();
+
 tgx_status devbuf_reserve(DevBuf& b, size_t bytes);
 void       devbuf_free(DevBuf& b);
 

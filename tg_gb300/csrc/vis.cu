@@ -1996,8 +1996,7 @@ extern "C" tgx_status tgx_frame_graph_create(tgx_ctx* c, const tgx_vis_job* jobs
     }
     const size_t jobs_off = table_bytes + scratch_bytes;
     const size_t total = jobs_off + al((size_t)n_jobs * sizeof(TileJob)) + 256;
-    if (cudaMalloc(&g->d_mem, total) != cudaSuccess) {
-        cudaGetLastError();
+    if (tgx_malloc(&g->d_mem, total) != cudaSuccess) {
         tgx_set_error("tgx_frame_graph_create: out of device memory (%zu bytes)", total);
         return fail(TGX_ERR_OUT_OF_MEMORY);
     }
