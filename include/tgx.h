@@ -142,6 +142,11 @@ typedef struct tgx_config
  * (where = 5).  Nothing faults; the context stays usable.  Never set it
  * outside such a test. */
 #define TGX_FLAG_TEST_LOST_COPY         2u
+/* Test of the failed-update path: every tgx_svo_build and tgx_svo_update stops,
+ * once its blocks have slots and are voxelised, as if a launch had failed there
+ * (TGX_ERR_CUDA).  A build frees what it had; an updated SVO is left with the
+ * blocks that no moved object touches.  Never set it outside such a test. */
+#define TGX_FLAG_TEST_FAILED_FILL       4u
 
 typedef struct tgx_device_error
 {

@@ -36,7 +36,11 @@ namespace {
 
 constexpr uint32_t kBlockSide = 32;
 constexpr uint32_t kBlockWords = 1024;
-constexpr uint32_t kMark = 0xffffffffu;      // table entry of a marked block
+// Table entries: 0 without a block, slot + 1 of one; with kMarked, a block that the
+// pass under way builds: kMark until it has a slot, then kMarked | its place in the
+// list of marked blocks, until k_svo_publish.
+constexpr uint32_t kMarked = 0x80000000u;
+constexpr uint32_t kMark = 0xffffffffu;
 constexpr uint32_t kNoBlock = 0xffffffffu;   // block of a candidate pair that failed its test
 constexpr uint32_t kWarpsPerVoxCta = 16;
 
@@ -364,7 +368,7 @@ __global__ void __launch_bounds__(128) k_svo_test_pairs(
 
 // Marked block m of n takes a slot from the end of the free list first
 // (free[n_free-1], free[n_free-2], ...), then fresh slots from `next_slot` on.
-// The table entry holds m + 1 until k_svo_publish puts the slot there: the
+// The table entry holds m, marked, until k_svo_publish puts the slot there: the
 // passes between group the pairs by m.
 __global__ void __launch_bounds__(256) k_svo_alloc(uint32_t* __restrict__ table, const uint32_t* __restrict__ marked,
                                                   uint32_t n, const uint32_t* __restrict__ free_list, uint32_t n_free,
@@ -377,7 +381,7 @@ __global__ void __launch_bounds__(256) k_svo_alloc(uint32_t* __restrict__ table,
     if (m >= n) return;
     const uint32_t blk = marked[m];
     const uint32_t slot = m < n_free ? free_list[n_free - 1u - m] : next_slot + (m - n_free);
-    table[blk] = m + 1u;
+    table[blk] = kMarked | m;
     slots[m] = slot;
     slot_block[slot] = blk;
     nonempty[slot] = 0u;
@@ -415,7 +419,7 @@ __global__ void __launch_bounds__(256) k_svo_pair_count(const SvoPair* __restric
     pdl_wait();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t blk = pairs[i].block;
-        if (blk != kNoBlock) atomicAdd(&cnt[table[blk] - 1u], 1u);
+        if (blk != kNoBlock) atomicAdd(&cnt[table[blk] & ~kMarked], 1u);
     }
 }
 
@@ -520,7 +524,7 @@ __global__ void __launch_bounds__(128) k_svo_pair_fill(const SvoPair* __restrict
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const SvoPair pr = pairs[i];
         if (pr.block == kNoBlock) continue;
-        pair_setup(objects, cluster_pointers, c2o, pr, mnx, mny, mnz, B, recs + atomicAdd(&cursor[table[pr.block] - 1u], 1u));
+        pair_setup(objects, cluster_pointers, c2o, pr, mnx, mny, mnz, B, recs + atomicAdd(&cursor[table[pr.block] & ~kMarked], 1u));
     }
 }
 
@@ -806,7 +810,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerVoxCta, 2) k_svo_voxelize(
 // 4. occupancy pyramid
 // ---------------------------------------------------------------------------
 
-// The slots of the marked blocks go into the table (which held m + 1).
+// The slots of the marked blocks go into the table.
 __global__ void __launch_bounds__(256) k_svo_publish(uint32_t* __restrict__ table, const uint32_t* __restrict__ marked,
                                                     const uint32_t* __restrict__ slots, uint32_t n)
 {
@@ -927,12 +931,28 @@ __global__ void __launch_bounds__(256) k_svo_release_dirty(uint32_t* __restrict_
     }
 }
 
-// Table entries still marked after an overflowed candidate pass go back to empty.
+// Table entries still marked after an overflowed candidate pass, or an update that
+// failed, go back to empty.
 __global__ void __launch_bounds__(256) k_svo_unmark(uint32_t* __restrict__ table, uint64_t n_table)
 {
     pdl_wait();
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_table; i += (uint64_t)gridDim.x * blockDim.x)
-        if (table[i] == kMark) table[i] = 0u;
+        if (table[i] & kMarked) table[i] = 0u;
+}
+
+// ... and the slots that it gave to blocks are nobody's: the pyramid pass goes by
+// slots, and a traversal that its bits led into a block without an entry would
+// read before the pool.
+__global__ void __launch_bounds__(256) k_svo_drop_slots(const uint32_t* __restrict__ table, uint32_t n_slots,
+                                                       uint32_t* __restrict__ slot_block, uint32_t* __restrict__ nonempty)
+{
+    pdl_wait();
+    const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
+    if (slot >= n_slots) return;
+    const uint32_t blk = slot_block[slot];
+    if (blk == 0xffffffffu || table[blk] == slot + 1u) return;
+    slot_block[slot] = 0xffffffffu;
+    nonempty[slot] = 0u;
 }
 
 }  // namespace
@@ -1089,6 +1109,24 @@ static tgx_status svo_candidates(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc, co
     return TGX_ERR_CAPACITY;
 }
 
+// Zeroes the pyramid, and the counts of pair ranges handed out and of non-empty blocks.
+static tgx_status svo_clear_pyramid(tgx_ctx* c, tgx_svo* s)
+{
+    TGX_CUDA(cudaMemsetAsync(s->d_counters + S_SLOTS, 0, 2 * 4, c->stream));
+    TGX_CUDA(cudaMemsetAsync(s->d_occ, 0, s->occ_words * 4, c->stream));
+    return TGX_OK;
+}
+
+// The occupancy pyramid of the blocks of n_slots slots, over zeroes.
+static tgx_status svo_pyramid(tgx_ctx* c, tgx_svo* s, uint32_t n_slots)
+{
+    if (n_slots)
+        TGX_LAUNCH_PDL(c, TR_SVO_PYRAMID, (n_slots + 255) / 256, 256, 0, k_svo_pyramid, s->d_slot_block, n_slots, s->d_nonempty,
+                   s->d_occ, (const uint64_t*)((char*)s->d_occ + svo_occ_off_bytes(s->occ_words)), s->n_levels, s->B,
+                   s->d_counters);
+    return TGX_OK;
+}
+
 // Slots for the n_marked marked blocks, voxelisation of the pairs, and the
 // occupancy pyramid of all n_slots slots (cleared first).
 static tgx_status svo_fill(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc, uint32_t n_cand, uint32_t n_marked,
@@ -1097,8 +1135,7 @@ static tgx_status svo_fill(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc, uint32_t
     uint32_t* counters = s->d_counters;
     const size_t sort_bytes = (size_t)n_marked * 4 * 4 + (size_t)s->n_pairs * sizeof(PairRec) + 64;
     TGX_TRY(devbuf_reserve(c->svo_sort, sort_bytes));
-    TGX_CUDA(cudaMemsetAsync(counters + S_SLOTS, 0, 2 * 4, c->stream));   // pair ranges handed out, non-empty
-    TGX_CUDA(cudaMemsetAsync(s->d_occ, 0, s->occ_words * 4, c->stream));
+    TGX_TRY(svo_clear_pyramid(c, s));
     if (n_marked) {
         // group the pairs by marked block: counts, ranges, placement
         const uint32_t* marked = svo_marked(c);
@@ -1135,13 +1172,33 @@ static tgx_status svo_fill(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc, uint32_t
         else if (split) VOXELIZE(false, 4);
         else VOXELIZE(false, 1);
 #undef VOXELIZE
+        if (c->flags & TGX_FLAG_TEST_FAILED_FILL) {
+            tgx_set_error("tgx_svo: TGX_FLAG_TEST_FAILED_FILL");
+            return TGX_ERR_CUDA;
+        }
         TGX_LAUNCH_PDL(c, TR_SVO_PYRAMID, mgrid, 256, 0, k_svo_publish, s->d_table, marked, slots, n_marked);
     }
-    if (n_slots)
-        TGX_LAUNCH_PDL(c, TR_SVO_PYRAMID, (n_slots + 255) / 256, 256, 0, k_svo_pyramid, s->d_slot_block, n_slots, s->d_nonempty,
-                   s->d_occ, (const uint64_t*)((char*)s->d_occ + svo_occ_off_bytes(s->occ_words)), s->n_levels, s->B,
-                   counters);
-    return TGX_OK;
+    return svo_pyramid(c, s, n_slots);
+}
+
+// After an update that failed with `why`: the blocks that no moved object touches
+// stay, with a pyramid of their own.  No mark stays in the table (a traversal would
+// take it for a slot), and the slots that were freed or given out are free.
+static tgx_status svo_drop_update(tgx_ctx* c, tgx_svo* s, tgx_status why)
+{
+    const uint64_t n_table = (uint64_t)s->B * s->B * s->B;
+    const uint32_t grid = (uint32_t)std::min<uint64_t>((n_table + 255) / 256, (uint64_t)c->num_sms * 32);
+    TGX_LAUNCH_PDL(c, TR_SVO_ALLOC, grid, 256, 0, k_svo_unmark, s->d_table, n_table);
+    TGX_LAUNCH_PDL(c, TR_SVO_ALLOC, (s->pool_cap + 255) / 256, 256, 0, k_svo_drop_slots, s->d_table, s->pool_cap,
+                   s->d_slot_block, s->d_nonempty);
+    TGX_TRY(svo_clear_pyramid(c, s));
+    TGX_TRY(svo_pyramid(c, s, s->n_slots));
+    TGX_CUDA(cudaMemcpyAsync(c->h_counter, s->d_counters, S_COUNT * 4, cudaMemcpyDeviceToHost, c->stream));
+    TGX_CUDA(cudaStreamSynchronize(c->stream));
+    const uint32_t n_freed = ((const uint32_t*)c->h_counter)[S_FREED];
+    s->n_free += n_freed;
+    s->n_blocks -= n_freed;
+    return why;
 }
 
 extern "C" tgx_status tgx_svo_build(tgx_ctx* c, const tgx_scene* sc, const float* mn, uint32_t L, tgx_svo** out)
@@ -1239,7 +1296,8 @@ extern "C" tgx_status tgx_svo_update(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc
     TGX_LAUNCH_PDL(c, TR_SVO_ALLOC, wgrid, 256, 0, k_svo_release_dirty, s->d_table, n_words, dirty, n_table, s->d_nonempty,
                s->d_slot_block, s->d_free + s->n_free, sc->d_objects, s->d_objs, sc->n_objects, counters);
     // pairs of the dirty blocks, into the pair storage the last build left (grown when short)
-    TGX_TRY(svo_candidates(c, s, sc, dirty, std::max<uint64_t>(1024, c->svo_pairs.bytes / kPairBytes)));
+    tgx_status st = svo_candidates(c, s, sc, dirty, std::max<uint64_t>(1024, c->svo_pairs.bytes / kPairBytes));
+    if (st != TGX_OK) return svo_drop_update(c, s, st);
     const uint32_t* hc = (const uint32_t*)c->h_counter;
     const uint32_t n_moved = hc[S_MOVED], n_freed = hc[S_FREED], n_marked = hc[S_MARKED], hc_pairs = hc[S_PAIRS], n_cand = hc[S_CAND];
     if (out_n_moved) *out_n_moved = n_moved;
@@ -1247,15 +1305,10 @@ extern "C" tgx_status tgx_svo_update(tgx_ctx* c, tgx_svo* s, const tgx_scene* sc
     const uint32_t n_free = s->n_free + n_freed;
     const uint32_t fresh = n_marked > n_free ? n_marked - n_free : 0u;
     const uint32_t need = s->n_slots + fresh;
-    tgx_status st = TGX_OK;
     if (need > s->pool_cap) st = svo_resize_slots(c, s, need + need / 4 + 64, s->n_slots, s->d_mat != nullptr);
     s->n_pairs = hc_pairs;
     if (st == TGX_OK) st = svo_fill(c, s, sc, n_cand, n_marked, n_free, s->n_slots, need);
-    if (st != TGX_OK) {   // no mark stays in the table: a traversal would take it for a slot
-        const uint32_t grid = (uint32_t)std::min<uint64_t>((n_table + 255) / 256, (uint64_t)c->num_sms * 32);
-        TGX_LAUNCH_PDL(c, TR_SVO_ALLOC, grid, 256, 0, k_svo_unmark, s->d_table, n_table);
-        return st;
-    }
+    if (st != TGX_OK) return svo_drop_update(c, s, st);
     s->n_free = n_free - (n_marked - fresh);
     s->n_slots = need;
     s->n_blocks = s->n_blocks - n_freed + n_marked;
