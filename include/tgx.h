@@ -139,8 +139,8 @@ typedef struct tgx_config
  * visibility tile waits for 64 bytes more than it copies, so its bounded wait
  * (about one second) runs out.  The tile then stops staging, the frame's
  * pixels are incomplete, and tgx_last_device_error reports TGX_ERR_TIMEOUT
- * (where = 5).  Nothing faults; the context stays usable.  Never set it
- * outside such a test. */
+ * (where = 5).  In a frame graph of several jobs only the first job's tiles do.
+ * Nothing faults; the context stays usable.  Never set it outside such a test. */
 #define TGX_FLAG_TEST_LOST_COPY         2u
 /* Test of the failed-update path: every tgx_svo_build and tgx_svo_update stops,
  * once its blocks have slots and are voxelised, as if a launch had failed there

@@ -1201,11 +1201,12 @@ __device__ __forceinline__ void gather_records(const TileJob& J, uint32_t base, 
 
 // Tile `slot` (in the job's heavy-first order) of one job: every pixel's
 // nearest packed word over the entries binned to the tile.  `phase` is the
-// parity of the CTA's bulk-copy mbarrier, carried across tiles.  Returns
-// false (the same in every thread) when a batch's copies did not complete in
-// time: the status word then holds TGX_ERR_TIMEOUT, the CTA has issued no
+// parity of the mbarrier that the CTA's copies arrive on, carried across tiles.
+// Returns false (the same in every thread) when a batch's copies did not complete
+// in time: the status word then holds TGX_ERR_TIMEOUT, the CTA has issued no
 // further copy, every thread's own have landed and it has written its pixels'
-// words so far; it must not stage another tile.
+// words so far; it must not stage another tile.  With kNoCopies the entries are
+// gathered without the mbarrier, as after an overflow.
 //
 // The tile's entries (sorted near to far by depth bucket) arrive kBatch at a
 // time (stage_entries); the first copies are issued before the pixels' rays are
@@ -1218,7 +1219,7 @@ __device__ __forceinline__ void gather_records(const TileJob& J, uint32_t base, 
 // The ring is drained at the end of each batch.  The minimum over a pixel's
 // pairs does not depend on the order they are evaluated in (every word is
 // distinct), so the buffer is the same bits as one DDA per pair in order.
-template <bool kCount = false>
+template <bool kCount = false, bool kNoCopies = false>
 __device__ __forceinline__ bool vis_tile(const TileJob& J, uint32_t slot, const TileSm& sm, uint32_t& phase,
                                          tgx_dev_status* __restrict__ status)
 {
@@ -1230,7 +1231,7 @@ __device__ __forceinline__ bool vis_tile(const TileJob& J, uint32_t slot, const 
     __syncthreads();   // the CTA's previous tile is done with the shared state
     const uint4 si = J.slot_info[slot];   // one load: the tile and its entry range
     // bins overflowed this frame: gather every record whose tile rectangle holds the tile (slow, exact)
-    const bool scan_all = J.counters[C_OVERFLOW] != 0u;
+    const bool scan_all = kNoCopies || J.counters[C_OVERFLOW] != 0u;
     const uint32_t begin = scan_all ? 0u : si.y;
     const uint32_t end = scan_all ? J.counters[C_RECORDS] : si.y + si.z;
     if (si.z == 0u) {   // the same in every thread
@@ -1445,6 +1446,28 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) k_vis_tiles_groups(
     vis_tile_groups<kGroups>(J, slot, sm, status);
 }
 
+// A CTA of the queue that lost a batch's copies still has the item that it drew
+// meanwhile (thread 0's), which no other one takes: it renders that one without
+// copies, and draws no more.  A function of its own: within the loop it took 1.4 %
+// of a batch of 20 views (registers).
+__device__ __noinline__ void vis_queue_last(const TileJob* jobs, uint32_t n_jobs, uint32_t total, uint32_t item, TileJob* job,
+                                            uint32_t* slot, tgx_dev_status* status)
+{
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        *slot = 0xffffffffu;
+        if (item < total) {
+            uint32_t k = 0;   // the last job whose first item is <= item
+            while (k + 1u < n_jobs && jobs[k + 1u].first <= item) k++;
+            *job = jobs[k];
+            if (item - job->first < job->counters[C_NONEMPTY]) *slot = item - job->first;
+        }
+    }
+    __syncthreads();
+    uint32_t phase = 0;
+    if (*slot != 0xffffffffu) vis_tile<false, true>(*job, *slot, tile_sm(), phase, status);
+}
+
 // Persistent form over several jobs (scenes, each with its views): CTAs take
 // tiles from one work queue in job order, each job's tiles heavy-first and those
 // without entries passed over, until all jobs' tiles are done.
@@ -1487,9 +1510,10 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_vis_tiles_queue(const 
             }
         }
         __syncthreads();
-        if (s_slot == 0xffffffffu) break;
-        if (!vis_tile(s_job, s_slot, sm, phase, status)) break;   // its shared staging is not reusable
+        if (s_slot == 0xffffffffu) return;
+        if (!vis_tile(s_job, s_slot, sm, phase, status)) break;   // its staging barrier is not reusable
     }
+    vis_queue_last(jobs, n_jobs, total, item, &s_job, &s_slot, status);
 }
 
 }  // namespace
@@ -2030,6 +2054,7 @@ extern "C" tgx_status tgx_frame_graph_create(tgx_ctx* c, const tgx_vis_job* jobs
         unsigned long long** d_outs = (unsigned long long**)(base + job.table_off + job.ptr_off);
         tjobs[j] = tile_job(c, job.scene, d_vc, d_outs, (uint32_t)job.views.size(), job.n_tiles, w);
         tjobs[j].first = j ? tjobs[j - 1].first + g->jobs[j - 1].n_tiles : 0u;
+        if (j == 0 && (c->flags & TGX_FLAG_TEST_LOST_COPY)) tjobs[j].extra_tx = 64u;
     }
     TileJob* d_jobs = (TileJob*)(base + jobs_off);
     uint32_t* d_queue = (uint32_t*)(base + jobs_off + al((size_t)n_jobs * sizeof(TileJob)));
