@@ -38,6 +38,7 @@
 // Every pair evaluates the same binary32 operations in the same order as the
 // CPU oracle's transcription of visibility.frag, so the buffer is bit-exact.
 
+#include "graph_bins.h"
 #include "tgx_internal.cuh"
 
 #include <climits>
@@ -2004,12 +2005,8 @@ extern "C" tgx_status tgx_frame_graph_create(tgx_ctx* c, const tgx_vis_job* jobs
         job.table_off = table_bytes;
         table_bytes += al(tables[j].size());
         job.rec_cap = (uint64_t)jb.scene->n_cluster_pointers * jb.n_views;
-        // Room for cameras that meet more than these ones: a replay that overflows scans all
-        // records for every tile (batches of 20 views at random poses, 16 of one scene: with a
-        // twelfth of this room, the same bytes when an entry had 96, 19 of 60 replays with new
-        // cameras overflowed and took 4 to 15 ms; with this room none of 100 does and they take 2).
-        job.bin_cap = std::max<uint64_t>(3u << 16, std::max<uint64_t>((uint64_t)job.n_tiles * 48, (uint64_t)entries * 18));
-        if (job.rec_cap > 0xffffffffull || job.bin_cap > 0xffffffffull || (uint64_t)total_tiles + job.n_tiles > 0xffffffffull) {
+        if (!graph_bin_capacity(job.n_tiles, entries, &job.bin_cap) || job.rec_cap > 0xffffffffull ||
+            (uint64_t)total_tiles + job.n_tiles > 0xffffffffull) {
             tgx_set_error("tgx_frame_graph_create: job %u has too many (view, cluster) pairs or tiles", j);
             return fail(TGX_ERR_CAPACITY);
         }
