@@ -1027,7 +1027,7 @@ static uint32_t* svo_marked(tgx_ctx* c)
 static uint64_t svo_device_bytes(const tgx_svo* s)
 {
     const uint64_t n_table = (uint64_t)s->B * s->B * s->B;
-    return n_table * 4 + (uint64_t)s->pool_cap * (kBlockWords * 4 + 128 + 4 + 4 + (s->d_mat ? 65536 : 0)) +
+    return n_table * 4 + (uint64_t)s->pool_cap * (kBlockWords * 4 + 128 + 4 + 4 + 4 + (s->d_mat ? 65536 : 0)) +
            s->occ_words * 4 + (uint64_t)s->n_objects * sizeof(tgx_object);
 }
 

@@ -401,10 +401,10 @@ tgx_status scene_finish(tgx_ctx* c, tgx_scene* s)
         if (cudaGetLastError() == cudaSuccess) c->launches++;
     }
     if (!s->d_inv) {
-        const cudaError_t e = tgx_malloc((void**)&s->d_inv, (size_t)s->n_objects * 4 * sizeof(float4));
+        const cudaError_t e = scene_malloc(c, s, (void**)&s->d_inv, (size_t)s->n_objects * 4 * sizeof(float4));
         if (e != cudaSuccess) {
             cudaGetLastError();
-            tgx_set_error("scene setup: out of device memory (%u object matrices)", s->n_objects);
+            tgx_set_error("scene setup: out of device memory or past the context's budget (%u object matrices)", s->n_objects);
             return e == cudaErrorMemoryAllocation ? TGX_ERR_OUT_OF_MEMORY : TGX_ERR_CUDA;
         }
     }

@@ -176,8 +176,7 @@ struct tgx_scene
     tgx_object* d_objects = nullptr;
     float*      d_inv_rot = nullptr;       // per object: 3x3 linear part of inverse(rotation), row-major
     float4*     d_inv = nullptr;           // per object: the 16 floats of inverse(rotation), column-major; the first one
-                                           // is NaN when some element is not a moderate number (inverse_is_plain).
-                                           // Derived from the objects, not counted in `bytes`
+                                           // is NaN when some element is not a moderate number (inverse_is_plain)
     uint32_t*   d_cluster_pointers = nullptr;
     uint32_t*   d_c2o = nullptr;
     uint32_t*   d_bits = nullptr;
