@@ -854,7 +854,7 @@ constexpr uint32_t kBatch = 48;                      // entries per staged batch
 constexpr uint32_t kQueue = 64;                      // ring entries per warp (an entry adds at most 32)
 constexpr uint32_t kWarpRays = 7 * kQueue;           // then the bounds of the warp's rays (warp_rays): 6 floats
 constexpr uint32_t kQueueWords = kWarpRays + 8;      // the ring: 6 float arrays + the packed word
-constexpr uint32_t kSmBar = 0, kSmN = 12, kSmLost = 16, kSmBars = 24;   // kSmBars: kStages - 1 more mbarriers
+constexpr uint32_t kSmBar = 0, kSmN = 12, kSmLost = 16, kSmBars = 24;   // kSmLost: two words; kSmBars: kStages - 1 more mbarriers
 constexpr uint32_t kSmStage = 128;                   // 16-byte aligned copy target
 constexpr uint32_t kStages = 2;                      // stages of a tile with several groups of threads (vis_tile_groups)
 // With several groups of threads a batch is up to four times as large: a group walks
@@ -879,7 +879,9 @@ struct TileSm
     __device__ __forceinline__ uint32_t bar() const { return smem_addr(p + kSmBar); }
     // mbarrier of stage i (stage 0's is that of the single-stage tiles)
     __device__ __forceinline__ uint32_t bar(uint32_t i) const { return smem_addr(p + (i ? kSmBars + 8u * (i - 1u) : kSmBar)); }
-    __device__ __forceinline__ volatile uint32_t& lost() const { return *(volatile uint32_t*)(p + kSmLost); }
+    // whether a wait of batch j ran out: batches take turns with two words, as a warp may be on the
+    // next batch while another one reads this one's
+    __device__ __forceinline__ volatile uint32_t& lost(uint32_t j) const { return *(volatile uint32_t*)(p + kSmLost + 4u * (j & 1u)); }
     __device__ __forceinline__ uint32_t& n() const { return *(uint32_t*)(p + kSmN); }
     __device__ __forceinline__ TileEntry* stage() const { return (TileEntry*)(p + kSmStage); }
     __device__ __forceinline__ unsigned long long* best() const { return (unsigned long long*)(p + best_off); }
@@ -1338,7 +1340,7 @@ __device__ __forceinline__ void vis_tile_groups(const TileJob& J, uint32_t slot,
         stage_entries(J, sm.bar(j % kStages), stage_of(j), si.y + first, min(batch, si.z - first), j == 0u ? J.extra_tx : 0u);
     };
     for (uint32_t j = 0; j < min(n_batches, kStages); j++) stage(j);
-    if (threadIdx.x == 0) sm.lost() = 0u;
+    if (threadIdx.x < 2u) sm.lost(threadIdx.x) = 0u;
     if (grp == 0u) sm.best()[pix] = ULLONG_MAX;
     __syncthreads();
     const uint32_t view = si.x;
@@ -1350,13 +1352,14 @@ __device__ __forceinline__ void vis_tile_groups(const TileJob& J, uint32_t slot,
     unsigned long long* const best0 = sm.best() + (pix & ~31u);
     warp_rays(P, (float*)q + kWarpRays);
     uint32_t j = 0;
+    bool lost = false;
     while (j < n_batches) {
         const uint32_t n = min(batch, si.z - j * batch);
         const TileEntry* const E = stage_of(j);
         const bool late = __any_sync(0xffffffffu, !mbar_wait_bounded(sm.bar(j % kStages), (j / kStages) & 1u));
         uint32_t lo = 0u;
         if (late) {
-            if (lane == 0) sm.lost() = 1u;
+            if (lane == 0) sm.lost(j) = 1u;
         } else {
             P.best_d24 = min(P.best_d24, (uint32_t)(best0[lane] >> 40));   // the other groups' words too
             tile_batch<false, kGroups>(J, E, grp, n, P, q, best0, nullptr);
@@ -1364,12 +1367,13 @@ __device__ __forceinline__ void vis_tile_groups(const TileJob& J, uint32_t slot,
         }
         // the batch is consumed; every pixel already nearer than the rest of the (bucket-sorted) entries: done
         const bool done = __syncthreads_and(!P.valid || P.best_d24 < lo);
+        lost = sm.lost(j) != 0u;
         j++;
-        if (done || sm.lost()) break;
+        if (done || lost) break;
         if (j + kStages - 1u < n_batches) stage(j + kStages - 1u);
     }
     own_copies_wait();   // none may land after the CTA is gone
-    if (threadIdx.x == 0 && sm.lost()) dev_error(status, TGX_ERR_TIMEOUT, 5, tile_index(vc, si.w));
+    if (threadIdx.x == 0 && lost) dev_error(status, TGX_ERR_TIMEOUT, 5, tile_index(vc, si.w));
     if (scan_all) {
         const uint32_t tx = si.w & 0xffffu, ty = si.w >> 16;
         const uint32_t n_rec = J.counters[C_RECORDS];
