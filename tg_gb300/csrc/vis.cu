@@ -1684,6 +1684,12 @@ static TileJob tile_job(const tgx_ctx* c, const tgx_scene* s, const ViewConst* d
 // 123 / 200 / 360; 16x16 tiles, 1 / 2 / 4: 640x360 200 / 108 / 76, 800x450 155 / 84 /
 // 88, 1280x720 100 / 97 / 151; 64 objects, 8x8: 640x360 31 / 22 / 18 / 21, 853x479
 // 25 / 20 / 18 / 29.
+// How far the heaviest tile stands out differs from frame to frame, so near a line
+// either side can be the better one: at 1280x720 two threads lose 4 us in the frame
+// above and win in others (whole frames, one / two threads: 512 objects, 8x8, two
+// seeds 88 / 93 and 71 / 64, 16x16 120 / 117 and 90 / 76; 256 objects, 8x8 79 / 79.5
+// and 49 / 47, 16x16 88 / 91 and 59 / 47; 64 objects, 8x8 37 / 33, 16x16 44 / 35).
+// The entries of an earlier frame would not tell: it may be any other scene's.
 static uint32_t vis_groups(const tgx_ctx* c, uint32_t pixels, uint32_t n_tiles)
 {
     const uint64_t unit = 1024ull * (uint64_t)c->num_sms;
