@@ -992,7 +992,6 @@ tgx_status cache_infer_counted(tgx_ctx* c, tgx_cache* k, const uint32_t* d_n, ui
     return cache_forward(c, k, d_n, max_n, d_x, d_rgb);
 }
 
-// Computes the batch gradient into the accumulator (no update); returns the loss if out_loss.
 // The fused training kernel over one network's n samples, or over two
 // networks' batches side by side in one launch; leaves each network's per-CTA
 // gradient slices in its scratch (parts[i] of them).

@@ -1,26 +1,34 @@
 // svo.cu -- one-bit SVO build on the GPU.
 //
 // Replaces tg's recursive single-threaded CPU builder tg_svo_create
-// (tg_sparse_voxel_octree.c:466-542) with four data-parallel passes that set
-// exactly the same world voxels:
+// (tg_sparse_voxel_octree.c:466-542) with data-parallel passes that set exactly the
+// same world voxels:
 //
 //   1. k_svo_candidates  one thread per cluster pointer: drops empty clusters
-//      (:515-531), finds the 32^3 blocks its box can touch, and for each runs
-//      the reference's OBB/AABB test (tg_physics.c:226-392) on every node on
-//      the path from the root's children down to the block, with the node
-//      boxes and ws2ms matrix of tg__construct_inner_node (:319-397).  A block
-//      whose whole path passes becomes a (cluster, block) pair; the block is
-//      marked in the dense block table.
+//      (:515-531) and lists the cluster with every 32^3 block that its world box
+//      can touch (in an update: every dirty one).
+//      k_svo_test_pairs  one thread per listed pair: the reference's OBB/AABB test
+//      (tg_physics.c:226-392) on the nodes on the path from the root's children
+//      down to the block, with the node boxes and ws2ms matrix of
+//      tg__construct_inner_node (:319-397), except where it surely passes.  The
+//      block of a pair that passes is marked in the dense block table.
 //   2. k_svo_alloc       gives every marked block a slot in the block pool.
-//   3. k_svo_voxelize    the pairs grouped by block (count, ranges, place; a
-//      record of its corners and range for each), then one CTA per marked block, one warp per pair: the leaf voxelisation
-//      of tg__construct_leaf_node (:102-317) -- corner lerp, [0,8)^3 test, bit
+//   3. k_svo_pair_count, _ranges, _fill: the pairs grouped by block, a record of
+//      corners and range for each.
+//      k_svo_voxelize    one CTA per marked block, or four (8 layers each) when
+//      few are marked; a warp per pair: the leaf voxelisation of
+//      tg__construct_leaf_node (:102-317) -- corner lerp, [0,8)^3 test, bit
 //      fetch -- into the block's image (and material grid) in shared memory,
 //      written out whole and coalesced, with no global atomics; and inside each
 //      block one bit per non-empty 4^3 and 8^3 cell (the sub-block levels the
 //      traversal steps through before single voxels).
+//      k_svo_publish     the slots go into the block table.
 //   4. k_svo_pyramid     one bit per non-empty block and per non-empty node of
 //      every coarser level.
+//
+// An update marks the blocks that moved objects touched or touch
+// (k_svo_mark_dirty), frees their slots (k_svo_release_dirty) and runs the same
+// passes over these blocks.
 //
 // The node encoding of the reference (u16 relative child pointers, 64-entry
 // leaf lists) is not kept; the voxel set is.  Side length 2^6 .. 2^14.
@@ -29,8 +37,6 @@
 
 #include <algorithm>
 #include <vector>
-
-
 
 namespace {
 
@@ -983,11 +989,14 @@ static void svo_free(tgx_svo* s)
 
 // An SVO's arrays come from a memory pool of the context that builds it, which
 // keeps up to kSvoPoolKeep bytes of freed arrays for the next build and gives the
-// rest back; the pool goes with the context (an array still in use keeps its
-// part alive), or sooner: on tgx_trim, and when an allocation of any context finds
-// no room (tgx_malloc).  A build of 18.4k blocks with materials (1.3 GB) and its free took
-// 1.1 ms in the driver's allocator beside 1.9 ms of GPU work.  Nothing waits when
-// a pool array is freed: svo_free and svo_resize_slots do before.
+// rest back; these go with the context (an array still in use keeps its part
+// alive), or sooner: on tgx_trim, and when an allocation of any context finds
+// no room (tgx_malloc).  A build of 18.4k blocks with materials (1.3 GB) and its free
+// took 1.1 ms in the driver's allocator beside 1.9 ms of GPU work.  That is saved
+// where a context builds again after it closed an SVO; its first build still pays
+// for the memory (first and later passes of a build, a frame and the free: 3.04 and
+// 1.73 ms).  Nothing waits when a pool array is freed: svo_free and
+// svo_resize_slots do before.
 constexpr uint64_t kSvoPoolKeep = 4ull << 30;
 
 static cudaError_t svo_malloc(tgx_ctx* c, void** p, uint64_t bytes)

@@ -1390,8 +1390,6 @@ __device__ __forceinline__ void vis_tile_groups(const TileJob& J, uint32_t slot,
     if (P.valid && grp == 0u) J.outs[view][(size_t)P.py * vc.width + P.px] = sm.best()[pix];
 }
 
-// Instantiated per block size (= tile pixels) so the register budget can be
-// bounded for the occupancy each size needs.  One CTA per tile of one job.
 // The slot (heavy-first order, the tiles without entries last) that CTA b of
 // t takes.  With interleave (outputs in host memory), the n non-empty tiles keep
 // their order but the e = t - n empty ones are spread over the first f = 3/2 e
@@ -1420,6 +1418,8 @@ __device__ __forceinline__ void publish_totals(const TileJob& J)
     }
 }
 
+// One CTA per tile of one job.  Instantiated per block size (= tile pixels) so the
+// register budget can be bounded for the occupancy each size needs.
 template <int kThreads, int kMinBlocks, bool kCount = false>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) k_vis_tiles(TileJob J, tgx_dev_status* __restrict__ status)
 {
@@ -1475,7 +1475,9 @@ __device__ __noinline__ void vis_queue_last(const TileJob* jobs, uint32_t n_jobs
 
 // Persistent form over several jobs (scenes, each with its views): CTAs take
 // tiles from one work queue in job order, each job's tiles heavy-first and those
-// without entries passed over, until all jobs' tiles are done.
+// without entries passed over, until all jobs' tiles are done.  One thread per pixel
+// whatever the jobs' sizes: several (vis_groups) are for the launches of a single
+// frame or job, so small views of several jobs take as long as their heaviest tile.
 template <int kThreads, int kMinBlocks>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) k_vis_tiles_queue(const TileJob* __restrict__ jobs,
                                                                           uint32_t n_jobs, uint32_t total,
@@ -1868,8 +1870,6 @@ tgx_status vis_render_device(tgx_ctx* c, const tgx_scene* s, const tgx_view* vie
         TGX_CUDA(cudaMemcpyAsync(c->vis_views.ptr, stage.data(), stage.size(), cudaMemcpyHostToDevice, c->stream));
     }
 
-    // bin capacity: grown from earlier frames' totals (read back without waiting); a frame
-    // that still overflows is rendered correctly by the tile kernel's record scan
     // Bin capacity.  Grown from earlier frames' totals, read back without
     // waiting.  A frame that could outgrow what is known (the first one, one
     // with more tiles or (view, cluster) pairs than before, or the one after an
