@@ -46,27 +46,38 @@ extern "C" const char* tgx_status_string(tgx_status s)
 }
 
 // The pools of all live contexts: memory that one of them keeps must not fail an
-// allocation of another.
-static std::mutex g_svo_pools_mutex;
-static std::vector<cudaMemPool_t> g_svo_pools;
+// allocation of another.  Never destroyed: a context may be closed at exit.
+struct SvoPools
+{
+    std::mutex mutex;
+    std::vector<cudaMemPool_t> open;
+};
+static SvoPools& svo_pools()
+{
+    static SvoPools* p = new SvoPools();
+    return *p;
+}
 
 void svo_pool_opened(cudaMemPool_t pool)
 {
-    std::lock_guard<std::mutex> lock(g_svo_pools_mutex);
-    g_svo_pools.push_back(pool);
+    SvoPools& p = svo_pools();
+    std::lock_guard<std::mutex> lock(p.mutex);
+    p.open.push_back(pool);
 }
 
 void svo_pool_close(cudaMemPool_t pool)
 {
-    std::lock_guard<std::mutex> lock(g_svo_pools_mutex);
-    g_svo_pools.erase(std::remove(g_svo_pools.begin(), g_svo_pools.end(), pool), g_svo_pools.end());
+    SvoPools& p = svo_pools();
+    std::lock_guard<std::mutex> lock(p.mutex);
+    p.open.erase(std::remove(p.open.begin(), p.open.end(), pool), p.open.end());
     cudaMemPoolDestroy(pool);
 }
 
 void svo_pools_trim()
 {
-    std::lock_guard<std::mutex> lock(g_svo_pools_mutex);
-    for (cudaMemPool_t pool : g_svo_pools) cudaMemPoolTrimTo(pool, 0);
+    SvoPools& p = svo_pools();
+    std::lock_guard<std::mutex> lock(p.mutex);
+    for (cudaMemPool_t pool : p.open) cudaMemPoolTrimTo(pool, 0);
 }
 
 cudaError_t tgx_malloc(void** p, size_t bytes)
